@@ -361,7 +361,7 @@ QWEN3_TTS_API int32_t q3t_launch_sample_logits_at(
  * "attention_mode" (process-wide, see q3t_set_attention_mode),
  * "tc_min_rows" (process-wide: projections with at least this many rows run on the tensor
  * cores, default 9; 65 keeps every row count on the SIMT kernels, whose results do not depend on
- * the batch size), "prefill_chunk" (prompt positions per decoder pass, 1..64, default 64: a
+ * the batch size), "prefill_chunk" (prompt positions per decoder pass, 1..2048, default 2048, at most 64 in the parity modes: a
  * prompt runs as the rows of skinny GEMMs instead of position by position (talker.cu:2750-3249
  * is the reference's prompt path); 1 restores the position-by-position path). */
 QWEN3_TTS_API int32_t q3t_model_set_option(Qwen3TtsModelHandle model, const char* key,

@@ -148,10 +148,10 @@ uint64_t KvPool::page_bytes() const { return (uint64_t)layers_ * 2 * page_elems_
 
 // ------------------------------------------------------------------ Workspace
 
-Workspace::Workspace(int capacity_, int device_) : capacity(capacity_), device(device_) {
+Workspace::Workspace(int capacity_, int device_, int rows) : capacity(capacity_), device(device_) {
     check_cuda(cudaSetDevice(device), "cudaSetDevice(workspace)");
     const size_t e = sizeof(bf16);
-    const size_t c = capacity;
+    size_t c = std::max(capacity, rows);
     hidden = DeviceBuffer(c * 2048 * e);
     qkv = DeviceBuffer(c * 4096 * e);
     attention = DeviceBuffer(c * 2048 * e);
@@ -160,11 +160,12 @@ Workspace::Workspace(int capacity_, int device_) : capacity(capacity_), device(d
     x_in = DeviceBuffer(c * 2048 * e);
     projection = DeviceBuffer(c * 2048 * e);
     normalized = DeviceBuffer(c * 2048 * e);
+    prompt_positions = DeviceBuffer(c * sizeof(int));
+    c = capacity;
     table = DeviceBuffer(sizeof(FrameTable));
     talker_pages = DeviceBuffer(c * kMaxPagesPerRow * sizeof(int));
     predictor_pages = DeviceBuffer(c * sizeof(int));
     predictor_positions = DeviceBuffer((size_t)kPredictorSequence * kMaxRows * sizeof(int));
-    prompt_positions = DeviceBuffer((size_t)kMaxRows * sizeof(int));
     counters = DeviceBuffer(c * 16 * sizeof(unsigned int));
     try {
         check_cuda(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -503,7 +504,7 @@ Workspace& Model::batch_workspace() {
 
 Workspace& Model::prefill_workspace() {
     std::lock_guard<std::mutex> lock(mutex);
-    if (!prefill_) prefill_.reset(new Workspace(kMaxRows, device_));
+    if (!prefill_) prefill_.reset(new Workspace(kMaxRows, device_, kMaxPromptRows));
     return *prefill_;
 }
 
@@ -521,9 +522,15 @@ struct Probe {
 
 void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWeights>& layers,
                     const uint32_t* rope_table, const KvPool& pool, const int* page_table, int table_stride,
-                    const int* positions, int n, int splits, cudaStream_t s, bool shared_cache = false,
+                    const int* positions, int n, int splits, cudaStream_t s, int prompt_base = -1,
                     const Probe* probe = nullptr) {
     const int qkv_width = d.q_width + 2 * d.kv_width;
+    // a prompt pass (prompt_base >= 0): the rows are consecutive positions of one session
+    const bool shared_cache = prompt_base >= 0;
+    auto project = [&](GemvArgs& g, const char* what) {
+        if (g.norm_w != nullptr && n >= tc_min_rows()) g.norm_out = w.normalized.as<bf16>();
+        check_launch(n > kMaxRows ? launch_int8_gemm_prompt(g, s) : launch_int8_gemm(g, s), what);
+    };
     for (size_t l = 0; l < layers.size(); ++l) {
         const LayerWeights& lw = layers[l];
         const int layer = static_cast<int>(l);
@@ -536,7 +543,7 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
         g.norm_w = lw.input_norm;
         if (probe != nullptr) g.norm_out = w.normalized.as<bf16>();
         g.in_features = d.hidden; g.out_features = qkv_width; g.rows = n; g.epilogue = EPI_PLAIN;
-        check_launch(launch_int8_gemm(g, s), "qkv projection");
+        project(g, "qkv projection");
         observe("input_norm", w.normalized.as<bf16>(), d.hidden, d.hidden);
         observe("q_projection", w.qkv.as<bf16>(), qkv_width, d.q_width);
         observe("k_projection", w.qkv.as<bf16>() + d.q_width, qkv_width, d.kv_width);
@@ -560,14 +567,20 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
         // the older cache rows all date from earlier launches (the kernel ignores this outside
         // plain decode steps).
         a.inputs_settled = 1;
-        if (shared_cache) {
+        if (shared_cache && n >= tc_min_rows() && attention_mode() != 0 && prompt_attention_supports(a)) {
+            // With the projections on the tensor cores nothing promises a row the bits it would have
+            // alone, and the positions share their passes over the cache.
+            check_launch(launch_prompt_attention(a, prompt_base, s), "prompt attention");
+        } else if (shared_cache) {
             // the rows are consecutive positions of one session: every row's K/V goes into the
             // cache first, then every row attends up to its own position
             a.append_mode = 1;
             check_launch(launch_attention(a, s), "prompt KV append");
             a.append_mode = 2;
+            check_launch(launch_attention(a, s), "prompt attention");
+        } else {
+            check_launch(launch_attention(a, s), "decode attention");
         }
-        check_launch(launch_attention(a, s), "decode attention");
         observe("attention", w.attention.as<bf16>(), d.q_width, d.q_width);
 
         GemvArgs o;
@@ -575,7 +588,7 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
         o.x = w.attention.as<bf16>(); o.y = w.hidden.as<bf16>();
         o.in_features = d.q_width; o.out_features = d.hidden; o.rows = n; o.epilogue = EPI_ADD;
         o.residual_settled = true;     // hidden was last written before the qkv projection
-        check_launch(launch_int8_gemm(o, s), "attention output projection");
+        project(o, "attention output projection");
         observe("attention_residual", w.hidden.as<bf16>(), d.hidden, d.hidden);
 
         GemvArgs u;
@@ -585,7 +598,7 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
         if (probe != nullptr) u.norm_out = w.normalized.as<bf16>();
         u.in_features = d.hidden; u.out_features = d.intermediate; u.rows = n;
         u.epilogue = EPI_GATE_UP_SILU;
-        check_launch(launch_int8_gemm(u, s), "gate/up projection");
+        project(u, "gate/up projection");
         observe("post_attention_norm", w.normalized.as<bf16>(), d.hidden, d.hidden);
         observe("gated_activation", w.gate.as<bf16>(), d.intermediate, d.intermediate);
 
@@ -595,7 +608,7 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
         dn.in_features = d.intermediate; dn.out_features = d.hidden; dn.rows = n;
         dn.epilogue = EPI_ADD;
         dn.residual_settled = true;    // hidden was last written by the output projection, two launches up
-        check_launch(launch_int8_gemm(dn, s), "down projection");
+        project(dn, "down projection");
         observe("layer_output", w.hidden.as<bf16>(), d.hidden, d.hidden);
     }
 }
@@ -636,7 +649,7 @@ void enqueue_text_projection(Workspace& w, Model& m, int n, bool residual, cudaS
     f1.w = m.text_fc1.data; f1.scales = m.text_fc1.scales;
     f1.x = w.x_in.as<bf16>(); f1.y = w.projection.as<bf16>(); f1.bias = m.text_fc1_bias;
     f1.in_features = H; f1.out_features = H; f1.rows = n; f1.epilogue = EPI_BIAS_SILU;
-    check_launch(launch_int8_gemm(f1, s), "text projection fc1");
+    check_launch(n > kMaxRows ? launch_int8_gemm_prompt(f1, s) : launch_int8_gemm(f1, s), "text projection fc1");
     GemvArgs f2;
     f2.w = m.text_fc2.data; f2.scales = m.text_fc2.scales;
     f2.x = w.projection.as<bf16>(); f2.bias = m.text_fc2_bias;
@@ -646,7 +659,7 @@ void enqueue_text_projection(Workspace& w, Model& m, int n, bool residual, cudaS
     } else {
         f2.y = w.hidden.as<bf16>(); f2.epilogue = EPI_BIAS;
     }
-    check_launch(launch_int8_gemm(f2, s), "text projection fc2");
+    check_launch(n > kMaxRows ? launch_int8_gemm_prompt(f2, s) : launch_int8_gemm(f2, s), "text projection fc2");
 }
 
 void enqueue_talker_head(Workspace& w, Model& m, int n, int advance, cudaStream_t s) {
@@ -703,7 +716,7 @@ void enqueue_prompt_chunk(Workspace& w, Model& m, const int* text_ids, const int
     if (probe != nullptr) probe->emit("input", -1, w.hidden.as<bf16>() + (size_t)probe->row * H, H);
     // page-table stride 0: every row reads and writes the cache of the session bound to row 0
     enqueue_layers(w, m.talker, m.talker_layers, m.talker_rope, *m.talker_pool, w.talker_pages.as<int>(), 0,
-                   w.prompt_positions.as<int>(), rows, splits, s, true, probe);
+                   w.prompt_positions.as<int>(), rows, splits, s, base, probe);
 }
 
 // ---- parity hooks of the prompt path --------------------------------------------------------
@@ -1270,8 +1283,10 @@ void Session::prefill(const int32_t* text_ids, const int32_t* codec_ids, int cou
     // A prompt runs as chunks of up to prefill_chunk positions per decoder pass (the rows of a
     // skinny GEMM) on the model's prompt workspace, one prompt at a time; with prefill_chunk = 1,
     // or a prompt of one position, it runs position by position on the session's own workspace.
-    const int chunk = std::min(std::max(m.prefill_chunk, 1), kMaxRows);
     const ParityHooks hooks = ParityHooks::from_environment(nullptr);
+    // Passes above kMaxRows exist on the tensor-core kernels only; the parity modes and hooks keep to it.
+    const int most = tc_min_rows() <= kMaxRows && attention_mode() != 0 && !hooks.active() ? kMaxPromptRows : kMaxRows;
+    const int chunk = std::min(std::max(m.prefill_chunk, 1), most);
     // the parity hooks observe the chunked pass (they synchronise, so nothing of it may be captured)
     const bool chunked = (chunk > 1 && count > 1) || hooks.active();
     std::unique_lock<std::mutex> one_prompt(m.prefill_mutex, std::defer_lock);

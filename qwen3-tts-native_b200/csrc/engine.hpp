@@ -114,7 +114,8 @@ class Session;
 
 // Activation buffers, frame table and captured graphs for up to `capacity` lockstep rows.
 struct Workspace {
-    Workspace(int capacity, int device);
+    // `rows`: activation rows of one pass when that is more than the `capacity` table rows (prompts)
+    Workspace(int capacity, int device, int rows = 0);
     ~Workspace();
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
@@ -134,7 +135,7 @@ struct Workspace {
     DeviceBuffer predictor_pages;    // [capacity][1]
     int* host_pages = nullptr;       // pinned staging for the two page tables
     DeviceBuffer predictor_positions;   // [16][kMaxRows], slot p filled with p
-    DeviceBuffer prompt_positions;      // [kMaxRows], positions of the rows of a prompt chunk
+    DeviceBuffer prompt_positions;      // [activation rows], positions of the rows of a prompt chunk
     DeviceBuffer scratch;
     DeviceBuffer counters;
     int scratch_splits = 0;
@@ -194,7 +195,7 @@ public:
     // frame or prompt during which it advanced cannot be trusted (check_device_errors throws).
     unsigned int device_errors() const;
     void check_device_errors(unsigned int count_at_enqueue) const;
-    int prefill_chunk = kMaxRows;       // prompt positions per pass (1: one position at a time)
+    int prefill_chunk = kMaxPromptRows; // prompt positions per pass (1: one position at a time)
     Workspace* batch_workspace_if_any() {
         std::lock_guard<std::mutex> lock(mutex);
         return batch_.get();

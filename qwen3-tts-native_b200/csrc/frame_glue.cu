@@ -299,7 +299,7 @@ cudaError_t launch_prompt_combine(const FrameTable* table, const int* text_ids, 
 cudaError_t launch_prompt_rows(const int* text_ids, const int* codec_ids, int base, int rows,
                                const bf16* text_embedding, int text_vocabulary, bf16* text_in,
                                int* positions, int width, cudaStream_t stream) {
-    if (rows < 1 || rows > kMaxRows) return cudaErrorInvalidValue;
+    if (rows < 1 || rows > kMaxPromptRows) return cudaErrorInvalidValue;
     prompt_rows_kernel<<<rows, kThreads, 0, stream>>>(text_ids, codec_ids, base, text_embedding,
                                                       text_vocabulary, text_in, positions, width);
     return cudaGetLastError();
@@ -308,7 +308,7 @@ cudaError_t launch_prompt_rows(const int* text_ids, const int* codec_ids, int ba
 cudaError_t launch_prompt_combine_rows(const int* text_ids, const int* codec_ids, int base, int rows,
                                        const bf16* codec_embedding, int codec_vocabulary, bf16* hidden,
                                        int width, cudaStream_t stream) {
-    if (rows < 1 || rows > kMaxRows) return cudaErrorInvalidValue;
+    if (rows < 1 || rows > kMaxPromptRows) return cudaErrorInvalidValue;
     prompt_combine_rows_kernel<<<rows, kThreads, 0, stream>>>(text_ids, codec_ids, base, codec_embedding,
                                                               codec_vocabulary, hidden, width);
     return cudaGetLastError();

@@ -28,14 +28,15 @@
 // its copies land, frees its TMEM columns and returns.
 
 #include "q3t_kernels.cuh"
-
-#include <cuda.h>
+#include "q3t_tcgen05.cuh"
 
 #include <cstdlib>
 #include <mutex>
 
 namespace q3t {
 namespace {
+
+using namespace tc;
 
 // Warp roles: 0 weight copies, 1 MMA issue, 2 activation copies, 3 TMEM allocation (one elected
 // thread each); 4..7 and 8..11 are the two dequantiser groups.  Warp w may touch TMEM lanes
@@ -74,145 +75,6 @@ struct TcParams {
     int residual_settled;     // GemvArgs::residual_settled
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ unsigned long long now_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// One lane of a converged warp.  Unlike a test of the lane index, this tells the compiler that
-// the code below runs in exactly one thread, which the instructions that take their operands
-// from uniform registers (TMA copies, MMA issue) need in order to be emitted without a loop
-// over the active lanes.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t chosen;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(chosen));
-    return chosen != 0;
-}
-
-// Shared by all roles of a CTA: deadline and an abort flag that turns every later wait into a no-op.
-struct Guard {
-    unsigned long long deadline;
-    volatile int* abort_flag;
-    __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity) const {
-        // the clock is read once per 1024 polls: a read of the global timer costs about as much
-        // as a whole pipeline stage
-        uint32_t polls = 0;
-        while (!mbar_try_wait(bar, parity)) {
-            if ((++polls & 63u) != 0) continue;
-            if (*abort_flag) return false;
-            if ((polls & 1023u) == 0 && now_ns() > deadline) {
-                *abort_flag = 1;
-                return false;
-            }
-        }
-        return true;
-    }
-};
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Hardware barrier over every thread of the cluster (one CTA per K-slice of a channel tile).
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// address of the same shared-memory location in the CTA of another rank of the cluster
-__device__ __forceinline__ uint32_t peer_smem(uint32_t local, uint32_t rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-
-// K-major, 128-byte-swizzled operand tile: rows at a 128-byte pitch, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-
-// A (128 x 16 bf16) from TMEM columns, B from shared memory
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
-
-// 32 consecutive columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_store_32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr),
-          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-          "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-          "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 ::"r"(smem_u32(bar)) : "memory");
-}
-
-
-// four int8 (one word) -> four bf16 (two words), exact
-__device__ __forceinline__ void dequant4(uint32_t word, uint32_t& lo, uint32_t& hi) {
-    const uint32_t u = word ^ 0x80808080u;
-    const unsigned long long bias = pack2(-8388736.0f, -8388736.0f);
-    const unsigned long long a = add2(pack2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7650)),
-                                            __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7651))), bias);
-    const unsigned long long b = add2(pack2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7652)),
-                                            __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7653))), bias);
-    // a small integer as fp32 has a zero low half: its high half is the bf16 of the same value
-    lo = __byte_perm(static_cast<uint32_t>(a), static_cast<uint32_t>(a >> 32), 0x7632);
-    hi = __byte_perm(static_cast<uint32_t>(b), static_cast<uint32_t>(b >> 32), 0x7632);
-}
-
 __device__ __forceinline__ float finish(const TcParams& p, float acc, float scale, int channel, size_t o,
                                         bool have_base, float base) {
     switch (p.epilogue) {
@@ -226,23 +88,6 @@ __device__ __forceinline__ float finish(const TcParams& p, float acc, float scal
         default: return acc * scale;
     }
 }
-
-// NCOL consecutive fp32 accumulator columns of this thread's TMEM lane
-template <int NCOL>
-__device__ __forceinline__ void tmem_load_row(uint32_t taddr, float (&v)[NCOL]) {
-#pragma unroll
-    for (int c = 0; c < NCOL; c += 8) {
-        uint32_t r[8];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-            : "r"(taddr + c));
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[c + i] = __uint_as_float(r[i]);
-    }
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 
 __device__ __forceinline__ void dequant_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(128 * kGroups) : "memory");
@@ -279,6 +124,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     const int lane = tid % kWarp;
     const int split = (int)cluster_rank();           // cluster = the K-slices of one channel tile
     const int tile = blockIdx.x / p.splits;
+    const int row_first = blockIdx.y * MT;           // activation rows of this CTA: a block of MT of them
+    const int rows = min(MT, p.rows - row_first);
     const int step_first = p.chunks * split / p.splits;             // slices may differ by one step
     const int nk = p.chunks * (split + 1) / p.splits - step_first;
     const int k_first = step_first * kBK;
@@ -366,8 +213,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 // that the MMA issuer has one thing to wait for per step
                 mbar_expect_tx(&full_a[sx], kXStageBytes);
                 unsigned char* dst = xs + sx * kXStageBytes;
-                tma_load_2d(dst, &x_map, k_first + i * kBK, 0, &full_a[sx]);
-                tma_load_2d(dst + kXAtomBytes, &x_map, k_first + i * kBK + 64, 0, &full_a[sx]);
+                tma_load_2d(dst, &x_map, k_first + i * kBK, row_first, &full_a[sx]);
+                tma_load_2d(dst + kXAtomBytes, &x_map, k_first + i * kBK + 64, row_first, &full_a[sx]);
             }
         }
     } else if (warp == 1) {
@@ -460,7 +307,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 int within = group * kCols - owner * rows_share;
 #pragma unroll
                 for (int j = 0; j < kCols; ++j) {
-                    if (group * kCols + j < p.rows) {
+                    if (group * kCols + j < rows) {
                         st_cluster(peer_smem(slot0 + (uint32_t)(within * kTileN) * 4u, (uint32_t)owner), v[j]);
                     }
                     if (++within == rows_share) {
@@ -482,11 +329,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     const bf16* base_src = p.epilogue == EPI_ADD ? p.y : p.resid;
     auto fetch_bases = [&]() {
         const int row0 = split * rows_share;
-        const int my_rows = min(rows_share, p.rows - row0);
+        const int my_rows = min(rows_share, rows - row0);
 #pragma unroll
         for (int u = 0; u < kBasePre; ++u) {
             const int j = tid / kPerRow + u * (kTcThreads / kPerRow);
-            base_pre[u] = j < my_rows ? bf2f(base_src[(size_t)(row0 + j) * N + channel]) : 0.0f;
+            base_pre[u] = j < my_rows ? bf2f(base_src[(size_t)(row_first + row0 + j) * N + channel]) : 0.0f;
         }
     };
     if (base_wanted && p.residual_settled != 0) fetch_bases();
@@ -497,7 +344,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     cluster_sync();       // the only cluster barrier: nothing remote is touched after it
     if (*abort_flag == 0 && channel < N) {
         const int row0 = split * rows_share;
-        const int my_rows = min(rows_share, p.rows - row0);
+        const int my_rows = min(rows_share, rows - row0);
         int u = 0;
 #pragma unroll 2
         for (int j = tid / kPerRow; j < my_rows; j += kTcThreads / kPerRow, ++u) {
@@ -520,7 +367,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                     acc_up += part_up[sp];
                 }
             }
-            const size_t out = (size_t)(row0 + j) * N + channel;
+            const size_t out = (size_t)(row_first + row0 + j) * N + channel;
             float val;
             if (GATEUP) {
                 const float gate = acc * scale;
@@ -554,36 +401,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------- host side
-
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                 CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-    static EncodeTiled fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult result;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &result) != cudaSuccess
-            || result != cudaDriverEntryPointSuccess) {
-            p = nullptr;
-        }
-        return reinterpret_cast<EncodeTiled>(p);
-    }();
-    return fn;
-}
-
-bool make_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t inner, uint64_t outer,
-              uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle) {
-    EncodeTiled fn = encode_tiled();
-    if (fn == nullptr) return false;
-    const cuuint64_t dims[2] = {inner, outer};
-    const cuuint64_t strides[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_inner, box_outer};
-    const cuuint32_t elem[2] = {1, 1};
-    return fn(map, type, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 
 // Per-device scratch of the tensor-core path: a buffer for normalised activations.  Allocated
 // once per device by configure_tc_kernels(); launches on one device that use it must be ordered
@@ -637,7 +454,7 @@ cudaError_t configure_one(int (&resident)[9]) {
 template <int MT, bool GATEUP>
 cudaError_t launch_mt(const CUtensorMap& wm, const CUtensorMap& xm, const TcParams& p, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.tiles * p.splits), 1, 1);
+    cfg.gridDim = dim3((unsigned)(p.tiles * p.splits), (unsigned)((p.rows + MT - 1) / MT), 1);
     cfg.blockDim = dim3(kTcThreads, 1, 1);
     cfg.dynamicSmemBytes = tc_smem_bytes<MT, GATEUP>();
     cfg.stream = stream;
@@ -684,7 +501,7 @@ cudaError_t configure_tc_kernels() {
 }
 
 bool gemm_tc_supports(const GemvArgs& a) {
-    if (a.rows < g_tc_min_rows || a.rows > kMaxRows) return false;
+    if (a.rows < g_tc_min_rows || a.rows > kMaxPromptRows) return false;
     if (a.in_features % kBK != 0 || a.in_features > 8192) return false;
     if ((reinterpret_cast<uintptr_t>(a.w) & 15u) != 0 || (reinterpret_cast<uintptr_t>(a.x) & 15u) != 0) return false;
     return scratch_for_current_device() != nullptr;
@@ -709,6 +526,7 @@ cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
         // RMSNorm as its own launch here: at 9+ rows one more launch is noise, and every CTA of the
         // GEMM reads the normalised rows
         bf16* normalized = a.norm_out != nullptr ? a.norm_out : scratch->normalized;
+        if (a.norm_out == nullptr && (size_t)a.rows * K > kNormalizedElems) return cudaErrorInvalidValue;
         const cudaError_t e = launch_rms_norm_rows(a.x, a.norm_w, normalized, a.rows, K, a.eps, stream);
         if (e != cudaSuccess) return e;
         x = normalized;
@@ -720,6 +538,7 @@ cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
     p.tiles = gateup ? (N + 63) / 64 : (N + kTileN - 1) / kTileN;
     p.residual_settled = a.residual_settled ? 1 : 0;
     const int nk = K / kBK;
+    const int row_blocks = (a.rows + mt - 1) / mt;
     // K-slices per tile = cluster size: as many as still let every cluster be resident at once (a
     // second wave would double the time); slices and row shares may be ragged
     const int (&resident)[9] = scratch->resident_clusters[mt == 16 ? 0 : (mt == 32 ? 1 : 2)][gateup ? 1 : 0];
@@ -730,7 +549,7 @@ cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
     }();
     int splits = 1;
     for (int s = 2; s <= split_cap && s <= nk; ++s) {
-        if (p.tiles <= resident[s]) splits = s;
+        if (p.tiles * row_blocks <= resident[s]) splits = s;
     }
     p.splits = splits;
     p.chunks = nk;

@@ -1,0 +1,408 @@
+// Int8 weight-only GEMM for the passes of a prompt: 65 to 2048 activation rows on the 5th-generation
+// tensor cores.
+//
+// Same operation and epilogues as gemm_int8_tc.cu, without its split of K: there are enough output
+// tiles here to fill the GPU.  A CTA owns NT tiles of 128 output channels (TMEM lanes) by 128
+// activation rows (TMEM columns).
+//
+// What bounds it: the tensor cores, if the operands arrive in time.  Per element of K a CTA with NT
+// = 2 fetches 256 bytes of weights and 256 bytes of activations for 8 cycles of MMA (4096 bf16 MACs a
+// cycle and SM), 64 bytes a cycle, about what the L2 delivers to one SM; with one channel tile of 128 the
+// same activations cost 96.  So NT = 2 wherever its tiles fill the GPU, NT = 1 for passes of few rows.
+// The two tiles of a gate/up projection are the gate rows and the up rows of the same 128 channels, so
+// that a thread finds both values of a channel in its own TMEM lane; with NT = 1 a tile holds 64 of
+// each and the up half crosses over through shared memory.
+//
+// Warp roles as in gemm_int8_tc.cu: 0 weight copies, 1 MMA issue, 2 activation copies, 3 TMEM; 4..7 and
+// 8..11 dequantise (a thread turns 128 int8 of its channel into bf16 and stores them to tensor memory as
+// the A operand; about 400 cycles a tile of 16 KB, two of them against the 1024 cycles of a step's MMAs),
+// then read the accumulators.  Every wait is bounded.
+
+#include "q3t_kernels.cuh"
+#include "q3t_tcgen05.cuh"
+
+namespace q3t {
+namespace {
+
+using namespace tc;
+
+constexpr int kGroups = 2;
+constexpr int kThreads = 128 + 128 * kGroups;
+constexpr int kTileN = 128;                   // channels per tile
+constexpr int kTileM = 128;                   // activation rows per CTA
+constexpr int kBK = 128;                      // K elements per step
+constexpr int kWStages = 5;
+constexpr int kXStages = 4;
+constexpr int kAStages = 4;
+constexpr int kWStageBytes = kTileN * kBK;            // 16 KB
+constexpr int kXAtomBytes = kTileM * 128;             // 128 rows x 64 bf16
+constexpr int kXStageBytes = 2 * kXAtomBytes;         // 32 KB
+constexpr int kAStageCols = kBK / 2;
+constexpr int kAStageBase = 256;                      // accumulators in columns [0, 256)
+constexpr uint32_t kTmemCols = 512;
+constexpr unsigned long long kBudgetNs = 2000000000ull;
+constexpr size_t kSmemBytes = 1024 + (size_t)kWStages * kWStageBytes + (size_t)kXStages * kXStageBytes
+    + (2 * kWStages + 2 * kXStages + 2 * kAStages + 1) * sizeof(uint64_t) + 64;
+
+__device__ unsigned int g_wide_errors = 0;
+__device__ unsigned int* g_wide_error_sink = nullptr;
+
+struct WideParams {
+    const float* scales;
+    bf16* y;
+    const bf16* bias;
+    bf16* resid;
+    int out_features;       // N (gate/up: channels, the matrix has 2N rows)
+    int rows;
+    int row_blocks;
+    int steps;              // K / kBK
+    int epilogue;
+};
+
+__device__ __forceinline__ void readers_barrier() {
+    asm volatile("bar.sync 1, %0;" ::"n"(128 * kGroups) : "memory");
+}
+
+template <int NT, bool GATEUP>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map,
+                 const WideParams p) {
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileM >> 3) << 17)
+                                | ((uint32_t)(kTileN >> 4) << 24);
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* w8 = smem;
+    unsigned char* xs = w8 + kWStages * kWStageBytes;
+    uint64_t* full_w = reinterpret_cast<uint64_t*>(xs + kXStages * kXStageBytes);
+    uint64_t* empty_w = full_w + kWStages;
+    uint64_t* full_x = empty_w + kWStages;
+    uint64_t* empty_x = full_x + kXStages;
+    uint64_t* full_a = empty_x + kXStages;
+    uint64_t* empty_a = full_a + kAStages;
+    uint64_t* acc_done = empty_a + kAStages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x;
+    const int warp = __shfl_sync(0xffffffffu, tid / kWarp, 0);
+    const int lane = tid % kWarp;
+    // row blocks fastest: the CTAs in flight share few weight tiles and all of the activations
+    const int tile = blockIdx.x / p.row_blocks;
+    const int row_base = (blockIdx.x % p.row_blocks) * kTileM;
+    const int N = p.out_features;
+    const int nk = p.steps;
+    constexpr int kChannels = GATEUP ? (NT == 2 ? 128 : 64) : NT * kTileN;    // output channels of the CTA
+
+    Guard guard;
+    guard.deadline = now_ns() + kBudgetNs;
+    guard.abort_flag = abort_flag;
+
+    if (tid == 0) {
+        for (int s = 0; s < kWStages; ++s) {
+            mbar_init(&full_w[s], 1);
+            mbar_init(&empty_w[s], 4);
+        }
+        for (int s = 0; s < kXStages; ++s) {
+            mbar_init(&full_x[s], 1);
+            mbar_init(&empty_x[s], 1);
+        }
+        for (int s = 0; s < kAStages; ++s) {
+            mbar_init(&full_a[s], 4);
+            mbar_init(&empty_a[s], 1);
+        }
+        mbar_init(acc_done, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 3) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    // weights never depend on the launch before; activations, residuals and outputs do
+    if (warp >= 1 && warp <= 3) {
+        pdl_wait();
+        if (warp == 1) pdl_trigger();
+    }
+
+    if (warp == 0) {
+        if (elect_one()) {
+            for (int item = 0; item < nk * NT; ++item) {
+                const int s = item % kWStages;
+                if (item >= kWStages && !guard.wait(&empty_w[s], ((item / kWStages) - 1) & 1)) break;
+                mbar_expect_tx(&full_w[s], kWStageBytes);
+                unsigned char* dst = w8 + s * kWStageBytes;
+                const int k = (item / NT) * kBK;
+                const int u = item % NT;
+                if (GATEUP && NT == 1) {
+                    tma_load_2d(dst, &w_map, k, tile * 64, &full_w[s]);
+                    tma_load_2d(dst + kWStageBytes / 2, &w_map, k, N + tile * 64, &full_w[s]);
+                } else if (GATEUP) {
+                    tma_load_2d(dst, &w_map, k, u * N + tile * kTileN, &full_w[s]);
+                } else {
+                    tma_load_2d(dst, &w_map, k, (tile * NT + u) * kTileN, &full_w[s]);
+                }
+            }
+        }
+    } else if (warp == 2) {
+        if (elect_one()) {
+            for (int i = 0; i < nk; ++i) {
+                const int s = i % kXStages;
+                if (i >= kXStages && !guard.wait(&empty_x[s], ((i / kXStages) - 1) & 1)) break;
+                mbar_expect_tx(&full_x[s], kXStageBytes);
+                unsigned char* dst = xs + s * kXStageBytes;
+                tma_load_2d(dst, &x_map, i * kBK, row_base, &full_x[s]);
+                tma_load_2d(dst + kXAtomBytes, &x_map, i * kBK + 64, row_base, &full_x[s]);
+            }
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            bool ok = true;
+            for (int i = 0; i < nk && ok; ++i) {
+                const int sx = i % kXStages;
+                ok = guard.wait(&full_x[sx], (i / kXStages) & 1);
+                if (!ok) break;
+                const uint32_t b_addr = smem_u32(xs + sx * kXStageBytes);
+#pragma unroll
+                for (int u = 0; u < NT; ++u) {
+                    const int item = i * NT + u;
+                    const int sa = item % kAStages;
+                    ok = ok && guard.wait(&full_a[sa], (item / kAStages) & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a_col = tmem_base + kAStageBase + sa * kAStageCols;
+#pragma unroll
+                    for (int j = 0; j < kBK / 16; ++j) {
+                        umma_f16_ts(tmem_base + u * kTileM, a_col + 8 * j,
+                                    umma_desc(b_addr + (j / 4) * kXAtomBytes + 32 * (j % 4)), kIdesc,
+                                    (i | j) != 0 ? 1u : 0u);
+                    }
+                    umma_commit(&empty_a[sa]);
+                }
+                if (ok) umma_commit(&empty_x[sx]);
+            }
+            umma_commit(acc_done);
+        }
+    } else if (warp >= 4) {
+        const int group = (warp - 4) / 4;
+        const int t = (warp % 4) * 32 + lane;        // channel within the tile = TMEM lane
+        const uint32_t lane_base = tmem_base + ((uint32_t)((warp % 4) * 32) << 16);
+        bool ok = true;
+        for (int item = group; item < nk * NT && ok; item += kGroups) {
+            const int s = item % kWStages;
+            const int sa = item % kAStages;
+            if (!__all_sync(0xffffffffu, guard.wait(&full_w[s], (item / kWStages) & 1))) { ok = false; break; }
+            const unsigned char* rowp = w8 + s * kWStageBytes + t * 128;
+            int4 raw[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                raw[c] = *reinterpret_cast<const int4*>(rowp + ((c ^ (t & 7)) << 4));
+            }
+            if (item >= kAStages
+                && !__all_sync(0xffffffffu, guard.wait(&empty_a[sa], ((item / kAStages) - 1) & 1))) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t out[32];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int4 v = raw[4 * h + c];
+                    dequant4(static_cast<uint32_t>(v.x), out[8 * c + 0], out[8 * c + 1]);
+                    dequant4(static_cast<uint32_t>(v.y), out[8 * c + 2], out[8 * c + 3]);
+                    dequant4(static_cast<uint32_t>(v.z), out[8 * c + 4], out[8 * c + 5]);
+                    dequant4(static_cast<uint32_t>(v.w), out[8 * c + 6], out[8 * c + 7]);
+                }
+                tmem_store_32(lane_base + kAStageBase + sa * kAStageCols + 32 * h, out);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&full_a[sa]);
+                mbar_arrive(&empty_w[s]);
+            }
+        }
+        if (ok) ok = guard.wait(acc_done, 0);
+        if (!ok) *abort_flag = 1;
+        pdl_wait();
+        readers_barrier();       // everybody agrees on whether the tile is complete
+        if (*abort_flag == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // Group g finishes the activation rows [64 g, 64 g + 64) of the CTA.
+            const int first_row = row_base + group * 64;
+            const bool up_lane = GATEUP && NT == 1 && t >= 64;
+            float* exchange = reinterpret_cast<float*>(smem) + (size_t)group * 64 * 64;   // the rings are idle now
+            if (GATEUP && NT == 1) {
+                if (up_lane) {
+#pragma unroll
+                    for (int c0 = 0; c0 < 64; c0 += 16) {
+                        float v[16];
+                        tmem_load_row<16>(lane_base + group * 64 + c0, v);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) exchange[(c0 + j) * 64 + t - 64] = v[j];
+                    }
+                }
+                readers_barrier();
+            }
+            if (!up_lane) {
+#pragma unroll 1
+                for (int u = 0; u < (GATEUP ? 1 : NT); ++u) {
+                    const int channel = tile * kChannels + u * kTileN + t;
+                    float scale = 0.0f, scale_up = 0.0f, bias = 0.0f;
+                    if (channel < N) {
+                        scale = p.scales[channel];
+                        if (GATEUP) scale_up = p.scales[N + channel];
+                        if (!GATEUP && p.bias != nullptr) bias = bf2f(p.bias[channel]);
+                    }
+                    const bool adds = !GATEUP && (p.epilogue == EPI_ADD || p.epilogue == EPI_BIAS_ADD);
+                    bf16* dst = (p.epilogue == EPI_BIAS_ADD ? p.resid : p.y) + channel;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < 64; c0 += 16) {
+                        const int row0 = first_row + c0;
+                        if (row0 >= p.rows) break;           // the same for the whole warp
+                        float base[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            base[j] = adds && channel < N && row0 + j < p.rows ? bf2f(dst[(size_t)(row0 + j) * N]) : 0.0f;
+                        }
+                        float v[16], w[16];
+                        tmem_load_row<16>(lane_base + u * kTileM + group * 64 + c0, v);
+                        if (GATEUP) {
+                            if (NT == 2) {
+                                tmem_load_row<16>(lane_base + kTileM + group * 64 + c0, w);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) w[j] = exchange[(c0 + j) * 64 + t];
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            float val;
+                            if (GATEUP) {
+                                const float gate = v[j] * scale;
+                                val = __fdividef(gate, 1.0f + __expf(-gate)) * (w[j] * scale_up);
+                            } else if (p.epilogue == EPI_ADD) {
+                                val = fmaf(v[j], scale, base[j]);
+                            } else if (p.epilogue == EPI_PLAIN) {
+                                val = v[j] * scale;
+                            } else {
+                                val = rbf(v[j] * scale) + bias;
+                                if (p.epilogue == EPI_BIAS_SILU) val = __fdividef(val, 1.0f + __expf(-val));
+                                else if (p.epilogue == EPI_BIAS_ADD) val = base[j] + rbf(val);
+                            }
+                            if (channel < N && row0 + j < p.rows) dst[(size_t)(row0 + j) * N] = f2bf(val);
+                        }
+                    }
+                }
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    if (*abort_flag) {
+        // copies still in flight get time to land before the CTA's memory is released
+        if (tid == 0) {
+            atomicAdd(&g_wide_errors, 1u);
+            if (g_wide_error_sink != nullptr) atomicAdd_system(g_wide_error_sink, 1u);
+        }
+        const unsigned long long until = now_ns() + 200000ull;
+        while (now_ns() < until) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 3) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
+                     : "memory");
+    }
+}
+
+template <int NT, bool GATEUP>
+cudaError_t launch_variant(const CUtensorMap& wm, const CUtensorMap& xm, const WideParams& p, int tiles, cudaStream_t stream) {
+    return launch_pdl(gemm_wide_kernel<NT, GATEUP>, dim3((unsigned)(tiles * p.row_blocks)), dim3(kThreads), kSmemBytes, stream,
+                      wm, xm, p);
+}
+
+}  // namespace
+
+cudaError_t configure_wide_kernels() {
+    cudaError_t e = cudaFuncSetAttribute(gemm_wide_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_wide_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_wide_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_wide_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    return e;
+}
+
+// `channel_tiles`: 1 or 2 (see the top of the file), 0 chooses
+cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int channel_tiles) {
+    const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
+    if (a.rows < 1 || a.rows > kMaxPromptRows || a.out_features < 1 || a.in_features % kBK != 0 || a.in_features < kBK
+        || a.w == nullptr || a.scales == nullptr || a.x == nullptr || a.norm_w != nullptr || a.y32 != nullptr
+        || (a.epilogue == EPI_BIAS_ADD ? a.resid == nullptr : a.y == nullptr)) {
+        return cudaErrorInvalidValue;
+    }
+    if ((a.epilogue == EPI_BIAS || a.epilogue == EPI_BIAS_SILU || a.epilogue == EPI_BIAS_ADD) && a.bias == nullptr) {
+        return cudaErrorInvalidValue;
+    }
+    WideParams p;
+    p.scales = a.scales; p.y = a.y; p.bias = a.bias; p.resid = a.resid;
+    p.out_features = a.out_features; p.rows = a.rows; p.epilogue = a.epilogue;
+    p.row_blocks = (a.rows + kTileM - 1) / kTileM;
+    p.steps = a.in_features / kBK;
+    const int per_single = gateup ? 64 : kTileN;                // output channels of a CTA with one tile
+    int nt = channel_tiles;
+    if (nt != 1 && nt != 2) {
+        // two tiles per CTA once even they come in more than one wave
+        const int ctas = (a.out_features + 2 * per_single - 1) / (2 * per_single) * p.row_blocks;
+        nt = ctas >= 148 ? 2 : 1;
+    }
+    const int tiles = (a.out_features + nt * per_single - 1) / (nt * per_single);
+    alignas(64) CUtensorMap wm, xm;
+    const uint64_t w_rows = gateup ? 2ull * a.out_features : (uint64_t)a.out_features;
+    const uint32_t box_rows = gateup && nt == 1 ? 64 : kTileN;
+    if (!make_map(&wm, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.w, a.in_features, w_rows, a.in_features, kBK, box_rows,
+                  CU_TENSOR_MAP_SWIZZLE_128B)
+        || !make_map(&xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.x, a.in_features, a.rows, (uint64_t)a.in_features * 2, 64, kTileM,
+                     CU_TENSOR_MAP_SWIZZLE_128B)) {
+        return cudaErrorInvalidValue;
+    }
+    if (gateup) return nt == 2 ? launch_variant<2, true>(wm, xm, p, tiles, stream) : launch_variant<1, true>(wm, xm, p, tiles, stream);
+    return nt == 2 ? launch_variant<2, false>(wm, xm, p, tiles, stream) : launch_variant<1, false>(wm, xm, p, tiles, stream);
+}
+
+// Which kernel takes a projection of a prompt pass.  Up to kBlockedRows rows the 64-row kernel of
+// gemm_int8_tc.cu, its row blocks side by side and K split where that still fits one wave; above it
+// this file's.
+cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
+    constexpr int kBlockedRows = 256;
+    GemvArgs a = args;
+    if (a.norm_w != nullptr) {
+        if (a.norm_out == nullptr) return cudaErrorInvalidValue;
+        const cudaError_t e = launch_rms_norm_rows(a.x, a.norm_w, a.norm_out, a.rows, a.in_features, a.eps, stream);
+        if (e != cudaSuccess) return e;
+        a.x = a.norm_out;
+        a.norm_w = nullptr;
+        a.norm_out = nullptr;
+    }
+    return a.rows <= kBlockedRows ? launch_int8_gemm_tc(a, stream) : launch_int8_gemm_wide(a, stream);
+}
+
+unsigned int gemm_wide_error_count() {
+    unsigned int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_wide_errors, sizeof(v)) != cudaSuccess) return ~0u;
+    return v;
+}
+
+cudaError_t set_wide_error_sink(unsigned int* device_visible_word) {
+    return cudaMemcpyToSymbol(g_wide_error_sink, &device_visible_word, sizeof(device_visible_word));
+}
+
+}  // namespace q3t

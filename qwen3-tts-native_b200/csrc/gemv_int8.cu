@@ -378,6 +378,7 @@ int gemv_mode() { return g_gemv_mode; }
 //   everything else, or gemv mode 0     SIMT kernel below, which keeps the reference's summation order
 //                                       bit for bit (mode 0 is for callers that need exactly that)
 cudaError_t launch_int8_gemm(const GemvArgs& a, cudaStream_t stream) {
+    if (a.rows > kMaxRows) return cudaErrorInvalidValue;      // prompt passes: launch_int8_gemm_prompt
     if (gemm_tc_supports(a)) return launch_int8_gemm_tc(a, stream);
     if (g_gemv_mode == 1 && gemv_mma_supports(a)) return launch_int8_gemv_mma(a, stream);
     return launch_int8_gemm_simt(a, stream);

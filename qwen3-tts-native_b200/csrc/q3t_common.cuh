@@ -14,6 +14,7 @@ constexpr float kRmsEps = 1.0e-6f;
 constexpr float kRopeTheta = 1.0e6f;
 constexpr int kPageTokens = 16;          // tokens per KV page
 constexpr int kMaxRows = 64;             // lockstep batch capacity
+constexpr int kMaxPromptRows = 2048;     // prompt positions of one decoder pass
 constexpr int kMaxVocab = 3072;
 constexpr int kPredictorVocab = 2048;
 constexpr int kCodebooks = 16;

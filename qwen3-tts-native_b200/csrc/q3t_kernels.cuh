@@ -35,7 +35,7 @@ struct GemvArgs {
     bf16* resid = nullptr;           // [rows][N] for EPI_BIAS_ADD
     int in_features = 0;             // K, multiple of 16
     int out_features = 0;            // N
-    int rows = 0;                    // 1..kMaxRows
+    int rows = 0;                    // 1..kMaxRows (launch_int8_gemm_prompt: up to kMaxPromptRows)
     int epilogue = EPI_PLAIN;
     float eps = kRmsEps;
     // EPI_ADD / EPI_BIAS_ADD: the accumulated-into values (y, resid) were last written two or more
@@ -91,6 +91,13 @@ cudaError_t configure_tc_kernels();      // also allocates the per-device scratc
 void set_tc_min_rows(int rows);          // 65 or more: never use the tensor-core path
 int tc_min_rows();
 unsigned int gemm_tc_error_count();
+// more than kMaxRows rows (prompt passes), K % 128 == 0, no norm prologue, no fp32 output
+// (gemm_int8_wide.cu); channel_tiles 1 or 2, 0 chooses
+cudaError_t launch_int8_gemm_wide(const GemvArgs& args, cudaStream_t stream, int channel_tiles = 0);
+cudaError_t configure_wide_kernels();
+// projections of a prompt pass of more than kMaxRows rows (needs norm_out when norm_w is given)
+cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream);
+unsigned int gemm_wide_error_count();
 
 cudaError_t launch_quantize_weight_rows(const bf16* weight, int8_t* quantized, float* scales,
                                         int in_features, int out_features, cudaStream_t stream);
@@ -193,6 +200,11 @@ cudaError_t set_attention_error_sink(unsigned int* device_visible_word);
 int set_attention_mode(int mode);
 int attention_mode();
 cudaError_t launch_attention(const AttentionArgs& args, cudaStream_t stream);
+// A prompt pass: rows are consecutive positions of one session (attention_prompt.cu).  Takes the packed
+// q | k | v projection, overwrites q, appends k and v, attends.
+bool prompt_attention_supports(const AttentionArgs& args);
+cudaError_t launch_prompt_attention(const AttentionArgs& args, int base, cudaStream_t stream);
+cudaError_t configure_prompt_kernels();
 // cos/sin of every (position, rotary pair), rounded to bf16 as the fused prologue rounds them;
 // computed by the same device expressions, so using the table changes no bit
 cudaError_t launch_build_rope_table(uint32_t* table, int positions, int head_dim, float theta,

@@ -1,0 +1,42 @@
+"""Prompt passes of more rows than a lockstep batch: the row-blocked and wide tensor-core GEMMs and the
+attention that shares its passes over the cache, against the position-by-position path."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [9, 33, 65, 128, 129, 257, 300, 385])
+def test_prompt_pass_tracks_single_positions(q3t, orc, gpu_model, n):
+    """Lengths around the row blocks (64), the attention blocks (32 positions, 64 tokens) and the change of
+    GEMM kernel (256).  Layer 0's keys and values have one GEMM chain behind them (text projection, q/k/v)
+    whose fp32 sums differ in order only: relative error below one bf16 rounding, 2^-8.  28 layers on, roundings
+    that fell the other way have spread: direction within 0.995, as for the passes of 64."""
+    rng = np.random.default_rng(n)
+    text = [int(t) for t in rng.integers(0, 151936, size=n)]
+    codec = [int(c) if i % 3 == 0 else -1 for i, c in enumerate(rng.integers(0, 2048, size=n))]
+
+    def run(chunk, tc_min_rows):
+        gpu_model.set_option("prefill_chunk", chunk)
+        gpu_model.set_option("tc_min_rows", tc_min_rows)
+        try:
+            s = gpu_model.create_session(512, 5)
+            s.prefill(text, codec)
+            hidden = orc.from_bf16(s.read_state()[0]).ravel()
+            kv = [[orc.from_bf16(x) for x in s.read_kv(layer, 0, n)] for layer in (0, 27)]
+            s.close()
+            return hidden, kv
+        finally:
+            gpu_model.set_option("prefill_chunk", 2048)
+            gpu_model.set_option("tc_min_rows", 9)
+
+    want_hidden, want = run(8, 65)            # passes of 8 rows: what one position alone gives, bit for bit
+    hidden, got = run(2048, 9)
+    again, _ = run(2048, 9)
+    assert np.array_equal(hidden, again)
+    for a, b in zip(got[0], want[0]):
+        assert np.linalg.norm(a - b) <= 2.0 ** -8 * np.linalg.norm(b)
+    for a, b in zip([hidden] + got[1], [want_hidden] + want[1]):
+        a, b = a.ravel(), b.ravel()
+        assert float(a @ b / np.sqrt((a @ a) * (b @ b))) > 0.995
+    assert q3t.library().q3t_kernel_error_count() == 0
