@@ -31,6 +31,7 @@ namespace q3t {
 cudaError_t set_gemv_mma_error_sink(unsigned int* device_visible_word);
 cudaError_t set_tc_error_sink(unsigned int* device_visible_word);
 cudaError_t set_wide_error_sink(unsigned int* device_visible_word);
+cudaError_t set_chain_error_sink(unsigned int* device_visible_word);
 
 namespace {
 std::atomic<unsigned int*> g_error_words[64];
@@ -52,6 +53,7 @@ cudaError_t configure_device() {
     if (e == cudaSuccess) e = configure_tc_kernels();
     if (e == cudaSuccess) e = configure_wide_kernels();
     if (e == cudaSuccess) e = configure_prompt_kernels();
+    if (e == cudaSuccess) e = configure_chain_kernels();
     if (e == cudaSuccess) e = configure_gemv_mma_kernels();
     if (e == cudaSuccess) e = configure_sampler_kernels();
     if (e == cudaSuccess && device >= 0 && device < 64 && g_error_words[device].load() == nullptr) {
@@ -64,6 +66,7 @@ cudaError_t configure_device() {
             e = set_gemv_mma_error_sink(word);
             if (e == cudaSuccess) e = set_tc_error_sink(word);
             if (e == cudaSuccess) e = set_wide_error_sink(word);
+            if (e == cudaSuccess) e = set_chain_error_sink(word);
             if (e == cudaSuccess) e = set_attention_error_sink(word);
             if (e == cudaSuccess) g_error_words[device].store(word, std::memory_order_release);
         }
@@ -1009,6 +1012,8 @@ int32_t q3t_model_set_option(Qwen3TtsModelHandle model, const char* key, int32_t
             m->use_graphs = value != 0;
         } else if (std::strcmp(key, "batch_host_codes") == 0) {
             m->batch_host_codes = value != 0;
+        } else if (std::strcmp(key, "decode_chain") == 0) {
+            m->use_chain = value != 0;
         } else if (std::strcmp(key, "prefill_chunk") == 0) {
             m->prefill_chunk = value < 1 ? 1 : (value > kMaxPromptRows ? kMaxPromptRows : value);
         } else if (std::strcmp(key, "tc_min_rows") == 0) {
@@ -1080,7 +1085,7 @@ int32_t q3t_test_report_device_wait_failure(int32_t device_index) {
 }
 
 uint32_t q3t_kernel_error_count(void) {
-    return gemm_tc_error_count() + gemm_wide_error_count() + gemv_mma_error_count();
+    return gemm_tc_error_count() + gemm_wide_error_count() + gemv_mma_error_count() + chain_error_count();
 }
 
 uint32_t q3t_attention_range_error_count(void) { return attention_range_error_count(); }

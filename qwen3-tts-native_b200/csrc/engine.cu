@@ -478,11 +478,69 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
         predictor_rope = predictor_rope_.as<uint32_t>();
     }
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(rope tables)");
+    build_chain();
     talker_pool.reset(new KvPool(talker.layers, talker.kv_width, 8));
     predictor_pool.reset(new KvPool(predictor.layers, predictor.kv_width, 6));
     finalized_ = true;
     *weight_bytes = weight_bytes_;
     *tensor_count = tensor_count_;
+}
+
+void Model::build_chain() {
+    if (!chain_available() || predictor.head_dim != 128) return;
+    auto table = [](DeviceBuffer& b, const void* host, size_t bytes) {
+        b = DeviceBuffer(bytes);
+        check_cuda(cudaMemcpy(b.as<void>(), host, bytes, cudaMemcpyHostToDevice), "cudaMemcpy(chain table)");
+    };
+    for (int t = 0; t < 2; ++t) {
+        const bool big = t == 1;
+        chain.streams[t] = DeviceBuffer(chain_stream_bytes(big));
+        chain.heads[t] = DeviceBuffer(chain_head_bytes(big));
+        std::vector<ChainLayer> constants;
+        const std::vector<LayerWeights>& layers = big ? talker_layers : predictor_layers;
+        for (size_t l = 0; l < layers.size(); ++l) {
+            const LayerWeights& lw = layers[l];
+            check_cuda(launch_pack_layer(big, static_cast<int>(l), lw.qkv.data, lw.o.data, lw.gate_up.data, lw.down.data,
+                                         chain.streams[t].as<uint8_t>(), upload_stream_), "pack layer");
+            constants.push_back({lw.qkv.scales, lw.o.scales, lw.gate_up.scales, lw.down.scales, lw.input_norm, lw.post_norm,
+                                 lw.q_norm, lw.k_norm});
+        }
+        table(chain.layers[t], constants.data(), constants.size() * sizeof(ChainLayer));
+        std::vector<const float*> scales;
+        for (int h = 0; h < (big ? 1 : kResidualCodebooks); ++h) {
+            const Quantized& head = big ? codec_head : predictor_heads[h];
+            check_cuda(launch_pack_head(big, h, head.data, chain.heads[t].as<uint8_t>(), upload_stream_), "pack head");
+            scales.push_back(head.scales);
+        }
+        table(chain.head_scales[t], scales.data(), scales.size() * sizeof(const float*));
+    }
+    // input row of predictor position p >= 1 for every token of codebook p - 1: the projection the frame would
+    // otherwise make of the token's embedding, by the same kernel (exact sums: same bits whatever rows run together)
+    const size_t PH = predictor.hidden;
+    std::vector<const bf16*> rows;
+    chain.projected_rows = DeviceBuffer(((size_t)kTalkerVocab + 14 * (size_t)kPredictorVocab) * PH * sizeof(bf16));
+    bf16* out = chain.projected_rows.as<bf16>();
+    for (int c = 0; c < kResidualCodebooks; ++c) {
+        const bf16* in = c == 0 ? codec_embedding : predictor_embeddings[c - 1];
+        const int tokens = c == 0 ? kTalkerVocab : kPredictorVocab;
+        rows.push_back(out);
+        for (int first = 0; first < tokens; first += kMaxRows) {
+            GemvArgs g;
+            g.w = small_to_mtp.data; g.scales = small_to_mtp.scales; g.bias = small_to_mtp_bias;
+            g.x = in + (size_t)first * talker.hidden; g.y = out + (size_t)first * PH;
+            g.in_features = talker.hidden; g.out_features = static_cast<int>(PH);
+            g.rows = std::min(kMaxRows, tokens - first); g.epilogue = EPI_BIAS;
+            check_cuda(launch_int8_gemv_mma(g, upload_stream_), "project embeddings");
+        }
+        out += (size_t)tokens * PH;
+    }
+    table(chain.projected, rows.data(), rows.size() * sizeof(const bf16*));
+    chain.exchange = DeviceBuffer(chain_exchange_bytes());
+    check_cuda(cudaMemsetAsync(chain.exchange.as<void>(), 0, chain_exchange_bytes(), upload_stream_), "cudaMemset(exchange)");
+    const uint32_t epoch[2] = {1u, 0u};
+    table(chain.epoch, epoch, sizeof(epoch));
+    check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(decode chain)");
+    chain.ready = true;
 }
 
 unsigned int Model::device_errors() const {
@@ -613,6 +671,46 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
     }
 }
 
+void enqueue_chain(Workspace& w, Model& m, bool talker, int n, cudaStream_t s) {
+    const Model::DecodeChain& c = m.chain;
+    const int t = talker ? 1 : 0;
+    const KvPool& pool = talker ? *m.talker_pool : *m.predictor_pool;
+    ChainLaunch a;
+    a.talker = talker;
+    a.stream = c.streams[t].as<uint8_t>(); a.heads = c.heads[t].as<uint8_t>();
+    a.layers = c.layers[t].as<ChainLayer>(); a.head_scales = c.head_scales[t].as<const float*>();
+    a.final_norm = talker ? m.talker_norm : m.predictor_norm;
+    a.hidden = w.hidden.as<bf16>();
+    a.table = w.table.as<FrameTable>();
+    if (talker) {
+        a.normalized = w.normalized.as<bf16>(); a.logits = w.logits.as<bf16>();
+        a.positions = w.table.as<FrameTable>()->position;
+        a.kv = pool.layout(0, w.talker_pages.as<int>(), Workspace::kMaxPagesPerRow);
+        a.rope_table = m.talker_rope;
+    } else {
+        a.projected = c.projected.as<const bf16*>();
+        a.kv = pool.layout(0, w.predictor_pages.as<int>(), 1);
+        a.rope_table = m.predictor_rope;
+    }
+    a.kv_layer_elems = 2 * pool.plane_elems();
+    a.exchange = c.exchange.as<void>(); a.epoch = c.epoch.as<uint32_t>();
+    a.rows = n;
+    check_launch(launch_decode_chain(a, s), talker ? "talker chain" : "predictor chain");
+}
+
+// The predictor's part of a frame as one chain; only the projection of the hidden state stays a launch of its own.
+void enqueue_predictor_chain(Workspace& w, Model& m, int n, cudaStream_t s) {
+    const int H = m.talker.hidden;
+    check_launch(launch_predictor_input(w.table.as<FrameTable>(), 0, m.codec_embedding, m.predictor_embedding_table,
+                                        w.x_in.as<bf16>(), H, n, s), "predictor input");
+    GemvArgs g;
+    g.w = m.small_to_mtp.data; g.scales = m.small_to_mtp.scales;
+    g.x = w.x_in.as<bf16>(); g.y = w.hidden.as<bf16>(); g.bias = m.small_to_mtp_bias;
+    g.in_features = H; g.out_features = m.predictor.hidden; g.rows = n; g.epilogue = EPI_BIAS;
+    check_launch(launch_int8_gemm(g, s), "predictor input projection");
+    enqueue_chain(w, m, false, n, s);
+}
+
 // 16 predictor positions, 15 sampled codebooks, packed codes (talker.cu:1549-1701)
 void enqueue_predictor(Workspace& w, Model& m, int n, cudaStream_t s) {
     const FrameTable* table = w.table.as<FrameTable>();
@@ -687,6 +785,65 @@ void enqueue_talker(Workspace& w, Model& m, int n, int splits, cudaStream_t s) {
     enqueue_layers(w, m.talker, m.talker_layers, m.talker_rope, *m.talker_pool, w.talker_pages.as<int>(),
                    Workspace::kMaxPagesPerRow, table->position, n, splits, s);
     enqueue_talker_head(w, m, n, 1, s);
+}
+
+void enqueue_talker_chain(Workspace& w, Model& m, int n, cudaStream_t s) {
+    FrameTable* table = w.table.as<FrameTable>();
+    const int H = m.talker.hidden;
+    check_launch(launch_talker_input(table, m.codec_embedding, m.predictor_embedding_table,
+                                   m.text_embedding, kTextVocab, w.hidden.as<bf16>(),
+                                   w.x_in.as<bf16>(), H, n, s), "talker input");
+    enqueue_text_projection(w, m, n, true, s);
+    enqueue_chain(w, m, true, n, s);
+    check_launch(launch_sample_table(table, w.logits.as<bf16>(), kTalkerVocab, kTalkerVocab, 1, 0, m.mask_eos, kEos, n, s),
+                 "sample talker logits");
+    check_launch(launch_frame_end(table, w.normalized.as<bf16>(), H, n, 1, s), "frame end");
+}
+
+// Chains wait between their CTAs, so two of them must not share the GPU's SMs: the chains of a device run one
+// after the other, whatever streams (and models) they come from.
+struct ChainOrder {
+    std::mutex mutex;
+    cudaEvent_t done = nullptr;
+    cudaStream_t last = nullptr;
+};
+ChainOrder g_chain_order[64];
+
+// Held while a frame with chains is enqueued; whatever was enqueued by then, the next holder's stream waits for it.
+class ChainTurn {
+public:
+    ChainTurn(ChainOrder* order, cudaStream_t stream) : order_(order), stream_(stream) {
+        if (order_ == nullptr) return;
+        lock_ = std::unique_lock<std::mutex>(order_->mutex);
+        if (order_->done == nullptr) {
+            check_cuda(cudaEventCreateWithFlags(&order_->done, cudaEventDisableTiming), "cudaEventCreate(chain order)");
+        } else if (order_->last != stream_) {
+            check_cuda(cudaStreamWaitEvent(stream_, order_->done, 0), "cudaStreamWaitEvent(chain order)");
+        }
+    }
+    ~ChainTurn() {
+        if (order_ == nullptr) return;
+        cudaEventRecord(order_->done, stream_);
+        order_->last = stream_;
+    }
+private:
+    ChainOrder* order_;
+    cudaStream_t stream_;
+    std::unique_lock<std::mutex> lock_;
+};
+
+// Whether a frame of these rows runs on the decode chain: few rows, the default kernels (it computes what they
+// compute), draws small enough for its sampler.
+bool frame_takes_chain(const Model& m, const FrameTable& t, int n) {
+    if (!m.chain.ready || m.use_chain == 0 || m.use_graphs == 0 || n > kChainRows || n >= tc_min_rows() || gemv_mode() != 1 || attention_mode() != 1
+        || m.device() < 0 || m.device() >= 64) {
+        return false;
+    }
+    for (int i = 0; i < n; ++i) {
+        const SamplingParams& p = t.predictor[i];
+        if (p.do_sample != 0 && (p.top_k < 1 || p.top_k > kChainTopK)) return false;
+    }
+    return true;
 }
 
 // one prompt position of row 0 (talker.cu:1058-1064 + one decoder pass)
@@ -1033,15 +1190,21 @@ void Session::bind_rows(Workspace& w, Session** s, int n) {
     for (int i = 0; i < n; ++i) w.bound[i] = s[i]->id_;
 }
 
-Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int splits) {
-    const auto key = std::make_pair(n, splits);
+Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int splits, bool chain) {
+    const auto key = std::make_pair(n, chain ? 0 : splits);
     auto found = w.graphs.find(key);
     if (found != w.graphs.end()) return found->second;
     Workspace::Graphs g;
-    g.predictor = capture(w.stream, [&] { enqueue_predictor(w, m, n, w.stream); },
+    g.predictor = capture(w.stream, [&] {
+                              if (chain) enqueue_predictor_chain(w, m, n, w.stream);
+                              else enqueue_predictor(w, m, n, w.stream);
+                          },
                           &g.predictor_kernels);
     try {
-        g.talker = capture(w.stream, [&] { enqueue_talker(w, m, n, splits, w.stream); },
+        g.talker = capture(w.stream, [&] {
+                               if (chain) enqueue_talker_chain(w, m, n, w.stream);
+                               else enqueue_talker(w, m, n, splits, w.stream);
+                           },
                            &g.talker_kernels);
     } catch (...) {
         cudaGraphExecDestroy(g.predictor);
@@ -1062,15 +1225,17 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
         w.destroy_graphs();
         w.option_epoch = m.option_epoch;
     }
-    w.ensure_scratch(splits);
+    const bool chain = frame_takes_chain(m, *w.host_table, n);
+    if (!chain) w.ensure_scratch(splits);
     bind_rows(w, s, n);
+    const ChainTurn turn(chain ? &g_chain_order[m.device()] : nullptr, w.stream);
     if (upload_table) {
         check_cuda(cudaMemcpyAsync(w.table.as<void>(), w.host_table, sizeof(FrameTable),
                                    cudaMemcpyHostToDevice, w.stream), "upload frame table");
         check_cuda(cudaEventRecord(w.table_uploaded, w.stream), "cudaEventRecord(table)");
     }
     if (m.use_graphs) {
-        Workspace::Graphs& g = frame_graphs(w, m, n, splits);
+        Workspace::Graphs& g = frame_graphs(w, m, n, splits, chain);
         check_cuda(cudaEventRecord(w.predictor_start, w.stream), "cudaEventRecord");
         check_cuda(cudaGraphLaunch(g.predictor, w.stream), "cudaGraphLaunch(predictor)");
         check_cuda(cudaEventRecord(w.predictor_stop, w.stream), "cudaEventRecord");
@@ -1085,7 +1250,8 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
         m.kernel_launches += static_cast<uint64_t>(g.predictor_kernels + g.talker_kernels);
     } else {
         check_cuda(cudaEventRecord(w.predictor_start, w.stream), "cudaEventRecord");
-        enqueue_predictor(w, m, n, w.stream);
+        if (chain) enqueue_predictor_chain(w, m, n, w.stream);
+        else enqueue_predictor(w, m, n, w.stream);
         check_cuda(cudaEventRecord(w.predictor_stop, w.stream), "cudaEventRecord");
         if (record_session_events) {
             for (int i = 0; i < n; ++i) {
@@ -1093,7 +1259,8 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
             }
         }
         check_cuda(cudaEventRecord(w.talker_start, w.stream), "cudaEventRecord");
-        enqueue_talker(w, m, n, splits, w.stream);
+        if (chain) enqueue_talker_chain(w, m, n, w.stream);
+        else enqueue_talker(w, m, n, splits, w.stream);
         check_cuda(cudaEventRecord(w.talker_stop, w.stream), "cudaEventRecord");
     }
     if (record_session_events) {

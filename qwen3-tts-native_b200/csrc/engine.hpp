@@ -147,7 +147,7 @@ struct Workspace {
         int predictor_kernels = 0;   // kernel nodes in each graph
         int talker_kernels = 0;
     };
-    std::map<std::pair<int, int>, Graphs> graphs;   // (rows, talker splits) -> graphs
+    std::map<std::pair<int, int>, Graphs> graphs;   // (rows, talker splits; 0: the decode chain) -> graphs
     cudaEvent_t predictor_start = nullptr, predictor_stop = nullptr;
     // frames launched on this workspace, and the GPU times of the frame `timed_frame` (every
     // session of a lockstep frame reports the same two numbers: they are read from the events once)
@@ -215,9 +215,17 @@ public:
     static constexpr int kRopePositions = 8192;
     const uint32_t* talker_rope = nullptr;
     const uint32_t* predictor_rope = nullptr;
+    // The decode chain's weights as per-CTA streams, the predictor's input rows of every token (embedding times
+    // small_to_mtp), its exchange buffers.  Built by finalize() where the device can hold the chain.
+    struct DecodeChain {
+        bool ready = false;
+        DeviceBuffer streams[2], heads[2], layers[2], head_scales[2];     // 0 predictor, 1 talker
+        DeviceBuffer projected_rows, projected, exchange, epoch;
+    } chain;
     std::mutex mutex;               // pools, workspaces
     int mask_eos = 0;
     int use_graphs = 1;
+    int use_chain = 1;              // frames of up to kChainRows sessions run as two cooperative launches
     int option_epoch = 0;           // bumped when an option that captured graphs bake in changes
     int batch_host_codes = 0;       // lockstep batches also mirror the 16 codes to pinned host memory
     std::atomic<uint64_t> kernel_launches{0};   // kernels of this library launched through frame graphs
@@ -235,6 +243,7 @@ private:
                         float* scales);
     Quantized allocate_quantized(uint64_t rows, uint64_t cols);
     Quantized add_quant_matrix(const std::string& name, uint64_t rows, uint64_t cols);
+    void build_chain();
     void plan_layers(const std::string& prefix, const ModelDims& d, std::vector<LayerWeights>& out);
 
     int device_;
@@ -317,7 +326,7 @@ private:
     void fill_row(FrameTable& t, int row, int trailing_text, const SamplingParams& talker,
                   const SamplingParams& predictor, bool host_codes) const;
     static void bind_rows(Workspace& w, Session** s, int n);
-    static Workspace::Graphs& frame_graphs(Workspace& w, Model& m, int n, int splits);
+    static Workspace::Graphs& frame_graphs(Workspace& w, Model& m, int n, int splits, bool chain);
     static void launch_frame(Workspace& w, Model& m, Session** s, int n, bool upload_table,
                              bool record_session_events);
 

@@ -265,6 +265,47 @@ struct FrameTable {
     SamplingParams predictor[kMaxRows];
 };
 
+// ---------------------------------------------------------------- decode chain (decode_chain.cu)
+// The predictor's 16 positions with their draws, or the talker's layers and head, of 1..8 rows in one
+// cooperative launch of 128 CTAs.  At most one chain may run on a device at a time.
+struct ChainLayer {                  // device array, one per layer
+    const float *qkv_s, *o_s, *gu_s, *down_s;
+    const bf16 *in_norm, *post_norm, *q_norm, *k_norm;
+};
+struct ChainLaunch {
+    bool talker = false;
+    const uint8_t* stream = nullptr;          // chain_stream_bytes(), filled by launch_pack_layer
+    const uint8_t* heads = nullptr;           // chain_head_bytes(), filled by launch_pack_head
+    const ChainLayer* layers = nullptr;
+    const float* const* head_scales = nullptr;    // device array: 15 (predictor) or 1
+    const bf16* final_norm = nullptr;
+    const bf16* hidden = nullptr;             // [rows][hidden]: talker input, or the predictor's at position 0
+    bf16* normalized = nullptr;               // talker out: [rows][hidden] after the final norm
+    bf16* logits = nullptr;                   // talker out: [rows][3072]
+    const bf16* const* projected = nullptr;   // predictor: device array of 15 tables [vocabulary][1024], the input row of
+                                              //   position p (1..15) for every token of codebook p - 1
+    FrameTable* table = nullptr;              // predictor: sampling, random states, tokens and codes
+    const int* positions = nullptr;           // talker: [rows]
+    KvLayout kv;                              // paged; offsets of layer 0
+    long long kv_layer_elems = 0;             // elements between the planes of consecutive layers
+    const uint32_t* rope_table = nullptr;
+    void* exchange = nullptr;                 // chain_exchange_bytes(), zeroed once
+    uint32_t* epoch = nullptr;                // two words, {1, 0} at first
+    int rows = 0;
+};
+constexpr int kChainRows = 8;
+constexpr int kChainTopK = 128;               // larger or unlimited top-k draws run outside the chain
+bool chain_available();
+cudaError_t configure_chain_kernels();
+size_t chain_stream_bytes(bool talker);
+size_t chain_head_bytes(bool talker);
+size_t chain_exchange_bytes();
+cudaError_t launch_pack_layer(bool talker, int layer, const int8_t* qkv, const int8_t* o, const int8_t* gate_up, const int8_t* down,
+                              uint8_t* stream_base, cudaStream_t stream);
+cudaError_t launch_pack_head(bool talker, int index, const int8_t* head, uint8_t* heads_base, cudaStream_t stream);
+cudaError_t launch_decode_chain(const ChainLaunch& chain, cudaStream_t stream);
+unsigned int chain_error_count();
+
 // Sampler over table rows: row r reads logits + r*logits_stride.  talker != 0: reserved
 // tokens masked, repetition penalty, token -> sampled[r] and appended to history[r];
 // talker == 0: token -> frame_tokens[r][store_index].

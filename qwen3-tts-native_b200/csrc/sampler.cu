@@ -19,18 +19,13 @@
 // denominator, the retained total and the final cumulative scan all read that one prefix.
 
 #include "q3t_kernels.cuh"
+#include "q3t_sampler.cuh"
 
 namespace q3t {
 namespace {
 
 constexpr int kSampleThreads = 512;
 constexpr int kSampleWarps = kSampleThreads / kWarp;
-
-__device__ __forceinline__ unsigned int order_key(float v) {
-    unsigned int u = __float_as_uint(v);
-    if (u == 0x80000000u) u = 0u;   // -0 ties with +0
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
 
 __device__ __forceinline__ float key_value(unsigned long long ckey) {
     const unsigned int k = static_cast<unsigned int>(ckey >> 12);
@@ -39,19 +34,6 @@ __device__ __forceinline__ float key_value(unsigned long long ckey) {
 
 __device__ __forceinline__ int key_index(unsigned long long ckey) {
     return 4095 - static_cast<int>(ckey & 0xfffull);
-}
-
-// xorshift64* (sampling_kernels.cu:53-69)
-__device__ float uniform_random(unsigned long long* state) {
-    unsigned long long v = *state;
-    if (v == 0) v = 0x9e3779b97f4a7c15ULL;
-    v ^= v >> 12;
-    v ^= v << 25;
-    v ^= v >> 27;
-    *state = v;
-    const unsigned long long r = v * 0x2545f4914f6cdd1dULL;
-    constexpr double scale = 1.0 / 9007199254740992.0;
-    return static_cast<float>(static_cast<double>(r >> 11) * scale);
 }
 
 __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v,
@@ -104,6 +86,8 @@ __device__ __forceinline__ void sample_one(const SamplerRow& r, unsigned char* s
         }
         __syncthreads();
     }
+    const bool small_k = r.do_sample != 0 && r.top_k >= 1 && min(r.top_k, V) <= kTopKMost;
+    unsigned int* short_keys = reinterpret_cast<unsigned int*>(smem_raw);     // small_k: [V], then the scratch
     for (int t = tid; t < V; t += kSampleThreads) {
         float v;
         if (r.suppress && t >= kPredictorVocab && (t != r.eos || r.mask_eos)) {
@@ -116,10 +100,27 @@ __device__ __forceinline__ void sample_one(const SamplerRow& r, unsigned char* s
                 v = v < 0.0f ? v * r.penalty : v / r.penalty;
             }
         }
-        keys[t] = (static_cast<unsigned long long>(order_key(v)) << 12)
-                  | static_cast<unsigned long long>(4095 - t);
+        if (small_k) {
+            short_keys[t] = order_key(v);
+        } else {
+            keys[t] = (static_cast<unsigned long long>(order_key(v)) << 12)
+                      | static_cast<unsigned long long>(4095 - t);
+        }
     }
     __syncthreads();
+
+    if (small_k) {
+        // the usual case: a handful of candidates, see q3t_sampler.cuh
+        TopKScratch& scratch = *reinterpret_cast<TopKScratch*>(smem_raw + (size_t)kMaxVocab * sizeof(unsigned int));
+        const int token = sample_top_k_block<kSampleThreads>(short_keys, V, min(r.top_k, V), r.top_p, r.temperature, r.rng,
+                                                             scratch, tid, [] { __syncthreads(); });
+        if (tid == 0) {
+            *r.selected = token;
+            if (r.store_a != nullptr) r.store_a[r.store_a_index] = token;
+            if (r.store_b != nullptr) r.store_b[count] = token;
+        }
+        return;
+    }
 
     const bool direct = r.do_sample != 0 && r.top_k == 0 && r.top_p >= 1.0f;
     const int selections = r.do_sample == 0 ? 1 : (r.top_k == 0 ? V : min(r.top_k, V));
@@ -379,6 +380,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_value_kernel(const Samp
 }
 
 constexpr size_t kSampleSmem = (size_t)kMaxVocab * 24;
+static_assert(kMaxVocab * sizeof(unsigned int) + sizeof(TopKScratch) <= kSampleSmem, "small-k layout");
 
 }  // namespace
 

@@ -1,0 +1,89 @@
+"""The decode chain (frames of up to eight sessions as two cooperative launches) against the frame made
+launch by launch, at the context lengths where its page walk and merges change."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# one page and its edges, the first page of a second class (16 x 16 tokens), several pages per warp
+POSITIONS = [1, 15, 16, 17, 255, 256, 700, 2100]
+
+
+@pytest.fixture(scope="module")
+def model(gpu_model):
+    gpu_model.set_option("mask_eos", 1)
+    yield gpu_model
+    gpu_model.set_option("decode_chain", 1)
+
+
+def frame(q3t, model, positions, chain, predictor=None, frames=1):
+    """(codes, next tokens, hidden rows, layer-0 and layer-1 K/V rows of the new token) after `frames` frames."""
+    model.set_option("decode_chain", chain)
+    sessions = []
+    for i, p in enumerate(positions):
+        s = model.create_session((p + frames + 32) // 16 * 16, 100 + i)
+        s.talker_sampling = q3t.SamplingConfig(True, 50, 0.9, 0.9, 1.05)
+        s.predictor_sampling = predictor or q3t.SamplingConfig(True, 50, 1.0, 0.9, 1.0)
+        s.synthetic_prefill(p, 1000 + i)
+        sessions.append(s)
+    for f in range(frames):
+        if len(sessions) == 1:
+            sessions[0].next_frame(7 + f)
+        else:
+            for p in model.batch_begin_device_frames(sessions, [7 + f] * len(sessions)):
+                p.finish_without_consumer()
+    out = []
+    for s, p in zip(sessions, positions):
+        hidden, tokens, rng = s.read_state()
+        kv = [np.stack(s.read_kv(layer, p, 1)) for layer in (0, 1)]
+        out.append((tokens, s.current_semantic_token, hidden, kv, rng))
+        s.close()
+    return out
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 5, 8])
+def test_chain_equals_launch_by_launch(q3t, orc, model, rows):
+    """The predictor's part is the same to the bit (codes, random state); so is the new token's K/V of layer 0.  The
+    talker merges a long context page by page instead of in chunks of 64 tokens: fp32 sums in another order.  From
+    there to layer 1's K lie eight bf16 roundings (attention, o, gate/up, down, q/k/v, norm twice, rotation), each of
+    which may fall the other way by an ulp, 2^-8 to 2^-7 of a value, in part of the elements: 8 x 2^-9 = 2^-6 at most.
+    After 28 layers: a direction within 0.995.  Within one page: to the bit."""
+    positions = POSITIONS[:rows] if rows != 3 else POSITIONS[5:8]
+    chained, launched = frame(q3t, model, positions, 1), frame(q3t, model, positions, 0)
+    for p, a, b in zip(positions, chained, launched):
+        assert np.array_equal(a[0], b[0]), p
+        assert np.array_equal(a[3][0], b[3][0])
+        if p < 16:
+            assert a[1] == b[1] and np.array_equal(a[2], b[2]) and a[4] == b[4]
+        ka, kb = orc.from_bf16(a[3][1]).ravel(), orc.from_bf16(b[3][1]).ravel()
+        assert np.linalg.norm(ka - kb) <= 2.0 ** -6 * np.linalg.norm(kb)
+        ha, hb = orc.from_bf16(a[2]).ravel(), orc.from_bf16(b[2]).ravel()
+        assert float(ha @ hb / np.sqrt((ha @ ha) * (hb @ hb))) > 0.995
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
+@pytest.mark.parametrize("rows", [2, 4, 7, 8])
+def test_row_does_not_depend_on_its_batch(q3t, model, rows):
+    together = frame(q3t, model, POSITIONS[-rows:], 1, frames=2)
+    for i, p in enumerate(POSITIONS[-rows:]):
+        # the same session alone: its seeds are those of its place in the batch
+        model.set_option("decode_chain", 1)
+        s = model.create_session((p + 34) // 16 * 16, 100 + i)
+        s.talker_sampling = q3t.SamplingConfig(True, 50, 0.9, 0.9, 1.05)
+        s.predictor_sampling = q3t.SamplingConfig(True, 50, 1.0, 0.9, 1.0)
+        s.synthetic_prefill(p, 1000 + i)
+        for f in range(2):
+            s.next_frame(7 + f)
+        hidden, tokens, rng = s.read_state()
+        assert np.array_equal(tokens, together[i][0]) and np.array_equal(hidden, together[i][2]) and rng == together[i][4]
+        s.close()
+
+
+@pytest.mark.parametrize("config", [(False, 0, 1.0), (True, 1, 1.0), (True, 128, 0.5), (True, 129, 0.9), (True, 0, 1.0)])
+def test_draws_inside_and_outside_the_chain(q3t, model, config):
+    """Greedy and top-k up to 128 are drawn inside the chain, the rest launch by launch: the codes are the same."""
+    do_sample, top_k, top_p = config
+    predictor = q3t.SamplingConfig(do_sample, top_k, top_p, 0.9, 1.0)
+    for positions in ([9], [9, 40, 3]):
+        for a, b in zip(frame(q3t, model, positions, 1, predictor), frame(q3t, model, positions, 0, predictor)):
+            assert np.array_equal(a[0], b[0])
