@@ -425,13 +425,17 @@ struct Chain {
                 if (i == 0 || at % kSlot < kTile) wait_slot(seq + at / kSlot);
                 w[i] = reinterpret_cast<const int4*>(smem + L::AtRing + (seq + at / kSlot) % L::Slots * kSlot + at % kSlot) + lane;
             }
-            int acc[G][NT][4];
+            constexpr int kChains = G * NT <= 4 ? 2 : 1;       // accumulators per tile (integers: any order)
+            int acc[G][NT][4], acc2[kChains == 2 ? G : 1][NT][4];
 #pragma unroll
             for (int i = 0; i < G; ++i)
 #pragma unroll
                 for (int q = 0; q < NT; ++q)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[i][q][e] = 0;
+                    for (int e = 0; e < 4; ++e) {
+                        acc[i][q][e] = 0;
+                        if (kChains == 2) acc2[kChains == 2 ? i : 0][q][e] = 0;
+                    }
 #pragma unroll
             for (int j = 0; j < S::J; ++j) {
                 uint32_t b[NT][4];
@@ -443,9 +447,18 @@ struct Chain {
 #pragma unroll
                     for (int q = 0; q < NT; ++q) {
                         imma(acc[i][q], wa.x, wb.x, wa.y, wb.y, b[q][0], b[q][1]);
-                        imma(acc[i][q], wa.z, wb.z, wa.w, wb.w, b[q][2], b[q][3]);
+                        if (kChains == 2) imma(acc2[kChains == 2 ? i : 0][q], wa.z, wb.z, wa.w, wb.w, b[q][2], b[q][3]);
+                        else imma(acc[i][q], wa.z, wb.z, wa.w, wb.w, b[q][2], b[q][3]);
                     }
                 }
+            }
+            if (kChains == 2) {
+#pragma unroll
+                for (int i = 0; i < G; ++i)
+#pragma unroll
+                    for (int q = 0; q < NT; ++q)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[i][q][e] += acc2[kChains == 2 ? i : 0][q][e];
             }
             if (kReleaseEarly<TILES> && t0 + G >= TILES) release(seq, off, TILES * kTile);
             const int t = lane & 3;
@@ -722,6 +735,18 @@ struct Chain {
     struct HeadNorm {
         bf16 q[4], k[4];
     };
+    // cos | sin of the head vectors this warp rotates: fixed for a launch (talker) or a position (predictor)
+    static constexpr int kJobs = (3 * ROWS + 7) / 8;
+    uint32_t cs[kJobs][2];
+    __device__ __forceinline__ void load_rotations() {
+#pragma unroll
+        for (int i = 0; i < kJobs; ++i) {
+            const int job = warp + 8 * i;
+            const uint32_t* at = a.rope_table + (size_t)misc->position[job < 3 * rows ? job / 3 : 0] * 64 + lane;
+            cs[i][0] = at[0];
+            cs[i][1] = at[32];
+        }
+    }
     // q heads of every row (and the new key where this CTA will need it) from the exchanged projections: per-head
     // RMSNorm and rotation, one warp per head vector, lane l dims l, l + 32, l + 64, l + 96
     template <class Needs>
@@ -729,13 +754,13 @@ struct Chain {
         const bf16* qkv = reinterpret_cast<const bf16*>(smem + L::AtQkv);
         float* qs = reinterpret_cast<float*>(smem + L::AtQ);
         bf16* knew = reinterpret_cast<bf16*>(smem + L::AtKNew);
-#pragma unroll 1
-        for (int job = warp; job < 3 * rows; job += kWorkers / kWarp) {
+#pragma unroll
+        for (int i = 0; i < kJobs; ++i) {
+            const int job = warp + 8 * i;
             const int r = job / 3, h = job % 3;
-            if (!needs(r, h == 2)) continue;
+            if (job >= 3 * rows || !needs(r, h == 2)) continue;
             const bf16* src = qkv + r * 512 + h * 128;
-            const uint32_t* cs = a.rope_table + (size_t)misc->position[r] * 64 + lane;
-            const uint32_t cs0 = cs[0], cs1 = cs[32];
+            const uint32_t cs0 = cs[i][0], cs1 = cs[i][1];
             float x[4], sq[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -797,19 +822,27 @@ struct Chain {
         sync_workers();
     }
 
-    // Talker: page p of a row belongs to CTA p % 16 of the group and there to class (p / 16) % 8; a class is
-    // walked by one warp (which one depends on the row, so that short rows spread over the warps), the classes
-    // and then the CTAs are merged in order.  The grouping of a row's pages depends on its length only.
+    // Talker: kBlock consecutive pages of a row go to one CTA, block after block over the group's 16 CTAs ("slots",
+    // counted from a CTA that depends on the row, so that the rows of a batch spread), and there to classes, one page
+    // to a class at first; a class is walked by one warp.  The classes and then the slots are merged in order.  The
+    // grouping of a row's pages depends on its length only.  (Blocks: the fewer CTAs hold parts of a row, the fewer
+    // partial results everybody has to collect; the more pages a CTA has to fetch.)
+    static constexpr int kBlock = 2;
+    static constexpr int kPageStep = 8 * kRanks;         // from a class's page to its next
     struct Walk {
         int row, page;
         bf16 *k, *v;          // its rows in layer 0
         bool any;
     };
     __device__ __forceinline__ int pages_of(int row) { return misc->position[row] / kPageTokens + 1; }
+    __device__ __forceinline__ int slots_of(int row) { return min(kRanks, (pages_of(row) + kBlock - 1) / kBlock); }
+    __device__ __forceinline__ int my_slot(int row) { return (rank - 2 * row) & (kRanks - 1); }
+    __device__ __forceinline__ int rank_of(int row, int slot) { return (slot + 2 * row) & (kRanks - 1); }
+    __device__ __forceinline__ int class_page(int slot, int cls) { return kBlock * (slot + kRanks * (cls / kBlock)) + cls % kBlock; }
     __device__ __forceinline__ Walk first_page() {
         Walk w{0, 0, nullptr, nullptr, false};
         for (w.row = 0; w.row < rows; ++w.row) {
-            w.page = rank + 16 * ((warp - w.row) & 7);
+            w.page = class_page(my_slot(w.row), (warp - w.row) & 7);
             if (w.page < pages_of(w.row)) {
                 w.k = page_at(a.kv, w.row, w.page, false);
                 w.v = page_at(a.kv, w.row, w.page, true);
@@ -829,7 +862,7 @@ struct Chain {
         float* out_s = l_s + ROWS * 8 * 2;                                        // [row][head][132]: max, sum, weighted V
         bf16* att = reinterpret_cast<bf16*>(smem + L::AtAtt);
         const float scale = rsqrtf(128.0f);
-        rotate_heads(hn, [&](int r, bool key) { return key ? (pages_of(r) - 1) % kRanks == rank : rank < pages_of(r); });
+        rotate_heads(hn, [&](int r, bool key) { return key ? (pages_of(r) - 1) / kBlock % kRanks == my_slot(r) : my_slot(r) < slots_of(r); });
         if (w0.any) {
             bool loaded = true;
 #pragma unroll 1
@@ -840,9 +873,9 @@ struct Chain {
                 for (int x = 0; x < 8; ++x)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) o[x][e] = 0.0f;
-                const int first = rank + 16 * cls;
+                const int first = class_page(my_slot(row), cls);
 #pragma unroll 1
-                for (int pg = first; pg < np; pg += 16 * 8) {
+                for (int pg = first; pg < np; pg += kPageStep) {
                     bf16 *kp = w0.k + layer_elems, *vp = w0.v + layer_elems;
                     if (!loaded) {
                         kp = page_at(a.kv, row, pg, false) + layer_elems;
@@ -898,9 +931,10 @@ struct Chain {
         const int g = tid >> 7, d = tid & 127;
 #pragma unroll 1
         for (int r = 0; r < rows; ++r) {
-            const int np = pages_of(r);
-            if (rank >= np) continue;
-            const int classes = min(8, (np - rank + 15) / 16);
+            const int np = pages_of(r), slot = my_slot(r);
+            if (slot >= slots_of(r)) continue;
+            int classes = 1;
+            while (classes < 8 && class_page(slot, classes) < np) ++classes;
             float M = -INFINITY;
             for (int c = 0; c < classes; ++c) M = fmaxf(M, m_s[(r * 8 + c) * 2 + g]);
             float Lsum = 0.0f, A = 0.0f;
@@ -924,40 +958,43 @@ struct Chain {
 #pragma unroll 1
         for (int i = tid; i < rows * 88; i += kWorkers) {
             const int r = i / 88, q = i % 88;
-            if (rank >= pages_of(r)) continue;
+            if (my_slot(r) >= slots_of(r)) continue;
             const float* src = out_s + (r * 2 + q / 44) * 132 + 3 * (q % 44);
             put_quad(group_at(kAtAttnPart, 88, b, rank, r) + q, __float_as_uint(src[0]), __float_as_uint(src[1]), __float_as_uint(src[2]), flag);
         }
         float* gathered = reinterpret_cast<float*>(smem + L::AtX);              // [rank][132] of a head
         auto fold = [&](const float* from, int stride, int ranks, int dim) {
-            float M = -INFINITY;
-            for (int k = 0; k < ranks; ++k) M = fmaxf(M, from[k * stride]);
+            // lane k holds what the fold needs of CTA k: its factor and sum
+            const float mine = lane < ranks ? from[lane * stride] : -INFINITY;
+            const float sum = lane < ranks ? from[lane * stride + 1] : 0.0f;
+            const float fac = expf(mine - warp_max_xor(mine));
             float Lsum = 0.0f, A = 0.0f;
+#pragma unroll 4
             for (int k = 0; k < ranks; ++k) {
-                const float fac = expf(from[k * stride] - M);
-                Lsum = fmaf(from[k * stride + 1], fac, Lsum);
-                A = fmaf(from[k * stride + 2 + dim], fac, A);
+                const float fk = __shfl_sync(0xffffffffu, fac, k);
+                Lsum = fmaf(__shfl_sync(0xffffffffu, sum, k), fk, Lsum);
+                A = fmaf(from[k * stride + 2 + dim], fk, A);
             }
             return A * (1.0f / Lsum);
         };
         sync_workers();        // out_s has been read; the area is written again below
         if constexpr (ROWS == 1) {
-            const int ranks = min(kRanks, pages_of(0));
+            const int ranks = slots_of(0);
 #pragma unroll 1
-            for (int i = tid; i < ranks * 88; i += 2 * kWorkers) {
-                const Quad* p[2];
-                Quad v[2];
-                float* dst[2];
+            for (int i = tid; i < ranks * 88; i += 3 * kWorkers) {
+                const Quad* p[3];
+                Quad v[3];
+                float* dst[3];
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
+                for (int k = 0; k < 3; ++k) {
                     const int n = min(i + k * kWorkers, ranks * 88 - 1);
                     const int rk = n / 88, q = n % 88;
-                    p[k] = group_at(kAtAttnPart, 88, b, rk, 0) + q;
+                    p[k] = group_at(kAtAttnPart, 88, b, rank_of(0, rk), 0) + q;
                     dst[k] = gathered + (rk * 2 + q / 44) * 132 + 3 * (q % 44);
                 }
                 poll(p, v, flag);
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
+                for (int k = 0; k < 3; ++k) {
                     dst[k][0] = __uint_as_float(v[k].x);
                     dst[k][1] = __uint_as_float(v[k].y);
                     dst[k][2] = __uint_as_float(v[k].z);
@@ -972,18 +1009,19 @@ struct Chain {
             const uint32_t flag_o = next_flag();
             bf16* mine = reinterpret_cast<bf16*>(smem + L::AtStage);
             if (row < rows) {
-                const int ranks = min(kRanks, pages_of(row));
+                const int ranks = slots_of(row);
 #pragma unroll 1
                 for (int i = tid; i < ranks * 44; i += kWorkers) {
                     const int rk = i / 44, q = i % 44;
-                    const Quad v = poll_one(group_at(kAtAttnPart, 88, b, rk, row) + head * 44 + q, flag);
+                    const Quad v = poll_one(group_at(kAtAttnPart, 88, b, rank_of(row, rk), row) + head * 44 + q, flag);
                     float* dst = gathered + rk * 132 + 3 * q;
                     dst[0] = __uint_as_float(v.x);
                     dst[1] = __uint_as_float(v.y);
                     dst[2] = __uint_as_float(v.z);
                 }
                 sync_workers();
-                if (tid < 132) mine[tid] = f2bf(tid < 128 ? fold(gathered, 132, ranks, tid) : 0.0f);
+                if (warp < 4) mine[tid] = f2bf(fold(gathered, 132, ranks, tid));
+                else if (tid < 132) mine[tid] = f2bf(0.0f);
                 sync_workers();
                 if (tid < 22) {
                     const uint32_t* w = reinterpret_cast<const uint32_t*>(mine) + 3 * tid;
@@ -1016,10 +1054,13 @@ struct Chain {
             hn.q[j] = lc.q_norm[lane + 32 * j];
             hn.k[j] = lc.k_norm[lane + 32 * j];
         }
-        // older cache rows
+        // older cache rows: asked into the L2 a layer ahead (a page of one head is 4 KB), fetched behind the q/k/v exchange
         page::Fragments f;
         const long long layer_elems = index * a.kv_layer_elems;
-        if (walk.any) page::load(f, walk.k + layer_elems, walk.v + layer_elems, TALKER ? older_in(walk.row, walk.page) : pos, lane);
+        if (TALKER && walk.any && lane < 2 && index + 1 < S::Layers) {
+            const bf16* p = (lane == 0 ? walk.k : walk.v) + layer_elems + a.kv_layer_elems;
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(kPageTokens * 128 * 2) : "memory");
+        }
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
             // scales of this half's outputs: q/k/v row (warp = activation row, lane = weight row) or channel
@@ -1044,6 +1085,9 @@ struct Chain {
 #pragma unroll
                     for (int w = 0; w < 8; ++w) sum += red[(w * rows + warp) * 32 + lane];
                     put_values(sum * scale, 32, group_at(kAtQkv, 6, b, rank, warp), flag);
+                }
+                if (walk.any) {
+                    page::load(f, walk.k + layer_elems, walk.v + layer_elems, TALKER ? older_in(walk.row, walk.page) : pos, lane);
                 }
                 release_full<2>();
                 collect_group<6, 16>(kAtQkv, b, flag, reinterpret_cast<uint32_t*>(smem + L::AtQkv), 256);
@@ -1214,6 +1258,7 @@ struct Chain {
         load_norm(lc.in_norm, nw);
         if constexpr (TALKER) {
             const Walk walk = first_page();
+            load_rotations();
             load_hidden([&](int r) { return a.hidden + (size_t)r * S::H; });
 #pragma unroll 1
             for (int l = 0; l < S::Layers; ++l) layer(l, 0, lc, nw, walk);
@@ -1249,6 +1294,7 @@ struct Chain {
                 if (tid < rows) misc->position[tid] = p;
                 if (p > 0 && warp < rows) __threadfence();      // cache rows appended by other CTAs at earlier positions
                 sync_workers();
+                load_rotations();
 #pragma unroll 1
                 for (int l = 0; l < S::Layers; ++l) layer(l, p, lc, nw, walk);
                 if (p > 0) predictor_head(p, head_scales);

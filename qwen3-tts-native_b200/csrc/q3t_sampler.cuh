@@ -38,11 +38,10 @@ struct TopKScratch {
     unsigned long long cand[kTopKCandidates];
     double weights[kTopKMost];
     double prefix[kTopKMost];
-    float value[kTopKMost];
     int index[kTopKMost];
     unsigned int hist[256];
     unsigned long long warp_best[32];
-    int bin, taken, counter, retained, token;
+    int counter, token;
 };
 
 // One draw from the `selections` largest of keys[0..V) (order keys; ties by lower index), 1 <= selections
@@ -70,55 +69,58 @@ __device__ __forceinline__ int sample_top_k_block(const unsigned int* keys, int 
     sync();
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) best = max(best, static_cast<unsigned int>(s.warp_best[w]));
-    int shift = 16;
+    // bin d lies at (d % 8) * 32 + d / 8: lane l then reads bins 8 l .. 8 l + 7 without bank conflicts
+    int shift = 16, last = -1, taken = 0;
     for (;; shift += 4) {
         for (int t = tid; t < V; t += THREADS) {
             const unsigned int d = (best - keys[t]) >> shift;
-            if (d < 256u) atomicAdd(&s.hist[d], 1u);
+            if (d < 256u) atomicAdd(&s.hist[(d & 7u) * 32u + (d >> 3)], 1u);
         }
         sync();
-        if (warp == 0) {
-            unsigned int mine[8];
-            unsigned int local = 0;
+        // every warp finds the bin of the `selections`-th key for itself
+        unsigned int mine[8];
+        unsigned int local = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            mine[j] = s.hist[32 * j + lane];
+            local += mine[j];
+        }
+        unsigned int incl = local;
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+            const unsigned int n = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += n;
+        }
+        const unsigned int ballot = __ballot_sync(0xffffffffu, static_cast<int>(incl) >= selections);
+        if (ballot != 0u) {            // with shift 28 every key is within 16 steps
+            const int owner = __ffs(ballot) - 1;
+            int c = static_cast<int>(incl - local);
+            int chosen = 7;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                mine[j] = s.hist[8 * lane + j];
-                local += mine[j];
-            }
-            unsigned int incl = local;
-#pragma unroll
-            for (int o = 1; o < kWarp; o <<= 1) {
-                const unsigned int n = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += n;
-            }
-            const unsigned int ballot = __ballot_sync(0xffffffffu, static_cast<int>(incl) >= selections);
-            if (ballot == 0u) {
-                if (lane == 0) s.bin = -1;
-            } else if (lane == __ffs(ballot) - 1) {
-                int c = static_cast<int>(incl - local);
-                int chosen = 7;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (c < selections) {
-                        c += static_cast<int>(mine[j]);
-                        chosen = j;
-                    }
+                if (c < selections) {
+                    c += static_cast<int>(mine[j]);
+                    chosen = j;
                 }
-                s.bin = 8 * lane + chosen;
-                s.taken = c;
             }
+            last = 8 * owner + __shfl_sync(0xffffffffu, chosen, owner);
+            taken = __shfl_sync(0xffffffffu, c, owner);
+            break;
         }
         sync();
-        if (s.bin >= 0) break;         // with shift 28 every key is within 16 steps
         for (int i = tid; i < 256; i += THREADS) s.hist[i] = 0u;
         sync();
     }
-    const int taken = s.taken;
+    const float maximum = order_value(best) / temperature;
+    auto place = [&](unsigned long long k, int rank) {
+        const float v = order_value(static_cast<unsigned int>(k >> 12));
+        s.index[rank] = 4095 - static_cast<int>(k & 0xfffull);
+        s.weights[rank] = exp(static_cast<double>(v / temperature - maximum));
+    };
     if (taken <= kTopKCandidates) {
-        const unsigned int last = static_cast<unsigned int>(s.bin);
         for (int t = tid; t < V; t += THREADS) {
             const unsigned int k = keys[t];
-            if (((best - k) >> shift) <= last) {
+            if (((best - k) >> shift) <= static_cast<unsigned int>(last)) {
                 const int p = atomicAdd(&s.counter, 1);
                 if (p < kTopKCandidates) s.cand[p] = (static_cast<unsigned long long>(k) << 12) | static_cast<unsigned long long>(4095 - t);
             }
@@ -129,22 +131,18 @@ __device__ __forceinline__ int sample_top_k_block(const unsigned int* keys, int 
             const int i = tid >> 2, part = tid & 3;
             const unsigned long long k = i < taken ? s.cand[i] : 0ull;
             int rank = 0;
+#pragma unroll 4
             for (int j = part; j < taken; j += 4) rank += s.cand[j] > k ? 1 : 0;
             rank += __shfl_xor_sync(0xffffffffu, rank, 1);
             rank += __shfl_xor_sync(0xffffffffu, rank, 2);
-            if (part == 0 && i < taken && rank < selections) {
-                s.value[rank] = order_value(static_cast<unsigned int>(k >> 12));
-                s.index[rank] = 4095 - static_cast<int>(k & 0xfffull);
-            }
+            if (part == 0 && i < taken && rank < selections) place(k, rank);
         } else {
             for (int i = tid; i < taken; i += THREADS) {
                 const unsigned long long k = s.cand[i];
                 int rank = 0;
+#pragma unroll 4
                 for (int j = 0; j < taken; ++j) rank += s.cand[j] > k ? 1 : 0;
-                if (rank < selections) {
-                    s.value[rank] = order_value(static_cast<unsigned int>(k >> 12));
-                    s.index[rank] = 4095 - static_cast<int>(k & 0xfffull);
-                }
+                if (rank < selections) place(k, rank);
             }
         }
     } else {
@@ -166,19 +164,12 @@ __device__ __forceinline__ int sample_top_k_block(const unsigned int* keys, int 
             sync();
             for (int w = 0; w < kWarps; ++w) top = s.warp_best[w] > top ? s.warp_best[w] : top;
             below = top;
-            if (tid == 0) {
-                s.value[r] = order_value(static_cast<unsigned int>(top >> 12));
-                s.index[r] = 4095 - static_cast<int>(top & 0xfffull);
-            }
+            if (tid == 0) place(top, r);
         }
     }
     sync();
-    const float maximum = s.value[0] / temperature;
-    for (int i = tid; i < selections; i += THREADS) {
-        s.weights[i] = exp(static_cast<double>(s.value[i] / temperature - maximum));
-    }
-    sync();
-    if (tid == 0) {
+    if (warp == 0) {
+    if (lane == 0) {
         // one thread, the reference's order of additions; eight loads at a time ahead of the chain
         double running = 0.0;
         int i = 0;
@@ -197,11 +188,11 @@ __device__ __forceinline__ int sample_top_k_block(const unsigned int* keys, int 
             s.prefix[i] = running;
         }
     }
-    sync();
+    __syncwarp();
     const double denominator = s.prefix[selections - 1];
-    for (int i = tid; i < selections; i += THREADS) s.weights[i] = s.weights[i] / denominator;
-    sync();
-    if (tid == 0) {
+    for (int i = lane; i < selections; i += kWarp) s.weights[i] = s.weights[i] / denominator;
+    __syncwarp();
+    if (lane == 0) {
         double cumulative = 0.0;
         int keep = selections;
         const double limit = static_cast<double>(top_p);
@@ -232,6 +223,7 @@ __device__ __forceinline__ int sample_top_k_block(const unsigned int* keys, int 
             }
         }
         s.token = s.index[first < keep ? first : keep - 1];
+    }
     }
     sync();
     return s.token;
