@@ -318,10 +318,17 @@ struct Chain {
         poll(q, v, flag);
         return v[0];
     }
+    // WRAPS: the phase is longer than the ring, so the slot's fill before this one may still be in flight for another
+    // warp, and its parity would pass for this one's.  A fill is asked for only once the one before it has been read.
+    template <bool WRAPS = false>
     __device__ __forceinline__ void wait_slot(uint32_t s) {
-        uint64_t* bar = &misc->full[s % L::Slots];
-        const uint32_t parity = (s / L::Slots) & 1u;
-        for (uint32_t polls = 0; !mbar_try_wait(bar, parity);) {
+        const uint32_t fill = s / L::Slots;
+        if (WRAPS) {
+            for (uint32_t polls = 0; *reinterpret_cast<volatile unsigned int*>(&misc->asked[s % L::Slots]) <= fill;) {
+                if ((++polls & 63u) == 0u && slow_check()) return;
+            }
+        }
+        for (uint32_t polls = 0; !mbar_try_wait(&misc->full[s % L::Slots], fill & 1u);) {
             if ((++polls & 63u) == 0u && slow_check()) return;
         }
     }
@@ -422,7 +429,7 @@ struct Chain {
 #pragma unroll
             for (int i = 0; i < G; ++i) {
                 const uint32_t at = off + (t0 + i) * kTile;
-                if (i == 0 || at % kSlot < kTile) wait_slot(seq + at / kSlot);
+                if (i == 0 || at % kSlot < kTile) wait_slot<(TILES * S::J > L::Slots)>(seq + at / kSlot);
                 w[i] = reinterpret_cast<const int4*>(smem + L::AtRing + (seq + at / kSlot) % L::Slots * kSlot + at % kSlot) + lane;
             }
             constexpr int kChains = G * NT <= 4 ? 2 : 1;       // accumulators per tile (integers: any order)

@@ -49,6 +49,7 @@ constexpr int kWStages = 6;            // int8 ring in shared memory
 constexpr int kXStages = 4;            // activation ring in shared memory (stage i pairs with A stage i)
 constexpr int kAStages = 4;            // dequantised A stages in TMEM
 constexpr int kWStageBytes = kTileN * kBK;          // 16 KB
+static_assert(kWStages % kGroups == 0 && kAStages % kGroups == 0, "a stage is always consumed by the same group");
 static_assert(kXStages == kAStages, "activation stage i and TMEM A stage i share their barriers");
 constexpr int kAStageCols = kBK / 2;   // 64 TMEM columns: two bf16 per 32-bit column
 constexpr int kAccCols = 64;           // accumulators sit in columns [0, 64), A stages follow
@@ -507,6 +508,39 @@ bool gemm_tc_supports(const GemvArgs& a) {
     return scratch_for_current_device() != nullptr;
 }
 
+namespace {
+int tile_rows(int rows) { return rows <= 16 ? 16 : (rows <= 32 ? 32 : 64); }
+// K-slices per tile = cluster size: as many as still let every cluster be resident at once (a second wave would
+// double the time); slices and row shares may be ragged
+int choose_splits(const TcScratch& scratch, const GemvArgs& a) {
+    const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
+    const int mt = tile_rows(a.rows), nk = a.in_features / kBK;
+    const int clusters = (gateup ? (a.out_features + 63) / 64 : (a.out_features + kTileN - 1) / kTileN) * ((a.rows + mt - 1) / mt);
+    const int (&resident)[9] = scratch.resident_clusters[mt == 16 ? 0 : (mt == 32 ? 1 : 2)][gateup ? 1 : 0];
+    static const int split_cap = [] {
+        const char* v = std::getenv("QWEN3_TTS_TC_MAX_SPLITS");
+        const int n = v != nullptr ? std::atoi(v) : 8;
+        return n < 1 ? 1 : (n > 8 ? 8 : n);
+    }();
+    int splits = 1;
+    for (int s = 2; s <= split_cap && s <= nk; ++s) {
+        if (clusters <= resident[s]) splits = s;
+    }
+    return splits;
+}
+}  // namespace
+
+float gemm_tc_estimate_us(const GemvArgs& a) {
+    TcScratch* scratch = scratch_for_current_device();
+    if (scratch == nullptr || a.in_features % kBK != 0) return 1.0e9f;
+    const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
+    const int mt = tile_rows(a.rows), splits = choose_splits(*scratch, a);
+    const int ctas = (gateup ? (a.out_features + 63) / 64 : (a.out_features + kTileN - 1) / kTileN) * ((a.rows + mt - 1) / mt) * splits;
+    const int waves = (ctas + scratch->sms - 1) / scratch->sms;
+    const int steps = (a.in_features / kBK + splits - 1) / splits;
+    return waves * ((splits > 1 ? 6.4f : 4.0f) + 0.5f * steps);
+}
+
 cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
     TcScratch* scratch = scratch_for_current_device();
     if (scratch == nullptr || !gemm_tc_supports(a) || a.out_features < 1 || a.w == nullptr
@@ -531,27 +565,14 @@ cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
         if (e != cudaSuccess) return e;
         x = normalized;
     }
-    const int mt = a.rows <= 16 ? 16 : (a.rows <= 32 ? 32 : 64);
+    const int mt = tile_rows(a.rows);
     TcParams p;
     p.scales = a.scales; p.y = a.y; p.y32 = a.y32; p.bias = a.bias; p.resid = a.resid;
     p.out_features = N; p.rows = a.rows; p.epilogue = a.epilogue;
     p.tiles = gateup ? (N + 63) / 64 : (N + kTileN - 1) / kTileN;
     p.residual_settled = a.residual_settled ? 1 : 0;
     const int nk = K / kBK;
-    const int row_blocks = (a.rows + mt - 1) / mt;
-    // K-slices per tile = cluster size: as many as still let every cluster be resident at once (a
-    // second wave would double the time); slices and row shares may be ragged
-    const int (&resident)[9] = scratch->resident_clusters[mt == 16 ? 0 : (mt == 32 ? 1 : 2)][gateup ? 1 : 0];
-    static const int split_cap = [] {
-        const char* v = std::getenv("QWEN3_TTS_TC_MAX_SPLITS");
-        const int n = v != nullptr ? std::atoi(v) : 8;
-        return n < 1 ? 1 : (n > 8 ? 8 : n);
-    }();
-    int splits = 1;
-    for (int s = 2; s <= split_cap && s <= nk; ++s) {
-        if (p.tiles * row_blocks <= resident[s]) splits = s;
-    }
-    p.splits = splits;
+    p.splits = choose_splits(*scratch, a);
     p.chunks = nk;
 
     alignas(64) CUtensorMap wm, xm;

@@ -13,10 +13,11 @@
 // that a thread finds both values of a channel in its own TMEM lane; with NT = 1 a tile holds 64 of
 // each and the up half crosses over through shared memory.
 //
-// Warp roles as in gemm_int8_tc.cu: 0 weight copies, 1 MMA issue, 2 activation copies, 3 TMEM; 4..7 and
-// 8..11 dequantise (a thread turns 128 int8 of its channel into bf16 and stores them to tensor memory as
-// the A operand; about 400 cycles a tile of 16 KB, two of them against the 1024 cycles of a step's MMAs),
-// then read the accumulators.  Every wait is bounded.
+// Warp roles as in gemm_int8_tc.cu: 0 weight copies, 1 MMA issue, 2 activation copies, 3 TMEM; 4..19 in four
+// groups dequantise (a thread turns 128 int8 of its channel into bf16 and stores them to tensor memory as the
+// A operand), then read the accumulators.  Every wait is bounded.
+// Measured (B200, 1500 rows): gate/up 2048 -> 2 x 6144 74 us, q/k/v 37 us, o 21 us, down 47 us, 0.6-1.0 PFLOP/s; a step
+// of 64 KB takes about 1350 cycles with or without its MMAs, the rate at which an SM takes data in.
 
 #include "q3t_kernels.cuh"
 #include "q3t_tcgen05.cuh"
@@ -26,14 +27,18 @@ namespace {
 
 using namespace tc;
 
-constexpr int kGroups = 2;
+constexpr int kGroups = 4;
 constexpr int kThreads = 128 + 128 * kGroups;
 constexpr int kTileN = 128;                   // channels per tile
 constexpr int kTileM = 128;                   // activation rows per CTA
 constexpr int kBK = 128;                      // K elements per step
-constexpr int kWStages = 5;
-constexpr int kXStages = 4;
+constexpr int kSms = 148;
+constexpr int kWStages = 8;
+constexpr int kXStages = 3;
 constexpr int kAStages = 4;
+// A slot's fills must be consumed by one group: copies may land out of order, and a group that waits for a fill two
+// phases ahead of the one in flight would read its parity as already complete.
+static_assert(kWStages % kGroups == 0 && kAStages % kGroups == 0, "one group per stage");
 constexpr int kWStageBytes = kTileN * kBK;            // 16 KB
 constexpr int kXAtomBytes = kTileM * 128;             // 128 rows x 64 bf16
 constexpr int kXStageBytes = 2 * kXAtomBytes;         // 32 KB
@@ -231,29 +236,39 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
                 mbar_arrive(&empty_w[s]);
             }
         }
+        // Group g finishes the activation rows [32 g, 32 g + 32) of the CTA; a thread has one channel of each tile.  What a
+        // residual epilogue adds to is requested a tile's 32 rows at a time, the first before the last MMAs are waited for.
+        constexpr int kShare = kTileM / kGroups;
+        const int first_row = row_base + group * kShare;
+        const int rows_here = min(kShare, p.rows - first_row);
+        const bool up_lane = GATEUP && NT == 1 && t >= 64;
+        const bool adds = !GATEUP && (p.epilogue == EPI_ADD || p.epilogue == EPI_BIAS_ADD);
+        bf16* out = (p.epilogue == EPI_BIAS_ADD ? p.resid : p.y) + (size_t)first_row * N;
+        bf16 base[kShare];
+        auto fetch_bases = [&](int channel) {
+#pragma unroll
+            for (int j = 0; j < kShare; ++j) {
+                base[j] = channel < N && j < rows_here ? out[(size_t)j * N + channel] : __ushort_as_bfloat16(0);
+            }
+        };
+        pdl_wait();
+        if (adds) fetch_bases(tile * kChannels + t);
         if (ok) ok = guard.wait(acc_done, 0);
         if (!ok) *abort_flag = 1;
-        pdl_wait();
         readers_barrier();       // everybody agrees on whether the tile is complete
-        if (*abort_flag == 0) {
+        if (*abort_flag == 0 && (rows_here > 0 || (GATEUP && NT == 1))) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // Group g finishes the activation rows [64 g, 64 g + 64) of the CTA.
-            const int first_row = row_base + group * 64;
-            const bool up_lane = GATEUP && NT == 1 && t >= 64;
-            float* exchange = reinterpret_cast<float*>(smem) + (size_t)group * 64 * 64;   // the rings are idle now
+            float* exchange = reinterpret_cast<float*>(smem) + (size_t)group * kShare * 64;   // the rings are idle now
             if (GATEUP && NT == 1) {
                 if (up_lane) {
+                    float v[kShare];
+                    tmem_load_row<kShare>(lane_base + group * kShare, v);
 #pragma unroll
-                    for (int c0 = 0; c0 < 64; c0 += 16) {
-                        float v[16];
-                        tmem_load_row<16>(lane_base + group * 64 + c0, v);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) exchange[(c0 + j) * 64 + t - 64] = v[j];
-                    }
+                    for (int j = 0; j < kShare; ++j) exchange[j * 64 + t - 64] = v[j];
                 }
                 readers_barrier();
             }
-            if (!up_lane) {
+            if (!up_lane && rows_here > 0) {
 #pragma unroll 1
                 for (int u = 0; u < (GATEUP ? 1 : NT); ++u) {
                     const int channel = tile * kChannels + u * kTileN + t;
@@ -263,22 +278,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
                         if (GATEUP) scale_up = p.scales[N + channel];
                         if (!GATEUP && p.bias != nullptr) bias = bf2f(p.bias[channel]);
                     }
-                    const bool adds = !GATEUP && (p.epilogue == EPI_ADD || p.epilogue == EPI_BIAS_ADD);
-                    bf16* dst = (p.epilogue == EPI_BIAS_ADD ? p.resid : p.y) + channel;
-#pragma unroll 1
-                    for (int c0 = 0; c0 < 64; c0 += 16) {
-                        const int row0 = first_row + c0;
-                        if (row0 >= p.rows) break;           // the same for the whole warp
-                        float base[16];
+                    if (adds && u > 0) fetch_bases(channel);
+                    bf16* dst = out + channel;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            base[j] = adds && channel < N && row0 + j < p.rows ? bf2f(dst[(size_t)(row0 + j) * N]) : 0.0f;
-                        }
+                    for (int c0 = 0; c0 < kShare; c0 += 16) {
                         float v[16], w[16];
-                        tmem_load_row<16>(lane_base + u * kTileM + group * 64 + c0, v);
+                        tmem_load_row<16>(lane_base + u * kTileM + group * kShare + c0, v);
                         if (GATEUP) {
                             if (NT == 2) {
-                                tmem_load_row<16>(lane_base + kTileM + group * 64 + c0, w);
+                                tmem_load_row<16>(lane_base + kTileM + group * kShare + c0, w);
                             } else {
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) w[j] = exchange[(c0 + j) * 64 + t];
@@ -291,15 +299,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
                                 const float gate = v[j] * scale;
                                 val = __fdividef(gate, 1.0f + __expf(-gate)) * (w[j] * scale_up);
                             } else if (p.epilogue == EPI_ADD) {
-                                val = fmaf(v[j], scale, base[j]);
+                                val = fmaf(v[j], scale, bf2f(base[c0 + j]));
                             } else if (p.epilogue == EPI_PLAIN) {
                                 val = v[j] * scale;
                             } else {
                                 val = rbf(v[j] * scale) + bias;
                                 if (p.epilogue == EPI_BIAS_SILU) val = __fdividef(val, 1.0f + __expf(-val));
-                                else if (p.epilogue == EPI_BIAS_ADD) val = base[j] + rbf(val);
+                                else if (p.epilogue == EPI_BIAS_ADD) val = bf2f(base[c0 + j]) + rbf(val);
                             }
-                            if (channel < N && row0 + j < p.rows) dst[(size_t)(row0 + j) * N] = f2bf(val);
+                            if (channel < N && c0 + j < rows_here) dst[(size_t)(c0 + j) * N] = f2bf(val);
                         }
                     }
                 }
@@ -341,7 +349,7 @@ cudaError_t configure_wide_kernels() {
     return e;
 }
 
-// `channel_tiles`: 1 or 2 (see the top of the file), 0 chooses
+// `channel_tiles`: 1 or 2 (see the top of the file)
 cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int channel_tiles) {
     const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
     if (a.rows < 1 || a.rows > kMaxPromptRows || a.out_features < 1 || a.in_features % kBK != 0 || a.in_features < kBK
@@ -358,12 +366,7 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
     p.row_blocks = (a.rows + kTileM - 1) / kTileM;
     p.steps = a.in_features / kBK;
     const int per_single = gateup ? 64 : kTileN;                // output channels of a CTA with one tile
-    int nt = channel_tiles;
-    if (nt != 1 && nt != 2) {
-        // two tiles per CTA once even they come in more than one wave
-        const int ctas = (a.out_features + 2 * per_single - 1) / (2 * per_single) * p.row_blocks;
-        nt = ctas >= 148 ? 2 : 1;
-    }
+    const int nt = channel_tiles == 2 ? 2 : 1;
     const int tiles = (a.out_features + nt * per_single - 1) / (nt * per_single);
     alignas(64) CUtensorMap wm, xm;
     const uint64_t w_rows = gateup ? 2ull * a.out_features : (uint64_t)a.out_features;
@@ -378,11 +381,12 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
     return nt == 2 ? launch_variant<2, false>(wm, xm, p, tiles, stream) : launch_variant<1, false>(wm, xm, p, tiles, stream);
 }
 
-// Which kernel takes a projection of a prompt pass.  Up to kBlockedRows rows the 64-row kernel of
-// gemm_int8_tc.cu, its row blocks side by side and K split where that still fits one wave; above it
-// this file's.
+// Which kernel takes a projection of a prompt pass: the one with the shortest estimate.  A wave of CTAs of this
+// file's kernel costs its steps (0.50 us each with one channel tile, 0.82 us with two: what an SM takes in) and 4
+// to 6 us of start and epilogue; the 64-row kernel of gemm_int8_tc.cu, its row blocks side by side and K split where
+// that fits one wave, is estimated there.  Within 20 % of the measured times of the talker's four shapes from 65 to
+// 2048 rows; the crossovers lie around 130 rows (gate/up), 200 (q/k/v), 300 (o, down).
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
-    constexpr int kBlockedRows = 256;
     GemvArgs a = args;
     if (a.norm_w != nullptr) {
         if (a.norm_out == nullptr) return cudaErrorInvalidValue;
@@ -392,7 +396,15 @@ cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
         a.norm_w = nullptr;
         a.norm_out = nullptr;
     }
-    return a.rows <= kBlockedRows ? launch_int8_gemm_tc(a, stream) : launch_int8_gemm_wide(a, stream);
+    const int per_single = a.epilogue == EPI_GATE_UP_SILU ? 64 : kTileN;
+    const int row_blocks = (a.rows + kTileM - 1) / kTileM, steps = a.in_features / kBK;
+    auto waves = [&](int tiles) {
+        return ((a.out_features + tiles * per_single - 1) / (tiles * per_single) * row_blocks + kSms - 1) / kSms;
+    };
+    const float one = waves(1) * (a.epilogue == EPI_GATE_UP_SILU ? 6.0f + 0.50f * steps : 4.3f + 0.50f * steps);
+    const float two = waves(2) * (5.5f + 0.82f * steps);
+    if (gemm_tc_estimate_us(a) <= (one < two ? one : two)) return launch_int8_gemm_tc(a, stream);
+    return launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
 }
 
 unsigned int gemm_wide_error_count() {

@@ -92,8 +92,9 @@ void set_tc_min_rows(int rows);          // 65 or more: never use the tensor-cor
 int tc_min_rows();
 unsigned int gemm_tc_error_count();
 // more than kMaxRows rows (prompt passes), K % 128 == 0, no norm prologue, no fp32 output
-// (gemm_int8_wide.cu); channel_tiles 1 or 2, 0 chooses
-cudaError_t launch_int8_gemm_wide(const GemvArgs& args, cudaStream_t stream, int channel_tiles = 0);
+// (gemm_int8_wide.cu); channel_tiles 1 or 2
+cudaError_t launch_int8_gemm_wide(const GemvArgs& args, cudaStream_t stream, int channel_tiles);
+float gemm_tc_estimate_us(const GemvArgs& args);     // what launch_int8_gemm_tc would take, for that choice
 cudaError_t configure_wide_kernels();
 // projections of a prompt pass of more than kMaxRows rows (needs norm_out when norm_w is given)
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream);
