@@ -259,3 +259,33 @@ def test_operator_benchmark_case_runs(q3t):
     us, kv_bytes = q3t.native.benchmark_decode_attention(0, rows=4, min_length=10, max_length=300, seed=5, iterations=2)
     assert us > 0.0
     assert kv_bytes % (1024 * 2 * 2) == 0 and 4 * 10 <= kv_bytes // 4096 <= 4 * 300      # tokens x 1024 x bf16 x (K, V)
+
+
+@pytest.mark.parametrize("rows", [1, 9, 130])
+def test_walk_edges(orc, ops, rows):
+    """The walk over (row, KV head, chunk) items at the edges of pages, chunks and warps' shares, over caches whose unused
+    places hold NaN: a new token that opens a page or a chunk, one that fills it, rows of one chunk beside rows of many,
+    more rows than one launch takes.  Fused over pages equals step by step over contiguous caches to the bit; those
+    are compared with the oracle like every other shape."""
+    qh, kvh, hd, cap = 16, 8, 128, 528
+    edges = [64, 0, 15, 16, 63, 65, 127, 128, 527, 512, 48]
+    positions = np.array([edges[(7 * r + rows) % len(edges)] if rows > 1 else 64 for r in range(rows)], dtype=np.int32)
+    rng = np.random.default_rng(rows)
+    qw, kvw = qh * hd, kvh * hd
+    q, k, v, pos = make(orc, 21, rows, qh, kvh, hd, cap, positions)
+    qkv = bf(orc, rng.standard_normal((rows, qw + 2 * kvw)))
+    ones = bf(orc, np.ones(hd))
+    q2 = ops.rope_rows_at(ops.head_rms_norm_rows(np.ascontiguousarray(qkv[:, :qw]), ones, rows, qh, hd), rows, qh, hd, pos)
+    k2 = ops.rope_rows_at(ops.head_rms_norm_rows(np.ascontiguousarray(qkv[:, qw:qw + kvw]), ones, rows, kvh, hd), rows, kvh, hd, pos)
+    kc = ops.kv_scatter_rows(k2.reshape(rows, kvw), k, pos)
+    vc = ops.kv_scatter_rows(np.ascontiguousarray(qkv[:, qw + kvw:]), v, pos)
+    plain = ops.attention_ex(q2.reshape(rows, qw), pos, qh, kvh, hd, k=kc, v=vc, want_f32=True)
+    want, want32 = orc.attention(q2.reshape(rows, qw), kc, vc, pos, qh, kvh, hd, fast=True, want_f32=True)
+    check(orc, plain["out"], plain["f32"], want, want32, hd)
+    for r in range(rows):
+        k[r, pos[r]:] = 0x7fc0
+        v[r, pos[r]:] = 0x7fc0
+    slabs, table = paged_copy(k, v, kvw, rng, per_slab=64)
+    fused = ops.attention_ex(qkv, pos, qh, kvh, hd, pages=slabs, page_table=table, slab_shift=6, q_norm_w=ones, k_norm_w=ones,
+                             fused=True, q_stride=qw + 2 * kvw, new_stride=qw + 2 * kvw)
+    assert np.array_equal(fused["out"], plain["out"])
