@@ -15,6 +15,10 @@ constexpr int kThreads = 256;
 __global__ void __launch_bounds__(kThreads)
 rms_norm_rows_kernel(const bf16* __restrict__ input, const bf16* __restrict__ weight,
                      bf16* __restrict__ output, int width, float eps) {
+    // First of all: the GEMM behind a norm then brings its barriers, its tensor memory and its first weight tiles up while
+    // the norm still waits (a frame of 23 sessions 4.76 -> 4.43 ms, of 64 6.86 -> 6.58; 150 prompt positions
+    // 2.51 -> 2.43 ms).  Attention, sampler and input kernels were no faster for it.
+    pdl_trigger();
     // the norm weights are constants: requested before the wait for the rows' producer
     constexpr int kPre = 8;                              // widths up to 2048 stay in registers
     const bool in_registers = width <= kPre * kThreads;
@@ -27,7 +31,6 @@ rms_norm_rows_kernel(const bf16* __restrict__ input, const bf16* __restrict__ we
         }
     }
     pdl_wait();
-    pdl_trigger();
     __shared__ float partial[kThreads];
     const bf16* xr = input + (size_t)blockIdx.x * width;
     bf16* yr = output + (size_t)blockIdx.x * width;

@@ -178,9 +178,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     const uint32_t tmem_base = *tmem_slot;
     // The weight copies (warp 0) start at once: weights never depend on the kernel before this
     // one.  Everyone else first waits for that kernel to complete (activations, residual), and
-    // only then is the kernel after this one let in: every kernel of the library signals its
-    // dependents after its own wait, so that a kernel may read, ahead of its wait, whatever was
-    // written two or more launches upstream.
+    // only then is the kernel after this one let in: every kernel of the library but the norm
+    // signals its dependents after its own wait, so that a kernel may read, ahead of its wait, whatever
+    // was written before the last such kernel upstream.
     // The dequantisers (warps 4..) touch only weights and tensor memory until the K-slice sum, so
     // they too run ahead and wait there.
     if (warp >= 1 && warp <= 3) {

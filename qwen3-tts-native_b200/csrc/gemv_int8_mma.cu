@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, NTMAX == 1 ? 2 : 1) gemv_mma_kernel(
 
     // Everything above touched only constants of the model.
     pdl_wait();
-    pdl_trigger();   // after the wait, as everywhere in the library.  (Triggering at kernel start was
+    pdl_trigger();   // after the wait, as everywhere but in the norm kernel.  (Triggering at kernel start was
                      // measured: the successor's bulk copies then collide with this kernel's fetch of
                      // its activations, which costs more than the earlier start of the copies gains.)
 
