@@ -73,22 +73,23 @@ DeviceBuffer::DeviceBuffer(size_t bytes) : bytes_(bytes) {
     }
     check_cuda(e, "cudaMalloc");
 }
-DeviceBuffer::DeviceBuffer(DeviceBuffer&& o) noexcept : ptr_(o.ptr_), bytes_(o.bytes_) {
+DeviceBuffer::DeviceBuffer(DeviceBuffer&& o) noexcept : ptr_(o.ptr_), bytes_(o.bytes_), owned_(o.owned_) {
     o.ptr_ = nullptr;
     o.bytes_ = 0;
 }
 DeviceBuffer& DeviceBuffer::operator=(DeviceBuffer&& o) noexcept {
     if (this != &o) {
-        if (ptr_ != nullptr) cudaFree(ptr_);
+        if (ptr_ != nullptr && owned_) cudaFree(ptr_);
         ptr_ = o.ptr_;
         bytes_ = o.bytes_;
+        owned_ = o.owned_;
         o.ptr_ = nullptr;
         o.bytes_ = 0;
     }
     return *this;
 }
 DeviceBuffer::~DeviceBuffer() {
-    if (ptr_ != nullptr) cudaFree(ptr_);
+    if (ptr_ != nullptr && owned_) cudaFree(ptr_);
 }
 
 // ------------------------------------------------------------------ KvPool
@@ -152,31 +153,32 @@ Workspace::Workspace(int capacity_, int device_, int rows) : capacity(capacity_)
     check_cuda(cudaSetDevice(device), "cudaSetDevice(workspace)");
     const size_t e = sizeof(bf16);
     size_t c = std::max(capacity, rows);
-    hidden = DeviceBuffer(c * 2048 * e);
-    qkv = DeviceBuffer(c * 4096 * e);
-    attention = DeviceBuffer(c * 2048 * e);
-    gate = DeviceBuffer(c * 6144 * e);
-    logits = DeviceBuffer(c * kTalkerVocab * e);
-    x_in = DeviceBuffer(c * 2048 * e);
-    projection = DeviceBuffer(c * 2048 * e);
-    normalized = DeviceBuffer(c * 2048 * e);
-    prompt_positions = DeviceBuffer(c * sizeof(int));
+    const size_t one = capacity;
+    // one allocation: a session's workspace is made when the session is, and fourteen of them were half of that
+    const std::pair<DeviceBuffer*, size_t> parts[] = {
+        {&table, sizeof(FrameTable)}, {&counters, one * 16 * sizeof(unsigned int)},
+        {&hidden, c * 2048 * e}, {&qkv, c * 4096 * e}, {&attention, c * 2048 * e}, {&gate, c * 6144 * e},
+        {&logits, c * kTalkerVocab * e}, {&x_in, c * 2048 * e}, {&projection, c * 2048 * e}, {&normalized, c * 2048 * e},
+        {&prompt_positions, c * sizeof(int)}, {&talker_pages, one * kMaxPagesPerRow * sizeof(int)},
+        {&predictor_pages, one * sizeof(int)}, {&predictor_positions, (size_t)kPredictorSequence * kMaxRows * sizeof(int)}};
+    size_t total = 0;
+    for (const auto& part : parts) total += align_up(part.second, 1024);
+    arena = DeviceBuffer(total);
+    size_t at = 0;
+    for (const auto& part : parts) {
+        *part.first = DeviceBuffer(arena, at, part.second);
+        at += align_up(part.second, 1024);
+    }
     c = capacity;
-    table = DeviceBuffer(sizeof(FrameTable));
-    talker_pages = DeviceBuffer(c * kMaxPagesPerRow * sizeof(int));
-    predictor_pages = DeviceBuffer(c * sizeof(int));
-    predictor_positions = DeviceBuffer((size_t)kPredictorSequence * kMaxRows * sizeof(int));
-    counters = DeviceBuffer(c * 16 * sizeof(unsigned int));
     try {
         check_cuda(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
-        check_cuda(cudaHostAlloc(reinterpret_cast<void**>(&host_table), sizeof(FrameTable),
-                                 cudaHostAllocDefault), "cudaHostAlloc(frame table)");
+        const size_t host_bytes = align_up(sizeof(FrameTable), 1024);
+        check_cuda(cudaHostAlloc(reinterpret_cast<void**>(&host_table), host_bytes + c * (kMaxPagesPerRow + 1) * sizeof(int),
+                                 cudaHostAllocDefault), "cudaHostAlloc(frame table, page tables)");
         std::memset(host_table, 0, sizeof(FrameTable));
-        check_cuda(cudaHostAlloc(reinterpret_cast<void**>(&host_pages),
-                                 c * (kMaxPagesPerRow + 1) * sizeof(int), cudaHostAllocDefault),
-                   "cudaHostAlloc(page tables)");
-        check_cuda(cudaMemset(table.as<void>(), 0, sizeof(FrameTable)), "cudaMemset(frame table)");
-        check_cuda(cudaMemset(counters.as<void>(), 0, counters.bytes()), "cudaMemset(counters)");
+        host_pages = reinterpret_cast<int*>(reinterpret_cast<char*>(host_table) + host_bytes);
+        check_cuda(cudaMemset(table.as<void>(), 0, align_up(table.bytes(), 1024) + counters.bytes()),
+                   "cudaMemset(frame table, counters)");
         std::vector<int> positions((size_t)kPredictorSequence * kMaxRows);
         for (int p = 0; p < kPredictorSequence; ++p)
             for (int r = 0; r < kMaxRows; ++r) positions[(size_t)p * kMaxRows + r] = p;
@@ -209,8 +211,7 @@ void Workspace::release() noexcept {
         if (*ev != nullptr) cudaEventDestroy(*ev);
         *ev = nullptr;
     }
-    if (host_pages != nullptr) cudaFreeHost(host_pages);
-    host_pages = nullptr;
+    host_pages = nullptr;            // behind the host table
     if (host_table != nullptr) cudaFreeHost(host_table);
     host_table = nullptr;
     if (stream != nullptr) cudaStreamDestroy(stream);
@@ -1055,10 +1056,9 @@ Session::Session(std::shared_ptr<Model> model, int max_sequence_length, uint64_t
         d_rng_ = reinterpret_cast<unsigned long long*>(base + off_rng);
         d_last_hidden_ = reinterpret_cast<bf16*>(base + off_hidden);
         d_history_ = reinterpret_cast<int*>(base + off_history);
-        check_cuda(cudaHostAlloc(reinterpret_cast<void**>(&h_token_), sizeof(int), cudaHostAllocMapped),
-                   "cudaHostAlloc(sampled token)");
-        check_cuda(cudaHostAlloc(reinterpret_cast<void**>(&h_codes_), kCodebooks * sizeof(unsigned short),
-                                 cudaHostAllocMapped), "cudaHostAlloc(frame codes)");
+        check_cuda(cudaHostAlloc(reinterpret_cast<void**>(&h_token_), 128 + kCodebooks * sizeof(unsigned short),
+                                 cudaHostAllocMapped), "cudaHostAlloc(sampled token, frame codes)");
+        h_codes_ = reinterpret_cast<unsigned short*>(reinterpret_cast<char*>(h_token_) + 128);
         *h_token_ = -1;
         {
             std::lock_guard<std::mutex> lock(model_->mutex);
@@ -1085,8 +1085,7 @@ void Session::release() noexcept {
         if (predictor_page_ >= 0) model_->predictor_pool->release(predictor_page_);
         predictor_page_ = -1;
     }
-    if (h_codes_ != nullptr) cudaFreeHost(h_codes_);
-    h_codes_ = nullptr;
+    h_codes_ = nullptr;              // behind the token
     if (h_token_ != nullptr) cudaFreeHost(h_token_);
     h_token_ = nullptr;
     if (semantic_ready_ != nullptr) cudaEventDestroy(semantic_ready_);

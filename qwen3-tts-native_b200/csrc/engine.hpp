@@ -53,6 +53,9 @@ class DeviceBuffer {
 public:
     DeviceBuffer() = default;
     explicit DeviceBuffer(size_t bytes);
+    // a part of another buffer, which has to outlive it
+    DeviceBuffer(const DeviceBuffer& whole, size_t offset, size_t bytes)
+        : ptr_(static_cast<char*>(whole.ptr_) + offset), bytes_(bytes), owned_(false) {}
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
     DeviceBuffer(DeviceBuffer&& o) noexcept;
@@ -63,6 +66,7 @@ public:
 private:
     void* ptr_ = nullptr;
     size_t bytes_ = 0;
+    bool owned_ = true;
 };
 
 struct ModelDims {
@@ -128,6 +132,7 @@ struct Workspace {
     int capacity;
     int device;
     cudaStream_t stream = nullptr;
+    DeviceBuffer arena;              // what the buffers below but `scratch` lie in: one allocation
     DeviceBuffer hidden, qkv, attention, gate, logits, x_in, projection, normalized;
     DeviceBuffer table;              // FrameTable
     FrameTable* host_table = nullptr;   // pinned mirror
