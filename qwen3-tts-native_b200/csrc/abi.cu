@@ -902,8 +902,9 @@ static int32_t attention_common(AttentionArgs& a, int max_sequence_length, void*
         const size_t cb = counters_bytes(a.rows, a.kv_heads);
         a.counters = static_cast<unsigned int*>(scratch);
         a.scratch = reinterpret_cast<float*>(static_cast<char*>(scratch) + cb);
-        const cudaError_t e = cudaMemsetAsync(scratch, 0, cb, stream);
+        const cudaError_t e = launch_zero_counters(a.counters, a.rows * a.kv_heads, stream);
         if (e != cudaSuccess) return static_cast<int32_t>(e);
+        a.inputs_settled = 2;
     }
     return static_cast<int32_t>(launch_attention(a, stream));
 }

@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(kAttnThreads, kWalkCtas) decode_attention_walk
     const int kn_stride = a.kv_new_stride > 0 ? a.kv_new_stride : kvw;
     const bool fused = a.fused != 0;
     const bool appends = fused && a.append_mode == 0;
-    const bool settled = appends && a.inputs_settled != 0;
+    const bool settled = (appends && a.inputs_settled != 0) || a.inputs_settled == 2;
     if (!settled) {
         pdl_wait();
         pdl_trigger();
@@ -1462,6 +1462,20 @@ cudaError_t launch_build_rope_table(uint32_t* table, int positions, int head_dim
     const int total = positions * (head_dim / 2);
     rope_table_kernel<<<(total + 255) / 256, 256, 0, stream>>>(table, positions, head_dim, theta);
     return cudaGetLastError();
+}
+
+namespace {
+__global__ void zero_counters_kernel(unsigned int* counters, int count) {
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) counters[i] = 0u;
+}
+}  // namespace
+
+cudaError_t launch_zero_counters(unsigned int* counters, int count, cudaStream_t stream) {
+    if (counters == nullptr || count < 1) return cudaErrorInvalidValue;
+    return launch_pdl(zero_counters_kernel, dim3((unsigned)((count + 255) / 256)), dim3(256), 0, stream, counters, count);
 }
 
 size_t attention_scratch_floats(int rows, int q_heads, int head_dim, int max_splits) {

@@ -168,6 +168,7 @@ struct AttentionArgs {
     // than this step's token were written before the last launch upstream that is not a norm, so the kernel
     // may fetch them ahead of its dependency wait (only q / k_new / v_new come from the launch directly
     // before).  Set by callers that build the whole launch sequence; 0 is always correct.
+    // 2, for any step: everything but the counters was (launch_zero_counters() directly before).
     int inputs_settled = 0;
     int units_per_cta = 0;              // splits one CTA walks (0: chosen from the grid size); no effect on results
     float eps = kRmsEps;
@@ -177,6 +178,9 @@ struct AttentionArgs {
 constexpr int kAttnChunk = 64;          // tokens per split
 size_t attention_scratch_floats(int rows, int q_heads, int head_dim, int max_splits);
 cudaError_t launch_decode_attention(const AttentionArgs& args, cudaStream_t stream);
+// Clears the tickets of a caller's scratch.  A launch of its own rather than a memset: the attention behind it is up, and
+// its first cache reads are under way, by the time it ends.
+cudaError_t launch_zero_counters(unsigned int* counters, int count, cudaStream_t stream);
 // Layout of a caller's scratch buffer for the split-KV kernel, shared by every entry point that
 // carves one up: ticket counters first (rounded to 256 bytes), the chunk partials behind them.
 inline size_t attention_counters_bytes(int rows, int kv_heads) {
