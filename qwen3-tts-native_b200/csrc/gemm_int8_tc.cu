@@ -18,8 +18,8 @@
 //                                   and the same epilogues as the SIMT path
 // K is split across the CTAs of a thread-block cluster (up to 8) so that every SM streams
 // weights; each CTA pushes the rows of its slice into the shared memory of the CTA that owns
-// them (distributed shared memory) and, after one cluster barrier, sums the rows it owns over
-// all slices in slice order (deterministic).
+// them (asynchronous stores to distributed shared memory, counted on a barrier there), which sums the
+// rows it owns over all slices in slice order (deterministic).
 //
 // The reference has no counterpart: its int8 path stops at 8 rows of SIMT FMAs
 // (int8_gemv.cu:329) and its larger row counts go through cuBLAS bf16 GEMMs.
@@ -54,7 +54,7 @@ static_assert(kXStages == kAStages, "activation stage i and TMEM A stage i share
 constexpr int kAStageCols = kBK / 2;   // 64 TMEM columns: two bf16 per 32-bit column
 constexpr int kAccCols = 64;           // accumulators sit in columns [0, 64), A stages follow
 constexpr uint32_t kTmemCols = 512;    // 64 + 4 * 64 rounded up to a power of two
-constexpr int kRedBytes = 36 * 1024;   // K-slice exchange: up to 8 slices x ceil(64 / slices) rows x 128 fp32
+constexpr int kRedBytes = 44 * 1024;   // K-slice exchange: up to 8 slices x ceil(64 / slices) rows, in fours, x 128 fp32
 constexpr unsigned long long kBudgetNs = 2000000000ull;   // 2 s for the whole kernel
 
 __device__ unsigned int g_tc_errors = 0;
@@ -117,7 +117,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     uint64_t* full_a = empty_x + kXStages;
     uint64_t* empty_a = full_a + kAStages;
     uint64_t* acc_done = empty_a + kAStages;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+    uint64_t* red_full = acc_done + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(red_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x;
@@ -131,7 +132,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     const int nk = p.chunks * (split + 1) / p.splits - step_first;
     const int k_first = step_first * kBK;
     const int N = p.out_features;
-    const int rows_share = (MT + p.splits - 1) / p.splits;      // rows a CTA owns in the K-slice sum
+    // Rows a CTA owns in the K-slice sum, in groups of four; the exchange buffer is [slice][group][channel][4].
+    const int share_groups = ((MT + p.splits - 1) / p.splits + 3) / 4;
+    const int row0 = split * share_groups * 4;
+    const int my_rows = max(0, min(share_groups * 4, rows - row0));
     const int row_a = GATEUP ? tile * 64 : tile * kTileN;          // first W row of the tile
     const int row_b = N + tile * 64;                               // GATEUP: first row of the "up" half
 
@@ -163,9 +167,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             mbar_init(&empty_a[s], 1);
         }
         mbar_init(acc_done, 1);
+        mbar_init(red_full, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // the other slices' parts of the rows owned here, counted in bytes (none: an arrival that completes at once)
+        mbar_expect_tx(red_full, (uint32_t)((p.splits - 1) * ((my_rows + 3) / 4) * kTileN * 16));
     }
     if (warp == 3) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -176,6 +183,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    // a peer's barriers have to be set up before anything is sent to it: waited for just before that
+    cluster_arrive();
     // The weight copies (warp 0) start at once: weights never depend on the kernel before this
     // one.  Everyone else first waits for that kernel to complete (activations, residual), and
     // only then is the kernel after this one let in: every kernel of the library but the norm
@@ -291,97 +300,105 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         if (!ok) *abort_flag = 1;
         // all accumulator readers meet here, so that they agree on whether the tile is complete
         dequant_barrier();
-        if (*abort_flag == 0) {
+        if (__all_sync(0xffffffffu, *abort_flag == 0)) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // each group takes half of the accumulator columns (= activation rows); every row of
             // this K-slice goes to the shared memory of the CTA that owns the row
             constexpr int kCols = MT / kGroups;
             float v[kCols];
             tmem_load_row<kCols>(lane_base + group * kCols, v);
-            if (p.splits == 1) {
-                // nothing to exchange: park the rows in this CTA's own shared memory
+            cluster_wait();
+            const uint32_t mine = smem_u32(red) + (uint32_t)((split * share_groups * kTileN + t) * 16);
+            int owner = (group * kCols / 4) / share_groups;      // one division, then counted up
+            int within = group * kCols / 4 - owner * share_groups;
 #pragma unroll
-                for (int j = 0; j < kCols; ++j) red[(group * kCols + j) * kTileN + t] = v[j];
-            } else {
-                const uint32_t slot0 = smem_u32(red) + (uint32_t)(split * rows_share * kTileN + t) * 4u;
-                int owner = (group * kCols) / rows_share;            // one division, then counted up
-                int within = group * kCols - owner * rows_share;
-#pragma unroll
-                for (int j = 0; j < kCols; ++j) {
-                    if (group * kCols + j < rows) {
-                        st_cluster(peer_smem(slot0 + (uint32_t)(within * kTileN) * 4u, (uint32_t)owner), v[j]);
-                    }
-                    if (++within == rows_share) {
-                        within = 0;
-                        ++owner;
+            for (int j = 0; j < kCols; j += 4) {
+                if (group * kCols + j < rows) {
+                    const uint32_t at = mine + (uint32_t)(within * kTileN * 16);
+                    if (owner == split) {
+                        *reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(red) + (at - smem_u32(red)))
+                            = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    } else {
+                        st_async_v4(peer_smem(at, (uint32_t)owner), v[j], v[j + 1], v[j + 2], v[j + 3],
+                                    peer_smem(smem_u32(red_full), (uint32_t)owner));
                     }
                 }
+                if (++within == share_groups) {
+                    within = 0;
+                    ++owner;
+                }
             }
+        } else {
+            cluster_wait();
         }
     }
+    if (warp < 4) {
+        __syncwarp();
+        cluster_wait();
+    }
 
-    // ---- the K-slices of a channel tile live in the CTAs of one cluster; CTA s owns rows
-    // [s * rows_share, (s + 1) * rows_share) and sums them over all slices in slice order ----------
-    // The values a residual epilogue adds to, requested before the cluster barrier hides their
+    // ---- the K-slices of a channel tile live in the CTAs of one cluster; each CTA sums the rows it owns over all slices
+    // in slice order, a thread four rows of a channel.  The slices' parts arrive as asynchronous stores counted on a barrier
+    // here: one way across the cluster, where a cluster barrier behind plain stores was three.
+    // The values a residual epilogue adds to, requested before the wait hides their
     // latency (and, when their writer is known to be long done, before the dependency wait).
-    constexpr int kBasePre = 3;
-    float base_pre[kBasePre];
+    constexpr int kStride = kTcThreads / kPerRow;      // row groups at a time
+    constexpr int kBasePre = 2;
+    float base_pre[kBasePre][4];
     const bool base_wanted = !GATEUP && channel < N && (p.epilogue == EPI_ADD || p.epilogue == EPI_BIAS_ADD);
     const bf16* base_src = p.epilogue == EPI_ADD ? p.y : p.resid;
     auto fetch_bases = [&]() {
-        const int row0 = split * rows_share;
-        const int my_rows = min(rows_share, rows - row0);
 #pragma unroll
-        for (int u = 0; u < kBasePre; ++u) {
-            const int j = tid / kPerRow + u * (kTcThreads / kPerRow);
-            base_pre[u] = j < my_rows ? bf2f(base_src[(size_t)(row_first + row0 + j) * N + channel]) : 0.0f;
-        }
+        for (int u = 0; u < kBasePre; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int j = 4 * (tid / kPerRow + u * kStride) + e;
+                base_pre[u][e] = j < my_rows ? bf2f(base_src[(size_t)(row_first + row0 + j) * N + channel]) : 0.0f;
+            }
     };
     if (base_wanted && p.residual_settled != 0) fetch_bases();
     if (warp == 0 || warp >= 4) pdl_wait();
     if (base_wanted && p.residual_settled == 0) fetch_bases();
-    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    cluster_sync();       // the only cluster barrier: nothing remote is touched after it
+    __syncthreads();                                   // this slice's own part
+    if (*abort_flag == 0 && !guard.wait(red_full, 0)) *abort_flag = 1;
     if (*abort_flag == 0 && channel < N) {
-        const int row0 = split * rows_share;
-        const int my_rows = min(rows_share, rows - row0);
         int u = 0;
-#pragma unroll 2
-        for (int j = tid / kPerRow; j < my_rows; j += kTcThreads / kPerRow, ++u) {
-            const float* at = red + j * kTileN + c;
-            float acc = at[0], acc_up = GATEUP ? at[64] : 0.0f;
-            if (p.splits > 1) {
-                float part[8], part_up[8];
+        for (int g = tid / kPerRow; 4 * g < my_rows; g += kStride, ++u) {
+            const float4* at = reinterpret_cast<const float4*>(red) + g * kTileN + c;
+            float acc[4], acc_up[4];
 #pragma unroll
-                for (int sp = 1; sp < 8; ++sp) {
-                    part[sp] = 0.0f;
-                    part_up[sp] = 0.0f;
-                    if (sp < p.splits) {
-                        part[sp] = at[sp * rows_share * kTileN];
-                        if (GATEUP) part_up[sp] = at[sp * rows_share * kTileN + 64];
+            for (int sp = 0; sp < 8; ++sp) {
+                if (sp < p.splits) {
+                    const float4 part = at[sp * share_groups * kTileN];
+                    const float4 part_up = GATEUP ? at[sp * share_groups * kTileN + 64] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    const float a4[4] = {part.x, part.y, part.z, part.w};
+                    const float u4[4] = {part_up.x, part_up.y, part_up.z, part_up.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        acc[e] = sp == 0 ? a4[e] : acc[e] + a4[e];
+                        acc_up[e] = sp == 0 ? u4[e] : acc_up[e] + u4[e];
                     }
                 }
+            }
 #pragma unroll
-                for (int sp = 1; sp < 8; ++sp) {
-                    acc += part[sp];
-                    acc_up += part_up[sp];
+            for (int e = 0; e < 4; ++e) {
+                const int j = 4 * g + e;
+                if (j >= my_rows) break;
+                const size_t out = (size_t)(row_first + row0 + j) * N + channel;
+                float val;
+                if (GATEUP) {
+                    const float gate = acc[e] * scale;
+                    const float up = acc_up[e] * scale_up;
+                    // hardware exp2/reciprocal (good to about 2^-21); this path is compared at bf16 tolerance
+                    val = __fdividef(gate, 1.0f + __expf(-gate)) * up;
+                } else {
+                    val = finish(p, acc[e], scale, channel, out, base_wanted && u < kBasePre, u == 0 ? base_pre[0][e] : base_pre[1][e]);
                 }
+                if (p.y32 != nullptr) p.y32[out] = val;
+                if (!GATEUP && p.epilogue == EPI_BIAS_ADD) p.resid[out] = f2bf(val);
+                else p.y[out] = f2bf(val);
             }
-            const size_t out = (size_t)(row_first + row0 + j) * N + channel;
-            float val;
-            if (GATEUP) {
-                const float gate = acc * scale;
-                const float up = acc_up * scale_up;
-                // hardware exp2/reciprocal (good to about 2^-21); this path is compared at bf16 tolerance
-                val = __fdividef(gate, 1.0f + __expf(-gate)) * up;
-            } else {
-                const float base = u == 0 ? base_pre[0] : (u == 1 ? base_pre[1] : base_pre[2]);
-                val = finish(p, acc, scale, channel, out, base_wanted && u < kBasePre, base);
-            }
-            if (p.y32 != nullptr) p.y32[out] = val;
-            if (!GATEUP && p.epilogue == EPI_BIAS_ADD) p.resid[out] = f2bf(val);
-            else p.y[out] = f2bf(val);
         }
     }
     __syncthreads();
@@ -394,6 +411,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         const unsigned long long until = now_ns() + 200000ull;
         while (now_ns() < until) __nanosleep(1000);
         __syncthreads();
+        // a slice that is merely late may still send here: stay until it has ended, well or not
+        cluster_sync();
     }
     if (warp == 3) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
@@ -426,7 +445,7 @@ TcScratch* scratch_for_current_device() {
 template <int MT, bool GATEUP>
 size_t tc_smem_bytes() {
     return 1024 + (size_t)kWStages * kWStageBytes + (size_t)kXStages * MT * 256 + kRedBytes
-        + (2 * kWStages + 2 * kAStages + 2 * kXStages + 1) * sizeof(uint64_t) + 64;
+        + (2 * kWStages + 2 * kAStages + 2 * kXStages + 2) * sizeof(uint64_t) + 64;
 }
 
 template <int MT, bool GATEUP>
