@@ -32,6 +32,7 @@
 
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 namespace q3t {
 namespace {
@@ -76,18 +77,16 @@ struct TcParams {
     int residual_settled;     // GemvArgs::residual_settled
 };
 
-__device__ __forceinline__ float finish(const TcParams& p, float acc, float scale, int channel, size_t o,
-                                        bool have_base, float base) {
-    switch (p.epilogue) {
-        case EPI_ADD: return fmaf(acc, scale, have_base ? base : bf2f(p.y[o]));
-        case EPI_BIAS: return rbf(acc * scale) + bf2f(p.bias[channel]);
-        case EPI_BIAS_SILU: {
-            float v = rbf(acc * scale) + bf2f(p.bias[channel]);
-            return __fdividef(v, 1.0f + __expf(-v));
-        }
-        case EPI_BIAS_ADD: return (have_base ? base : bf2f(p.resid[o])) + rbf(rbf(acc * scale) + bf2f(p.bias[channel]));
-        default: return acc * scale;
+template <int EPI>
+__device__ __forceinline__ float finish(float acc, float scale, float bias, float base) {
+    if (EPI == EPI_ADD) return fmaf(acc, scale, base);
+    if (EPI == EPI_BIAS) return rbf(acc * scale) + bias;
+    if (EPI == EPI_BIAS_SILU) {
+        const float v = rbf(acc * scale) + bias;
+        return __fdividef(v, 1.0f + __expf(-v));
     }
+    if (EPI == EPI_BIAS_ADD) return base + rbf(rbf(acc * scale) + bias);
+    return acc * scale;
 }
 
 __device__ __forceinline__ void dequant_barrier() {
@@ -153,6 +152,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     guard.deadline = now_ns() + kBudgetNs;
     guard.abort_flag = abort_flag;
 
+    if (tid == 32) prefetch_map(&w_map);
+    if (tid == 64) prefetch_map(&x_map);
     if (tid == 0) {
         for (int s = 0; s < kWStages; ++s) {
             mbar_init(&full_w[s], 1);
@@ -363,41 +364,63 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     __syncthreads();                                   // this slice's own part
     if (*abort_flag == 0 && !guard.wait(red_full, 0)) *abort_flag = 1;
     if (*abort_flag == 0 && channel < N) {
-        int u = 0;
-        for (int g = tid / kPerRow; 4 * g < my_rows; g += kStride, ++u) {
-            const float4* at = reinterpret_cast<const float4*>(red) + g * kTileN + c;
-            float acc[4], acc_up[4];
+        bf16* dst = (!GATEUP && p.epilogue == EPI_BIAS_ADD ? p.resid : p.y) + (size_t)(row_first + row0) * N + channel;
+        // one loop per epilogue: what a row costs here is instructions behind the last wait of the launch
+        auto finish_rows = [&](auto which) {
+            constexpr int EPI = decltype(which)::value;
+            const float bias = EPI == EPI_BIAS || EPI == EPI_BIAS_SILU || EPI == EPI_BIAS_ADD ? bf2f(p.bias[channel]) : 0.0f;
+            int u = 0;
+            for (int g = tid / kPerRow; 4 * g < my_rows; g += kStride, ++u) {
+                const float4* at = reinterpret_cast<const float4*>(red) + g * kTileN + c;
+                float acc[4], acc_up[4];
 #pragma unroll
-            for (int sp = 0; sp < 8; ++sp) {
-                if (sp < p.splits) {
-                    const float4 part = at[sp * share_groups * kTileN];
-                    const float4 part_up = GATEUP ? at[sp * share_groups * kTileN + 64] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    const float a4[4] = {part.x, part.y, part.z, part.w};
-                    const float u4[4] = {part_up.x, part_up.y, part_up.z, part_up.w};
+                for (int sp = 0; sp < 8; ++sp) {
+                    if (sp < p.splits) {
+                        const float4 part = at[sp * share_groups * kTileN];
+                        const float a4[4] = {part.x, part.y, part.z, part.w};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        acc[e] = sp == 0 ? a4[e] : acc[e] + a4[e];
-                        acc_up[e] = sp == 0 ? u4[e] : acc_up[e] + u4[e];
+                        for (int e = 0; e < 4; ++e) acc[e] = sp == 0 ? a4[e] : acc[e] + a4[e];
+                        if (GATEUP) {
+                            const float4 part_up = at[sp * share_groups * kTileN + 64];
+                            const float u4[4] = {part_up.x, part_up.y, part_up.z, part_up.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc_up[e] = sp == 0 ? u4[e] : acc_up[e] + u4[e];
+                        }
+                    }
+                }
+                bf16* row = dst + (size_t)(4 * g) * N;
+                float base[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    base[e] = u == 0 ? base_pre[0][e] : base_pre[1][e];
+                    if ((EPI == EPI_ADD || EPI == EPI_BIAS_ADD) && u >= kBasePre && 4 * g + e < my_rows) base[e] = bf2f(row[(size_t)e * N]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float val;
+                    if (GATEUP) {
+                        const float gate = acc[e] * scale;
+                        // hardware exp2/reciprocal (good to about 2^-21); this path is compared at bf16 tolerance
+                        val = __fdividef(gate, 1.0f + __expf(-gate)) * (acc_up[e] * scale_up);
+                    } else {
+                        val = finish<EPI>(acc[e], scale, bias, base[e]);
+                    }
+                    if (4 * g + e < my_rows) {
+                        if (p.y32 != nullptr) p.y32[(size_t)(row_first + row0 + 4 * g + e) * N + channel] = val;
+                        row[(size_t)e * N] = f2bf(val);
                     }
                 }
             }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = 4 * g + e;
-                if (j >= my_rows) break;
-                const size_t out = (size_t)(row_first + row0 + j) * N + channel;
-                float val;
-                if (GATEUP) {
-                    const float gate = acc[e] * scale;
-                    const float up = acc_up[e] * scale_up;
-                    // hardware exp2/reciprocal (good to about 2^-21); this path is compared at bf16 tolerance
-                    val = __fdividef(gate, 1.0f + __expf(-gate)) * up;
-                } else {
-                    val = finish(p, acc[e], scale, channel, out, base_wanted && u < kBasePre, u == 0 ? base_pre[0][e] : base_pre[1][e]);
-                }
-                if (p.y32 != nullptr) p.y32[out] = val;
-                if (!GATEUP && p.epilogue == EPI_BIAS_ADD) p.resid[out] = f2bf(val);
-                else p.y[out] = f2bf(val);
+        };
+        if (GATEUP) {
+            finish_rows(std::integral_constant<int, EPI_GATE_UP_SILU>());
+        } else {
+            switch (p.epilogue) {
+                case EPI_ADD: finish_rows(std::integral_constant<int, EPI_ADD>()); break;
+                case EPI_BIAS: finish_rows(std::integral_constant<int, EPI_BIAS>()); break;
+                case EPI_BIAS_SILU: finish_rows(std::integral_constant<int, EPI_BIAS_SILU>()); break;
+                case EPI_BIAS_ADD: finish_rows(std::integral_constant<int, EPI_BIAS_ADD>()); break;
+                default: finish_rows(std::integral_constant<int, EPI_PLAIN>()); break;
             }
         }
     }
