@@ -49,6 +49,13 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
+// 2^x, x <= 0: as exp2f, but what would be subnormal (below 2^-126 of the largest weight) is zero
+__device__ __forceinline__ float exp2_ftz(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 struct PromptArgs {
     bf16* qkv;                 // [rows][qkv_stride]: q | k | v; q is normalised and rotated in place by the append
     const bf16* q_norm_w;
@@ -140,9 +147,9 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
     const int warp = tid / kWarp;
     const int gid = lane >> 2;
     const int tig = lane & 3;
-    const int kvh = blockIdx.y;
-    // the last positions have the longest context: they go first
-    const int block = gridDim.x - 1 - blockIdx.x;
+    // the last positions have the longest context: they go first, all KV heads of a block together
+    const int kvh = (int)blockIdx.x % a.kv_heads;
+    const int block = ((int)gridDim.x - 1 - (int)blockIdx.x) / a.kv_heads;
     const int row0 = block * kBlockPositions;
     const int head = kvh * 2 + (warp >> 1);
     const int my_row = row0 + (warp & 1) * 16;            // rows my_row + gid and + 8 of this lane
@@ -154,21 +161,25 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
 
     auto load_step = [&](int step, int buffer) {
         const uint32_t kdst = smem_addr(smem) + buffer * 2 * kTileBytes;
-        // 64 tokens x 16 pieces of K and as many of V: thread t takes piece t % 16 of the tokens t / 16 + 8 i
+        // 64 tokens x 16 pieces of K and as many of V: thread t takes piece t % 16 of the tokens t / 16 + 8 i, two of a page
         const int piece = tid & 15;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int t = (tid >> 4) + 8 * i;
-            const int token = step * kStepTokens + t;
-            const uint32_t off = tile_offset(t, piece);
-            if (token < length) {
-                const size_t in_page = (size_t)(token % kPageTokens) * kHd + piece * 8;
-                copy16(kdst + off, page_of(a, token, kvh, false) + in_page);
-                copy16(kdst + kTileBytes + off, page_of(a, token, kvh, true) + in_page);
-            } else {
-                // past the end: the scores are masked, but 0 * (stale bits that decode as NaN) is not zero
-                *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + off) = make_int4(0, 0, 0, 0);
-                *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + kTileBytes + off) = make_int4(0, 0, 0, 0);
+        for (int page = 0; page < kStepTokens / kPageTokens; ++page) {
+            const int first = step * kStepTokens + page * kPageTokens;
+            const bf16* k = first < length ? page_of(a, first, kvh, false) + (size_t)(tid >> 4) * kHd + piece * 8 : nullptr;
+            const bf16* v = k + (a.kv.v_offset - a.kv.k_offset);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int t = page * kPageTokens + 8 * half + (tid >> 4);
+                const uint32_t off = tile_offset(t, piece);
+                if (step * kStepTokens + t < length) {
+                    copy16(kdst + off, k + 8 * half * kHd);
+                    copy16(kdst + kTileBytes + off, v + 8 * half * kHd);
+                } else {
+                    // past the end: the scores are masked, but 0 * (stale bits that decode as NaN) is not zero
+                    *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + off) = make_int4(0, 0, 0, 0);
+                    *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + kTileBytes + off) = make_int4(0, 0, 0, 0);
+                }
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -233,41 +244,46 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
         }
         // ---- running softmax
         const bool masked = t0 + kStepTokens - 1 > a.base + my_row;       // some row of the warp ends in this step
-        float mx[2] = {m[0], m[1]};
+        if (masked) {
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (t0 + 8 * n + 2 * tig + (e & 1) > (e < 2 ? last_lo : last_hi)) s[n][e] = -INFINITY;
+        }
+        float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float v = s[n][e] * scale;
-                if (masked && t0 + 8 * n + 2 * tig + (e & 1) > (e < 2 ? last_lo : last_hi)) v = -INFINITY;
-                s[n][e] = v;
-                mx[e >> 1] = fmaxf(mx[e >> 1], v);
-            }
+            for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
             mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+            mx[h] = fmaxf(m[h], mx[h] * scale);
         }
         // token 0 is visible to every row, so the maximum is finite from the first step on
-        float f[2];
+        if (__any_sync(0xffffffffu, mx[0] != m[0] || mx[1] != m[1])) {       // seldom, once the context is some steps long
+            float f[2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            f[h] = exp2f(m[h] - mx[h]);
-            m[h] = mx[h];
-            l[h] *= f[h];
+            for (int h = 0; h < 2; ++h) {
+                f[h] = exp2_ftz(m[h] - mx[h]);
+                m[h] = mx[h];
+                l[h] *= f[h];
+            }
+#pragma unroll
+            for (int n = 0; n < 16; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[n][e] *= f[e >> 1];
         }
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float pr = exp2f(s[n][e] - m[e >> 1]);
+                const float pr = exp2_ftz(fmaf(s[n][e], scale, -m[e >> 1]));
                 s[n][e] = pr;
                 l[e >> 1] += pr;
             }
-#pragma unroll
-        for (int n = 0; n < 16; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[n][e] *= f[e >> 1];
         // ---- output: P (16 x 64) V (64 x 128), P as hi + lo
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -337,7 +353,7 @@ cudaError_t launch_prompt_attention(const AttentionArgs& a, int base, cudaStream
     p.q_heads = a.q_heads; p.kv_heads = a.kv_heads; p.eps = a.eps;
     const cudaError_t e = launch_pdl(prompt_append_kernel, dim3((unsigned)a.rows), dim3(256), 0, stream, p);
     if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)((a.rows + kBlockPositions - 1) / kBlockPositions), (unsigned)a.kv_heads);
+    const dim3 grid((unsigned)((a.rows + kBlockPositions - 1) / kBlockPositions * a.kv_heads));
     return launch_pdl(prompt_attention_kernel, grid, dim3(kFlashThreads), kFlashSmem, stream, p);
 }
 
