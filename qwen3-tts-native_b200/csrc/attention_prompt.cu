@@ -8,9 +8,13 @@
 // Here a CTA takes 32 positions of the two query heads of a KV head (64 rows of MMA) and walks their
 // common context once, 64 tokens at a time, with a running softmax.
 //
-// What bounds it: mma.sync issue.  The probabilities go through the second product as bf16 hi + lo (16
-// bits kept), so a 64-row, 64-token step is 3 x 64 x 64 x 128 MACs.  Four warps of 16 rows, K and V of
-// the next step in flight (cp.async, two buffers of 32 KB): three CTAs fit an SM.
+// What bounds it: the chain of a step, 64 tokens' scores, softmax and products, times the steps of the longest
+// context.  The probabilities go through the second product as bf16 hi + lo (16 bits kept), so a 64-row, 64-token step is
+// 3 x 64 x 64 x 128 MACs: 0.9 us of an SM's mma.sync rate, 31 steps an SM for 1500 positions.  Two groups of four
+// warps of 16 rows take half of every step's tokens each and meet at the end; K and V of the next step are in flight
+// (cp.async, two buffers of 32 KB); two CTAs fit an SM at 128 registers (the query fragments come from shared memory).
+// 1500 positions: 71 us a layer; four warps on whole steps 81, with a page lookup per token, masks on every score
+// and heads one after the other 118.
 
 #include "q3t_kernels.cuh"
 
@@ -20,9 +24,11 @@ namespace {
 constexpr int kHd = 128;
 constexpr int kBlockPositions = 32;
 constexpr int kStepTokens = 64;
-constexpr int kFlashThreads = 128;
+constexpr int kFlashThreads = 256;
 constexpr int kTileBytes = kStepTokens * kHd * 2;       // 16 KB of K or V
-constexpr size_t kFlashSmem = 4 * kTileBytes;           // two buffers of (K, V)
+constexpr int kFlashCtas = 2;
+constexpr int kHalfTokens = kStepTokens / 2;            // of a step, to each group of four warps
+constexpr size_t kFlashSmem = 5 * kTileBytes;           // two buffers of (K, V), the queries
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -140,11 +146,12 @@ __global__ void __launch_bounds__(256) prompt_append_kernel(const PromptArgs a) 
 // eight rows of an ldmatrix fall into different banks
 __device__ __forceinline__ uint32_t tile_offset(int t, int piece) { return (uint32_t)(t * 256 + ((piece ^ (t & 7)) << 4)); }
 
-__global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(const PromptArgs a) {
+__global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_kernel(const PromptArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x;
     const int lane = tid % kWarp;
-    const int warp = tid / kWarp;
+    const int group = tid / (kFlashThreads / 2);          // tokens 32 group .. + 31 of every step
+    const int warp = tid / kWarp % 4;
     const int gid = lane >> 2;
     const int tig = lane & 3;
     // the last positions have the longest context: they go first, all KV heads of a block together
@@ -161,45 +168,37 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
 
     auto load_step = [&](int step, int buffer) {
         const uint32_t kdst = smem_addr(smem) + buffer * 2 * kTileBytes;
-        // 64 tokens x 16 pieces of K and as many of V: thread t takes piece t % 16 of the tokens t / 16 + 8 i, two of a page
+        // 64 tokens x 16 pieces of K and as many of V: thread t takes piece t % 16 of token t / 16 of every page
         const int piece = tid & 15;
 #pragma unroll
         for (int page = 0; page < kStepTokens / kPageTokens; ++page) {
-            const int first = step * kStepTokens + page * kPageTokens;
-            const bf16* k = first < length ? page_of(a, first, kvh, false) + (size_t)(tid >> 4) * kHd + piece * 8 : nullptr;
-            const bf16* v = k + (a.kv.v_offset - a.kv.k_offset);
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int t = page * kPageTokens + 8 * half + (tid >> 4);
-                const uint32_t off = tile_offset(t, piece);
-                if (step * kStepTokens + t < length) {
-                    copy16(kdst + off, k + 8 * half * kHd);
-                    copy16(kdst + kTileBytes + off, v + 8 * half * kHd);
-                } else {
-                    // past the end: the scores are masked, but 0 * (stale bits that decode as NaN) is not zero
-                    *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + off) = make_int4(0, 0, 0, 0);
-                    *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + kTileBytes + off) = make_int4(0, 0, 0, 0);
-                }
+            const int t = page * kPageTokens + (tid >> 4);
+            const uint32_t off = tile_offset(t, piece);
+            if (step * kStepTokens + t < length) {
+                const bf16* k = page_of(a, step * kStepTokens + page * kPageTokens, kvh, false) + (size_t)(tid >> 4) * kHd + piece * 8;
+                copy16(kdst + off, k);
+                copy16(kdst + kTileBytes + off, k + (a.kv.v_offset - a.kv.k_offset));
+            } else {
+                // past the end: the scores are masked, but 0 * (stale bits that decode as NaN) is not zero
+                *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + off) = make_int4(0, 0, 0, 0);
+                *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + kTileBytes + off) = make_int4(0, 0, 0, 0);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    load_step(0, 0);
-
-    // query fragments: eight k-steps of 16 dims
-    uint32_t qa[8][4];
+    // the queries: row 32 head + position, as the K tiles
     {
-        const int r_lo = my_row + gid, r_hi = my_row + gid + 8;
-        const bf16* q_lo = a.qkv + (size_t)min(r_lo, a.rows - 1) * a.qkv_stride + (size_t)head * kHd;
-        const bf16* q_hi = a.qkv + (size_t)min(r_hi, a.rows - 1) * a.qkv_stride + (size_t)head * kHd;
+        const uint32_t to = smem_addr(smem) + 4 * kTileBytes;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            qa[k][0] = *reinterpret_cast<const uint32_t*>(q_lo + 16 * k + 2 * tig);
-            qa[k][1] = *reinterpret_cast<const uint32_t*>(q_hi + 16 * k + 2 * tig);
-            qa[k][2] = *reinterpret_cast<const uint32_t*>(q_lo + 16 * k + 2 * tig + 8);
-            qa[k][3] = *reinterpret_cast<const uint32_t*>(q_hi + 16 * k + 2 * tig + 8);
+        for (int i = 0; i < 4; ++i) {
+            const int row = (tid >> 4) + 16 * i;
+            const bf16* q = a.qkv + (size_t)min(row0 + row % kBlockPositions, a.rows - 1) * a.qkv_stride
+                            + (size_t)(kvh * 2 + row / kBlockPositions) * kHd;
+            copy16(to + tile_offset(row, tid & 15), q + 8 * (tid & 15));
         }
     }
+    load_step(0, 0);
+
     float o[16][4];
 #pragma unroll
     for (int n = 0; n < 16; ++n)
@@ -220,40 +219,44 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        const uint32_t kt = smem_addr(smem) + buffer * 2 * kTileBytes;
+        const uint32_t kt = smem_addr(smem) + buffer * 2 * kTileBytes + group * kHalfTokens * 256;
         const uint32_t vt = kt + kTileBytes;
-        const int t0 = step * kStepTokens;
-        // ---- scores of 16 rows x 64 tokens
-        float s[8][4];
+        const uint32_t qt = smem_addr(smem) + 4 * kTileBytes;
+        const int t0 = step * kStepTokens + group * kHalfTokens;
+        // ---- scores of 16 rows x 32 tokens
+        float s[4][4];
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
+        for (int n = 0; n < 4; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) s[n][e] = 0.0f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
+            // matrices: rows 16 warp .. + 7 and + 8 .. + 15, dims 16 k .. + 7, then dims 16 k + 8 .. + 15
+            uint32_t qa[4];
+            ldmatrix_x4(qt + tile_offset(16 * warp + (lane & 15), 2 * k + (lane >> 4)), qa);
 #pragma unroll
-            for (int n2 = 0; n2 < 4; ++n2) {
+            for (int n2 = 0; n2 < 2; ++n2) {
                 // matrices: tokens 16 n2 .. + 7 and + 8 .. + 15, dims 16 k .. + 7 and + 8 .. + 15
                 const int t = 16 * n2 + (lane & 7) + ((lane >> 4) << 3);
                 const int piece = 2 * k + ((lane >> 3) & 1);
                 uint32_t b[4];
                 ldmatrix_x4(kt + tile_offset(t, piece), b);
-                mma_16816(s[2 * n2], qa[k], b[0], b[1]);
-                mma_16816(s[2 * n2 + 1], qa[k], b[2], b[3]);
+                mma_16816(s[2 * n2], qa, b[0], b[1]);
+                mma_16816(s[2 * n2 + 1], qa, b[2], b[3]);
             }
         }
         // ---- running softmax
-        const bool masked = t0 + kStepTokens - 1 > a.base + my_row;       // some row of the warp ends in this step
+        const bool masked = t0 + kHalfTokens - 1 > a.base + my_row;       // some row of the warp ends in this step
         if (masked) {
 #pragma unroll
-            for (int n = 0; n < 8; ++n)
+            for (int n = 0; n < 4; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     if (t0 + 8 * n + 2 * tig + (e & 1) > (e < 2 ? last_lo : last_hi)) s[n][e] = -INFINITY;
         }
         float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
+        for (int n = 0; n < 4; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
 #pragma unroll
@@ -262,12 +265,12 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
             mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
             mx[h] = fmaxf(m[h], mx[h] * scale);
         }
-        // token 0 is visible to every row, so the maximum is finite from the first step on
         if (__any_sync(0xffffffffu, mx[0] != m[0] || mx[1] != m[1])) {       // seldom, once the context is some steps long
             float f[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                f[h] = exp2_ftz(m[h] - mx[h]);
+                // a half whose tokens so far all lie past the row has no maximum yet, and zeros to scale
+                f[h] = m[h] == -INFINITY ? 0.0f : exp2_ftz(m[h] - mx[h]);
                 m[h] = mx[h];
                 l[h] *= f[h];
             }
@@ -277,16 +280,16 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
                 for (int e = 0; e < 4; ++e) o[n][e] *= f[e >> 1];
         }
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
+        for (int n = 0; n < 4; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float pr = exp2_ftz(fmaf(s[n][e], scale, -m[e >> 1]));
+                const float pr = s[n][e] == -INFINITY ? 0.0f : exp2_ftz(fmaf(s[n][e], scale, -m[e >> 1]));
                 s[n][e] = pr;
                 l[e >> 1] += pr;
             }
-        // ---- output: P (16 x 64) V (64 x 128), P as hi + lo
+        // ---- output: P (16 x 32) V (32 x 128), P as hi + lo
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < 2; ++k) {
             uint32_t hi[4], lo[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -314,7 +317,38 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
     }
-    const float inv[2] = {1.0f / l[0], 1.0f / l[1]};
+    // ---- the two halves of every row meet: the second group's in shared memory (the last barrier of the loop has freed it)
+    float* meet = reinterpret_cast<float*>(smem) + (warp * kWarp + lane);
+    constexpr int kPlane = 4 * kWarp;                     // one value of every thread of a group
+    if (group == 1) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            meet[h * kPlane] = m[h];
+            meet[(2 + h) * kPlane] = l[h];
+        }
+#pragma unroll
+        for (int n = 0; n < 16; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) meet[(4 + 4 * n + e) * kPlane] = o[n][e];
+    }
+    __syncthreads();
+    if (group == 1) return;
+    float inv[2], f1[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        // token 0 is visible to every row: the first group's maximum is finite
+        const float m1 = meet[h * kPlane];
+        const float top = fmaxf(m[h], m1);
+        const float f0 = exp2_ftz(m[h] - top);
+        f1[h] = exp2_ftz(m1 - top);
+        inv[h] = 1.0f / (l[h] * f0 + meet[(2 + h) * kPlane] * f1[h]);
+        f1[h] *= inv[h];
+        inv[h] *= f0;
+    }
+#pragma unroll
+    for (int n = 0; n < 16; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] = fmaf(meet[(4 + 4 * n + e) * kPlane], f1[e >> 1], o[n][e] * inv[e >> 1]);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int row = my_row + gid + 8 * h;
@@ -322,7 +356,7 @@ __global__ void __launch_bounds__(kFlashThreads, 3) prompt_attention_kernel(cons
             bf16* dst = a.out + (size_t)row * a.q_heads * kHd + (size_t)head * kHd + 2 * tig;
 #pragma unroll
             for (int n = 0; n < 16; ++n) {
-                *reinterpret_cast<uint32_t*>(dst + 8 * n) = pack_pair(o[n][2 * h] * inv[h], o[n][2 * h + 1] * inv[h]);
+                *reinterpret_cast<uint32_t*>(dst + 8 * n) = pack_pair(o[n][2 * h], o[n][2 * h + 1]);
             }
         }
     }
