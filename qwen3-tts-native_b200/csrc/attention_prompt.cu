@@ -102,42 +102,60 @@ __global__ void __launch_bounds__(256) prompt_append_kernel(const PromptArgs a) 
     pdl_wait();
     pdl_trigger();
     const int t = pos % kPageTokens;
-    for (int job = warp; job < a.q_heads + a.kv_heads; job += 8) {
-        const bool is_key = job >= a.q_heads;
-        bf16* src = a.qkv + (size_t)row * a.qkv_stride + (size_t)job * kHd;
-        float x[4], sq[4];
+    // three heads a warp at a time (all of the talker's 16 + 8), requested together: one latency
+    constexpr int kJobs = 3;
+    const int total = a.q_heads + a.kv_heads;
+    for (int first = warp; first < total; first += 8 * kJobs) {
+        bf16 raw[kJobs][4], value[kJobs][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            x[j] = bf2f(src[lane + 32 * j]);
-            sq[j] = fmaf(x[j], x[j], 0.0f);
-        }
-        float c = (sq[0] + sq[2]) + (sq[1] + sq[3]);
-        c = warp_sum_down(c);
-        c = __shfl_sync(0xffffffffu, c, 0);
-        const float inv = rsqrtf(c / static_cast<float>(kHd) + a.eps);
-        float y[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) y[j] = rbf(rbf(x[j] * inv) * (is_key ? wk[j] : wq[j]));
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            float o1, o2;
-            rope_pair_cs(y[j], y[j + 2], bf_lo(cs[j]), bf_hi(cs[j]), o1, o2);
-            y[j] = o1;
-            y[j + 2] = o2;
-        }
-        if (is_key) {
-            const int kvh = job - a.q_heads;
-            bf16* kdst = page_of(a, pos, kvh, false) + (size_t)t * kHd;
-            bf16* vdst = page_of(a, pos, kvh, true) + (size_t)t * kHd;
-            const bf16* vsrc = src + (size_t)a.kv_heads * kHd;
+        for (int u = 0; u < kJobs; ++u) {
+            const int job = first + 8 * u;
+            const bf16* src = a.qkv + (size_t)row * a.qkv_stride + (size_t)job * kHd;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                kdst[lane + 32 * j] = f2bf(y[j]);
-                vdst[lane + 32 * j] = vsrc[lane + 32 * j];
+                if (job < total) raw[u][j] = src[lane + 32 * j];
+                if (job >= a.q_heads && job < total) value[u][j] = src[(size_t)a.kv_heads * kHd + lane + 32 * j];
             }
-        } else {
+        }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) src[lane + 32 * j] = f2bf(y[j]);
+        for (int u = 0; u < kJobs; ++u) {
+            const int job = first + 8 * u;
+            if (job >= total) break;
+            const bool is_key = job >= a.q_heads;
+            float x[4], sq[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                x[j] = bf2f(raw[u][j]);
+                sq[j] = fmaf(x[j], x[j], 0.0f);
+            }
+            float c = (sq[0] + sq[2]) + (sq[1] + sq[3]);
+            c = warp_sum_down(c);
+            c = __shfl_sync(0xffffffffu, c, 0);
+            const float inv = rsqrtf(c / static_cast<float>(kHd) + a.eps);
+            float y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[j] = rbf(rbf(x[j] * inv) * (is_key ? wk[j] : wq[j]));
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float o1, o2;
+                rope_pair_cs(y[j], y[j + 2], bf_lo(cs[j]), bf_hi(cs[j]), o1, o2);
+                y[j] = o1;
+                y[j + 2] = o2;
+            }
+            if (is_key) {
+                const int kvh = job - a.q_heads;
+                bf16* kdst = page_of(a, pos, kvh, false) + (size_t)t * kHd;
+                bf16* vdst = page_of(a, pos, kvh, true) + (size_t)t * kHd;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    kdst[lane + 32 * j] = f2bf(y[j]);
+                    vdst[lane + 32 * j] = value[u][j];
+                }
+            } else {
+                bf16* dst = a.qkv + (size_t)row * a.qkv_stride + (size_t)job * kHd;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dst[lane + 32 * j] = f2bf(y[j]);
+            }
         }
     }
 }
