@@ -59,6 +59,16 @@ def test_residual(orc, ops, n, k, rows):
     check_bf16(orc, got, orc.int8_gemm_rows(w, s, x, y_in=base, mode=1), summand=base)
 
 
+@pytest.mark.parametrize("rows", [33, 47, 48, 49])
+def test_row_tile_edges(orc, ops, rows):
+    """Around the tile of 48 rows, with K in ragged slices and a last channel tile that is not full."""
+    n, k = 1100, 1408
+    w, s, x = case(orc, rows, n, k, rows)
+    base = orc.to_bf16(np.random.default_rng(rows).standard_normal((rows, n)).astype(np.float32))
+    got = ops.int8_gemm_rows(w, s, x, y_in=base, mode=1)
+    check_bf16(orc, got, orc.int8_gemm_rows(w, s, x, y_in=base, mode=1), summand=base)
+
+
 @pytest.mark.parametrize("n,k,rows", [(6144, 2048, 64), (3072, 1024, 16), (100, 128, 9), (64, 64, 33)])
 def test_gate_up_silu(orc, ops, n, k, rows):
     rng = np.random.default_rng(3)
