@@ -7,9 +7,8 @@
 //   TMA, 128-byte swizzle           int8 W tile 128 x 128 -> shared ring (6 stages of 16 KB)
 //   TMA, 128-byte swizzle           bf16 x tile MT x 128  -> shared ring (4 stages), UMMA K-major
 //   2 x 4 warps, steps in turn      a thread owns a channel: 128 int8 of its row -> bf16 in
-//                                   registers (exact: XOR, PRMT into the mantissa of 2^23, packed
-//                                   subtract, PRMT of the high halves) -> tcgen05.st into the TMEM
-//                                   columns of an A stage.  The dequantised weights never touch
+//                                   registers (exact: PRMT, two masks, packed subtract) ->
+//                                   tcgen05.st into the TMEM columns of an A stage.  The dequantised weights never touch
 //                                   shared memory, whose bandwidth bounds this kernel.
 //   1 thread                        tcgen05.mma.cta_group::1.kind::f16 with A from TMEM and B
 //                                   (activations) from shared memory, 128 x MT x 16 per

@@ -145,17 +145,14 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 
 
-// four int8 (one word) -> four bf16 (two words), exact
+// Four int8 (one word) -> four bf16 (two words), exact.  Behind the byte 0x43 the low seven bits of a weight read as
+// 128 + those bits, and its sign bit alone as 128 or, set, 256: their difference is the weight.  Six integer instructions
+// and two subtractions; by way of fp32 (2^23 + byte, minus the bias, high halves) it was seven and two, and the integer
+// pipe bounds a step of the skinny GEMM (16 projections of 48 rows 123.9 against 119.9 us).
 __device__ __forceinline__ void dequant4(uint32_t word, uint32_t& lo, uint32_t& hi) {
-    const uint32_t u = word ^ 0x80808080u;
-    const unsigned long long bias = pack2(-8388736.0f, -8388736.0f);
-    const unsigned long long a = add2(pack2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7650)),
-                                            __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7651))), bias);
-    const unsigned long long b = add2(pack2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7652)),
-                                            __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7653))), bias);
-    // a small integer as fp32 has a zero low half: its high half is the bf16 of the same value
-    lo = __byte_perm(static_cast<uint32_t>(a), static_cast<uint32_t>(a >> 32), 0x7632);
-    hi = __byte_perm(static_cast<uint32_t>(b), static_cast<uint32_t>(b >> 32), 0x7632);
+    const uint32_t p = __byte_perm(word, 0x43434343u, 0x4140), q = __byte_perm(word, 0x43434343u, 0x4342);
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(p & 0xff7fff7fu), "r"(p & 0xff80ff80u));
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"(q & 0xff7fff7fu), "r"(q & 0xff80ff80u));
 }
 
 // NCOL consecutive fp32 accumulator columns of this thread's TMEM lane
