@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from dataclasses import dataclass
 from typing import Iterable, Optional, Sequence, Tuple
 
@@ -51,6 +52,9 @@ class DeviceFrameViewV2C(C.Structure):   # 40 bytes, align 8
     _fields_ = [("struct_size", C.c_uint32), ("code_count", C.c_uint32),
                 ("device_codes", C.c_void_p), ("ready_event", C.c_void_p),
                 ("lease_id", C.c_uint64), ("device_index", C.c_int32), ("reserved", C.c_uint32)]
+
+
+_EMPTY_VIEW = bytes(DeviceFrameViewV2C(struct_size=C.sizeof(DeviceFrameViewV2C)))
 
 
 class StateInfoC(C.Structure):        # 40 bytes
@@ -214,6 +218,22 @@ class NativeTalkerStatusError(RuntimeError):
 _ERR_CAP = 512
 
 
+class _Scratch(threading.local):
+    """Out-parameters of the calls a frame makes, one set per thread and read before the next call: making them anew
+    for every session of every frame was a tenth of a 64-session frame, most of it with the GPU idle."""
+
+    def __init__(self):
+        self.err = C.create_string_buffer(_ERR_CAP)
+        self.codes = (C.c_uint16 * CODEBOOKS)()
+        self.next = C.c_uint16(0)
+        self.next_ref = C.byref(self.next)
+        self.info = FrameInfoC()
+        self.info_ref = C.byref(self.info)
+
+
+_scratch = _Scratch()
+
+
 def _check(status: int, err) -> None:
     if status != STATUS_OK:
         raise NativeTalkerStatusError(status, err.value.decode("utf-8", "replace"))
@@ -243,6 +263,14 @@ class SamplingConfig:
     def to_c(self) -> SamplingConfigC:
         return SamplingConfigC(int(self.do_sample), int(self.top_k), float(self.top_p),
                                float(self.temperature), float(self.repetition_penalty))
+
+    def _image(self) -> bytes:
+        """The bytes of to_c(), made once: the object never changes."""
+        image = self.__dict__.get("_c_image")
+        if image is None:
+            image = bytes(self.to_c())
+            object.__setattr__(self, "_c_image", image)
+        return image
 
 
 @dataclass(frozen=True)
@@ -396,15 +424,12 @@ class NativeTalkerModel:
                                   trailing_text_ids: Sequence[int]) -> list:
         """One lockstep frame for all sessions (native_talker.rs:314-380)."""
         n = len(sessions)
-        handles = (C.c_void_p * n)(*[s._handle for s in sessions])
+        handles = (C.c_void_p * n)(*[s._handle.value for s in sessions])
         trailing = (C.c_int32 * n)(*[int(t) for t in trailing_text_ids])
-        talker = (SamplingConfigC * n)(*[s.talker_sampling.to_c() for s in sessions])
-        predictor = (SamplingConfigC * n)(*[s.predictor_sampling.to_c() for s in sessions])
-        views = (DeviceFrameViewV2C * n)()
-        for v in views:
-            v.struct_size = C.sizeof(DeviceFrameViewV2C)
-            v.reserved = 0
-        err = C.create_string_buffer(_ERR_CAP)
+        talker = (SamplingConfigC * n).from_buffer_copy(b"".join([s.talker_sampling._image() for s in sessions]))
+        predictor = (SamplingConfigC * n).from_buffer_copy(b"".join([s.predictor_sampling._image() for s in sessions]))
+        views = (DeviceFrameViewV2C * n).from_buffer_copy(_EMPTY_VIEW * n)
+        err = _scratch.err
         _check(library().qwen3_tts_model_batch_next_frame_begin_v2(
             self._handle, handles, n, trailing, talker, predictor, views, err, _ERR_CAP), err)
         out = []
@@ -516,15 +541,12 @@ class NativeTalkerSession:
         """Host-visible frame (native_talker.rs:1279-1334)."""
         if self.ended:
             return None
-        codes = (C.c_uint16 * CODEBOOKS)()
-        nxt = C.c_uint16(0)
-        info = FrameInfoC()
-        err = C.create_string_buffer(_ERR_CAP)
+        t = _scratch
         _check(library().qwen3_tts_session_next_frame(
             self._handle, self.current_semantic_token, trailing_text_id, self.talker_sampling.to_c(),
-            self.predictor_sampling.to_c(), codes, CODEBOOKS, C.byref(nxt), C.byref(info), err,
-            _ERR_CAP), err)
-        return self._advance(tuple(int(c) for c in codes), nxt.value, info)
+            self.predictor_sampling.to_c(), t.codes, CODEBOOKS, t.next_ref, t.info_ref, t.err,
+            _ERR_CAP), t.err)
+        return self._advance(tuple(t.codes), t.next.value, t.info)
 
     def begin_device_frame(self, trailing_text_id: int = 0) -> Optional[PendingTalkerFrame]:
         """Device-resident frame (native_talker.rs:1340-1420)."""
@@ -540,21 +562,17 @@ class NativeTalkerSession:
         return PendingTalkerFrame(self, view)
 
     def _finish(self, lease_id: int, consumer_done_event: int) -> StreamingCodecFrame:
-        nxt = C.c_uint16(0)
-        info = FrameInfoC()
-        err = C.create_string_buffer(_ERR_CAP)
+        t = _scratch
         _check(library().qwen3_tts_session_next_frame_finish_v2(
-            self._handle, lease_id, C.c_void_p(consumer_done_event or None), C.byref(nxt),
-            C.byref(info), err, _ERR_CAP), err)
-        return self._advance((), nxt.value, info)
+            self._handle, lease_id, consumer_done_event or None, t.next_ref, t.info_ref, t.err, _ERR_CAP), t.err)
+        return self._advance((), t.next.value, t.info)
 
     def _advance(self, codes, nxt: int, info: FrameInfoC) -> StreamingCodecFrame:
-        self.current_semantic_token = int(nxt)
+        self.current_semantic_token = nxt
         self.frames_emitted += 1
-        self.ended = bool(info.ended_by_eos)
-        return StreamingCodecFrame(codes, int(nxt), bool(info.ended_by_eos), int(info.talker_position),
-                                   float(info.predictor_gpu_milliseconds),
-                                   float(info.talker_gpu_milliseconds))
+        self.ended = ended = bool(info.ended_by_eos)
+        return StreamingCodecFrame(codes, nxt, ended, info.talker_position, info.predictor_gpu_milliseconds,
+                                   info.talker_gpu_milliseconds)
 
     def runtime_state(self) -> SessionRuntimeState:
         out = StateInfoC()
