@@ -538,7 +538,7 @@ def run_ours(args, rank: int, local_rank: int, world: int) -> None:
             ps.prefill(ids, [-1] * 128)
             prompt_ms.append((time.perf_counter() - t0) * 1e3)
             ps.close()
-        line["prefill"] = {"positions": 128, "ms": min(prompt_ms), "positions_per_pass": 64,
+        line["prefill"] = {"positions": 128, "ms": min(prompt_ms), "positions_per_pass": 128,
                            "api": "qwen3_tts_session_prefill"}
         # ---- a 128-id prompt, then 375 frames (30 s of audio at 12.5 frames/s), B=1 and B=64;
         # the end-of-sequence code stays masked so that all 375 frames run on synthetic weights
