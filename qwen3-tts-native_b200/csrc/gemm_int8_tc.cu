@@ -552,9 +552,12 @@ bool gemm_tc_supports(const GemvArgs& a) {
 }
 
 namespace {
-// the smallest tile that takes the rows at once: activations and exchange cost what the tile has, used or not (16
-// projections of 48 rows: 128.4 us by a tile of 64, 124.0 by one of 48)
-int tile_rows(int rows) { return rows > 48 ? 64 : (rows + 15) / 16 * 16; }
+// The smallest tile that takes the rows at once, or in as many blocks as tiles of 64 would: activations and exchange
+// cost what the tile has, used or not (16 projections of 48 rows: 128.4 us by a tile of 64, 124.0 by one of 48).
+int tile_rows(int rows) {
+    if (rows <= 48) return (rows + 15) / 16 * 16;
+    return rows <= (rows + 63) / 64 * 48 ? 48 : 64;
+}
 // K-slices per tile = cluster size: as many as still let every cluster be resident at once (a second wave would
 // double the time); slices and row shares may be ragged
 int choose_splits(const TcScratch& scratch, const GemvArgs& a) {
