@@ -607,12 +607,17 @@ struct Plan {
 };
 
 constexpr int kSmemBudgetAlone = 200 * 1024;   // one CTA per SM: launches of three or more activation rows
+constexpr int kSmemBudgetGateUp = 150 * 1024;  // gate/up of one or two rows
 
 // Shared memory of a launch.  When every tile of a CTA can be resident at once, the last stage is
 // only as long as the longest last tile needs (a CTA's channels rarely fill their last tile).
 bool plan_with_budget(const GemvArgs& a, int rows, size_t budget, Plan& plan);
 
 bool plan_for(const GemvArgs& a, int rows, Plan& plan) {
+    // Gate/up streams twice a projection's weights: four stages ahead of the wait are worth more than room for the next
+    // launch beside them, whose copies start while this one ends (four layers of projections, one row 83.8 -> 79.1 us, two
+    // rows 84.5 -> 81.7; the same slices resident all at once 79.0 and 82.1).  What fits the smaller budget is unchanged.
+    if (rows <= 2 && a.epilogue == EPI_GATE_UP_SILU && plan_with_budget(a, rows, kSmemBudgetGateUp, plan)) return true;
     // one or two rows: room for two CTAs per SM if the shape allows, else the SM to itself
     if (rows <= 2 && plan_with_budget(a, rows, kSmemBudget, plan)) return true;
     return plan_with_budget(a, rows, kSmemBudgetAlone, plan);
