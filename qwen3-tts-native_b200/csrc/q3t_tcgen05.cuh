@@ -101,7 +101,8 @@ __device__ __forceinline__ uint32_t peer_smem(uint32_t local, uint32_t rank) {
     return r;
 }
 // the two halves of cluster_sync(); a thread that has exited counts as arrived
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// (relaxed: what it announces, barriers set up, has its own fence, and a release would wait for loads in flight)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // sixteen bytes to another CTA's shared memory, counted on an mbarrier of that CTA
 __device__ __forceinline__ void st_async_v4(uint32_t addr, float a, float b, float c, float d, uint32_t bar) {
