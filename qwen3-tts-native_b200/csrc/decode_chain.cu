@@ -104,6 +104,7 @@ constexpr int kAttnPartQuads = 2 * kSlices * kRanks * kRowsMost * 88;
 constexpr int kAttnQuads = 2 * kSlices * kRanks * 22;
 constexpr int kLogitQuads = 2 * kCtas * kRowsMost * 3;
 constexpr int kTokenQuads = 2 * kRowsMost;
+constexpr int kAppendedQuads = 2 * kSlices * kRowsMost;
 constexpr int kAtHidden = kPartQuads;
 constexpr int kAtQkv = kAtHidden + kHiddenQuads;
 constexpr int kAtAct = kAtQkv + kQkvQuads;
@@ -111,7 +112,8 @@ constexpr int kAtAttnPart = kAtAct + kActQuads;
 constexpr int kAtAttn = kAtAttnPart + kAttnPartQuads;
 constexpr int kAtLogits = kAtAttn + kAttnQuads;
 constexpr int kAtTokens = kAtLogits + kLogitQuads;
-constexpr int kExchangeQuads = kAtTokens + kTokenQuads;
+constexpr int kAtAppended = kAtTokens + kTokenQuads;
+constexpr int kExchangeQuads = kAtAppended + kAppendedQuads;
 
 __device__ unsigned int g_chain_errors = 0;
 __device__ unsigned int* g_chain_error_sink = nullptr;
@@ -134,6 +136,17 @@ __device__ __forceinline__ Quad get_quad(const Quad* p) {
         : "l"(p)
         : "memory");
     return v;
+}
+
+// A number that stands for plain stores: whoever reads it may read what was stored (by this thread, or by others that
+// met it at a barrier) before it was put.
+__device__ __forceinline__ void put_behind(Quad* p, uint32_t number) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&p->flag), "r"(number) : "memory");
+}
+__device__ __forceinline__ uint32_t get_ahead(const Quad* p) {
+    uint32_t number;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(number) : "l"(&p->flag) : "memory");
+    return number;
 }
 
 struct LayerConst {
@@ -290,7 +303,7 @@ struct Chain {
     uint32_t flips = 0;            // buffer in use, one bit per kind of exchange
     unsigned long long deadline = 0;
 
-    enum Kind { kPart = 0, kHid = 1, kQkv = 2, kAct = 3, kAttnPart = 4, kAttn = 5, kLogits = 6, kTokens = 7 };
+    enum Kind { kPart = 0, kHid = 1, kQkv = 2, kAct = 3, kAttnPart = 4, kAttn = 5, kLogits = 6, kTokens = 7, kAppended = 8 };
 
     __device__ Chain(const ChainArgs& args, unsigned char* s)
         : a(args), smem(s), misc(reinterpret_cast<Misc*>(s + L::AtMisc)), tid(threadIdx.x), lane(threadIdx.x % kWarp),
@@ -317,6 +330,26 @@ struct Chain {
         Quad v[1];
         poll(q, v, flag);
         return v[0];
+    }
+    // The predictor's cache rows are appended by one CTA of the group (rank r for row r) with plain stores and read by the
+    // others at the next position: the appending warp says so when its position is done, the reading ones look before
+    // their first load.  (The talker's rows are read by the next launch.)
+    uint32_t appended_flag = 0;
+    const Quad* appended_at = nullptr;
+    __device__ __forceinline__ void say_appended(bool last) {
+        const int b = flip(kAppended);
+        appended_flag = next_flag();
+        Quad* at = a.exchange + kAtAppended + (b * kSlices + slice) * kRowsMost + min(warp, rows - 1);
+        appended_at = at;
+        if (!last && warp < rows && rank == warp && lane == 0) put_behind(at, appended_flag);
+    }
+    __device__ __forceinline__ void await_appended() {
+        if (lane == 0) {
+            for (uint32_t polls = 0; get_ahead(appended_at) != appended_flag;) {
+                if ((++polls & 31u) == 0u && slow_check()) break;
+            }
+        }
+        __syncwarp();
     }
     // WRAPS: the phase is longer than the ring, so the slot's fill before this one may still be in flight for another
     // warp, and its parity would pass for this one's.  A fill is asked for only once the one before it has been read.
@@ -1094,6 +1127,7 @@ struct Chain {
                     put_values(sum * scale, 32, group_at(kAtQkv, 6, b, rank, warp), flag);
                 }
                 if (walk.any) {
+                    if (!TALKER && index == 0 && pos > 0) await_appended();
                     page::load(f, walk.k + layer_elems, walk.v + layer_elems, TALKER ? older_in(walk.row, walk.page) : pos, lane);
                 }
                 release_full<2>();
@@ -1299,13 +1333,12 @@ struct Chain {
                     return p == 0 ? a.hidden + (size_t)r * S::H : a.projected[p - 1] + (size_t)min(max(misc->token[r], 0), most) * S::H;
                 });
                 if (tid < rows) misc->position[tid] = p;
-                if (p > 0 && warp < rows) __threadfence();      // cache rows appended by other CTAs at earlier positions
                 sync_workers();
                 load_rotations();
 #pragma unroll 1
                 for (int l = 0; l < S::Layers; ++l) layer(l, p, lc, nw, walk);
                 if (p > 0) predictor_head(p, head_scales);
-                if (warp < rows) __threadfence();               // and this CTA's own
+                say_appended(p + 1 == kCodebooks);
             }
             if (ROWS == 1 ? blockIdx.x == 0 && tid == 0 : rank == 0 && slice < rows && tid == 0) {
                 const int r = ROWS == 1 ? 0 : slice;
