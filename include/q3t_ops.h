@@ -412,6 +412,10 @@ QWEN3_TTS_API void q3t_test_fail_launch_after(int32_t launches);
 QWEN3_TTS_API void q3t_test_fail_allocation_after(int32_t allocations);
 QWEN3_TTS_API int32_t q3t_test_report_device_wait_failure(int32_t device_index);
 
+/* Test hook: puts a model whose frames run as a decode chain where it would be after `used` exchanges, the run that
+ * started at number `given_up` having been given up.  No frame may be in flight. */
+QWEN3_TTS_API int32_t q3t_test_set_chain_numbers(Qwen3TtsModelHandle model, uint64_t used, uint32_t given_up);
+
 /* Number of this library's kernels launched so far through frame graphs of the model. */
 QWEN3_TTS_API int32_t q3t_model_kernel_launches(Qwen3TtsModelHandle model, uint64_t* launches,
                                                 char* error, size_t error_capacity);

@@ -1085,6 +1085,10 @@ int32_t q3t_test_report_device_wait_failure(int32_t device_index) {
     return QWEN3_TTS_TALKER_STATUS_OK;
 }
 
+int32_t q3t_test_set_chain_numbers(Qwen3TtsModelHandle model, uint64_t used, uint32_t given_up) {
+    return protect([&] { model_of(model)->set_chain_numbers(used, given_up); }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
+}
+
 uint32_t q3t_kernel_error_count(void) {
     return gemm_tc_error_count() + gemm_wide_error_count() + gemv_mma_error_count() + chain_error_count();
 }

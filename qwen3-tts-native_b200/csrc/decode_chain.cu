@@ -26,7 +26,8 @@
 // Exchanges carry their own flags: a 16-byte store holds three words of data and the exchange's number, the
 // reader polls the data itself (single-copy atomic 128-bit relaxed accesses), so a hand-over is one trip
 // through the L2 and needs no fence or counter.  Buffers alternate by exchange; a CTA can be at most one
-// exchange of a kind ahead of the slowest reader (it has read what that reader wrote after reading).
+// exchange of a kind ahead of the slowest reader (it has read what that reader wrote after reading).  The numbers
+// are 32 bits and are restarted, buffers cleared, long before they would come round (restart_chain_numbers).
 //
 // Weights: at load time every CTA's share is laid out as one contiguous stream in the order the chain uses
 // it, each 1 KB block holding the MMA fragments of 16 rows x 64 K as the lanes read them.  It flows through a
@@ -1510,6 +1511,15 @@ cudaError_t launch_decode_chain(const ChainLaunch& c, cudaStream_t stream) {
     a.table = c.table; a.positions = c.positions; a.kv = c.kv; a.kv_layer_elems = c.kv_layer_elems; a.rope_table = c.rope_table;
     a.exchange = static_cast<Quad*>(c.exchange); a.epoch = c.epoch; a.rows = c.rows; a.eps = kRmsEps;
     return c.talker ? launch_rows<true>(a, stream) : launch_rows<false>(a, stream);
+}
+
+// The last number used becomes 0, the run given up one that no launch reaches before the next restart, and no word of
+// the exchange carries a number that will be used.
+cudaError_t restart_chain_numbers(void* exchange, uint32_t* epoch, cudaStream_t stream) {
+    cudaError_t e = cudaMemsetAsync(exchange, 0, chain_exchange_bytes(), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(epoch, 0, sizeof(uint32_t), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(epoch + 1, 0xff, sizeof(uint32_t), stream);
+    return e;
 }
 
 unsigned int chain_error_count() {

@@ -537,11 +537,18 @@ void Model::build_chain() {
     }
     table(chain.projected, rows.data(), rows.size() * sizeof(const bf16*));
     chain.exchange = DeviceBuffer(chain_exchange_bytes());
-    check_cuda(cudaMemsetAsync(chain.exchange.as<void>(), 0, chain_exchange_bytes(), upload_stream_), "cudaMemset(exchange)");
-    const uint32_t epoch[2] = {1u, 0u};
-    table(chain.epoch, epoch, sizeof(epoch));
+    chain.epoch = DeviceBuffer(2 * sizeof(uint32_t));
+    check_cuda(restart_chain_numbers(chain.exchange.as<void>(), chain.epoch.as<uint32_t>(), upload_stream_), "chain numbers");
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(decode chain)");
     chain.ready = true;
+}
+
+void Model::set_chain_numbers(uint64_t used, uint32_t given_up) {
+    if (!chain.ready) return;
+    const uint32_t epoch[2] = {static_cast<uint32_t>(used), given_up};
+    check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(chain numbers)");
+    check_cuda(cudaMemcpy(chain.epoch.as<void>(), epoch, sizeof(epoch), cudaMemcpyHostToDevice), "cudaMemcpy(chain numbers)");
+    chain.numbers = used;
 }
 
 unsigned int Model::device_errors() const {
@@ -1232,6 +1239,10 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
         check_cuda(cudaMemcpyAsync(w.table.as<void>(), w.host_table, sizeof(FrameTable),
                                    cudaMemcpyHostToDevice, w.stream), "upload frame table");
         check_cuda(cudaEventRecord(w.table_uploaded, w.stream), "cudaEventRecord(table)");
+    }
+    if (chain && (m.chain.numbers += kChainNumbersPerFrame) > kChainNumbers) {
+        check_cuda(restart_chain_numbers(m.chain.exchange.as<void>(), m.chain.epoch.as<uint32_t>(), w.stream), "chain numbers");
+        m.chain.numbers = kChainNumbersPerFrame;
     }
     if (m.use_graphs) {
         Workspace::Graphs& g = frame_graphs(w, m, n, splits, chain);

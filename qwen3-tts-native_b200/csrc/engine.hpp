@@ -199,6 +199,8 @@ public:
     // count when it enqueues work and compares at the host synchronisation point that follows: a
     // frame or prompt during which it advanced cannot be trusted (check_device_errors throws).
     unsigned int device_errors() const;
+    // Test hook: as if `used` numbers had gone by and the run that started at `given_up` had been given up.
+    void set_chain_numbers(uint64_t used, uint32_t given_up);
     void check_device_errors(unsigned int count_at_enqueue) const;
     int prefill_chunk = kMaxPromptRows; // prompt positions per pass (1: one position at a time)
     Workspace* batch_workspace_if_any() {
@@ -226,6 +228,7 @@ public:
         bool ready = false;
         DeviceBuffer streams[2], heads[2], layers[2], head_scales[2];     // 0 predictor, 1 talker
         DeviceBuffer projected_rows, projected, exchange, epoch;
+        uint64_t numbers = 0;           // of exchanges, at most, since they were restarted (guarded as the device's chains are)
     } chain;
     std::mutex mutex;               // pools, workspaces
     int mask_eos = 0;

@@ -293,8 +293,8 @@ struct ChainLaunch {
     KvLayout kv;                              // paged; offsets of layer 0
     long long kv_layer_elems = 0;             // elements between the planes of consecutive layers
     const uint32_t* rope_table = nullptr;
-    void* exchange = nullptr;                 // chain_exchange_bytes(), zeroed once
-    uint32_t* epoch = nullptr;                // two words, {1, 0} at first
+    void* exchange = nullptr;                 // chain_exchange_bytes(); with epoch, set up by restart_chain_numbers
+    uint32_t* epoch = nullptr;                // two words
     int rows = 0;
 };
 constexpr int kChainRows = 8;
@@ -308,6 +308,11 @@ cudaError_t launch_pack_layer(bool talker, int layer, const int8_t* qkv, const i
                               uint8_t* stream_base, cudaStream_t stream);
 cudaError_t launch_pack_head(bool talker, int index, const int8_t* head, uint8_t* heads_base, cudaStream_t stream);
 cudaError_t launch_decode_chain(const ChainLaunch& chain, cudaStream_t stream);
+// Exchanges are numbered through all launches of a model in 32 bits.  Numbers that came round would meet words of rows
+// that have not been used since, and the number of a run that was given up: before kChainNumbers are used they start again.
+constexpr uint64_t kChainNumbers = 1ull << 31;
+constexpr uint64_t kChainNumbersPerFrame = 1024;     // at most: 16 x (5 x 6 + 1) + 15 x 2 by the predictor, 28 x 8 by the talker
+cudaError_t restart_chain_numbers(void* exchange, uint32_t* epoch, cudaStream_t stream);
 unsigned int chain_error_count();
 
 // Sampler over table rows: row r reads logits + r*logits_stride.  talker != 0: reserved

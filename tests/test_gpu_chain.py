@@ -87,3 +87,18 @@ def test_draws_inside_and_outside_the_chain(q3t, model, config):
     for positions in ([9], [9, 40, 3]):
         for a, b in zip(frame(q3t, model, positions, 1, predictor), frame(q3t, model, positions, 0, predictor)):
             assert np.array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("used,given_up", [(2 ** 31 - 1024, 2 ** 32 - 1), (2 ** 31 - 1023, 2 ** 31 - 1023), (2 ** 32 - 300, 2 ** 32 - 300)])
+def test_exchange_numbers_start_again(q3t, model, used, given_up):
+    """Exchanges are numbered in 32 bits.  At the last frame before a restart, at the first behind it, and where numbers
+    would come round within a frame; the latter two where the run that was once given up bore the next run's number."""
+    import ctypes as C
+    lib = q3t.library()
+    lib.q3t_test_set_chain_numbers.argtypes = [C.c_void_p, C.c_uint64, C.c_uint32]
+    want = frame(q3t, model, [40, 9, 700], 1, frames=3)
+    assert lib.q3t_test_set_chain_numbers(model._handle, used, given_up) == 0
+    got = frame(q3t, model, [40, 9, 700], 1, frames=3)
+    for a, b in zip(got, want):
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2]) and a[4] == b[4]
+    assert lib.q3t_kernel_error_count() == 0
