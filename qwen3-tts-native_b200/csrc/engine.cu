@@ -489,6 +489,9 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
 
 void Model::build_chain() {
     if (!chain_available() || predictor.head_dim != 128) return;
+    // The streams are made from the weights as they lie there now: what a caller has enqueued on streams of its own to fill
+    // adopted storage has to be done.
+    check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(adopted weights)");
     auto table = [](DeviceBuffer& b, const void* host, size_t bytes) {
         b = DeviceBuffer(bytes);
         check_cuda(cudaMemcpy(b.as<void>(), host, bytes, cudaMemcpyHostToDevice), "cudaMemcpy(chain table)");

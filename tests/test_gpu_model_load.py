@@ -1,0 +1,60 @@
+"""What a model makes of its weights when it is finalised, and what it does without when memory is short."""
+import importlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def replica_of(q3t, model, names, delay_cycles=0):
+    """A second model, not yet finalised, whose storage is being filled from the first one's on torch's stream."""
+    import torch
+    dp = importlib.import_module("qwen3-tts-native_b200.dp")
+    replica = q3t.NativeTalkerModel.create(0)
+    if delay_cycles:
+        torch.cuda._sleep(delay_cycles)
+    for name in names:
+        for (src, n), (dst, _) in zip(dp.image_spans(model.tensor_image(name)), dp.image_spans(replica.tensor_image(name))):
+            dp.device_bytes(dst, n, 0).copy_(dp.device_bytes(src, n, 0))
+        replica.adopt_tensor(name)
+    return replica
+
+
+def frames(q3t, model, sessions=1, count=2, seed=11):
+    """(codes, next tokens, hidden row) of `count` frames of sessions that start on synthetic contexts."""
+    model.set_option("mask_eos", 1)
+    ss = []
+    for i in range(sessions):
+        s = model.create_session(128, seed + i)
+        s.talker_sampling = q3t.SamplingConfig(True, 50, 0.9, 0.9, 1.05)
+        s.predictor_sampling = q3t.SamplingConfig(True, 50, 1.0, 0.9, 1.0)
+        s.synthetic_prefill(40 + i, seed + i)
+        ss.append(s)
+    out = []
+    for f in range(count):
+        if sessions == 1:
+            ss[0].next_frame(7 + f)
+        else:
+            for p in model.batch_begin_device_frames(ss, [7 + f] * sessions):
+                p.finish_without_consumer()
+        out += [(s.current_semantic_token, *(np.array(x) for x in s.read_state()[:2])) for s in ss]
+    for s in ss:
+        s.close()
+    return out
+
+
+def same(a, b):
+    return all(x[0] == y[0] and np.array_equal(x[1], y[1]) and np.array_equal(x[2], y[2]) for x, y in zip(a, b))
+
+
+def test_weights_that_are_still_being_filled(q3t, gpu_model, checkpoint):
+    """Adopted storage is filled by work that the caller has enqueued and not waited for: finalize makes its streams of the
+    weights that will be there, not of what lies there when it is called."""
+    want = frames(q3t, gpu_model), frames(q3t, gpu_model, 3)
+    replica = replica_of(q3t, gpu_model, checkpoint.keys(), delay_cycles=1_000_000_000)
+    try:
+        replica.finalize()
+        assert same(frames(q3t, replica), want[0]) and same(frames(q3t, replica, 3), want[1])
+    finally:
+        replica.close()
