@@ -25,6 +25,8 @@ constexpr int kPredictorSequence = 16;
 constexpr int kEos = 2150;
 constexpr uint32_t kPhaseCreated = 0, kPhaseReady = 1, kPhasePrefilled = 2, kPhaseEnded = 3;
 
+constexpr size_t kChainLeaves = 4ull << 30;      // device memory that has to stay free behind the decode chain's image
+
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 int env_int(const char* name, int fallback) {
@@ -479,7 +481,13 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
         predictor_rope = predictor_rope_.as<uint32_t>();
     }
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(rope tables)");
-    build_chain();
+    try {
+        build_chain();
+    } catch (const std::bad_alloc&) {
+        // frames run launch by launch without it
+        cudaStreamSynchronize(upload_stream_);
+        chain = DecodeChain();
+    }
     talker_pool.reset(new KvPool(talker.layers, talker.kv_width, 8));
     predictor_pool.reset(new KvPool(predictor.layers, predictor.kv_width, 6));
     finalized_ = true;
@@ -489,6 +497,12 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
 
 void Model::build_chain() {
     if (!chain_available() || predictor.head_dim != 128) return;
+    // The chain is a second image of the decode matrices, for speed alone: it is not to take the memory that sessions and
+    // prompts need.
+    size_t free_bytes = 0, total_bytes = 0;
+    check_cuda(cudaMemGetInfo(&free_bytes, &total_bytes), "cudaMemGetInfo");
+    const size_t wanted = chain_stream_bytes(false) + chain_stream_bytes(true) + chain_head_bytes(false) + chain_head_bytes(true);
+    if (free_bytes < wanted + kChainLeaves) return;
     // The streams are made from the weights as they lie there now: what a caller has enqueued on streams of its own to fill
     // adopted storage has to be done.
     check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(adopted weights)");

@@ -58,3 +58,26 @@ def test_weights_that_are_still_being_filled(q3t, gpu_model, checkpoint):
         assert same(frames(q3t, replica), want[0]) and same(frames(q3t, replica, 3), want[1])
     finally:
         replica.close()
+
+
+def test_without_memory_for_the_chain(q3t, gpu_model, checkpoint):
+    """The decode chain's second image of the weights is optional: where it cannot be allocated the model loads all the same and
+    its frames run launch by launch (hundreds of kernels instead of a dozen), with the codes that the chain gives."""
+    lib = q3t.library()
+    want = frames(q3t, gpu_model, 2, count=1)
+    replica = replica_of(q3t, gpu_model, checkpoint.keys())
+    try:
+        lib.q3t_test_fail_allocation_after(6)          # behind what every model needs (the table of embeddings, the rotations)
+        replica.finalize()
+        lib.q3t_test_fail_allocation_after(0)
+        before = replica.kernel_launches()
+        got = frames(q3t, replica, 2, count=1)
+        assert replica.kernel_launches() - before > 300
+        before = gpu_model.kernel_launches()
+        frames(q3t, gpu_model, 2, count=1)
+        assert gpu_model.kernel_launches() - before < 30
+        for a, b in zip(got, want):
+            assert np.array_equal(a[2], b[2])
+    finally:
+        lib.q3t_test_fail_allocation_after(0)
+        replica.close()
