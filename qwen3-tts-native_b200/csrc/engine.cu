@@ -151,16 +151,16 @@ uint64_t KvPool::page_bytes() const { return (uint64_t)layers_ * 2 * page_elems_
 
 // ------------------------------------------------------------------ Workspace
 
-Workspace::Workspace(int capacity_, int device_, int rows) : capacity(capacity_), device(device_) {
+Workspace::Workspace(int capacity_, int device_, int rows_) : capacity(capacity_), rows(std::max(capacity_, rows_)), device(device_) {
     check_cuda(cudaSetDevice(device), "cudaSetDevice(workspace)");
     const size_t e = sizeof(bf16);
-    size_t c = std::max(capacity, rows);
+    size_t c = rows;
     const size_t one = capacity;
     // one allocation: a session's workspace is made when the session is, and fourteen of them were half of that
     const std::pair<DeviceBuffer*, size_t> parts[] = {
         {&table, sizeof(FrameTable)}, {&counters, one * 16 * sizeof(unsigned int)},
         {&hidden, c * 2048 * e}, {&qkv, c * 4096 * e}, {&attention, c * 2048 * e}, {&gate, c * 6144 * e},
-        {&logits, c * kTalkerVocab * e}, {&x_in, c * 2048 * e}, {&projection, c * 2048 * e}, {&normalized, c * 2048 * e},
+        {&logits, one * kTalkerVocab * e}, {&x_in, c * 2048 * e}, {&projection, c * 2048 * e}, {&normalized, c * 2048 * e},
         {&prompt_positions, c * sizeof(int)}, {&talker_pages, one * kMaxPagesPerRow * sizeof(int)},
         {&predictor_pages, one * sizeof(int)}, {&predictor_positions, (size_t)kPredictorSequence * kMaxRows * sizeof(int)}};
     size_t total = 0;
@@ -587,7 +587,13 @@ Workspace& Model::batch_workspace() {
 
 Workspace& Model::prefill_workspace() {
     std::lock_guard<std::mutex> lock(mutex);
-    if (!prefill_) prefill_.reset(new Workspace(kMaxRows, device_, kMaxPromptRows));
+    if (!prefill_) {
+        try {
+            prefill_.reset(new Workspace(kMaxRows, device_, kMaxPromptRows));
+        } catch (const std::bad_alloc&) {
+            prefill_.reset(new Workspace(kMaxRows, device_));       // 3 MB instead of 85: prompts in passes of 64
+        }
+    }
     return *prefill_;
 }
 
@@ -1480,12 +1486,13 @@ void Session::prefill(const int32_t* text_ids, const int32_t* codec_ids, int cou
     const ParityHooks hooks = ParityHooks::from_environment(nullptr);
     // Passes above kMaxRows exist on the tensor-core kernels only; the parity modes and hooks keep to it.
     const int most = tc_min_rows() <= kMaxRows && attention_mode() != 0 && !hooks.active() ? kMaxPromptRows : kMaxRows;
-    const int chunk = std::min(std::max(m.prefill_chunk, 1), most);
+    int chunk = std::min(std::max(m.prefill_chunk, 1), most);
     // the parity hooks observe the chunked pass (they synchronise, so nothing of it may be captured)
     const bool chunked = (chunk > 1 && count > 1) || hooks.active();
     std::unique_lock<std::mutex> one_prompt(m.prefill_mutex, std::defer_lock);
     if (chunked) one_prompt.lock();
     Workspace& w = chunked ? m.prefill_workspace() : *solo_;
+    if (chunked) chunk = std::min(chunk, w.rows);
     position_ = 0;
     generated_ = 0;
     const unsigned int errors_before = m.device_errors();

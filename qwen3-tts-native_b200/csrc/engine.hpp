@@ -130,6 +130,7 @@ struct Workspace {
     uint64_t bytes() const;
 
     int capacity;
+    int rows;
     int device;
     cudaStream_t stream = nullptr;
     DeviceBuffer arena;              // what the buffers below but `scratch` lie in: one allocation

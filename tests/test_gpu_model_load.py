@@ -60,7 +60,7 @@ def test_weights_that_are_still_being_filled(q3t, gpu_model, checkpoint):
         replica.close()
 
 
-def test_without_memory_for_the_chain(q3t, gpu_model, checkpoint):
+def test_without_memory_for_the_chain_and_for_long_passes(q3t, gpu_model, checkpoint):
     """The decode chain's second image of the weights is optional: where it cannot be allocated the model loads all the same and
     its frames run launch by launch (hundreds of kernels instead of a dozen), with the codes that the chain gives."""
     lib = q3t.library()
@@ -78,6 +78,29 @@ def test_without_memory_for_the_chain(q3t, gpu_model, checkpoint):
         assert gpu_model.kernel_launches() - before < 30
         for a, b in zip(got, want):
             assert np.array_equal(a[2], b[2])
+
+        # likewise the workspace of prompts in one pass: without it they run in passes of 64
+        rng = np.random.default_rng(3)
+        text, codec = [int(t) for t in rng.integers(0, 151936, size=150)], [-1] * 150
+
+        def prompt(model):
+            s = model.create_session(160, 5)
+            s.prefill(text, codec)
+            out = s.current_semantic_token, s.read_state()[0], s.read_kv(27, 0, 150)
+            s.close()
+            return out
+
+        gpu_model.set_option("prefill_chunk", 64)
+        want = prompt(gpu_model)
+        gpu_model.set_option("prefill_chunk", 2048)
+        s = replica.create_session(160, 5)
+        lib.q3t_test_fail_allocation_after(1)
+        s.prefill(text, codec)
+        lib.q3t_test_fail_allocation_after(0)
+        s.close()
+        got = prompt(replica)
+        assert got[0] == want[0] and np.array_equal(got[1], want[1]) and all(np.array_equal(a, b) for a, b in zip(got[2], want[2]))
     finally:
+        gpu_model.set_option("prefill_chunk", 2048)
         lib.q3t_test_fail_allocation_after(0)
         replica.close()
