@@ -1123,13 +1123,15 @@ __global__ void __launch_bounds__(kAttnThreads, kWalkCtas) decode_attention_walk
         for (int p = 0; p < kPages; ++p) mx = fmaxf(mx, fmaxf(fmaxf(pr[p][0][0], pr[p][0][1]), fmaxf(pr[p][1][0], pr[p][1][1])));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        // a chunk whose scores are all -inf has probabilities of zero and counts for nothing in the merge
+        const float top = mx == -INFINITY ? 0.0f : mx;
         // probabilities as hi + lo bf16, 2^-16 from the fp32 ones
         uint32_t ph[kPages][2], pl[kPages][2];
 #pragma unroll
         for (int p = 0; p < kPages; ++p)
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                const float p0 = expf(pr[p][nt][0] - mx), p1 = expf(pr[p][nt][1] - mx);
+                const float p0 = expf(pr[p][nt][0] - top), p1 = expf(pr[p][nt][1] - top);
                 lsum += p0;
                 lsum += p1;
                 ph[p][nt] = pack_bf16x2(p0, p1);

@@ -289,3 +289,20 @@ def test_walk_edges(orc, ops, rows):
     fused = ops.attention_ex(qkv, pos, qh, kvh, hd, pages=slabs, page_table=table, slab_shift=6, q_norm_w=ones, k_norm_w=ones,
                              fused=True, q_stride=qw + 2 * kvw, new_stride=qw + 2 * kvw)
     assert np.array_equal(fused["out"], plain["out"])
+
+
+@pytest.mark.parametrize("length", [65, 128, 190, 200])
+@pytest.mark.parametrize("masked", [(0, 64), (64, 128), (3, 60)])
+def test_scores_of_minus_infinity(orc, ops, length, masked):
+    """Keys whose products overflow to -inf have no weight, also where they fill a 64-token chunk, the first, a middle or the
+    last one; what is left is compared with the oracle."""
+    qh, kvh, hd, cap = 16, 8, 128, 256
+    rng = np.random.default_rng(length)
+    q, k, v, pos = make(orc, 31, 2, qh, kvh, hd, cap, np.array([length - 1, length], dtype=np.int32))
+    q = bf(orc, -1e20 * (1 + rng.random((2, qh * hd))))
+    k = bf(orc, rng.standard_normal(k.shape) * 1e-20)
+    k[:, masked[0]:masked[1]] = bf(orc, np.full(hd, 1e20)).reshape(-1)[0]
+    got = ops.attention_ex(q, pos, qh, kvh, hd, k=k, v=v, want_f32=True)
+    want, want32 = orc.attention(q, k, v, pos, qh, kvh, hd, fast=True, want_f32=True)
+    assert np.isfinite(want32).all()
+    check(orc, got["out"], got["f32"], want, want32, hd)
