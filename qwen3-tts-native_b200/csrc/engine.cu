@@ -94,6 +94,20 @@ DeviceBuffer::~DeviceBuffer() {
     if (ptr_ != nullptr && owned_) cudaFree(ptr_);
 }
 
+namespace {
+// Clears (source null) or fills device memory before it returns.  cudaMemset and cudaMemcpy are of no use for that: they may
+// return before their work on the default stream is done, which the engine's streams do not wait for.
+void set_now(void* destination, const void* source, size_t bytes, const char* what) {
+    cudaStream_t s = nullptr;
+    check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), what);
+    cudaError_t e = source == nullptr ? cudaMemsetAsync(destination, 0, bytes, s)
+                                      : cudaMemcpyAsync(destination, source, bytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+    check_cuda(e, what);
+}
+}  // namespace
+
 // ------------------------------------------------------------------ KvPool
 
 KvPool::KvPool(int layers, int kv_width, int slab_shift)
@@ -101,7 +115,7 @@ KvPool::KvPool(int layers, int kv_width, int slab_shift)
       page_elems_((long long)kPageTokens * kv_width),
       plane_elems_(((long long)1 << slab_shift) * kPageTokens * kv_width),
       slab_table_(kMaxSlabs * sizeof(bf16*)) {
-    check_cuda(cudaMemset(slab_table_.as<void>(), 0, kMaxSlabs * sizeof(bf16*)), "cudaMemset(slab table)");
+    set_now(slab_table_.as<void>(), nullptr, kMaxSlabs * sizeof(bf16*), "clear slab table");
 }
 
 void KvPool::add_slab() {
@@ -110,8 +124,7 @@ void KvPool::add_slab() {
     DeviceBuffer slab(bytes);
     bf16* base = slab.as<bf16>();
     const int index = static_cast<int>(slabs_.size());
-    check_cuda(cudaMemcpy(slab_table_.as<bf16*>() + index, &base, sizeof(base), cudaMemcpyHostToDevice),
-               "cudaMemcpy(slab table)");
+    set_now(slab_table_.as<bf16*>() + index, &base, sizeof(base), "fill slab table");
     slabs_.push_back(std::move(slab));
     const int per = 1 << slab_shift_;
     for (int i = per - 1; i >= 0; --i) free_.push_back(index * per + i);
@@ -179,13 +192,13 @@ Workspace::Workspace(int capacity_, int device_, int rows_) : capacity(capacity_
                                  cudaHostAllocDefault), "cudaHostAlloc(frame table, page tables)");
         std::memset(host_table, 0, sizeof(FrameTable));
         host_pages = reinterpret_cast<int*>(reinterpret_cast<char*>(host_table) + host_bytes);
-        check_cuda(cudaMemset(table.as<void>(), 0, align_up(table.bytes(), 1024) + counters.bytes()),
+        check_cuda(cudaMemsetAsync(table.as<void>(), 0, align_up(table.bytes(), 1024) + counters.bytes(), stream),
                    "cudaMemset(frame table, counters)");
         std::vector<int> positions((size_t)kPredictorSequence * kMaxRows);
         for (int p = 0; p < kPredictorSequence; ++p)
             for (int r = 0; r < kMaxRows; ++r) positions[(size_t)p * kMaxRows + r] = p;
-        check_cuda(cudaMemcpy(predictor_positions.as<void>(), positions.data(),
-                              positions.size() * sizeof(int), cudaMemcpyHostToDevice),
+        check_cuda(cudaMemcpyAsync(predictor_positions.as<void>(), positions.data(),
+                                   positions.size() * sizeof(int), cudaMemcpyHostToDevice, stream),
                    "cudaMemcpy(predictor positions)");
         check_cuda(cudaEventCreate(&predictor_start), "cudaEventCreate");
         check_cuda(cudaEventCreate(&predictor_stop), "cudaEventCreate");
@@ -464,9 +477,7 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(upload)");
     staging_ = DeviceBuffer();
     embedding_ptrs_ = DeviceBuffer(kResidualCodebooks * sizeof(const bf16*));
-    check_cuda(cudaMemcpy(embedding_ptrs_.as<void>(), predictor_embeddings.data(),
-                          kResidualCodebooks * sizeof(const bf16*), cudaMemcpyHostToDevice),
-               "cudaMemcpy(embedding table)");
+    set_now(embedding_ptrs_.as<void>(), predictor_embeddings.data(), kResidualCodebooks * sizeof(const bf16*), "embedding table");
     predictor_embedding_table = embedding_ptrs_.as<const bf16*>();
     talker_rope_ = DeviceBuffer((size_t)kRopePositions * (talker.head_dim / 2) * sizeof(uint32_t));
     check_cuda(launch_build_rope_table(talker_rope_.as<uint32_t>(), kRopePositions, talker.head_dim,
@@ -508,7 +519,7 @@ void Model::build_chain() {
     check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(adopted weights)");
     auto table = [](DeviceBuffer& b, const void* host, size_t bytes) {
         b = DeviceBuffer(bytes);
-        check_cuda(cudaMemcpy(b.as<void>(), host, bytes, cudaMemcpyHostToDevice), "cudaMemcpy(chain table)");
+        set_now(b.as<void>(), host, bytes, "chain table");
     };
     for (int t = 0; t < 2; ++t) {
         const bool big = t == 1;
@@ -564,7 +575,7 @@ void Model::set_chain_numbers(uint64_t used, uint32_t given_up) {
     if (!chain.ready) return;
     const uint32_t epoch[2] = {static_cast<uint32_t>(used), given_up};
     check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(chain numbers)");
-    check_cuda(cudaMemcpy(chain.epoch.as<void>(), epoch, sizeof(epoch), cudaMemcpyHostToDevice), "cudaMemcpy(chain numbers)");
+    set_now(chain.epoch.as<void>(), epoch, sizeof(epoch), "chain numbers");
     chain.numbers = used;
 }
 
@@ -1078,7 +1089,7 @@ Session::Session(std::shared_ptr<Model> model, int max_sequence_length, uint64_t
         const size_t off_history = align_up(off_hidden + 2048 * sizeof(bf16), 256);
         const size_t total = off_history + (size_t)max_seq_ * sizeof(int);
         state_ = DeviceBuffer(total);
-        check_cuda(cudaMemset(state_.as<void>(), 0, total), "cudaMemset(session state)");
+        check_cuda(cudaMemsetAsync(state_.as<void>(), 0, total, stream_), "cudaMemset(session state)");
         char* base = state_.as<char>();
         d_frame_tokens_ = reinterpret_cast<int*>(base + off_tokens);
         d_frame_codes_ = reinterpret_cast<unsigned short*>(base + off_codes);
