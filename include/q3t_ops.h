@@ -356,8 +356,10 @@ QWEN3_TTS_API int32_t q3t_launch_sample_logits_at(
 
 /* Options: "mask_eos" (1: the talker sampler also masks EOS, for synthetic weights whose
  * logits would otherwise end a run at random), "use_graphs" (0: launch kernels one by one),
- * "decode_chain" (1, default: frames of up to 8 sessions run as two cooperative launches; 0: launch by
- * launch; with "use_graphs" 0 always launch by launch),
+ * "decode_chain" (1, default: frames of up to 8 sessions run as two cooperative launches, or, while the
+ * device is at work on a prompt, on larger frames or on three and more sessions stepped alone, launch by launch with
+ * the same results to the bit; 2: always the latter; 0: launch by launch with the operators' attention; with
+ * "use_graphs" 0 always as with 0),
  * "batch_host_codes" (1: lockstep batches also mirror each frame's 16 codes to host memory),
  * "gemv_mode" (process-wide, see q3t_set_gemv_mode),
  * "attention_mode" (process-wide, see q3t_set_attention_mode),

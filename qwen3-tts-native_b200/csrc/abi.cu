@@ -1014,7 +1014,7 @@ int32_t q3t_model_set_option(Qwen3TtsModelHandle model, const char* key, int32_t
         } else if (std::strcmp(key, "batch_host_codes") == 0) {
             m->batch_host_codes = value != 0;
         } else if (std::strcmp(key, "decode_chain") == 0) {
-            m->use_chain = value != 0;
+            m->use_chain = value < 0 || value > 2 ? 1 : value;
         } else if (std::strcmp(key, "prefill_chunk") == 0) {
             m->prefill_chunk = value < 1 ? 1 : (value > kMaxPromptRows ? kMaxPromptRows : value);
         } else if (std::strcmp(key, "tc_min_rows") == 0) {

@@ -801,23 +801,14 @@ struct Chain {
             const int r = job / 3, h = job % 3;
             if (job >= 3 * rows || !needs(r, h == 2)) continue;
             const bf16* src = qkv + r * 512 + h * 128;
-            const uint32_t cs0 = cs[i][0], cs1 = cs[i][1];
-            float x[4], sq[4];
+            float x[4], o[4];
+            bf16 w[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 x[j] = bf2f(src[lane + 32 * j]);
-                sq[j] = fmaf(x[j], x[j], 0.0f);
+                w[j] = h == 2 ? hn.k[j] : hn.q[j];
             }
-            float c = (sq[0] + sq[2]) + (sq[1] + sq[3]);
-            c = warp_sum_down(c);
-            c = __shfl_sync(0xffffffffu, c, 0);
-            const float inv = rsqrtf(c / 128.0f + a.eps);
-            float y[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) y[j] = rbf(rbf(x[j] * inv) * bf2f(h == 2 ? hn.k[j] : hn.q[j]));
-            float o[4];
-            rope_pair_cs(y[0], y[2], bf_lo(cs0), bf_hi(cs0), o[0], o[2]);
-            rope_pair_cs(y[1], y[3], bf_lo(cs1), bf_hi(cs1), o[1], o[3]);
+            page::rotate(x, w, cs[i][0], cs[i][1], a.eps, o);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (h == 2) knew[r * 128 + lane + 32 * j] = f2bf(o[j]);
@@ -863,27 +854,23 @@ struct Chain {
         sync_workers();
     }
 
-    // Talker: kBlock consecutive pages of a row go to one CTA, block after block over the group's 16 CTAs ("slots",
-    // counted from a CTA that depends on the row, so that the rows of a batch spread), and there to classes, one page
-    // to a class at first; a class is walked by one warp.  The classes and then the slots are merged in order.  The
-    // grouping of a row's pages depends on its length only.  (Blocks: the fewer CTAs hold parts of a row, the fewer
-    // partial results everybody has to collect; the more pages a CTA has to fetch.)
-    static constexpr int kBlock = 2;
-    static constexpr int kPageStep = 8 * kRanks;         // from a class's page to its next
+    // Talker: the slots of a row (q3t_attention_page.cuh) are the group's 16 CTAs, counted from one that depends on the
+    // row, so that the rows of a batch spread.  (Blocks: the fewer CTAs hold parts of a row, the fewer partial results
+    // everybody has to collect; the more pages a CTA has to fetch.)
+    static_assert(kRanks == page::kSlots && kWorkers / kWarp == page::kClasses, "a CTA per slot, a warp per class");
     struct Walk {
         int row, page;
         bf16 *k, *v;          // its rows in layer 0
         bool any;
     };
     __device__ __forceinline__ int pages_of(int row) { return misc->position[row] / kPageTokens + 1; }
-    __device__ __forceinline__ int slots_of(int row) { return min(kRanks, (pages_of(row) + kBlock - 1) / kBlock); }
+    __device__ __forceinline__ int slots_of(int row) { return page::slots_of(pages_of(row)); }
     __device__ __forceinline__ int my_slot(int row) { return (rank - 2 * row) & (kRanks - 1); }
     __device__ __forceinline__ int rank_of(int row, int slot) { return (slot + 2 * row) & (kRanks - 1); }
-    __device__ __forceinline__ int class_page(int slot, int cls) { return kBlock * (slot + kRanks * (cls / kBlock)) + cls % kBlock; }
     __device__ __forceinline__ Walk first_page() {
         Walk w{0, 0, nullptr, nullptr, false};
         for (w.row = 0; w.row < rows; ++w.row) {
-            w.page = class_page(my_slot(w.row), (warp - w.row) & 7);
+            w.page = page::class_page(my_slot(w.row), (warp - w.row) & 7);
             if (w.page < pages_of(w.row)) {
                 w.k = page_at(a.kv, w.row, w.page, false);
                 w.v = page_at(a.kv, w.row, w.page, true);
@@ -903,20 +890,17 @@ struct Chain {
         float* out_s = l_s + ROWS * 8 * 2;                                        // [row][head][132]: max, sum, weighted V
         bf16* att = reinterpret_cast<bf16*>(smem + L::AtAtt);
         const float scale = rsqrtf(128.0f);
-        rotate_heads(hn, [&](int r, bool key) { return key ? (pages_of(r) - 1) / kBlock % kRanks == my_slot(r) : my_slot(r) < slots_of(r); });
+        rotate_heads(hn, [&](int r, bool key) { return key ? (pages_of(r) - 1) / page::kBlock % kRanks == my_slot(r) : my_slot(r) < slots_of(r); });
         if (w0.any) {
             bool loaded = true;
 #pragma unroll 1
             for (int row = w0.row; row < rows; ++row) {
                 const int np = pages_of(row), cls = (warp - row) & 7;
-                float m = -INFINITY, l = 0.0f, o[8][4];
-#pragma unroll
-                for (int x = 0; x < 8; ++x)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) o[x][e] = 0.0f;
-                const int first = class_page(my_slot(row), cls);
+                page::Running run;
+                page::start(run);
+                const int first = page::class_page(my_slot(row), cls);
 #pragma unroll 1
-                for (int pg = first; pg < np; pg += kPageStep) {
+                for (int pg = first; pg < np; pg += page::kPageStep) {
                     bf16 *kp = w0.k + layer_elems, *vp = w0.v + layer_elems;
                     if (!loaded) {
                         kp = page_at(a.kv, row, pg, false) + layer_elems;
@@ -932,39 +916,9 @@ struct Chain {
                     float mp, lp, op[8][4];
                     page::attend(f, reinterpret_cast<const float*>(smem + L::AtQ) + row * 256, min(kPageTokens, t_new + 1), scale, lane,
                                  mp, lp, op);
-                    // the first page replaces nothing: m is -inf, its factor 0 and the page's own 1, exactly
-                    const float top = fmaxf(m, mp);
-                    const float fo = pg == first ? 0.0f : expf(m - top), fn = expf(mp - top);
-                    l = pg == first ? lp : l * fo + lp * fn;
-                    m = top;
-                    // columns 2 tig and 2 tig + 1 are heads; only tig = 0 holds real ones
-                    const float fo0 = __shfl_sync(0xffffffffu, fo, 0), fo1 = __shfl_sync(0xffffffffu, fo, 4);
-                    const float fn0 = __shfl_sync(0xffffffffu, fn, 0), fn1 = __shfl_sync(0xffffffffu, fn, 4);
-#pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        o[x][0] = fmaf(o[x][0], fo0, op[x][0] * fn0);
-                        o[x][2] = fmaf(o[x][2], fo0, op[x][2] * fn0);
-                        o[x][1] = fmaf(o[x][1], fo1, op[x][1] * fn1);
-                        o[x][3] = fmaf(o[x][3], fo1, op[x][3] * fn1);
-                    }
+                    page::add(run, pg == first, mp, lp, op);
                 }
-                if (first < np && (lane & 3) == 0) {
-                    const int gid = lane >> 2;
-                    if (gid < 2) {
-                        m_s[(row * 8 + cls) * 2 + gid] = m;
-                        l_s[(row * 8 + cls) * 2 + gid] = l;
-                    }
-                    float* d0 = acc_s + (row * 8 + cls) * 256 + 8 * gid;
-#pragma unroll
-                    for (int c = 0; c < 2; ++c)
-#pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            const int e = 2 * half + c;
-                            float4* d4 = reinterpret_cast<float4*>(d0 + 128 * c + 64 * half);
-                            d4[0] = make_float4(o[0][e], o[1][e], o[2][e], o[3][e]);
-                            d4[1] = make_float4(o[4][e], o[5][e], o[6][e], o[7][e]);
-                        }
-                }
+                if (first < np) page::put_class(run, acc_s + (row * 8 + cls) * 256, m_s + (row * 8 + cls) * 2, l_s + (row * 8 + cls) * 2, lane);
             }
         }
         sync_workers();
@@ -974,16 +928,8 @@ struct Chain {
         for (int r = 0; r < rows; ++r) {
             const int np = pages_of(r), slot = my_slot(r);
             if (slot >= slots_of(r)) continue;
-            int classes = 1;
-            while (classes < 8 && class_page(slot, classes) < np) ++classes;
-            float M = -INFINITY;
-            for (int c = 0; c < classes; ++c) M = fmaxf(M, m_s[(r * 8 + c) * 2 + g]);
-            float Lsum = 0.0f, A = 0.0f;
-            for (int c = 0; c < classes; ++c) {
-                const float fac = expf(m_s[(r * 8 + c) * 2 + g] - M);
-                Lsum = fmaf(l_s[(r * 8 + c) * 2 + g], fac, Lsum);
-                A = fmaf(acc_s[(r * 8 + c) * 256 + g * 128 + d], fac, A);
-            }
+            float M, Lsum, A;
+            page::merge_classes(acc_s + r * 8 * 256, m_s + r * 8 * 2, l_s + r * 8 * 2, slot, np, g, d, M, Lsum, A);
             float* dst = out_s + (r * 2 + g) * 132;
             if (d == 0) {
                 dst[0] = M;
@@ -1005,18 +951,7 @@ struct Chain {
         }
         float* gathered = reinterpret_cast<float*>(smem + L::AtX);              // [rank][132] of a head
         auto fold = [&](const float* from, int stride, int ranks, int dim) {
-            // lane k holds what the fold needs of CTA k: its factor and sum
-            const float mine = lane < ranks ? from[lane * stride] : -INFINITY;
-            const float sum = lane < ranks ? from[lane * stride + 1] : 0.0f;
-            const float fac = expf(mine - warp_max_xor(mine));
-            float Lsum = 0.0f, A = 0.0f;
-#pragma unroll 4
-            for (int k = 0; k < ranks; ++k) {
-                const float fk = __shfl_sync(0xffffffffu, fac, k);
-                Lsum = fmaf(__shfl_sync(0xffffffffu, sum, k), fk, Lsum);
-                A = fmaf(from[k * stride + 2 + dim], fk, A);
-            }
-            return A * (1.0f / Lsum);
+            return page::fold([&](int k, int n) { return from[k * stride + n]; }, ranks, dim, lane);
         };
         sync_workers();        // out_s has been read; the area is written again below
         if constexpr (ROWS == 1) {

@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstddef>
 #include <cstdlib>
@@ -62,6 +63,158 @@ void check_launch(cudaError_t status, const char* what) {
     if (status == cudaSuccess && countdown_fires(g_fail_launch)) status = cudaErrorLaunchOutOfResources;
     check_cuda(status, what);
 }
+
+// ------------------------------------------------------------------ what runs on a device at the moment
+
+namespace {
+
+// Chains wait between their CTAs, so two of them must not share the GPU's SMs: the chains of a device run one after the
+// other, whatever streams (and models) they come from.  And a chain takes 128 SMs whole: launches of other frames or of a
+// prompt beside it get on between two chains only (a frame of 23 sessions beside one session stepped alone took 25 ms
+// instead of 6, a prompt of 64 positions 10 ms instead of 3.5).  So a frame that could run as a chain is made launch by
+// launch, with the same bits, while the device is at work on something that is no chain.
+//
+// Frames are known by the workspace that they run on: its last frame's end is the event talker_stop.
+struct Traffic {
+    enum Kind { kChain, kInPlaceOfChain, kOther };
+    struct Entry {
+        const Workspace* workspace;
+        int rows;
+        Kind kind;
+        bool enqueued;          // the whole frame is on its stream, talker_stop behind it
+    };
+    std::mutex mutex;
+    std::vector<Entry> entries;
+    cudaEvent_t chain_done = nullptr;
+    cudaStream_t chain_stream = nullptr;
+    std::chrono::steady_clock::time_point crowd_until{}, shared_until{};
+
+    Entry* find(const Workspace* w) {
+        for (Entry& e : entries) if (e.workspace == w) return &e;
+        return nullptr;
+    }
+    void drop_finished() {
+        for (size_t i = 0; i < entries.size();) {
+            if (entries[i].enqueued && cudaEventQuery(entries[i].workspace->talker_stop) == cudaSuccess) {
+                entries[i] = entries.back();
+                entries.pop_back();
+            } else {
+                ++i;
+            }
+        }
+        cudaGetLastError();     // "not ready" is no error
+    }
+    // Whether a frame of n rows that may run as a chain should.  Three and more sessions stepped alone get on faster side by
+    // side, launch by launch, than chain after chain (frames/s of 3, 4, 6, 8, 16 of them: 737, 784, 841, 791, 802 against 635);
+    // two are as fast either way (643 and 637), so that a second one joins a first that is made launch by launch instead of
+    // waiting for it.  Their frames end together and begin one after the other, so that the first of a round sees nobody:
+    // a crowd is remembered for a while.  Beside a lockstep frame the chain's is the shorter one (8 sessions and 3 alone
+    // 8.0 ms against 9.6).
+    bool chain_pays(const Workspace* w, int n) {
+        const auto now = std::chrono::steady_clock::now();
+        int alone = n == 1 ? 1 : 0;
+        bool lockstep = n > 1, launches = false;
+        for (const Entry& e : entries) {
+            if (e.workspace == w) continue;
+            if (e.kind == kOther) {
+                shared_until = now + std::chrono::milliseconds(5);       // past the host's part between two prompts
+                return false;
+            }
+            if (e.kind == kInPlaceOfChain && !e.enqueued) return false;
+            launches = launches || e.kind == kInPlaceOfChain;
+            if (e.rows == 1) ++alone;
+            else lockstep = true;
+        }
+        if (now < shared_until) return false;
+        if (lockstep) return true;
+        if (alone >= 3) crowd_until = now + std::chrono::milliseconds(20);
+        return !launches && now >= crowd_until;
+    }
+    void enter(const Workspace* w, int rows, Kind kind) {
+        Entry* e = find(w);
+        if (e != nullptr) *e = Entry{w, rows, kind, false};
+        else entries.push_back(Entry{w, rows, kind, false});
+    }
+    void leave(const Workspace* w) {
+        for (size_t i = 0; i < entries.size(); ++i) {
+            if (entries[i].workspace == w) {
+                entries[i] = entries.back();
+                entries.pop_back();
+                return;
+            }
+        }
+    }
+};
+Traffic* traffic_of(int device) {
+    static Traffic* const all = new Traffic[64];       // outlives every session
+    return device >= 0 && device < 64 ? &all[device] : nullptr;
+}
+
+// A prompt or a frame in the census, from its construction until it is known to have ended.
+class InFlight {
+public:
+    InFlight(Traffic* traffic, const Workspace& w, int rows, Traffic::Kind kind) : traffic_(traffic), workspace_(&w) {
+        if (traffic_ == nullptr) return;
+        std::lock_guard<std::mutex> lock(traffic_->mutex);
+        traffic_->enter(workspace_, rows, kind);
+    }
+    // a frame that may run as a chain: kind() tells whether it does
+    InFlight(Traffic* traffic, const Workspace& w, int rows, bool never_chain) : traffic_(traffic), workspace_(&w) {
+        std::lock_guard<std::mutex> lock(traffic_->mutex);
+        traffic_->drop_finished();
+        kind_ = !never_chain && traffic_->chain_pays(workspace_, rows) ? Traffic::kChain : Traffic::kInPlaceOfChain;
+        traffic_->enter(workspace_, rows, kind_);
+    }
+    InFlight(const InFlight&) = delete;
+    InFlight& operator=(const InFlight&) = delete;
+    // from here on the workspace's talker_stop tells the end
+    void enqueued() {
+        if (traffic_ == nullptr) return;
+        std::lock_guard<std::mutex> lock(traffic_->mutex);
+        if (Traffic::Entry* e = traffic_->find(workspace_)) e->enqueued = true;
+        traffic_ = nullptr;
+    }
+    ~InFlight() {
+        if (traffic_ == nullptr) return;
+        std::lock_guard<std::mutex> lock(traffic_->mutex);
+        traffic_->leave(workspace_);
+    }
+    Traffic::Kind kind() const { return kind_; }
+private:
+    Traffic* traffic_;
+    const Workspace* workspace_;
+    Traffic::Kind kind_ = Traffic::kOther;
+};
+
+// Held while a frame's chains are enqueued; whatever chain was enqueued by then, the next holder's stream waits for it, and
+// for the frames that stand in for one.
+class ChainTurn {
+public:
+    ChainTurn(Traffic* traffic, const Workspace& w) : traffic_(traffic), stream_(w.stream) {
+        if (traffic_ == nullptr) return;
+        lock_ = std::unique_lock<std::mutex>(traffic_->mutex);
+        if (traffic_->chain_done == nullptr) {
+            check_cuda(cudaEventCreateWithFlags(&traffic_->chain_done, cudaEventDisableTiming), "cudaEventCreate(chain order)");
+        } else if (traffic_->chain_stream != stream_) {
+            check_cuda(cudaStreamWaitEvent(stream_, traffic_->chain_done, 0), "cudaStreamWaitEvent(chain order)");
+        }
+        for (const Traffic::Entry& e : traffic_->entries) {
+            if (e.workspace == &w || e.kind != Traffic::kInPlaceOfChain || !e.enqueued) continue;
+            check_cuda(cudaStreamWaitEvent(stream_, e.workspace->talker_stop, 0), "cudaStreamWaitEvent(frame)");
+        }
+    }
+    ~ChainTurn() {
+        if (traffic_ == nullptr) return;
+        cudaEventRecord(traffic_->chain_done, stream_);
+        traffic_->chain_stream = stream_;
+    }
+private:
+    Traffic* traffic_;
+    cudaStream_t stream_;
+    std::unique_lock<std::mutex> lock_;
+};
+
+}  // namespace
 
 // ------------------------------------------------------------------ DeviceBuffer
 
@@ -172,6 +325,7 @@ Workspace::Workspace(int capacity_, int device_, int rows_) : capacity(capacity_
     // one allocation: a session's workspace is made when the session is, and fourteen of them were half of that
     const std::pair<DeviceBuffer*, size_t> parts[] = {
         {&table, sizeof(FrameTable)}, {&counters, one * 16 * sizeof(unsigned int)},
+        {&chain_order_scratch, chain_order_scratch_floats(std::min(capacity, kChainRows), 8) * sizeof(float)},
         {&hidden, c * 2048 * e}, {&qkv, c * 4096 * e}, {&attention, c * 2048 * e}, {&gate, c * 6144 * e},
         {&logits, one * kTalkerVocab * e}, {&x_in, c * 2048 * e}, {&projection, c * 2048 * e}, {&normalized, c * 2048 * e},
         {&prompt_positions, c * sizeof(int)}, {&talker_pages, one * kMaxPagesPerRow * sizeof(int)},
@@ -236,6 +390,10 @@ void Workspace::release() noexcept {
 Workspace::~Workspace() {
     cudaSetDevice(device);
     if (stream != nullptr) cudaStreamSynchronize(stream);
+    if (Traffic* traffic = traffic_of(device)) {
+        std::lock_guard<std::mutex> lock(traffic->mutex);
+        traffic->leave(this);
+    }
     release();
 }
 
@@ -260,7 +418,7 @@ uint64_t Workspace::bytes() const {
     return hidden.bytes() + qkv.bytes() + attention.bytes() + gate.bytes() + logits.bytes()
         + x_in.bytes() + projection.bytes() + normalized.bytes() + table.bytes()
         + talker_pages.bytes() + predictor_pages.bytes() + predictor_positions.bytes()
-        + counters.bytes() + scratch.bytes();
+        + counters.bytes() + scratch.bytes() + chain_order_scratch.bytes();
 }
 
 // ------------------------------------------------------------------ Model
@@ -623,7 +781,7 @@ struct Probe {
 void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWeights>& layers,
                     const uint32_t* rope_table, const KvPool& pool, const int* page_table, int table_stride,
                     const int* positions, int n, int splits, cudaStream_t s, int prompt_base = -1,
-                    const Probe* probe = nullptr) {
+                    const Probe* probe = nullptr, bool chain_order = false) {
     const int qkv_width = d.q_width + 2 * d.kv_width;
     // a prompt pass (prompt_base >= 0): the rows are consecutive positions of one session
     const bool shared_cache = prompt_base >= 0;
@@ -678,6 +836,9 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
             check_launch(launch_attention(a, s), "prompt KV append");
             a.append_mode = 2;
             check_launch(launch_attention(a, s), "prompt attention");
+        } else if (chain_order) {
+            a.scratch = w.chain_order_scratch.as<float>();
+            check_launch(launch_chain_order_attention(a, s), "decode attention");
         } else {
             check_launch(launch_attention(a, s), "decode attention");
         }
@@ -698,6 +859,7 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
         if (probe != nullptr) u.norm_out = w.normalized.as<bf16>();
         u.in_features = d.hidden; u.out_features = d.intermediate; u.rows = n;
         u.epilogue = EPI_GATE_UP_SILU;
+        u.leave_room = chain_order;
         project(u, "gate/up projection");
         observe("post_attention_norm", w.normalized.as<bf16>(), d.hidden, d.hidden);
         observe("gated_activation", w.gate.as<bf16>(), d.intermediate, d.intermediate);
@@ -817,7 +979,8 @@ void enqueue_talker_head(Workspace& w, Model& m, int n, int advance, cudaStream_
 }
 
 // next talker input, 28 layers, head, sample (talker.cu:1703-1880)
-void enqueue_talker(Workspace& w, Model& m, int n, int splits, cudaStream_t s) {
+// `chain_order`: with the bits of enqueue_talker_chain
+void enqueue_talker(Workspace& w, Model& m, int n, int splits, cudaStream_t s, bool chain_order = false) {
     FrameTable* table = w.table.as<FrameTable>();
     const int H = m.talker.hidden;
     check_launch(launch_talker_input(table, m.codec_embedding, m.predictor_embedding_table,
@@ -825,7 +988,7 @@ void enqueue_talker(Workspace& w, Model& m, int n, int splits, cudaStream_t s) {
                                    w.x_in.as<bf16>(), H, n, s), "talker input");
     enqueue_text_projection(w, m, n, true, s);
     enqueue_layers(w, m.talker, m.talker_layers, m.talker_rope, *m.talker_pool, w.talker_pages.as<int>(),
-                   Workspace::kMaxPagesPerRow, table->position, n, splits, s);
+                   Workspace::kMaxPagesPerRow, table->position, n, splits, s, -1, nullptr, chain_order);
     enqueue_talker_head(w, m, n, 1, s);
 }
 
@@ -842,43 +1005,11 @@ void enqueue_talker_chain(Workspace& w, Model& m, int n, cudaStream_t s) {
     check_launch(launch_frame_end(table, w.normalized.as<bf16>(), H, n, 1, s), "frame end");
 }
 
-// Chains wait between their CTAs, so two of them must not share the GPU's SMs: the chains of a device run one
-// after the other, whatever streams (and models) they come from.
-struct ChainOrder {
-    std::mutex mutex;
-    cudaEvent_t done = nullptr;
-    cudaStream_t last = nullptr;
-};
-ChainOrder g_chain_order[64];
-
-// Held while a frame with chains is enqueued; whatever was enqueued by then, the next holder's stream waits for it.
-class ChainTurn {
-public:
-    ChainTurn(ChainOrder* order, cudaStream_t stream) : order_(order), stream_(stream) {
-        if (order_ == nullptr) return;
-        lock_ = std::unique_lock<std::mutex>(order_->mutex);
-        if (order_->done == nullptr) {
-            check_cuda(cudaEventCreateWithFlags(&order_->done, cudaEventDisableTiming), "cudaEventCreate(chain order)");
-        } else if (order_->last != stream_) {
-            check_cuda(cudaStreamWaitEvent(stream_, order_->done, 0), "cudaStreamWaitEvent(chain order)");
-        }
-    }
-    ~ChainTurn() {
-        if (order_ == nullptr) return;
-        cudaEventRecord(order_->done, stream_);
-        order_->last = stream_;
-    }
-private:
-    ChainOrder* order_;
-    cudaStream_t stream_;
-    std::unique_lock<std::mutex> lock_;
-};
-
-// Whether a frame of these rows runs on the decode chain: few rows, the default kernels (it computes what they
+// Whether a frame of these rows may run on the decode chain: few rows, the default kernels (it computes what they
 // compute), draws small enough for its sampler.
-bool frame_takes_chain(const Model& m, const FrameTable& t, int n) {
+bool frame_may_chain(const Model& m, const FrameTable& t, int n) {
     if (!m.chain.ready || m.use_chain == 0 || m.use_graphs == 0 || n > kChainRows || n >= tc_min_rows() || gemv_mode() != 1 || attention_mode() != 1
-        || m.device() < 0 || m.device() >= 64) {
+        || traffic_of(m.device()) == nullptr) {
         return false;
     }
     for (int i = 0; i < n; ++i) {
@@ -1230,8 +1361,9 @@ void Session::bind_rows(Workspace& w, Session** s, int n) {
     for (int i = 0; i < n; ++i) w.bound[i] = s[i]->id_;
 }
 
-Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int splits, bool chain) {
-    const auto key = std::make_pair(n, chain ? 0 : splits);
+Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int splits, Way way) {
+    const bool chain = way == Way::kChain;
+    const auto key = std::make_pair(n, chain ? 0 : (way == Way::kInItsPlace ? -1 : splits));
     auto found = w.graphs.find(key);
     if (found != w.graphs.end()) return found->second;
     Workspace::Graphs g;
@@ -1243,7 +1375,7 @@ Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int spli
     try {
         g.talker = capture(w.stream, [&] {
                                if (chain) enqueue_talker_chain(w, m, n, w.stream);
-                               else enqueue_talker(w, m, n, splits, w.stream);
+                               else enqueue_talker(w, m, n, splits, w.stream, way == Way::kInItsPlace);
                            },
                            &g.talker_kernels);
     } catch (...) {
@@ -1265,36 +1397,31 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
         w.destroy_graphs();
         w.option_epoch = m.option_epoch;
     }
-    const bool chain = frame_takes_chain(m, *w.host_table, n);
-    if (!chain) w.ensure_scratch(splits);
-    bind_rows(w, s, n);
-    const ChainTurn turn(chain ? &g_chain_order[m.device()] : nullptr, w.stream);
-    if (upload_table) {
-        check_cuda(cudaMemcpyAsync(w.table.as<void>(), w.host_table, sizeof(FrameTable),
-                                   cudaMemcpyHostToDevice, w.stream), "upload frame table");
-        check_cuda(cudaEventRecord(w.table_uploaded, w.stream), "cudaEventRecord(table)");
-    }
-    if (chain && (m.chain.numbers += kChainNumbersPerFrame) > kChainNumbers) {
-        check_cuda(restart_chain_numbers(m.chain.exchange.as<void>(), m.chain.epoch.as<uint32_t>(), w.stream), "chain numbers");
-        m.chain.numbers = kChainNumbersPerFrame;
-    }
-    if (m.use_graphs) {
-        Workspace::Graphs& g = frame_graphs(w, m, n, splits, chain);
-        check_cuda(cudaEventRecord(w.predictor_start, w.stream), "cudaEventRecord");
-        check_cuda(cudaGraphLaunch(g.predictor, w.stream), "cudaGraphLaunch(predictor)");
-        check_cuda(cudaEventRecord(w.predictor_stop, w.stream), "cudaEventRecord");
-        if (record_session_events) {
-            for (int i = 0; i < n; ++i) {
-                check_cuda(cudaEventRecord(s[i]->codes_ready_, w.stream), "cudaEventRecord(codes)");
-            }
-        }
-        check_cuda(cudaEventRecord(w.talker_start, w.stream), "cudaEventRecord");
-        check_cuda(cudaGraphLaunch(g.talker, w.stream), "cudaGraphLaunch(talker)");
-        check_cuda(cudaEventRecord(w.talker_stop, w.stream), "cudaEventRecord");
-        m.kernel_launches += static_cast<uint64_t>(g.predictor_kernels + g.talker_kernels);
+    Traffic* const traffic = traffic_of(m.device());
+    std::unique_ptr<InFlight> in_flight;
+    Way way = Way::kLaunches;
+    if (frame_may_chain(m, *w.host_table, n)) {
+        in_flight.reset(new InFlight(traffic, w, n, m.use_chain == 2));
+        way = in_flight->kind() == Traffic::kChain ? Way::kChain : Way::kInItsPlace;
     } else {
+        in_flight.reset(new InFlight(traffic, w, n, Traffic::kOther));
+    }
+    if (way == Way::kLaunches) w.ensure_scratch(splits);
+    bind_rows(w, s, n);
+    Workspace::Graphs* const g = m.use_graphs ? &frame_graphs(w, m, n, splits, way) : nullptr;
+    {
+        const ChainTurn turn(way == Way::kChain ? traffic : nullptr, w);
+        if (upload_table) {
+            check_cuda(cudaMemcpyAsync(w.table.as<void>(), w.host_table, sizeof(FrameTable),
+                                       cudaMemcpyHostToDevice, w.stream), "upload frame table");
+            check_cuda(cudaEventRecord(w.table_uploaded, w.stream), "cudaEventRecord(table)");
+        }
+        if (way == Way::kChain && (m.chain.numbers += kChainNumbersPerFrame) > kChainNumbers) {
+            check_cuda(restart_chain_numbers(m.chain.exchange.as<void>(), m.chain.epoch.as<uint32_t>(), w.stream), "chain numbers");
+            m.chain.numbers = kChainNumbersPerFrame;
+        }
         check_cuda(cudaEventRecord(w.predictor_start, w.stream), "cudaEventRecord");
-        if (chain) enqueue_predictor_chain(w, m, n, w.stream);
+        if (g != nullptr) check_cuda(cudaGraphLaunch(g->predictor, w.stream), "cudaGraphLaunch(predictor)");
         else enqueue_predictor(w, m, n, w.stream);
         check_cuda(cudaEventRecord(w.predictor_stop, w.stream), "cudaEventRecord");
         if (record_session_events) {
@@ -1303,10 +1430,12 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
             }
         }
         check_cuda(cudaEventRecord(w.talker_start, w.stream), "cudaEventRecord");
-        if (chain) enqueue_talker_chain(w, m, n, w.stream);
+        if (g != nullptr) check_cuda(cudaGraphLaunch(g->talker, w.stream), "cudaGraphLaunch(talker)");
         else enqueue_talker(w, m, n, splits, w.stream);
         check_cuda(cudaEventRecord(w.talker_stop, w.stream), "cudaEventRecord");
+        if (g != nullptr) m.kernel_launches += static_cast<uint64_t>(g->predictor_kernels + g->talker_kernels);
     }
+    in_flight->enqueued();
     if (record_session_events) {
         for (int i = 0; i < n; ++i) {
             check_cuda(cudaEventRecord(s[i]->semantic_ready_, w.stream), "cudaEventRecord(semantic)");
@@ -1504,6 +1633,7 @@ void Session::prefill(const int32_t* text_ids, const int32_t* codec_ids, int cou
     if (chunked) one_prompt.lock();
     Workspace& w = chunked ? m.prefill_workspace() : *solo_;
     if (chunked) chunk = std::min(chunk, w.rows);
+    const InFlight in_flight(traffic_of(device_), w, 1, Traffic::kOther);      // until the call returns
     position_ = 0;
     generated_ = 0;
     const unsigned int errors_before = m.device_errors();

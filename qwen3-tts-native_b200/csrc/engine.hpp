@@ -143,6 +143,7 @@ struct Workspace {
     DeviceBuffer predictor_positions;   // [16][kMaxRows], slot p filled with p
     DeviceBuffer prompt_positions;      // [activation rows], positions of the rows of a prompt chunk
     DeviceBuffer scratch;
+    DeviceBuffer chain_order_scratch;   // of frames that stand in for the chain's
     DeviceBuffer counters;
     int scratch_splits = 0;
     int option_epoch = 0;            // Model::option_epoch the captured graphs were built under
@@ -153,7 +154,8 @@ struct Workspace {
         int predictor_kernels = 0;   // kernel nodes in each graph
         int talker_kernels = 0;
     };
-    std::map<std::pair<int, int>, Graphs> graphs;   // (rows, talker splits; 0: the decode chain) -> graphs
+    // (rows, talker splits; 0: the decode chain, -1: launch by launch in its place) -> graphs
+    std::map<std::pair<int, int>, Graphs> graphs;
     cudaEvent_t predictor_start = nullptr, predictor_stop = nullptr;
     // frames launched on this workspace, and the GPU times of the frame `timed_frame` (every
     // session of a lockstep frame reports the same two numbers: they are read from the events once)
@@ -234,7 +236,9 @@ public:
     std::mutex mutex;               // pools, workspaces
     int mask_eos = 0;
     int use_graphs = 1;
-    int use_chain = 1;              // frames of up to kChainRows sessions run as two cooperative launches
+    // Frames of up to kChainRows sessions: 1 as two cooperative launches, or launch by launch with the same bits where
+    // the device is shared; 2 always the latter; 0 launch by launch.
+    int use_chain = 1;
     int option_epoch = 0;           // bumped when an option that captured graphs bake in changes
     int batch_host_codes = 0;       // lockstep batches also mirror the 16 codes to pinned host memory
     std::atomic<uint64_t> kernel_launches{0};   // kernels of this library launched through frame graphs
@@ -335,7 +339,8 @@ private:
     void fill_row(FrameTable& t, int row, int trailing_text, const SamplingParams& talker,
                   const SamplingParams& predictor, bool host_codes) const;
     static void bind_rows(Workspace& w, Session** s, int n);
-    static Workspace::Graphs& frame_graphs(Workspace& w, Model& m, int n, int splits, bool chain);
+    enum class Way { kChain, kInItsPlace, kLaunches };      // of a frame
+    static Workspace::Graphs& frame_graphs(Workspace& w, Model& m, int n, int splits, Way way);
     static void launch_frame(Workspace& w, Model& m, Session** s, int n, bool upload_table,
                              bool record_session_events);
 

@@ -150,5 +150,112 @@ __device__ __forceinline__ void attend(const Fragments& f, const float* q, int c
     }
 }
 
+// ---- a row's pages over sixteen slots of eight classes -------------------------------------------------------------
+// kBlock consecutive pages go to one slot (a CTA), block after block over the slots, and there to classes, one page to a
+// class at first; a class is walked by one warp.  The classes of a slot and then the slots are merged in order.  The
+// grouping depends on the row's length only, so whoever computes it, the decode chain or a launch of its own, gets the
+// same bits.
+constexpr int kSlots = 16;
+constexpr int kClasses = 8;
+constexpr int kBlock = 2;
+constexpr int kPageStep = kClasses * kSlots;             // from a class's page to its next
+__device__ __forceinline__ int slots_of(int pages) { return min(kSlots, (pages + kBlock - 1) / kBlock); }
+__device__ __forceinline__ int class_page(int slot, int cls) { return kBlock * (slot + kSlots * (cls / kBlock)) + cls % kBlock; }
+
+// One head vector, lane l dims l, l + 32, l + 64, l + 96: RMSNorm, then the rotation cs0 (dims l, l + 64) and cs1.
+__device__ __forceinline__ void rotate(const float (&x)[4], const bf16 (&w)[4], uint32_t cs0, uint32_t cs1, float eps, float (&o)[4]) {
+    float sq[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sq[j] = fmaf(x[j], x[j], 0.0f);
+    float c = (sq[0] + sq[2]) + (sq[1] + sq[3]);
+    c = warp_sum_down(c);
+    c = __shfl_sync(0xffffffffu, c, 0);
+    const float inv = rsqrtf(c / 128.0f + eps);
+    float y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) y[j] = rbf(rbf(x[j] * inv) * bf2f(w[j]));
+    rope_pair_cs(y[0], y[2], bf_lo(cs0), bf_hi(cs0), o[0], o[2]);
+    rope_pair_cs(y[1], y[3], bf_lo(cs1), bf_hi(cs1), o[1], o[3]);
+}
+
+// What a class has so far: maximum, sum and weighted V, as attend() leaves a page's.
+struct Running {
+    float m, l, o[8][4];
+};
+__device__ __forceinline__ void start(Running& r) {
+    r.m = -INFINITY;
+    r.l = 0.0f;
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r.o[x][e] = 0.0f;
+}
+__device__ __forceinline__ void add(Running& r, bool first, float mp, float lp, const float (&op)[8][4]) {
+    // the first page replaces nothing: m is -inf, its factor 0 and the page's own 1, exactly
+    const float top = fmaxf(r.m, mp);
+    const float fo = first ? 0.0f : expf(r.m - top), fn = expf(mp - top);
+    r.l = first ? lp : fmaf(r.l, fo, lp * fn);
+    r.m = top;
+    // columns 2 tig and 2 tig + 1 are heads; only tig = 0 holds real ones
+    const float fo0 = __shfl_sync(0xffffffffu, fo, 0), fo1 = __shfl_sync(0xffffffffu, fo, 4);
+    const float fn0 = __shfl_sync(0xffffffffu, fn, 0), fn1 = __shfl_sync(0xffffffffu, fn, 4);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        r.o[x][0] = fmaf(r.o[x][0], fo0, op[x][0] * fn0);
+        r.o[x][2] = fmaf(r.o[x][2], fo0, op[x][2] * fn0);
+        r.o[x][1] = fmaf(r.o[x][1], fo1, op[x][1] * fn1);
+        r.o[x][3] = fmaf(r.o[x][3], fo1, op[x][3] * fn1);
+    }
+}
+// acc: [head][128], m and l: [head], of this class
+__device__ __forceinline__ void put_class(const Running& r, float* acc, float* m, float* l, int lane) {
+    if ((lane & 3) != 0) return;
+    const int gid = lane >> 2;
+    if (gid < 2) {
+        m[gid] = r.m;
+        l[gid] = r.l;
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int e = 2 * half + c;
+            float4* d4 = reinterpret_cast<float4*>(acc + 8 * gid + 128 * c + 64 * half);
+            d4[0] = make_float4(r.o[0][e], r.o[1][e], r.o[2][e], r.o[3][e]);
+            d4[1] = make_float4(r.o[4][e], r.o[5][e], r.o[6][e], r.o[7][e]);
+        }
+}
+// the classes of a slot in order, for dim d of head g: acc [class][head][128], m and l [class][head]
+__device__ __forceinline__ void merge_classes(const float* acc, const float* m, const float* l, int slot, int pages, int g, int d,
+                                              float& top, float& sum, float& value) {
+    int classes = 1;
+    while (classes < kClasses && class_page(slot, classes) < pages) ++classes;
+    top = -INFINITY;
+    for (int c = 0; c < classes; ++c) top = fmaxf(top, m[c * 2 + g]);
+    sum = 0.0f;
+    value = 0.0f;
+    for (int c = 0; c < classes; ++c) {
+        const float fac = expf(m[c * 2 + g] - top);
+        sum = fmaf(l[c * 2 + g], fac, sum);
+        value = fmaf(acc[c * 256 + g * 128 + d], fac, value);
+    }
+}
+// the slots in order, by a warp: get(k, 0) is slot k's maximum, get(k, 1) its sum, get(k, 2 + dim) its weighted V
+template <class Get>
+__device__ __forceinline__ float fold(Get get, int slots, int dim, int lane) {
+    // lane k holds what the fold needs of slot k: its factor and sum
+    const float mine = lane < slots ? get(lane, 0) : -INFINITY;
+    const float sum = lane < slots ? get(lane, 1) : 0.0f;
+    const float fac = expf(mine - warp_max_xor(mine));
+    float total = 0.0f, value = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < slots; ++k) {
+        const float fk = __shfl_sync(0xffffffffu, fac, k);
+        total = fmaf(__shfl_sync(0xffffffffu, sum, k), fk, total);
+        value = fmaf(get(k, 2 + dim), fk, value);
+    }
+    return value * (1.0f / total);
+}
+
 }  // namespace page
 }  // namespace q3t

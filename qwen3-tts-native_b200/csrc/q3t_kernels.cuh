@@ -42,6 +42,9 @@ struct GemvArgs {
     // upstream of this one in its stream that is not a norm, so they may be fetched ahead of the dependency wait.  Set only by callers that build the whole
     // launch sequence; false is always correct.
     bool residual_settled = false;
+    // Other streams' launches run beside this one: room for two CTAs per SM where the shape allows, rather than one
+    // with more of its weights ahead (same result).
+    bool leave_room = false;
 };
 
 // Launch with programmatic stream serialisation (QWEN3_TTS_PDL=0 turns it into an ordinary
@@ -314,6 +317,10 @@ constexpr uint64_t kChainNumbers = 1ull << 31;
 constexpr uint64_t kChainNumbersPerFrame = 1024;     // at most: 16 x (5 x 6 + 1) + 15 x 2 by the predictor, 28 x 8 by the talker
 cudaError_t restart_chain_numbers(void* exchange, uint32_t* epoch, cudaStream_t stream);
 unsigned int chain_error_count();
+// The talker's decode attention with the bits of the chain's, as a launch (attention_blocks.cu): fused, paged, settled
+// inputs, a.scratch of chain_order_scratch_floats().
+size_t chain_order_scratch_floats(int rows, int kv_heads);
+cudaError_t launch_chain_order_attention(const AttentionArgs& args, cudaStream_t stream);
 
 // Sampler over table rows: row r reads logits + r*logits_stride.  talker != 0: reserved
 // tokens masked, repetition penalty, token -> sampled[r] and appended to history[r];

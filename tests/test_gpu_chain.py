@@ -102,3 +102,71 @@ def test_exchange_numbers_start_again(q3t, model, used, given_up):
     for a, b in zip(got, want):
         assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2]) and a[4] == b[4]
     assert lib.q3t_kernel_error_count() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 5, 8])
+def test_launches_in_the_chains_place(q3t, model, rows):
+    """Where the device is shared a frame is made launch by launch instead of as a chain: the same bits, for contexts of one
+    page, one slot, several slots and several pages to a class (2,048 tokens and more), and for the frames that follow."""
+    positions = POSITIONS[-rows:]
+    for a, b in zip(frame(q3t, model, positions, 2, frames=3), frame(q3t, model, positions, 1, frames=3)):
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2]) and a[4] == b[4]
+        assert all(np.array_equal(x, y) for x, y in zip(a[3], b[3]))
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
+def test_frames_do_not_depend_on_what_else_runs(q3t, model):
+    """Sessions stepped alone from threads of their own, a lockstep batch and prompts, all at once: every session decodes what
+    it decodes on a quiet device, whichever way its frames were made."""
+    import threading
+    model.set_option("decode_chain", 1)
+    rng = np.random.default_rng(8)
+    prompts = {n: ([int(t) for t in rng.integers(0, 151936, size=n)], [-1] * n) for n in (70, 300)}
+    steps = 12
+
+    def session(seed, position):
+        s = model.create_session(position + steps + 32, seed)
+        s.talker_sampling = q3t.SamplingConfig(True, 50, 0.9, 0.9, 1.05)
+        s.predictor_sampling = q3t.SamplingConfig(True, 50, 1.0, 0.9, 1.0)
+        s.synthetic_prefill(position, seed)
+        return s
+
+    def alone(seed, position):
+        s = session(seed, position)
+        out = [s.next_frame(5 + i) for i in range(steps)]
+        out = [(f.codes, f.next_semantic_token) for f in out] + [s.read_state()[0].tobytes()]
+        s.close()
+        return out
+
+    def together(count, seed):
+        ss = [session(seed + i, 100 + 50 * i) for i in range(count)]
+        out = []
+        for i in range(steps):
+            out.append([p.finish_without_consumer().next_semantic_token for p in model.batch_begin_device_frames(ss, [5 + i] * count)])
+        out.append([s.read_state()[0].tobytes() for s in ss])
+        for s in ss:
+            s.close()
+        return out
+
+    def prompt(n):
+        out = []
+        for _ in range(4):
+            s = model.create_session(n + 16, 3)
+            s.prefill(*prompts[n])
+            out.append((s.current_semantic_token, s.read_state()[0].tobytes()))
+            s.close()
+        return out
+
+    jobs = [lambda i=i: alone(300 + i, 20 + 150 * i) for i in range(4)] + [lambda: together(3, 400), lambda: prompt(70), lambda: prompt(300)]
+    quiet = [job() for job in jobs]
+    assert all(len(set(q)) == 1 for q in quiet[-2:])
+    for some in ([0, 1], [0, 1, 2, 3], [0, 4], [0, 1, 2, 4], [0, 5], [4, 6], list(range(len(jobs)))):
+        got = {}
+        threads = [threading.Thread(target=lambda i=i: got.__setitem__(i, jobs[i]())) for i in some]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for i in some:
+            assert got.get(i) == quiet[i], (some, i)
+    assert q3t.library().q3t_kernel_error_count() == 0
