@@ -250,25 +250,21 @@ DeviceBuffer::~DeviceBuffer() {
 namespace {
 // Clears (source null) or fills device memory before it returns.  cudaMemset and cudaMemcpy are of no use for that: they may
 // return before their work on the default stream is done, which the engine's streams do not wait for.
-void set_now(void* destination, const void* source, size_t bytes, const char* what) {
-    cudaStream_t s = nullptr;
-    check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), what);
-    cudaError_t e = source == nullptr ? cudaMemsetAsync(destination, 0, bytes, s)
-                                      : cudaMemcpyAsync(destination, source, bytes, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
-    check_cuda(e, what);
+void set_now(void* destination, const void* source, size_t bytes, cudaStream_t s, const char* what) {
+    check_cuda(source == nullptr ? cudaMemsetAsync(destination, 0, bytes, s)
+                                 : cudaMemcpyAsync(destination, source, bytes, cudaMemcpyHostToDevice, s), what);
+    check_cuda(cudaStreamSynchronize(s), what);
 }
 }  // namespace
 
 // ------------------------------------------------------------------ KvPool
 
-KvPool::KvPool(int layers, int kv_width, int slab_shift)
-    : layers_(layers), kv_width_(kv_width), slab_shift_(slab_shift),
+KvPool::KvPool(int layers, int kv_width, int slab_shift, cudaStream_t stream)
+    : stream_(stream), layers_(layers), kv_width_(kv_width), slab_shift_(slab_shift),
       page_elems_((long long)kPageTokens * kv_width),
       plane_elems_(((long long)1 << slab_shift) * kPageTokens * kv_width),
       slab_table_(kMaxSlabs * sizeof(bf16*)) {
-    set_now(slab_table_.as<void>(), nullptr, kMaxSlabs * sizeof(bf16*), "clear slab table");
+    set_now(slab_table_.as<void>(), nullptr, kMaxSlabs * sizeof(bf16*), stream_, "clear slab table");
 }
 
 void KvPool::add_slab() {
@@ -277,7 +273,7 @@ void KvPool::add_slab() {
     DeviceBuffer slab(bytes);
     bf16* base = slab.as<bf16>();
     const int index = static_cast<int>(slabs_.size());
-    set_now(slab_table_.as<bf16*>() + index, &base, sizeof(base), "fill slab table");
+    set_now(slab_table_.as<bf16*>() + index, &base, sizeof(base), stream_, "fill slab table");
     slabs_.push_back(std::move(slab));
     const int per = 1 << slab_shift_;
     for (int i = per - 1; i >= 0; --i) free_.push_back(index * per + i);
@@ -635,7 +631,8 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(upload)");
     staging_ = DeviceBuffer();
     embedding_ptrs_ = DeviceBuffer(kResidualCodebooks * sizeof(const bf16*));
-    set_now(embedding_ptrs_.as<void>(), predictor_embeddings.data(), kResidualCodebooks * sizeof(const bf16*), "embedding table");
+    set_now(embedding_ptrs_.as<void>(), predictor_embeddings.data(), kResidualCodebooks * sizeof(const bf16*), upload_stream_,
+            "embedding table");
     predictor_embedding_table = embedding_ptrs_.as<const bf16*>();
     talker_rope_ = DeviceBuffer((size_t)kRopePositions * (talker.head_dim / 2) * sizeof(uint32_t));
     check_cuda(launch_build_rope_table(talker_rope_.as<uint32_t>(), kRopePositions, talker.head_dim,
@@ -657,8 +654,8 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
         cudaStreamSynchronize(upload_stream_);
         chain = DecodeChain();
     }
-    talker_pool.reset(new KvPool(talker.layers, talker.kv_width, 8));
-    predictor_pool.reset(new KvPool(predictor.layers, predictor.kv_width, 6));
+    talker_pool.reset(new KvPool(talker.layers, talker.kv_width, 8, upload_stream_));
+    predictor_pool.reset(new KvPool(predictor.layers, predictor.kv_width, 6, upload_stream_));
     finalized_ = true;
     *weight_bytes = weight_bytes_;
     *tensor_count = tensor_count_;
@@ -675,9 +672,9 @@ void Model::build_chain() {
     // The streams are made from the weights as they lie there now: what a caller has enqueued on streams of its own to fill
     // adopted storage has to be done.
     check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(adopted weights)");
-    auto table = [](DeviceBuffer& b, const void* host, size_t bytes) {
+    auto table = [this](DeviceBuffer& b, const void* host, size_t bytes) {
         b = DeviceBuffer(bytes);
-        set_now(b.as<void>(), host, bytes, "chain table");
+        set_now(b.as<void>(), host, bytes, upload_stream_, "chain table");
     };
     for (int t = 0; t < 2; ++t) {
         const bool big = t == 1;
@@ -733,7 +730,7 @@ void Model::set_chain_numbers(uint64_t used, uint32_t given_up) {
     if (!chain.ready) return;
     const uint32_t epoch[2] = {static_cast<uint32_t>(used), given_up};
     check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(chain numbers)");
-    set_now(chain.epoch.as<void>(), epoch, sizeof(epoch), "chain numbers");
+    set_now(chain.epoch.as<void>(), epoch, sizeof(epoch), upload_stream_, "chain numbers");
     chain.numbers = used;
 }
 

@@ -92,7 +92,7 @@ struct LayerWeights {
 // `pages_per_slab` pages: slab[layer][k|v][page][kv_head][16][head_dim] (head-major pages).
 class KvPool {
 public:
-    KvPool(int layers, int kv_width, int slab_shift);
+    KvPool(int layers, int kv_width, int slab_shift, cudaStream_t stream);     // its table is filled on `stream`
     int allocate();                 // page id; grows by one slab when empty
     void release(int page);
     KvLayout layout(int layer, const int* page_table, int table_stride) const;
@@ -107,6 +107,7 @@ public:
     static constexpr int kMaxSlabs = 512;
 private:
     void add_slab();
+    cudaStream_t stream_;
     int layers_, kv_width_, slab_shift_;
     long long page_elems_, plane_elems_;
     std::vector<DeviceBuffer> slabs_;
