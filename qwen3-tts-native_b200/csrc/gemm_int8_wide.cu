@@ -1,9 +1,9 @@
 // Int8 weight-only GEMM for the passes of a prompt: 65 to 2048 activation rows on the 5th-generation
 // tensor cores.
 //
-// Same operation and epilogues as gemm_int8_tc.cu, without its split of K: there are enough output
-// tiles here to fill the GPU.  A CTA owns NT tiles of 128 output channels (TMEM lanes) by 128
-// activation rows (TMEM columns).
+// Same operation as gemm_int8_tc.cu and the same epilogues but the bias with a residual, which no prompt has, without
+// its split of K: there are enough output tiles here to fill the GPU.  A CTA owns NT tiles of 128 output channels (TMEM
+// lanes) by 128 activation rows (TMEM columns).
 //
 // What bounds it: the tensor cores, if the operands arrive in time.  Per element of K a CTA with NT
 // = 2 fetches 256 bytes of weights and 256 bytes of activations for 8 cycles of MMA (4096 bf16 MACs a
@@ -56,7 +56,6 @@ struct WideParams {
     const float* scales;
     bf16* y;
     const bf16* bias;
-    bf16* resid;
     int out_features;       // N (gate/up: channels, the matrix has 2N rows)
     int rows;
     int row_blocks;
@@ -242,8 +241,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         const int first_row = row_base + group * kShare;
         const int rows_here = min(kShare, p.rows - first_row);
         const bool up_lane = GATEUP && NT == 1 && t >= 64;
-        const bool adds = !GATEUP && (p.epilogue == EPI_ADD || p.epilogue == EPI_BIAS_ADD);
-        bf16* out = (p.epilogue == EPI_BIAS_ADD ? p.resid : p.y) + (size_t)first_row * N;
+        const bool adds = !GATEUP && p.epilogue == EPI_ADD;
+        bf16* out = p.y + (size_t)first_row * N;
         bf16 base[kShare];
         auto fetch_bases = [&](int channel) {
 #pragma unroll
@@ -305,7 +304,6 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
                             } else {
                                 val = rbf(v[j] * scale) + bias;
                                 if (p.epilogue == EPI_BIAS_SILU) val = __fdividef(val, 1.0f + __expf(-val));
-                                else if (p.epilogue == EPI_BIAS_ADD) val = bf2f(base[c0 + j]) + rbf(val);
                             }
                             if (channel < N && c0 + j < rows_here) dst[(size_t)(c0 + j) * N] = f2bf(val);
                         }
@@ -354,14 +352,14 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
     const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
     if (a.rows < 1 || a.rows > kMaxPromptRows || a.out_features < 1 || a.in_features % kBK != 0 || a.in_features < kBK
         || a.w == nullptr || a.scales == nullptr || a.x == nullptr || a.norm_w != nullptr || a.y32 != nullptr
-        || (a.epilogue == EPI_BIAS_ADD ? a.resid == nullptr : a.y == nullptr)) {
+        || a.y == nullptr || a.epilogue == EPI_BIAS_ADD) {
         return cudaErrorInvalidValue;
     }
-    if ((a.epilogue == EPI_BIAS || a.epilogue == EPI_BIAS_SILU || a.epilogue == EPI_BIAS_ADD) && a.bias == nullptr) {
+    if ((a.epilogue == EPI_BIAS || a.epilogue == EPI_BIAS_SILU) && a.bias == nullptr) {
         return cudaErrorInvalidValue;
     }
     WideParams p;
-    p.scales = a.scales; p.y = a.y; p.bias = a.bias; p.resid = a.resid;
+    p.scales = a.scales; p.y = a.y; p.bias = a.bias;
     p.out_features = a.out_features; p.rows = a.rows; p.epilogue = a.epilogue;
     p.row_blocks = (a.rows + kTileM - 1) / kTileM;
     p.steps = a.in_features / kBK;
@@ -384,8 +382,12 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
 // Which kernel takes a projection of a prompt pass: the one with the shortest estimate.  A wave of CTAs of this
 // file's kernel costs its steps (0.50 us each with one channel tile, 0.82 us with two: what an SM takes in) and 4
 // to 6 us of start and epilogue; the 64-row kernel of gemm_int8_tc.cu, its row blocks side by side and K split where
-// that fits one wave, is estimated there.  Within 20 % of the measured times of the talker's four shapes from 65 to
-// 2048 rows; the crossovers lie around 130 rows (gate/up), 200 (q/k/v), 300 (o, down).
+// that fits one wave, is estimated there.  For the talker's shapes that puts the lines at 65 rows (gate/up; two tiles
+// from 129), 257 (q/k/v; two tiles from 513) and 577 (o, down and the text projection; two tiles from about 1,200).
+// Measured from 65 to 2000 rows (us, row blocks / one tile / two tiles): gate/up 128 rows 21.1 / 15.6 / 18.1, 129
+// 21.4 / 27.0 / 18.5; q/k/v 256 12.1 / 12.6 / 19.4, 257 18.6 / 13.1 / 19.3; down 576 27.1 / 29.8 / 47.7, 577
+// 45.8 / 30.0 / 47.7.  The choice is within 4 % of the best everywhere but for o between 384 and 576 rows (6 to 11 %:
+// 13.4 to 14.1 us against 12.4 to 12.7 by one tile).
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     GemvArgs a = args;
     if (a.norm_w != nullptr) {
@@ -403,7 +405,8 @@ cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     };
     const float one = waves(1) * (a.epilogue == EPI_GATE_UP_SILU ? 6.0f + 0.50f * steps : 4.3f + 0.50f * steps);
     const float two = waves(2) * (5.5f + 0.82f * steps);
-    if (gemm_tc_estimate_us(a) <= (one < two ? one : two)) return launch_int8_gemm_tc(a, stream);
+    // (a bias with a residual, which no prompt has, exists there only)
+    if (a.epilogue == EPI_BIAS_ADD || gemm_tc_estimate_us(a) <= (one < two ? one : two)) return launch_int8_gemm_tc(a, stream);
     return launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
 }
 
