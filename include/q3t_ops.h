@@ -76,6 +76,9 @@ typedef struct Q3tGemmDesc {
     float epsilon;
 } Q3tGemmDesc;
 QWEN3_TTS_API int32_t q3t_launch_int8_gemm_ex(const Q3tGemmDesc* desc, void* stream);
+/* Test hook: a projection of a prompt pass, up to 2048 rows.  kernel 0: the one that a prompt takes; 1 and 2: 128 rows and
+ * one or two tiles of channels a CTA; 3: the lockstep kernel with its row blocks side by side. */
+QWEN3_TTS_API int32_t q3t_test_prompt_gemm(const Q3tGemmDesc* desc, int32_t kernel, void* stream);
 
 /* launch_quantize_weight_rows (int8_gemv.cu:302-317) */
 QWEN3_TTS_API int32_t q3t_launch_quantize_weight_rows(const uint16_t* weight, int8_t* quantized,
@@ -335,6 +338,10 @@ typedef struct Q3tAttentionDesc {
     size_t scratch_bytes;
 } Q3tAttentionDesc;
 QWEN3_TTS_API int32_t q3t_launch_decode_attention_ex(const Q3tAttentionDesc* desc, void* stream);
+/* Test hook: the attention of a prompt pass.  The rows are the positions base, base + 1, ... of the session whose pages
+ * row 0 of the table lists; query, key_new and value_new are the parts of one packed projection, of which the query part is
+ * overwritten.  Returns when it is done. */
+QWEN3_TTS_API int32_t q3t_test_prompt_attention(const Q3tAttentionDesc* desc, int32_t base);
 
 /* ---- sampler (sampling_kernels.cu) ------------------------------------------------------- */
 

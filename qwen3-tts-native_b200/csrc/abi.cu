@@ -621,18 +621,30 @@ int32_t q3t_launch_int8_gate_up_silu_rows(const int8_t* weight, const float* sca
                      EPI_GATE_UP_SILU, stream);
 }
 
-int32_t q3t_launch_int8_gemm_ex(const Q3tGemmDesc* d, void* stream) {
+static int32_t gemm_args(const Q3tGemmDesc* d, GemvArgs& a) {
     if (d == nullptr || d->struct_size != sizeof(Q3tGemmDesc)) return cudaErrorInvalidValue;
     if (d->epilogue < Q3T_EPI_PLAIN || d->epilogue > Q3T_EPI_GATE_UP_SILU) return cudaErrorInvalidValue;
     if (const int32_t e = ready()) return e;
-    GemvArgs a;
     a.w = d->weight; a.scales = d->scales; a.x = B(d->input); a.y = B(d->output);
     a.y32 = d->output_f32; a.norm_w = B(d->norm_weight); a.norm_out = B(d->norm_output);
     a.bias = B(d->bias); a.resid = B(d->residual);
     a.in_features = d->in_features; a.out_features = d->out_features; a.rows = d->rows;
     a.epilogue = d->epilogue;
     a.eps = d->epsilon > 0.0f ? d->epsilon : kRmsEps;
+    return 0;
+}
+
+int32_t q3t_launch_int8_gemm_ex(const Q3tGemmDesc* d, void* stream) {
+    GemvArgs a;
+    if (const int32_t e = gemm_args(d, a)) return e;
     return static_cast<int32_t>(launch_int8_gemm(a, S(stream)));
+}
+
+int32_t q3t_test_prompt_gemm(const Q3tGemmDesc* d, int32_t kernel, void* stream) {
+    GemvArgs a;
+    if (const int32_t e = gemm_args(d, a)) return e;
+    if (kernel == 0) return static_cast<int32_t>(launch_int8_gemm_prompt(a, S(stream)));
+    return static_cast<int32_t>(kernel == 3 ? launch_int8_gemm_tc(a, S(stream)) : launch_int8_gemm_wide(a, S(stream), kernel));
 }
 
 int32_t q3t_launch_quantize_weight_rows(const uint16_t* weight, int8_t* quantized, float* scales,
@@ -925,12 +937,11 @@ int32_t q3t_launch_batch_causal_gqa_attention_fast(
     return attention_common(a, max_sequence_length, scratch, scratch_bytes, S(stream));
 }
 
-int32_t q3t_launch_decode_attention_ex(const Q3tAttentionDesc* d, void* stream) {
+static int32_t attention_args(const Q3tAttentionDesc* d, AttentionArgs& a) {
     if (d == nullptr || d->struct_size != sizeof(Q3tAttentionDesc) || d->rows < 1
         || d->max_sequence_length < 1) {
         return cudaErrorInvalidValue;
     }
-    AttentionArgs a;
     a.q = B(d->query); a.k_new = B(d->key_new); a.v_new = B(d->value_new);
     a.q_norm_w = B(d->query_norm_weight); a.k_norm_w = B(d->key_norm_weight);
     a.positions = d->positions;
@@ -949,7 +960,32 @@ int32_t q3t_launch_decode_attention_ex(const Q3tAttentionDesc* d, void* stream) 
     a.head_dim = d->head_dimension; a.fused = d->fused;
     a.eps = d->epsilon > 0.0f ? d->epsilon : kRmsEps;
     a.theta = d->theta > 0.0f ? d->theta : kRopeTheta;
+    return 0;
+}
+
+int32_t q3t_launch_decode_attention_ex(const Q3tAttentionDesc* d, void* stream) {
+    AttentionArgs a;
+    if (const int32_t e = attention_args(d, a)) return e;
     return attention_common(a, d->max_sequence_length, d->scratch, d->scratch_bytes, S(stream));
+}
+
+int32_t q3t_test_prompt_attention(const Q3tAttentionDesc* d, int32_t base) {
+    AttentionArgs a;
+    if (const int32_t e = attention_args(d, a)) return e;
+    if (const int32_t e = ready()) return e;
+    if (base < 0 || d->rows > 8192 - base) return cudaErrorInvalidValue;
+    cudaError_t e = cudaSuccess;
+    const int32_t status = protect([&] {
+        DeviceBuffer table((size_t)(base + d->rows) * (d->head_dimension / 2) * sizeof(uint32_t));
+        a.rope_table = table.as<uint32_t>();
+        a.rope_positions = base + d->rows;
+        a.kv.table_stride = 0;
+        e = launch_build_rope_table(table.as<uint32_t>(), a.rope_positions, a.head_dim, a.theta, nullptr);
+        if (e == cudaSuccess) e = launch_prompt_attention(a, base, nullptr);
+        const cudaError_t done = cudaStreamSynchronize(nullptr);
+        if (e == cudaSuccess) e = done;
+    }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
+    return status != 0 ? status : static_cast<int32_t>(e);
 }
 
 static int32_t sample_common(const uint16_t* logits, int vocabulary, int suppress, int eos,

@@ -67,8 +67,9 @@ def _ok(rc: int, what: str) -> None:
 
 
 def int8_gemm(w, scales, x, *, epilogue=EPI_PLAIN, y_in=None, norm_w=None, bias=None, resid=None,
-              want_f32=False, want_norm=False, eps=1.0e-6):
-    """Returns dict(y=..., f32=..., norm=..., resid=...) for one fused GEMV/GEMM launch."""
+              want_f32=False, want_norm=False, eps=1.0e-6, prompt_kernel=None):
+    """Returns dict(y=..., f32=..., norm=..., resid=...) for one fused GEMV/GEMM launch; `prompt_kernel`: see
+    q3t_test_prompt_gemm."""
     lib = native.library()
     wr, k = w.shape
     n = wr // 2 if epilogue == EPI_GATE_UP_SILU else wr
@@ -92,7 +93,10 @@ def int8_gemm(w, scales, x, *, epilogue=EPI_PLAIN, y_in=None, norm_w=None, bias=
     d.bias = db.data_ptr() if db is not None else None
     d.residual = dr.data_ptr() if dr is not None else None
     d.in_features, d.out_features, d.rows, d.epsilon = k, n, rows, eps
-    _ok(lib.q3t_launch_int8_gemm_ex(C.byref(d), None), "q3t_launch_int8_gemm_ex")
+    if prompt_kernel is None:
+        _ok(lib.q3t_launch_int8_gemm_ex(C.byref(d), None), "q3t_launch_int8_gemm_ex")
+    else:
+        _ok(lib.q3t_test_prompt_gemm(C.byref(d), prompt_kernel, None), "q3t_test_prompt_gemm")
     return dict(y=_u16(dy), f32=d32.cpu().numpy() if d32 is not None else None,
                 norm=_u16(dno) if dno is not None else None,
                 resid=_u16(dr) if dr is not None else None)
@@ -266,8 +270,8 @@ def attention_contiguous_noalloc(q, k, v, positions, q_heads, kv_heads, head_dim
 def attention_ex(q, positions, q_heads, kv_heads, head_dim, *, k=None, v=None, pages=None,
                  page_table=None, slab_shift=0, k_new=None, v_new=None, q_norm_w=None,
                  k_norm_w=None, fused=False, q_stride=0, new_stride=0, max_seq=None,
-                 want_f32=False, theta=1.0e6, eps=1.0e-6):
-    """Full-form attention.  Contiguous: k, v [rows][capacity][kvw].  Paged: `pages` is a list
+                 want_f32=False, theta=1.0e6, eps=1.0e-6, prompt_base=None):
+    """Full-form attention; `prompt_base`: that of a prompt pass (q3t_test_prompt_attention).  Contiguous: k, v [rows][capacity][kvw].  Paged: `pages` is a list
     of slabs, each [2][pages_per_slab][kv_heads][16][head_dim] (K plane then V plane; a page is
     head-major: the 16 tokens of one KV head are contiguous), page_table
     [rows][stride].  Returns dict(out, f32, k, v | pages) with caches after the append."""
@@ -328,7 +332,10 @@ def attention_ex(q, positions, q_heads, kv_heads, head_dim, *, k=None, v=None, p
     nbytes = int(lib.q3t_attention_scratch_bytes(rows, q_heads, kv_heads, head_dim, max_seq))
     scratch = torch.empty((max(nbytes, 16),), dtype=torch.uint8, device="cuda")
     d.scratch, d.scratch_bytes = scratch.data_ptr(), nbytes
-    _ok(lib.q3t_launch_decode_attention_ex(C.byref(d), None), "q3t_launch_decode_attention_ex")
+    if prompt_base is None:
+        _ok(lib.q3t_launch_decode_attention_ex(C.byref(d), None), "q3t_launch_decode_attention_ex")
+    else:
+        _ok(lib.q3t_test_prompt_attention(C.byref(d), prompt_base), "q3t_test_prompt_attention")
     return dict(out=_u16(do), f32=d32.cpu().numpy() if d32 is not None else None,
                 k=_u16(dk) if dk is not None else None, v=_u16(dv) if dv is not None else None,
                 pages=[_u16(s) for s in dslabs])

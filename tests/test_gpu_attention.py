@@ -306,3 +306,36 @@ def test_scores_of_minus_infinity(orc, ops, length, masked):
     want, want32 = orc.attention(q, k, v, pos, qh, kvh, hd, fast=True, want_f32=True)
     assert np.isfinite(want32).all()
     check(orc, got["out"], got["f32"], want, want32, hd)
+
+
+@pytest.mark.parametrize("base,rows", [(0, 9), (0, 32), (0, 33), (0, 64), (0, 97), (31, 40), (64, 65), (100, 70), (250, 129)])
+def test_prompt_attention(orc, ops, base, rows):
+    """Consecutive positions of one session that share their walk over the cache, against the oracle row by row: first and
+    later passes, at the edges of pages, of blocks of 32 positions and of steps of 64 tokens; places behind the last position
+    hold NaN, so that a token let through the mask would show."""
+    qh, kvh, hd = 16, 8, 128
+    qw, kvw = qh * hd, kvh * hd
+    end = base + rows
+    cap = (end + 15) // 16 * 16 + 16
+    rng = np.random.default_rng(base + rows)
+    qkv = bf(orc, rng.standard_normal((rows, qw + 2 * kvw)))
+    wq, wk = (bf(orc, 1 + 0.1 * rng.standard_normal(hd)) for _ in range(2))
+    k, v = (bf(orc, rng.standard_normal((1, cap, kvw))) for _ in range(2))
+    pos = np.arange(base, end, dtype=np.int32)
+    q2 = ops.rope_rows_at(ops.head_rms_norm_rows(np.ascontiguousarray(qkv[:, :qw]), wq, rows, qh, hd), rows, qh, hd, pos)
+    k2 = ops.rope_rows_at(ops.head_rms_norm_rows(np.ascontiguousarray(qkv[:, qw:qw + kvw]), wk, rows, kvh, hd), rows, kvh, hd, pos)
+    full_k, full_v = k.copy(), v.copy()
+    full_k[0, base:end], full_v[0, base:end] = k2.reshape(rows, kvw), qkv[:, qw + kvw:]
+    k[0, base:], v[0, base:] = 0x7fc0, 0x7fc0
+    slabs, table = paged_copy(k, v, kvw, rng, per_slab=64)
+    got = ops.attention_ex(qkv, pos, qh, kvh, hd, pages=slabs, page_table=table, slab_shift=6, q_norm_w=wq, k_norm_w=wk, fused=True,
+                           q_stride=qw + 2 * kvw, new_stride=qw + 2 * kvw, prompt_base=base)
+    want, _ = orc.attention(q2.reshape(rows, qw), np.repeat(full_k, rows, axis=0), np.repeat(full_v, rows, axis=0), pos, qh, kvh, hd,
+                            fast=True, want_f32=True)
+    check_bf16(orc, got["out"], want, hd)
+    # the rows that the pass appends, and nothing behind them
+    for which, full in ((0, full_k), (1, full_v)):
+        for t in range(cap):
+            pid = int(table[0, t // 16])
+            row = got["pages"][pid // 64][which, pid % 64, :, t % 16].reshape(-1)
+            assert np.array_equal(row, full[0, t] if t < end else np.full(kvw, 0x7fc0, dtype=np.uint16)), t

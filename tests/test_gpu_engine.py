@@ -314,7 +314,7 @@ def test_chunked_prompt_equals_position_by_position(q3t, orc, model):
             s.close()
             return first, hidden, rng_state, frames
         finally:
-            model.set_option("prefill_chunk", 64)
+            model.set_option("prefill_chunk", 2048)
             model.set_option("tc_min_rows", 9)
             model.set_option("gemv_mode", 1)
 

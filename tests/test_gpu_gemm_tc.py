@@ -111,3 +111,59 @@ def test_deterministic_and_healthy(q3t, orc, ops):
     c = ops.int8_gemm_rows(w, s, x[:40])
     assert np.array_equal(a[:40], c)
     assert q3t.library().q3t_kernel_error_count() == 0
+
+
+def prompt_case(orc, n, k, rows, gate_up=False):
+    w, s, x = case(orc, n + rows, 2 * n if gate_up else n, k, rows)
+    rng = np.random.default_rng(rows)
+    return w, s, x, orc.to_bf16((0.1 * rng.standard_normal(n)).astype(np.float32)), orc.to_bf16(rng.standard_normal((rows, n)).astype(np.float32))
+
+
+@pytest.mark.parametrize("kernel", [1, 2, 3])
+@pytest.mark.parametrize("n,k,rows", [(300, 384, 65), (128, 128, 128), (129, 1152, 129), (640, 256, 161), (257, 512, 300), (1100, 2048, 128)])
+def test_prompt_kernels(q3t, orc, ops, kernel, n, k, rows):
+    """Projections of more than 64 rows: 128 rows and one or two tiles of channels a CTA (1, 2), or the lockstep kernel's row
+    blocks side by side (3), with every epilogue that they have, at the edges of row blocks and of channel tiles (a last tile
+    that is short, a second one that is not there), fewer steps than the rings hold and more."""
+    w, s, x, bias, base = prompt_case(orc, n, k, rows)
+    plain = orc.int8_gemm_rows(w, s, x)
+    check_bf16(orc, ops.int8_gemm(w, s, x, prompt_kernel=kernel)["y"], plain)
+    check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=ops.EPI_ADD, y_in=base, prompt_kernel=kernel)["y"],
+               orc.int8_gemm_rows(w, s, x, y_in=base, mode=1), summand=base)
+    # the product is rounded to bf16 before the bias is added, and its rounding may fall the other way: an ulp of it, at most
+    # 2^-7 |product|, through SiLU (slope at most 1.1) and a rounding of the result, 2^-8 (|product| + |bias|)
+    summand = orc.to_bf16(1.6 * (np.abs(orc.from_bf16(plain)) + np.abs(orc.from_bf16(bias))).astype(np.float32))
+    for epilogue, silu in ((ops.EPI_BIAS, False), (ops.EPI_BIAS_SILU, True)):
+        check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=epilogue, bias=bias, prompt_kernel=kernel)["y"],
+                   orc.bias_activation_rows(plain, bias, silu), summand=summand)
+    w, s, x, _, _ = prompt_case(orc, n, k, rows, gate_up=True)
+    check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=ops.EPI_GATE_UP_SILU, prompt_kernel=kernel)["y"],
+               orc.int8_gate_up_silu_rows(w, s, x))
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
+@pytest.mark.parametrize("n,k,rows,gate_up", [(2048, 6144, 700, False), (4096, 2048, 1200, False), (2048, 2048, 2048, False), (6144, 2048, 600, True)])
+def test_prompt_kernels_over_several_waves(q3t, orc, ops, n, k, rows, gate_up):
+    """More CTAs than the GPU holds at once, at the talker's shapes; rows are compared with the lockstep kernel's, each within
+    a rounding step of the other (both sum in fp32, in another order), and the choice by estimate is one of the three."""
+    w, s, x, _, base = prompt_case(orc, n, k, rows, gate_up)
+    args = dict(epilogue=ops.EPI_GATE_UP_SILU) if gate_up else dict(epilogue=ops.EPI_ADD, y_in=base)
+    outs = [ops.int8_gemm(w, s, x, prompt_kernel=i, **args)["y"] for i in (0, 1, 2, 3)]
+    blocks = np.concatenate([ops.int8_gemm(w, s, x[i:i + 64], **dict(args, **({} if gate_up else {"y_in": base[i:i + 64]})))["y"]
+                             for i in range(0, rows, 64)])
+    for out in outs:
+        check_bf16(orc, out, blocks, summand=None if gate_up else base)
+    assert any(np.array_equal(outs[0], out) for out in outs[1:])
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
+def test_prompt_kernels_refuse(ops, orc):
+    w, s, x, bias, base = prompt_case(orc, 128, 128, 65)
+    for bad in (dict(epilogue=ops.EPI_BIAS_ADD, bias=bias, resid=base), dict(want_f32=True), dict(epilogue=ops.EPI_BIAS)):
+        for kernel in (1, 2):
+            with pytest.raises(RuntimeError):
+                ops.int8_gemm(w, s, x, prompt_kernel=kernel, **bad)
+    with pytest.raises(RuntimeError):
+        ops.int8_gemm(w[:, :64].copy(), s, x[:, :64].copy(), prompt_kernel=1)      # K in steps of 128
+    with pytest.raises(RuntimeError):
+        ops.int8_gemm(w, s, np.resize(x, (2049, 128)), prompt_kernel=1)
