@@ -933,6 +933,8 @@ void enqueue_predictor(Workspace& w, Model& m, int n, cudaStream_t s) {
             h.w = m.predictor_heads[p - 1].data; h.scales = m.predictor_heads[p - 1].scales;
             h.x = w.hidden.as<bf16>(); h.y = w.logits.as<bf16>(); h.norm_w = m.predictor_norm;
             h.in_features = PH; h.out_features = kPredictorVocab; h.rows = n; h.epilogue = EPI_PLAIN;
+            // (not the tensor-core path's own buffer: another model may be running on the device)
+            if (n >= tc_min_rows()) h.norm_out = w.normalized.as<bf16>();
             check_launch(launch_int8_gemm(h, s), "predictor head");
             check_launch(launch_sample_table(table, w.logits.as<bf16>(), kPredictorVocab,
                                            kPredictorVocab, 0, p, 0, kEos, n, s),

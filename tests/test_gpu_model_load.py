@@ -104,3 +104,25 @@ def test_without_memory_for_the_chain_and_for_long_passes(q3t, gpu_model, checkp
         gpu_model.set_option("prefill_chunk", 2048)
         lib.q3t_test_fail_allocation_after(0)
         replica.close()
+
+
+def test_two_models_on_one_device(q3t, gpu_model, checkpoint):
+    """Two replicas that decode at the same time from threads of their own, in large batches (tensor cores, norms as launches of
+    their own) and in small ones (decode chain), decode what each decodes alone: nothing that a frame writes is shared."""
+    import threading
+    replica = replica_of(q3t, gpu_model, checkpoint.keys())
+    try:
+        replica.finalize()
+        for sessions in (12, 3):
+            want = frames(q3t, gpu_model, sessions, count=25)
+            for _ in range(3):
+                got = {}
+                threads = [threading.Thread(target=lambda i=i, m=m: got.__setitem__(i, frames(q3t, m, sessions, count=25)))
+                           for i, m in enumerate((gpu_model, replica))]
+                for t in threads:
+                    t.start()
+                for t in threads:
+                    t.join()
+                assert same(got[0], want) and same(got[1], want)
+    finally:
+        replica.close()
