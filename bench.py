@@ -566,8 +566,8 @@ def run_ours(args, rank: int, local_rank: int, world: int) -> None:
         runs = gemv_runs
         g = runs[len(runs) // 2]
         gemv_s = g.mean_launch_microseconds * 1e-6
-        line["roofline"] = {"bound": "hbm", "kernel": "gemv_mma_kernel<4,false,false,1> 2048->6144 (configs[0]); the kernel the B=1 frame "
-                                      "dispatches for all its projections (gemv mode 1)",
+        line["roofline"] = {"bound": "hbm", "kernel": "gemv_mma_kernel<4,false,false,1> 2048->6144 (configs[0]): projections of 1..8 rows as "
+                                      "operator calls and in frames made launch by launch (gemv mode 1)",
                             "achieved": GEMV_BYTES / gemv_s / 1e9, "peak": hbm_peak, "unit": "GB/s",
                             "frac": GEMV_BYTES / gemv_s / 1e9 / hbm_peak, "peak_kind": peak_kind,
                             "frac_of_8TBs": GEMV_BYTES / gemv_s / 8.0e12,

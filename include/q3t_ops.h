@@ -67,7 +67,8 @@ typedef struct Q3tGemmDesc {
     uint16_t* output;            /* [rows][out_features] */
     float* output_f32;           /* optional: the fp32 value before the last bf16 round */
     const uint16_t* norm_weight; /* optional: RMSNorm(input) * norm_weight feeds the GEMM */
-    uint16_t* norm_output;       /* optional: the normalized rows */
+    uint16_t* norm_output;       /* optional: the normalized rows (without it, calls of 9 and more rows on
+                                  * one device share a buffer for them and have to be ordered) */
     const uint16_t* bias;        /* bias epilogues */
     uint16_t* residual;          /* Q3T_EPI_BIAS_ADD */
     int32_t in_features;

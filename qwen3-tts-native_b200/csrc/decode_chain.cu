@@ -16,12 +16,15 @@
 //                                                                                  -> exchange over the grid
 //     gate/up, SiLU  1/16 of the group's eighth of the channels, all of K         -> exchange in the group
 //     down           partial sums over the group's channels                       -> exchange over the grid
-//   Four exchanges a layer (five where pages are spread) instead of five launches.
+//   Dependent hand-overs a layer, instead of five launches: an exchange over the grid is one hop where every CTA adds up
+//   all columns itself (the predictor at one row) and two elsewhere (partial sums, then the new hidden rows in the
+//   group); talker attention adds one (pages' partials), with several rows two (folded heads).  Predictor 4 at one row
+//   and 6 at more, talker 7 and 8.
 //
 // The eight partial sums of a K-split projection are the eight K-slices that gemv_int8_mma.cu gives its eight
 // warps: same fixed-point conversion per slice, exact integer sums, the slices added in the same order.
-// A frame made here is bit for bit the frame made launch by launch, and a row's result does not depend on
-// the rows beside it.
+// A frame made here is bit for bit the frame made launch by launch with attention_blocks.cu for the talker's
+// attention, and a row's result does not depend on the rows beside it.
 //
 // Exchanges carry their own flags: a 16-byte store holds three words of data and the exchange's number, the
 // reader polls the data itself (single-copy atomic 128-bit relaxed accesses), so a hand-over is one trip
