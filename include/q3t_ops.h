@@ -185,7 +185,8 @@ typedef struct Q3tTensorImage {
 QWEN3_TTS_API int32_t q3t_model_tensor_image(Qwen3TtsModelHandle model, const char* name,
                                              Q3tTensorImage* image, char* error, size_t error_capacity);
 /* Declares the tensor's device storage filled by the caller; counts like an upload (a second
- * upload or adoption of the same name is an error, as in the reference's upload path). */
+ * upload or adoption of the same name is an error, as in the reference's upload path).  The fill has to be
+ * enqueued, on any stream, before qwen3_tts_model_finalize is called, which waits for it. */
 QWEN3_TTS_API int32_t q3t_model_adopt_tensor(Qwen3TtsModelHandle model, const char* name, char* error,
                                              size_t error_capacity);
 
