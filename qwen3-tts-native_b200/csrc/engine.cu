@@ -1386,9 +1386,9 @@ Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int spli
 
 // Enqueues one frame for rows s[0..n) on w.stream.  The host table must be filled.
 void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool upload_table,
-                           bool record_session_events) {
+                           bool record_session_events, int ahead) {
     int max_length = 1;
-    for (int i = 0; i < n; ++i) max_length = std::max(max_length, w.host_table->position[i] + 1);
+    for (int i = 0; i < n; ++i) max_length = std::max(max_length, w.host_table->position[i] + ahead + 1);
     const int splits = split_bucket(max_length);
     ++w.frame_serial;
     if (w.option_epoch != m.option_epoch) {
@@ -1758,9 +1758,7 @@ void Session::run_frames(Model* model, Session** s, int n, int frames, int trail
         for (cudaEvent_t& ev : marks) check_cuda(cudaEventCreate(&ev), "cudaEventCreate(frame mark)");
         check_cuda(cudaEventRecord(marks[0], w.stream), "cudaEventRecord(frame mark)");
         for (int f = 0; f < frames; ++f) {
-            // the device table advances itself; the host mirror follows for the graph key
-            launch_frame(w, *model, s, n, f == 0, false);
-            for (int i = 0; i < n; ++i) w.host_table->position[i] += 1;
+            launch_frame(w, *model, s, n, f == 0, false, f);        // the device table advances itself
             check_cuda(cudaEventRecord(marks[f + 1], w.stream), "cudaEventRecord(frame mark)");
         }
         check_cuda(cudaStreamSynchronize(w.stream), "cudaStreamSynchronize(frame loop)");

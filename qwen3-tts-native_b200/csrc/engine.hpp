@@ -342,8 +342,10 @@ private:
     static void bind_rows(Workspace& w, Session** s, int n);
     enum class Way { kChain, kInItsPlace, kLaunches };      // of a frame
     static Workspace::Graphs& frame_graphs(Workspace& w, Model& m, int n, int splits, Way way);
+    // `ahead`: frames enqueued since the host table was filled (their rows advance on the device; the host table stays as
+    // it is, since its upload may not have run yet)
     static void launch_frame(Workspace& w, Model& m, Session** s, int n, bool upload_table,
-                             bool record_session_events);
+                             bool record_session_events, int ahead = 0);
 
     std::shared_ptr<Model> model_;
     const uint64_t id_;             // unique for the life of the process

@@ -170,3 +170,35 @@ def test_frames_do_not_depend_on_what_else_runs(q3t, model):
         for i in some:
             assert got.get(i) == quiet[i], (some, i)
     assert q3t.library().q3t_kernel_error_count() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 3, 12])
+def test_frame_loop_behind_other_frames(q3t, model, rows):
+    """A frame loop whose stream has to wait for frames of other sessions: its rows start where they are, not where the host,
+    which is done enqueueing by then, has counted them to."""
+    model.set_option("decode_chain", 1)
+
+    def run(others):
+        busy = []
+        for i in range(others):
+            b = model.create_session(256, 800 + i)
+            b.synthetic_prefill(200, 800 + i)
+            busy.append((b, b.begin_device_frame(3)))
+        ss = []
+        for i in range(rows):
+            s = model.create_session(64 + 40 * i + 32, 60 + i)
+            s.synthetic_prefill(20 + 40 * i, 60 + i)
+            ss.append(s)
+        for b, p in busy:
+            p.finish_without_consumer()
+        pending = [b.begin_device_frame(3) for b, _ in busy]
+        model.run_frames(ss, 9, 11)
+        out = [tuple(np.array(x).tobytes() for x in s.read_state()) for s in ss]
+        for p in pending:
+            p.finish_without_consumer()
+        for s in ss + [b for b, _ in busy]:
+            s.close()
+        return out
+
+    quiet = run(0)
+    assert run(1) == quiet and run(2) == quiet and run(4) == quiet
