@@ -1,9 +1,9 @@
 // Int8 weight-only GEMM for the passes of a prompt: 65 to 2048 activation rows on the 5th-generation
 // tensor cores.
 //
-// Same operation as gemm_int8_tc.cu and the same epilogues but the bias with a residual, which no prompt has, without
-// its split of K: there are enough output tiles here to fill the GPU.  A CTA owns NT tiles of 128 output channels (TMEM
-// lanes) by 128 activation rows (TMEM columns).
+// Same operation and epilogues as gemm_int8_tc.cu, without its split of K: there are enough output
+// tiles here to fill the GPU.  A CTA owns NT tiles of 128 output channels (TMEM lanes) by 128
+// activation rows (TMEM columns).
 //
 // What bounds it: the tensor cores, if the operands arrive in time.  Per element of K a CTA with NT
 // = 2 fetches 256 bytes of weights and 256 bytes of activations for 8 cycles of MMA (4096 bf16 MACs a
@@ -56,6 +56,7 @@ struct WideParams {
     const float* scales;
     bf16* y;
     const bf16* bias;
+    bf16* resid;
     int out_features;       // N (gate/up: channels, the matrix has 2N rows)
     int rows;
     int row_blocks;
@@ -241,8 +242,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         const int first_row = row_base + group * kShare;
         const int rows_here = min(kShare, p.rows - first_row);
         const bool up_lane = GATEUP && NT == 1 && t >= 64;
-        const bool adds = !GATEUP && p.epilogue == EPI_ADD;
-        bf16* out = p.y + (size_t)first_row * N;
+        const bool adds = !GATEUP && (p.epilogue == EPI_ADD || p.epilogue == EPI_BIAS_ADD);
+        bf16* out = (p.epilogue == EPI_BIAS_ADD ? p.resid : p.y) + (size_t)first_row * N;
         bf16 base[kShare];
         auto fetch_bases = [&](int channel) {
 #pragma unroll
@@ -304,6 +305,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
                             } else {
                                 val = rbf(v[j] * scale) + bias;
                                 if (p.epilogue == EPI_BIAS_SILU) val = __fdividef(val, 1.0f + __expf(-val));
+                                else if (p.epilogue == EPI_BIAS_ADD) val = bf2f(base[c0 + j]) + rbf(val);
                             }
                             if (channel < N && c0 + j < rows_here) dst[(size_t)(c0 + j) * N] = f2bf(val);
                         }
@@ -352,14 +354,14 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
     const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
     if (a.rows < 1 || a.rows > kMaxPromptRows || a.out_features < 1 || a.in_features % kBK != 0 || a.in_features < kBK
         || a.w == nullptr || a.scales == nullptr || a.x == nullptr || a.norm_w != nullptr || a.y32 != nullptr
-        || a.y == nullptr || a.epilogue == EPI_BIAS_ADD) {
+        || (a.epilogue == EPI_BIAS_ADD ? a.resid == nullptr : a.y == nullptr)) {
         return cudaErrorInvalidValue;
     }
-    if ((a.epilogue == EPI_BIAS || a.epilogue == EPI_BIAS_SILU) && a.bias == nullptr) {
+    if ((a.epilogue == EPI_BIAS || a.epilogue == EPI_BIAS_SILU || a.epilogue == EPI_BIAS_ADD) && a.bias == nullptr) {
         return cudaErrorInvalidValue;
     }
     WideParams p;
-    p.scales = a.scales; p.y = a.y; p.bias = a.bias;
+    p.scales = a.scales; p.y = a.y; p.bias = a.bias; p.resid = a.resid;
     p.out_features = a.out_features; p.rows = a.rows; p.epilogue = a.epilogue;
     p.row_blocks = (a.rows + kTileM - 1) / kTileM;
     p.steps = a.in_features / kBK;
@@ -405,8 +407,7 @@ cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     };
     const float one = waves(1) * (a.epilogue == EPI_GATE_UP_SILU ? 6.0f + 0.50f * steps : 4.3f + 0.50f * steps);
     const float two = waves(2) * (5.5f + 0.82f * steps);
-    // (a bias with a residual, which no prompt has, exists there only)
-    if (a.epilogue == EPI_BIAS_ADD || gemm_tc_estimate_us(a) <= (one < two ? one : two)) return launch_int8_gemm_tc(a, stream);
+    if (gemm_tc_estimate_us(a) <= (one < two ? one : two)) return launch_int8_gemm_tc(a, stream);
     return launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
 }
 

@@ -136,6 +136,9 @@ def test_prompt_kernels(q3t, orc, ops, kernel, n, k, rows):
     for epilogue, silu in ((ops.EPI_BIAS, False), (ops.EPI_BIAS_SILU, True)):
         check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=epilogue, bias=bias, prompt_kernel=kernel)["y"],
                    orc.bias_activation_rows(plain, bias, silu), summand=summand)
+    got = ops.int8_gemm(w, s, x, epilogue=ops.EPI_BIAS_ADD, bias=bias, resid=base, prompt_kernel=kernel)["resid"]
+    check_bf16(orc, got, orc.add(base, orc.bias_activation_rows(plain, bias, False)).reshape(rows, n),
+               summand=orc.to_bf16(np.maximum(np.abs(orc.from_bf16(base)), orc.from_bf16(summand)).astype(np.float32)))
     w, s, x, _, _ = prompt_case(orc, n, k, rows, gate_up=True)
     check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=ops.EPI_GATE_UP_SILU, prompt_kernel=kernel)["y"],
                orc.int8_gate_up_silu_rows(w, s, x))
@@ -159,7 +162,7 @@ def test_prompt_kernels_over_several_waves(q3t, orc, ops, n, k, rows, gate_up):
 
 def test_prompt_kernels_refuse(ops, orc):
     w, s, x, bias, base = prompt_case(orc, 128, 128, 65)
-    for bad in (dict(epilogue=ops.EPI_BIAS_ADD, bias=bias, resid=base), dict(want_f32=True), dict(epilogue=ops.EPI_BIAS)):
+    for bad in (dict(epilogue=ops.EPI_BIAS_ADD, bias=bias), dict(want_f32=True), dict(epilogue=ops.EPI_BIAS)):
         for kernel in (1, 2):
             with pytest.raises(RuntimeError):
                 ops.int8_gemm(w, s, x, prompt_kernel=kernel, **bad)
