@@ -386,10 +386,10 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
 // to 6 us of start and epilogue; the 64-row kernel of gemm_int8_tc.cu, its row blocks side by side and K split where
 // that fits one wave, is estimated there.  For the talker's shapes that puts the lines at 65 rows (gate/up; two tiles
 // from 129), 257 (q/k/v; two tiles from 513) and 577 (o, down and the text projection; two tiles from about 1,200).
-// Measured from 65 to 2000 rows (us, row blocks / one tile / two tiles): gate/up 128 rows 21.1 / 15.6 / 18.1, 129
-// 21.4 / 27.0 / 18.5; q/k/v 256 12.1 / 12.6 / 19.4, 257 18.6 / 13.1 / 19.3; down 576 27.1 / 29.8 / 47.7, 577
-// 45.8 / 30.0 / 47.7.  The choice is within 4 % of the best everywhere but for o between 384 and 576 rows (6 to 11 %:
-// 13.4 to 14.1 us against 12.4 to 12.7 by one tile).
+// Measured from 65 to 2000 rows (us, row blocks / one tile / two tiles): gate/up 128 rows 20.7 / 15.4 / 17.9, 129
+// 21.3 / 27.0 / 18.2; q/k/v 256 11.8 / 11.7 / 18.4, 257 18.4 / 12.4 / 18.2; down 576 26.4 / 29.4 / 45.1, 577
+// 45.7 / 29.2 / 45.1.  The choice is within 2 % of the best everywhere but for o between 384 and 576 rows (3 to 6 %:
+// 13.1 to 13.9 us against 12.7 to 13.3 by one tile).
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     GemvArgs a = args;
     if (a.norm_w != nullptr) {
