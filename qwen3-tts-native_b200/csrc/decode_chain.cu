@@ -34,9 +34,8 @@
 //
 // Weights: at load time every CTA's share is laid out as one contiguous stream in the order the chain uses
 // it, each 1 KB block holding the MMA fragments of 16 rows x 64 K as the lanes read them.  It flows through a
-// ring in shared memory in 8 KB bulk copies, each requested by the warp that empties its slot, as far ahead
-// as the ring reaches, so that HBM (talker) or the L2 (predictor) keeps delivering while the CTAs wait for
-// each other.
+// ring in shared memory in 8 KB bulk copies, requested by a warp of their own as far ahead as the ring
+// reaches, so that HBM (talker) or the L2 (predictor) keeps delivering while the CTAs wait for each other.
 //
 // The launch is cooperative (all CTAs resident or none) and the engine orders the chains of a device one
 // after the other.  Every wait is bounded by a deadline; a wait that gives up marks the run, all others then
@@ -59,7 +58,12 @@ using tc::smem_u32;
 constexpr int kSlices = 8;
 constexpr int kRanks = 16;
 constexpr int kCtas = kSlices * kRanks;
-constexpr int kWorkers = 256;                        // eight warps: two per scheduler, so a thread may hold 255 registers
+constexpr int kWorkers = 256;                        // eight warps that compute
+constexpr int kThreads = kWorkers + 4 * kWarp;       // and a group of four, one of which requests weights
+// Registers are handed out to groups of four warps: 168 a thread at launch, 232 to those that compute and 40 to the others
+// (256 * 232 + 128 * 40 = 384 * 168).
+constexpr int kWorkerRegisters = 232, kRequestRegisters = 40;
+static_assert(kWorkers * kWorkerRegisters + 4 * kWarp * kRequestRegisters <= kThreads * 168, "registers of the block");
 constexpr int kSlot = 8192;                          // bytes of a ring slot
 constexpr int kSlotUnits = 4;                        // a slot is free once all of its 2 KB units have been read
 constexpr int kLimbs = 3;
@@ -102,17 +106,16 @@ struct alignas(16) Quad {
 };
 constexpr int kPartQuads = 2 * kSlices * kRanks * kRowsMost * 48;
 constexpr int kHiddenQuads = 2 * kSlices * kRanks * kRowsMost * 24;
-constexpr int kQkvQuads = 2 * kSlices * kRanks * kRowsMost * 6;
-constexpr int kActQuads = 2 * kSlices * kRanks * kRowsMost * 8;
+constexpr int kGroupRow = 8;                         // quads of a CTA's q/k/v rows (6) or gate/up channels (4 or 8) of an activation row
+constexpr int kGroupQuads = 2 * kSlices * kRanks * kRowsMost * kGroupRow;
 constexpr int kAttnPartQuads = 2 * kSlices * kRanks * kRowsMost * 88;
 constexpr int kAttnQuads = 2 * kSlices * kRanks * 22;
 constexpr int kLogitQuads = 2 * kCtas * kRowsMost * 3;
 constexpr int kTokenQuads = 2 * kRowsMost;
 constexpr int kAppendedQuads = 2 * kSlices * kRowsMost;
 constexpr int kAtHidden = kPartQuads;
-constexpr int kAtQkv = kAtHidden + kHiddenQuads;
-constexpr int kAtAct = kAtQkv + kQkvQuads;
-constexpr int kAtAttnPart = kAtAct + kActQuads;
+constexpr int kAtGroup = kAtHidden + kHiddenQuads;
+constexpr int kAtAttnPart = kAtGroup + kGroupQuads;
 constexpr int kAtAttn = kAtAttnPart + kAttnPartQuads;
 constexpr int kAtLogits = kAtAttn + kAttnQuads;
 constexpr int kAtTokens = kAtLogits + kLogitQuads;
@@ -190,7 +193,7 @@ struct Layout {
     static constexpr int UBytesC = TALKER && ROWS == 1 ? 16 * 2 * 132 * 4 : 0;     // gathered attention partials
     static constexpr int UBytes = UBytesA > UBytesB ? (UBytesA > UBytesC ? UBytesA : UBytesC) : (UBytesB > UBytesC ? UBytesB : UBytesC);
     static constexpr int QkvBytes = ROWS * 1024;                   // [rows][512] bf16; also [rows][256] fp32 partial squares
-    static constexpr int AttBytes = ROWS * 512;                    // [rows][256] bf16
+    static constexpr int AttBytes = ROWS * S::Slice * 2;           // [rows][256] bf16, each row as long as one of the next
     static constexpr int ActBytes = ROWS * S::Slice * 2;           // [rows][Slice] bf16
     static constexpr bool OneHop = !TALKER && ROWS == 1;           // every CTA sums all columns itself
     static constexpr int OwnBytes = OneHop ? S::H * 2 : ROWS * S::Out * 2;
@@ -210,7 +213,13 @@ struct Layout {
     static constexpr int AtSample = AtStage + StageBytes;
     static constexpr int AtMisc = AtSample + (SampleBytes + 15) / 16 * 16;
     static constexpr int MiscBytes = 1024;
-    static constexpr int AtRing = (AtMisc + MiscBytes + 127) / 128 * 128;
+    // One or two rows of the predictor: every CTA of a group keeps the group's cache, one page of 16 tokens a layer, to
+    // itself (K as rows, V with the tokens of a dimension side by side): nothing to fetch, nothing to publish.
+    static constexpr bool LocalKv = !TALKER && ROWS <= 2;
+    static constexpr int KvPage = 2 * kPageTokens * 128 * 2;
+    static constexpr int AtConst = AtMisc + MiscBytes;             // the layers' constants
+    static constexpr int AtKv = (AtConst + S::Layers * (int)sizeof(LayerConst) + 127) / 128 * 128;
+    static constexpr int AtRing = AtKv + (LocalKv ? ROWS * S::Layers * KvPage : 0);
     static constexpr int Budget = 227 * 1024;
     static constexpr int SlotsFit = (Budget - AtRing) / kSlot;
     static constexpr int Slots = SlotsFit > 24 ? 24 : SlotsFit;
@@ -224,14 +233,16 @@ struct Layout {
 
 struct Misc {
     uint64_t full[24];
+    uint64_t empty[24];            // counts the units of the slot that have been read
     unsigned int asked[24];        // copies requested into the slot
-    unsigned int read[24];         // units of the slot read so far
     uint32_t base;
     int abort;
     int position[kRowsMost];
     int token[kRowsMost];
     float unscale[kRowsMost];
+    float inverse[kRowsMost];      // of the rows' root mean squares
     unsigned long long rng[kRowsMost];
+    unsigned short codes[kRowsMost][kCodebooks];
 };
 static_assert(sizeof(Misc) <= 1024, "misc area");
 
@@ -307,7 +318,7 @@ struct Chain {
     uint32_t flips = 0;            // buffer in use, one bit per kind of exchange
     unsigned long long deadline = 0;
 
-    enum Kind { kPart = 0, kHid = 1, kQkv = 2, kAct = 3, kAttnPart = 4, kAttn = 5, kLogits = 6, kTokens = 7, kAppended = 8 };
+    enum Kind { kPart = 0, kHid = 1, kGroup = 2, kAttnPart = 4, kAttn = 5, kLogits = 6, kTokens = 7, kAppended = 8 };
 
     __device__ Chain(const ChainArgs& args, unsigned char* s)
         : a(args), smem(s), misc(reinterpret_cast<Misc*>(s + L::AtMisc)), tid(threadIdx.x), lane(threadIdx.x % kWarp),
@@ -380,45 +391,66 @@ struct Chain {
     // ---- ring ----------------------------------------------------------------------------------------------
     static constexpr uint32_t kLayerSlots = S::Layers * S::LayerSlots;
     static constexpr uint32_t kAllSlots = TALKER ? kLayerSlots + S::HeadSlots : kCodebooks * kLayerSlots + 15 * S::HeadSlots;
-    // requests slot `s` of the CTA's stream into the ring (one thread)
-    __device__ __forceinline__ void request(uint32_t s) {
-        if (s >= kAllSlots || given_up()) return;
-        const uint8_t* src;
+    // The requesting warp's one thread: slot after slot of the CTA's stream, each once what lay in its place has been read.
+    __device__ __forceinline__ void request_weights() {
         const uint8_t* layers = a.stream + (size_t)blockIdx.x * S::Layers * S::LayerBytes;
-        if (TALKER) {
-            src = s < kLayerSlots ? layers + (size_t)s * kSlot
-                                  : a.heads + (size_t)blockIdx.x * S::HeadBytes + (size_t)(s - kLayerSlots) * kSlot;
-        } else {
-            // position 0 has no head; position p >= 1 ends with head p - 1
-            const uint32_t t = s < kLayerSlots ? s : s - kLayerSlots;
-            const uint32_t p = s < kLayerSlots ? 0u : t / (kLayerSlots + S::HeadSlots) + 1u;
-            const uint32_t in = s < kLayerSlots ? s : t % (kLayerSlots + S::HeadSlots);
-            src = in < kLayerSlots ? layers + (size_t)in * kSlot
-                                   : a.heads + ((size_t)blockIdx.x * 15 + (p - 1)) * S::HeadBytes + (size_t)(in - kLayerSlots) * kSlot;
+        const uint8_t* heads = a.heads + (size_t)blockIdx.x * (TALKER ? 1 : 15) * S::HeadBytes;
+        // the layers, then a head; the predictor's sixteen positions all read the layers, and position 0 has no head
+        const uint8_t* src = layers;
+        uint32_t left = kLayerSlots, at = 0, fill = 0;
+        bool in_layers = true, headless = !TALKER;
+#pragma unroll 1
+        for (uint32_t s = 0; s < kAllSlots; ++s) {
+            uint64_t* bar = &misc->full[at];
+            if (fill > 0) {
+                for (uint32_t polls = 0; !mbar_try_wait(&misc->empty[at], (fill - 1) & 1u);) {
+                    if ((++polls & 15u) == 0u && slow_check()) return;
+                }
+            }
+            *reinterpret_cast<volatile unsigned int*>(&misc->asked[at]) = fill + 1;
+            mbar_expect_tx(bar, kSlot);
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                ::"r"(smem_u32(smem + L::AtRing + at * kSlot)), "l"(src), "r"(kSlot), "r"(smem_u32(bar))
+                : "memory");
+            src += kSlot;
+            if (++at == L::Slots) {
+                at = 0;
+                ++fill;
+            }
+            if (--left == 0) {
+                if (in_layers && !headless) {
+                    src = heads;
+                    heads += S::HeadBytes;
+                    left = S::HeadSlots;
+                    in_layers = false;
+                } else {
+                    src = layers;
+                    left = kLayerSlots;
+                    in_layers = true;
+                    headless = false;
+                }
+            }
         }
-        uint64_t* bar = &misc->full[s % L::Slots];
-        misc->asked[s % L::Slots] = s / L::Slots + 1;
-        mbar_expect_tx(bar, kSlot);
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-            ::"r"(smem_u32(smem + L::AtRing + (s % L::Slots) * kSlot)), "l"(src), "r"(kSlot), "r"(smem_u32(bar))
-            : "memory");
     }
-    // Gives back bytes [off, off + len) of the phase that started at slot `first`, lane i the i-th slot touched.  Who
-    // reads the last 2 KB of a slot requests what comes into it next.
+    // Gives back bytes [off, off + len) of the phase that started at slot `first`, lane i the i-th slot touched.
     __device__ __forceinline__ void release(uint32_t first, uint32_t off, uint32_t len) {
         __syncwarp();
         const uint32_t lo = off / kSlot, hi = (off + len - 1) / kSlot;
         if (lo + lane <= hi) {
-            const uint32_t at = max(off, (lo + lane) * kSlot), end = min(off + len, (lo + lane + 1) * kSlot);
-            const uint32_t units = (end - at) / (kSlot / kSlotUnits);
-            const uint32_t s = first + lo + lane;
-            const unsigned int before = atomicAdd(&misc->read[s % L::Slots], units);
-            if ((before + units) % kSlotUnits == 0u) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                request(s + L::Slots);
-            }
+            const uint32_t from = max(off, (lo + lane) * kSlot), end = min(off + len, (lo + lane + 1) * kSlot);
+            give_back(first + lo + lane, (end - from) / (kSlot / kSlotUnits));
         }
+    }
+    __device__ __forceinline__ void give_back(uint32_t s, uint32_t units) {
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&misc->empty[s % L::Slots])), "r"(units) : "memory");
+    }
+    // The predictor's ring is deeper than a layer: one warp gives back everything up to slot `end` behind a barrier that all
+    // readers have met at, instead of every warp its own on the way from one exchange to the next.
+    uint32_t given_back = 0;
+    __device__ __forceinline__ void release_all(uint32_t end) {
+        if (warp == kWorkers / kWarp - 1 && given_back + lane < end) give_back(given_back + lane, kSlotUnits);
+        given_back = end;
     }
 
     // ---- MMA -----------------------------------------------------------------------------------------------
@@ -445,76 +477,124 @@ struct Chain {
             part[half] *= unscale;
         }
     }
-    // Projection over all of K: warp w has K-slice w of every row; its sums go to red[w][row][16 TILES].  G tiles side by
-    // side.  The weights' slots are given back by the caller (release_full), off the critical path, except where the
-    // phase fills much of the ring (the talker's gate/up): there each warp gives its own back at once, since what it
-    // waits for may have to come into the slots of the others.
-    template <int TILES>
-    static constexpr bool kReleaseEarly = 2 * TILES * S::J > L::Slots;       // TILES * J: slots of the phase
-    template <int TILES, int G>
-    __device__ __forceinline__ void mma_full(float unscale_mine) {
-        constexpr uint32_t kTile = S::J * 1024;                 // a tile's blocks lie in one slot
-        const uint32_t off = warp * (TILES * kTile);
-        float* red = reinterpret_cast<float*>(smem + L::AtU) + (size_t)warp * rows * (TILES * 16);
+    // Projection over all of K: warp w has K-slice w of every row; its sums go to red[w][row][kRedRow].  `tiles` is not known
+    // to the compiler, so that all projections of this kind share one copy of the code.
+    //
+    // kAhead: one or two rows of the predictor take the weights of a projection and of the K-split one behind it from the ring
+    // to registers while the exchange before them is under way.  The wait for a slot (110 cycles, data there or not) and the
+    // reads then cost nothing between one exchange and the next (a predictor layer at one row 18.2 -> 16.9 thousand cycles).
+    static constexpr int kRedRow = L::RedRows;
+    static constexpr bool kAhead = !TALKER && ROWS <= 2;
+    static constexpr int kSide = TALKER ? 2 : S::GuTiles;      // tiles side by side (the predictor: all of a phase)
+    static constexpr int kSliceBlocks = S::Slice / 64;         // of the down projection; the o projection has 4
+    static constexpr int kSliceSide = TALKER ? 2 : kSliceBlocks;
+    static constexpr uint32_t kTile = S::J * 1024;              // a tile's blocks lie in one slot
+    // A phase longer than the ring: its later slots come in only once the earlier ones of other warps have been used.
+    static constexpr bool kWraps = S::GuTiles * S::J > L::Slots;
+    static_assert(S::OutTiles * kSliceBlocks <= 8 * L::Slots && (TALKER || 2 * S::LayerSlots / 3 <= L::Slots), "phases held fit the ring");
+    int4 held_full[2 * kSide * S::J], held_slice[2 * kSliceSide];
+    __device__ __forceinline__ const int4* ring_at(uint32_t first, uint32_t at) {
+        return reinterpret_cast<const int4*>(smem + L::AtRing + (first + at / kSlot) % L::Slots * kSlot + at % kSlot) + lane;
+    }
+    __device__ __forceinline__ void hold_full(uint32_t first, int tiles, int t0) {
+        const uint32_t off = (warp * tiles + t0) * kTile;
+#pragma unroll
+        for (int i = 0; i < kSide; ++i) {
+            if (!TALKER && i >= tiles) break;
+            const uint32_t at = off + i * kTile;
+            if (i == 0 || at % kSlot < kTile) wait_slot<kWraps>(first + at / kSlot);
+            const int4* w = ring_at(first, at);
+#pragma unroll
+            for (int j = 0; j < 2 * S::J; ++j) held_full[2 * S::J * i + j] = w[kWarp * j];
+        }
+    }
+    __device__ __forceinline__ void hold_slice(uint32_t first, int blocks, int j0) {
+        // two blocks at a time: 2 KB units never cross a slot
+#pragma unroll
+        for (int j = 0; j < kSliceSide; j += 2) {
+            if (!TALKER && j >= blocks) break;
+            const uint32_t at = (warp % S::OutTiles * blocks + j0 + j) * 1024u;
+            if ((kAhead ? j : j0 + j) == 0 || at % kSlot == 0) wait_slot(first + at / kSlot);
+            const int4* w = ring_at(first, at);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) held_slice[2 * j + i] = w[kWarp * i];
+        }
+    }
+    // the weights of a layer's half, or of a head (blocks = 0)
+    __device__ __forceinline__ void hold_ahead(int tiles, int blocks) {
+        if constexpr (kAhead) {
+            hold_full(seq, tiles, 0);
+            if (blocks > 0 && warp < S::OutTiles) hold_slice(seq + tiles * S::J, blocks, 0);
+        }
+    }
+    __device__ __forceinline__ void mma_full(int tiles, float unscale_mine) {
+        float* red = reinterpret_cast<float*>(smem + L::AtU) + (size_t)warp * rows * kRedRow;
         const unsigned char* xs = smem + L::AtX + warp * 64 * S::J + 16 * (lane & 3);
         float u[NT];                                            // of the row this lane will hold: 2 q + t / 2
 #pragma unroll
         for (int q = 0; q < NT; ++q) u[q] = __shfl_sync(0xffffffffu, unscale_mine, 2 * q + ((lane >> 1) & 1));
 #pragma unroll 1
-        for (int t0 = 0; t0 < TILES; t0 += G) {
-            const int4* w[G];
+        for (int t0 = 0; t0 < tiles; t0 += kSide) {
+            if (!kAhead) hold_full(seq, tiles, t0);
+            constexpr int kChains = kSide * NT <= 4 ? 2 : 1;   // accumulators per tile (integers: any order)
+            int acc[kChains][kSide][NT][4];
 #pragma unroll
-            for (int i = 0; i < G; ++i) {
-                const uint32_t at = off + (t0 + i) * kTile;
-                if (i == 0 || at % kSlot < kTile) wait_slot<(TILES * S::J > L::Slots)>(seq + at / kSlot);
-                w[i] = reinterpret_cast<const int4*>(smem + L::AtRing + (seq + at / kSlot) % L::Slots * kSlot + at % kSlot) + lane;
-            }
-            constexpr int kChains = G * NT <= 4 ? 2 : 1;       // accumulators per tile (integers: any order)
-            int acc[G][NT][4], acc2[kChains == 2 ? G : 1][NT][4];
+            for (int c = 0; c < kChains; ++c)
 #pragma unroll
-            for (int i = 0; i < G; ++i)
-#pragma unroll
-                for (int q = 0; q < NT; ++q)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        acc[i][q][e] = 0;
-                        if (kChains == 2) acc2[kChains == 2 ? i : 0][q][e] = 0;
-                    }
-#pragma unroll
-            for (int j = 0; j < S::J; ++j) {
-                uint32_t b[NT][4];
-#pragma unroll
-                for (int q = 0; q < NT; ++q) load_b(xs + 64 * j, q, b[q]);
-#pragma unroll
-                for (int i = 0; i < G; ++i) {
-                    const int4 wa = w[i][64 * j], wb = w[i][64 * j + kWarp];
-#pragma unroll
-                    for (int q = 0; q < NT; ++q) {
-                        imma(acc[i][q], wa.x, wb.x, wa.y, wb.y, b[q][0], b[q][1]);
-                        if (kChains == 2) imma(acc2[kChains == 2 ? i : 0][q], wa.z, wb.z, wa.w, wb.w, b[q][2], b[q][3]);
-                        else imma(acc[i][q], wa.z, wb.z, wa.w, wb.w, b[q][2], b[q][3]);
-                    }
-                }
-            }
-            if (kChains == 2) {
-#pragma unroll
-                for (int i = 0; i < G; ++i)
+                for (int i = 0; i < kSide; ++i)
 #pragma unroll
                     for (int q = 0; q < NT; ++q)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) acc[i][q][e] += acc2[kChains == 2 ? i : 0][q][e];
+                        for (int e = 0; e < 4; ++e) acc[c][i][q][e] = 0;
+            // all of B first where the registers allow it (the talker's is twice as long)
+            uint32_t b[TALKER ? 1 : S::J][NT][4];
+            auto fetch_b = [&](int j) {
+#pragma unroll
+                for (int q = 0; q < NT; ++q) load_b(xs + 64 * j, q, b[TALKER ? 0 : j][q]);
+            };
+            auto multiply = [&](int i, int j) {
+                const int4 wa = held_full[2 * (S::J * i + j)], wb = held_full[2 * (S::J * i + j) + 1];
+#pragma unroll
+                for (int q = 0; q < NT; ++q) {
+                    const uint32_t (&bq)[4] = b[TALKER ? 0 : j][q];
+                    imma(acc[0][i][q], wa.x, wb.x, wa.y, wb.y, bq[0], bq[1]);
+                    imma(acc[kChains - 1][i][q], wa.z, wb.z, wa.w, wb.w, bq[2], bq[3]);
+                }
+            };
+            if (TALKER) {
+#pragma unroll
+                for (int j = 0; j < S::J; ++j) {
+                    fetch_b(j);
+#pragma unroll
+                    for (int i = 0; i < kSide; ++i) multiply(i, j);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < S::J; ++j) fetch_b(j);
+#pragma unroll
+                for (int i = 0; i < kSide; ++i) {
+                    if (i >= tiles) break;
+#pragma unroll
+                    for (int j = 0; j < S::J; ++j) multiply(i, j);
+                }
             }
-            if (kReleaseEarly<TILES> && t0 + G >= TILES) release(seq, off, TILES * kTile);
+            // the talker's gate/up is as long as its ring: what comes next has to come into its places at once
+            if (TALKER && tiles == S::GuTiles) release(seq, (warp * tiles + t0) * kTile, kSide * kTile);
             const int t = lane & 3;
 #pragma unroll
-            for (int q = 0; q < NT; ++q) {
-                const int row = 2 * q + (t >> 1);
+            for (int i = 0; i < kSide; ++i) {
+                if (!TALKER && i >= tiles) break;
 #pragma unroll
-                for (int i = 0; i < G; ++i) {
+                for (int q = 0; q < NT; ++q) {
+                    const int row = 2 * q + (t >> 1);
+                    if (kChains == 2) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[0][i][q][e] += acc[kChains - 1][i][q][e];
+                    }
                     float part[2];
-                    combine(acc[i][q], u[q], part);
+                    combine(acc[0][i][q], u[q], part);
                     if ((t & 1) == 0 && row < rows) {
-                        float* out = red + row * (TILES * 16) + (t0 + i) * 16 + (lane >> 2);
+                        float* out = red + row * kRedRow + (t0 + i) * 16 + (lane >> 2);
                         out[0] = part[0];
                         out[8] = part[1];
                     }
@@ -522,47 +602,50 @@ struct Chain {
             }
         }
     }
-    template <int TILES>
-    __device__ __forceinline__ void release_full() {
-        constexpr uint32_t kLen = TILES * S::J * 1024;
-        if (!kReleaseEarly<TILES>) release(seq, warp * kLen, kLen);
-        seq += 8 * kLen / kSlot;
+    // behind the barrier that joins the sums (predictor), or once they are on their way
+    __device__ __forceinline__ void end_full(int tiles) {
+        const uint32_t first = seq;
+        seq += tiles * S::J;
+        if (!TALKER) release_all(seq);
+        else if (tiles != S::GuTiles) release(first, warp * tiles * kTile, tiles * kTile);
     }
-    // K-split projection: warp w < OutTiles has 16 of the CTA's outputs over the whole slice and sends its partial
-    // sums to everybody: six quads of three columns per row.
+    // K-split projection: a warp has 16 of the CTA's outputs over the whole slice and sends its partial sums to everybody: six
+    // quads of three columns per row.  The predictor has four such tiles: with several column groups its warps w and w + 4
+    // share one, half of the groups each, with one the upper four are done without.
+    static constexpr int kShare = S::OutTiles == 4 && NT > 1 ? 2 : 1;
+    static constexpr int kSliceWarps = S::OutTiles * kShare;
     __device__ __forceinline__ void mma_slice(int blocks, int b, uint32_t flag) {
-        const uint32_t len = blocks * 1024u, off = warp * len;
-        if (warp < S::OutTiles) {
+        if (warp < kSliceWarps) {
+            constexpr int NQ = NT / kShare;
+            const int tile = warp % S::OutTiles, q0 = kShare == 1 ? 0 : warp / S::OutTiles * NQ;
             const unsigned char* xs = smem + L::AtX + 16 * (lane & 3);
-            int acc[2][NT][4];
+            int acc[2][NQ][4];
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int q = 0; q < NT; ++q)
+                for (int q = 0; q < NQ; ++q)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[i][q][e] = 0;
-            // two blocks at a time: 2 KB units never cross a slot
 #pragma unroll 1
-            for (int j = 0; j < blocks; j += 2) {
-                const uint32_t at = off + j * 1024u;
-                if (j == 0 || at % kSlot == 0) wait_slot(seq + at / kSlot);
-                const int4* w = reinterpret_cast<const int4*>(smem + L::AtRing + (seq + at / kSlot) % L::Slots * kSlot + at % kSlot) + lane;
+            for (int j0 = 0; j0 < blocks; j0 += kSliceSide) {
+                if (!kAhead) hold_slice(seq, blocks, j0);
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int4 wa = w[64 * i], wb = w[64 * i + kWarp];
+                for (int j = 0; j < kSliceSide; ++j) {
+                    if (!TALKER && j >= blocks) break;
+                    const int4 wa = held_slice[2 * j], wb = held_slice[2 * j + 1];
 #pragma unroll
-                    for (int q = 0; q < NT; ++q) {
+                    for (int q = 0; q < NQ; ++q) {
                         uint32_t bf[4];
-                        load_b(xs + 64 * (j + i), q, bf);
-                        imma(acc[i][q], wa.x, wb.x, wa.y, wb.y, bf[0], bf[1]);
-                        imma(acc[i][q], wa.z, wb.z, wa.w, wb.w, bf[2], bf[3]);
+                        load_b(xs + 64 * (j0 + j), q0 + q, bf);
+                        imma(acc[j & 1][q], wa.x, wb.x, wa.y, wb.y, bf[0], bf[1]);
+                        imma(acc[j & 1][q], wa.z, wb.z, wa.w, wb.w, bf[2], bf[3]);
                     }
                 }
             }
 #pragma unroll
-            for (int q = 0; q < NT; ++q) {
+            for (int q = 0; q < NQ; ++q) {
                 const int t = lane & 3;
-                const int row = 2 * q + (t >> 1);
+                const int row = 2 * (q0 + q) + (t >> 1);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[0][q][e] += acc[1][q][e];
                 float part[2];
@@ -577,13 +660,13 @@ struct Chain {
                     const float hi = __shfl_sync(0xffffffffu, part[1], 4 * (c & 7) + 2 * pair);
                     v[e] = __float_as_uint(c < 8 ? lo : hi);
                 }
-                if (quad < 6 && 2 * q + pair < rows) {
-                    put_quad(part_at(b, slice, rank, 2 * q + pair) + warp * 6 + quad, v[0], v[1], v[2], flag);
+                if (quad < 6 && 2 * (q0 + q) + pair < rows) {
+                    put_quad(part_at(b, slice, rank, 2 * (q0 + q) + pair) + tile * 6 + quad, v[0], v[1], v[2], flag);
                 }
             }
-            release(seq, off, len);
+            if (TALKER) release(seq, warp * blocks * 1024u, blocks * 1024u);
         }
-        seq += (uint32_t)(S::OutTiles * blocks * 1024) / kSlot;
+        seq += (uint32_t)(S::OutTiles * blocks * 1024) / kSlot;         // (predictor: given back with the next phase)
     }
 
     // ---- norm and conversion ----------------------------------------------------------------------------------
@@ -591,24 +674,47 @@ struct Chain {
     __device__ __forceinline__ float norm_to_limbs(const uint32_t (&nw)[S::J], bf16* norm_out) {
         const bf16* hid = reinterpret_cast<const bf16*>(smem + L::AtU);
         float* partial = reinterpret_cast<float*>(smem + L::AtQkv);
-#pragma unroll(ROWS <= 2 ? ROWS : 2)
-        for (int r = 0; r < rows; ++r) {
-            float ss = 0.0f;
+        // thread t of the stand-alone kernel sums elements t, t + 256, ...
+        if (ROWS <= 2) {
 #pragma unroll
-            for (int i = 0; i < S::H / kWorkers; ++i) {
-                const float v = bf2f(hid[r * S::H + tid + i * kWorkers]);
-                ss = fmaf(v, v, ss);
+            for (int r = 0; r < ROWS; ++r) {
+                float ss = 0.0f;
+#pragma unroll
+                for (int i = 0; i < S::H / kWorkers; ++i) {
+                    const float v = bf2f(hid[r * S::H + tid + i * kWorkers]);
+                    ss = fmaf(v, v, ss);
+                }
+                partial[r * kWorkers + tid] = ss;
             }
-            partial[r * kWorkers + tid] = ss;
+            sync_workers();
+        } else {
+            // two such threads' sums to a thread, two rows at a time; then a warp per row instead of every warp every row
+            // (8 rows: a norm 4,370 cycles before)
+#pragma unroll 2
+            for (int r = tid >> 7; r < rows; r += 2) {
+                float lo = 0.0f, hi = 0.0f;
+#pragma unroll
+                for (int i = 0; i < S::H / kWorkers; ++i) {
+                    const uint32_t x = reinterpret_cast<const uint32_t*>(hid + r * S::H + i * kWorkers)[tid & 127];
+                    lo = fmaf(bf_lo(x), bf_lo(x), lo);
+                    hi = fmaf(bf_hi(x), bf_hi(x), hi);
+                }
+                reinterpret_cast<float2*>(partial + r * kWorkers)[tid & 127] = make_float2(lo, hi);
+            }
+            sync_workers();
+            if (warp < rows) {
+                const float total = tree_sum_256(partial + warp * kWorkers, lane);
+                if (lane == 0) misc->inverse[warp] = rsqrtf(total / static_cast<float>(S::H) + a.eps);
+            }
+            sync_workers();
         }
-        sync_workers();
         float unscale_mine = 1.0f;
         const int at = warp * 64 * S::J + 2 * S::J * lane;
         unsigned char* xs = smem + L::AtX;
-#pragma unroll(ROWS <= 2 ? ROWS : 2)
+#pragma unroll(ROWS <= 4 ? ROWS : 4)
         for (int r = 0; r < rows; ++r) {
-            const float total = tree_sum_256(partial + r * kWorkers, lane);
-            const float inv = rsqrtf(total / static_cast<float>(S::H) + a.eps);
+            const float inv = ROWS <= 2 ? rsqrtf(tree_sum_256(partial + r * kWorkers, lane) / static_cast<float>(S::H) + a.eps)
+                                        : misc->inverse[r];
             uint32_t raw[S::J];
             const uint32_t* src = reinterpret_cast<const uint32_t*>(hid + r * S::H + at);
 #pragma unroll
@@ -729,14 +835,15 @@ struct Chain {
                 store_group(mine, g, packed);
                 put_quad(group_at(kAtHidden, S::Groups, bh, rank, r) + g, packed[0], packed[1], packed[2], flag_h);
             }
-            // two quads at a time per thread
+            // a thread's quads, up to six, requested together
+            constexpr int kEach = (ROWS * kRanks * S::Groups + kWorkers - 1) / kWorkers < 6 ? (ROWS * kRanks * S::Groups + kWorkers - 1) / kWorkers : 6;
 #pragma unroll 1
-            for (int i = tid; i < kRanks * rows * S::Groups; i += 2 * kWorkers) {
-                const Quad* p[2];
-                Quad v[2];
-                int at[2], g[2];
+            for (int i = tid; i < kRanks * rows * S::Groups; i += kEach * kWorkers) {
+                const Quad* p[kEach];
+                Quad v[kEach];
+                int at[kEach], g[kEach];
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
+                for (int k = 0; k < kEach; ++k) {
                     const int n = min(i + k * kWorkers, kRanks * rows * S::Groups - 1);
                     g[k] = n % S::Groups;
                     const int r = n / S::Groups % rows, rk = n / S::Groups / rows;
@@ -745,7 +852,7 @@ struct Chain {
                 }
                 poll(p, v, flag_h);
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
+                for (int k = 0; k < kEach; ++k) {
                     const uint32_t packed[3] = {v[k].x, v[k].y, v[k].z};
                     store_group(hid + at[k], g[k], packed);
                 }
@@ -753,18 +860,28 @@ struct Chain {
         }
         sync_workers();
     }
-    // quads of six bf16 from every CTA of the group ([rank][row][per_row]) -> rows of `row_words` words in shared memory,
-    // rank after rank (`rank_words` words each)
-    template <int PerRow, int RankWords>
-    __device__ __forceinline__ void collect_group(int kind_base, int b, uint32_t flag, uint32_t* dst, int row_words) {
-#pragma unroll 1
-        for (int i = tid; i < kRanks * rows * PerRow; i += kWorkers) {
-            const int g = i % PerRow, r = i / PerRow % rows, rk = i / PerRow / rows;
-            const Quad v = poll_one(group_at(kind_base, PerRow, b, rk, r) + g, flag);
-            uint32_t* d = dst + r * row_words + rk * RankWords + 3 * g;
-            d[0] = v.x;
-            if (3 * g + 1 < RankWords) d[1] = v.y;
-            if (3 * g + 2 < RankWords) d[2] = v.z;
+    // quads of six bf16 from every CTA of the group ([rank][row][kGroupRow], the first per_row of them) -> rows of `row_words`
+    // words in shared memory, rank after rank (`rank_words` words each).  A thread's quads are requested together.
+    __device__ __forceinline__ void collect_group(int per_row, int rank_words, int b, uint32_t flag, uint32_t* dst, int row_words) {
+        constexpr int kEach = (ROWS * kRanks * kGroupRow + kWorkers - 1) / kWorkers;
+        const int g = tid % kGroupRow, rk = tid / kGroupRow % kRanks;
+        const Quad* p[kEach];
+        Quad v[kEach];
+        const int r0 = tid / (kGroupRow * kRanks);
+        if (g < per_row && r0 < rows) {
+#pragma unroll
+            for (int i = 0; i < kEach; ++i) p[i] = group_at(kAtGroup, kGroupRow, b, rk, min(r0 + 2 * i, rows - 1)) + g;
+            poll(p, v, flag);
+#pragma unroll
+            for (int i = 0; i < kEach; ++i) {
+                const int r = r0 + 2 * i;
+                if (r < rows) {
+                    uint32_t* d = dst + r * row_words + rk * rank_words + 3 * g;
+                    d[0] = v[i].x;
+                    if (3 * g + 1 < rank_words) d[1] = v[i].y;
+                    if (3 * g + 2 < rank_words) d[2] = v[i].z;
+                }
+            }
         }
         sync_workers();
     }
@@ -780,7 +897,7 @@ struct Chain {
         bf16 q[4], k[4];
     };
     // cos | sin of the head vectors this warp rotates: fixed for a launch (talker) or a position (predictor)
-    static constexpr int kJobs = (3 * ROWS + 7) / 8;
+    static constexpr int kJobs = L::LocalKv ? 1 : (3 * ROWS + 7) / 8;       // (LocalKv: the rows are at one position)
     uint32_t cs[kJobs][2];
     __device__ __forceinline__ void load_rotations() {
 #pragma unroll
@@ -825,7 +942,95 @@ struct Chain {
         reinterpret_cast<uint2*>(v)[lane] = reinterpret_cast<const uint2*>(vnew)[lane];
     }
 
-    // The predictor's caches are one page: warp r of every CTA of the group attends for row r.
+    // ---- the predictor's attention over pages in shared memory (LocalKv)
+    // 16-byte piece of K of token `t`: pieces of odd tokens change halves, so that a fragment load meets every bank once
+    static __device__ __forceinline__ int k_piece(int t, int piece) { return t * 256 + ((piece ^ ((t & 1) << 2)) << 4); }
+    // byte of V of token `t` behind its dimension's 32: the words of an MMA lane, tokens 2 tig (+ 1) and 8 more, lie together
+    static __device__ __forceinline__ int v_token(int t) { return ((t & 7) >> 1) * 8 + (t >> 3) * 4 + (t & 1) * 2; }
+    __device__ __forceinline__ unsigned char* local_page(int row, int index) {
+        return smem + L::AtKv + (row * S::Layers + index) * L::KvPage;
+    }
+    __device__ __forceinline__ void clear_local_values() {
+        // places of tokens to come: their probability is zero, and zero times what lies there has to be zero
+        for (int i = tid; i < ROWS * S::Layers * (L::KvPage / 2 / 16); i += kWorkers) {
+            const int page = i / (L::KvPage / 2 / 16), at = i % (L::KvPage / 2 / 16);
+            reinterpret_cast<int4*>(smem + L::AtKv + page * L::KvPage + L::KvPage / 2)[at] = make_int4(0, 0, 0, 0);
+        }
+    }
+    // A row's scores are computed by all of its warps (8 / ROWS), its 128 dimensions, 16 to a tile, are dealt to them.
+    // The arithmetic is that of q3t_attention_page.cuh: a value does not depend on the tile that it is computed in.
+    __device__ __forceinline__ void local_attention(const HeadNorm& hn, int index, int pos) {
+        const bf16* qkv = reinterpret_cast<const bf16*>(smem + L::AtQkv);
+        bf16* qs = reinterpret_cast<bf16*>(smem + L::AtQ);                 // [row][head][128]
+#pragma unroll
+        for (int i = 0; i < (4 * ROWS + 7) / 8; ++i) {
+            // four vectors a row: two query heads, key, value
+            const int job = warp + 8 * i, r = job >> 2, h = job & 3;
+            if (job >= 4 * rows) continue;
+            unsigned char* page = local_page(r, index);
+            const bf16* src = qkv + r * 512 + h * 128;
+            if (h == 3) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    *reinterpret_cast<bf16*>(page + L::KvPage / 2 + (lane + 32 * j) * 32 + v_token(pos)) = src[lane + 32 * j];
+                continue;
+            }
+            float x[4], o[4];
+            bf16 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                x[j] = bf2f(src[lane + 32 * j]);
+                w[j] = h == 2 ? hn.k[j] : hn.q[j];
+            }
+            page::rotate(x, w, cs[0][0], cs[0][1], a.eps, o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                bf16* at = h == 2 ? reinterpret_cast<bf16*>(page + k_piece(pos, 4 * j + (lane >> 3))) + (lane & 7)
+                                  : qs + r * 256 + h * 128 + lane + 32 * j;
+                *at = f2bf(o[j]);
+            }
+        }
+        sync_workers();
+        constexpr int kWarpsRow = 8 / ROWS;
+        const int r = warp / kWarpsRow, gid = lane >> 2, tig = lane & 3;
+        const unsigned char* page = local_page(r, index);
+        float sc[2][4] = {};
+        const bool real = gid < 2;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+            const int4 q = real ? *reinterpret_cast<const int4*>(qs + r * 256 + gid * 128 + 32 * jj + 8 * tig) : make_int4(0, 0, 0, 0);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                const int4 k = *reinterpret_cast<const int4*>(page + k_piece(8 * nt + gid, 4 * jj + tig));
+                page::mma_bf16_16816(sc[nt], (uint32_t)q.x, 0u, (uint32_t)q.y, 0u, (uint32_t)k.x, (uint32_t)k.y);
+                page::mma_bf16_16816(sc[nt], (uint32_t)q.z, 0u, (uint32_t)q.w, 0u, (uint32_t)k.z, (uint32_t)k.w);
+            }
+        }
+        float mx, lsum;
+        uint32_t ph[2], pl[2];
+        page::probabilities(sc, pos + 1, rsqrtf(128.0f), tig, mx, lsum, ph, pl);
+        const float inv0 = 1.0f / __shfl_sync(0xffffffffu, lsum, 0);
+        const float inv1 = 1.0f / __shfl_sync(0xffffffffu, lsum, 4);
+        bf16* att = reinterpret_cast<bf16*>(smem + L::AtAtt) + r * S::Slice;
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+            const int dim = 16 * (warp % kWarpsRow * ROWS + u) + gid;
+            const uint2 lo = *reinterpret_cast<const uint2*>(page + L::KvPage / 2 + dim * 32 + tig * 8);
+            const uint2 hi = *reinterpret_cast<const uint2*>(page + L::KvPage / 2 + (dim + 8) * 32 + tig * 8);
+            float o[4] = {};
+            page::mma_bf16_16816(o, lo.x, hi.x, lo.y, hi.y, ph[0], ph[1]);
+            page::mma_bf16_16816(o, lo.x, hi.x, lo.y, hi.y, pl[0], pl[1]);
+            if (tig == 0) {
+                att[dim] = f2bf(o[0] * inv0);
+                att[128 + dim] = f2bf(o[1] * inv1);
+                att[dim + 8] = f2bf(o[2] * inv0);
+                att[128 + dim + 8] = f2bf(o[3] * inv1);
+            }
+        }
+        sync_workers();
+    }
+
+    // More rows: the predictor's caches are one page; warp r of every CTA of the group attends for row r.
     __device__ __forceinline__ void predictor_attention(const HeadNorm& hn, page::Fragments& f, bf16* k, bf16* v, int pos) {
         const bf16* qkv = reinterpret_cast<const bf16*>(smem + L::AtQkv);
         const bf16* knew = reinterpret_cast<const bf16*>(smem + L::AtKNew);
@@ -839,7 +1044,7 @@ struct Chain {
             const float inv0 = 1.0f / __shfl_sync(0xffffffffu, lsum, 0);
             const float inv1 = 1.0f / __shfl_sync(0xffffffffu, lsum, 4);
             if ((lane & 3) == 0) {
-                bf16* att = reinterpret_cast<bf16*>(smem + L::AtAtt) + r * 256 + 8 * (lane >> 2);
+                bf16* att = reinterpret_cast<bf16*>(smem + L::AtAtt) + r * S::Slice + 8 * (lane >> 2);
 #pragma unroll
                 for (int c = 0; c < 2; ++c)
 #pragma unroll
@@ -1011,7 +1216,7 @@ struct Chain {
             for (int i = tid; i < 2 * rows * 22; i += kWorkers) {
                 const int rk = i / 22, q = i % 22;
                 const Quad v = poll_one(a.exchange + kAtAttn + ((bo * kSlices + slice) * kRanks + rk) * 22 + q, flag_o);
-                uint32_t* dst = reinterpret_cast<uint32_t*>(att + rk * 128) + 3 * q;
+                uint32_t* dst = reinterpret_cast<uint32_t*>(att + (rk >> 1) * S::Slice + (rk & 1) * 128) + 3 * q;
                 dst[0] = v.x;
                 if (q < 21) {
                     dst[1] = v.y;
@@ -1022,11 +1227,12 @@ struct Chain {
         sync_workers();
     }
 
+    __device__ __forceinline__ const LayerConst& constants(int index) { return reinterpret_cast<const LayerConst*>(smem + L::AtConst)[index]; }
     // ---- a layer -------------------------------------------------------------------------------------------------
-    // In: hidden rows in U, this CTA's residual columns in Own, the layer's constants and input norm weights (they
-    // are fetched ahead).  Out: the same for the next layer.
-    __device__ __forceinline__ void layer(int index, int pos, LayerConst& lc, uint32_t (&nw)[S::J], const Walk& walk) {
-        const LayerConst next = a.layers[index + 1 < S::Layers ? index + 1 : 0];
+    // In: hidden rows in U, this CTA's residual columns in Own, the layer's input norm weights and q/k/v weights (they are
+    // fetched ahead).  Out: the same for what comes next, a projection of `next_tiles` tiles.
+    __device__ __forceinline__ void layer(int index, int pos, int next_tiles, uint32_t (&nw)[S::J], const Walk& walk) {
+        const LayerConst& lc = constants(index);
         HeadNorm hn;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -1042,67 +1248,62 @@ struct Chain {
         }
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
-            // scales of this half's outputs: q/k/v row (warp = activation row, lane = weight row) or channel
+            // the units of this half's sums: an activation row's 32 q/k/v rows, or 24 of its channels (gate and up)
+            constexpr int kChunks = S::Gu / 24;
+            const int n = half == 0 ? 32 : 24, chunk = half == 0 ? 0 : warp % kChunks;
             const int qkv_row = rank < 8 ? 256 * slice + 32 * rank
                                          : (rank < 12 ? 2048 + 128 * slice + 32 * (rank - 8) : 3072 + 128 * slice + 32 * (rank - 12));
-            constexpr int kChunks = S::Gu / 24;                  // 24 channels: four quads
-            const int channel = slice * S::Slice + rank * S::Gu + 24 * (warp % kChunks) + min(lane, 23);
+            const int channel = slice * S::Slice + rank * S::Gu + 24 * chunk + min(lane, 23);
             const float scale = half == 0 ? lc.qkv_s[qkv_row + lane] : lc.gu_s[channel];
             const float scale_up = half == 0 ? 0.0f : lc.gu_s[S::I + channel];
             const float u = norm_to_limbs(nw, nullptr);
-            load_norm(half == 0 ? lc.post_norm : next.in_norm, nw);
+            load_norm(half == 0 ? lc.post_norm : constants(index + 1 < S::Layers ? index + 1 : 0).in_norm, nw);
             sync_workers();           // everybody has read the hidden rows: their place takes the sums
+            mma_full(half == 0 ? 2 : S::GuTiles, u);
+            sync_workers();
+            const int bp = flip(kPart), b = flip(kGroup);
+            const uint32_t flag_g = next_flag();
             const float* red = reinterpret_cast<const float*>(smem + L::AtU);
-            const int bp = flip(kPart);
-            if (half == 0) {
-                mma_full<2, 2>(u);
-                sync_workers();
-                const int b = flip(kQkv);
-                const uint32_t flag = next_flag();
-                if (warp < rows) {
-                    float sum = 0.0f;
-#pragma unroll
-                    for (int w = 0; w < 8; ++w) sum += red[(w * rows + warp) * 32 + lane];
-                    put_values(sum * scale, 32, group_at(kAtQkv, 6, b, rank, warp), flag);
-                }
-                if (walk.any) {
-                    if (!TALKER && index == 0 && pos > 0) await_appended();
-                    page::load(f, walk.k + layer_elems, walk.v + layer_elems, TALKER ? older_in(walk.row, walk.page) : pos, lane);
-                }
-                release_full<2>();
-                collect_group<6, 16>(kAtQkv, b, flag, reinterpret_cast<uint32_t*>(smem + L::AtQkv), 256);
-                if (TALKER) talker_attention(hn, layer_elems, f, walk);
-                else predictor_attention(hn, f, walk.k + layer_elems, walk.v + layer_elems, pos);
-                // output projection over the group's 256 attention values
-                slice_to_limbs<4>(smem + L::AtAtt, 512);
-            } else {
-                mma_full<S::GuTiles, 3>(u);
-                sync_workers();
-                const int b = flip(kAct);
-                const uint32_t flag = next_flag();
-                constexpr int kG = S::Gu / 6;
 #pragma unroll 1
-                for (int unit = warp; unit < rows * kChunks; unit += 8) {
-                    const int r = unit / kChunks, ch = 24 * (warp % kChunks) + min(lane, 23);    // 8 is a multiple of kChunks
-                    float sum = 0.0f, sum_up = 0.0f;
+            for (int unit = warp; unit < (half == 0 ? rows : rows * kChunks); unit += 8) {
+                const int r = half == 0 ? unit : unit / kChunks;              // (8 is a multiple of kChunks)
+                const float* at = red + r * kRedRow + 24 * chunk + min(lane, n - 1);
+                float sum = 0.0f;
 #pragma unroll
-                    for (int w = 0; w < 8; ++w) {
-                        sum += red[(w * rows + r) * (2 * S::Gu) + ch];
-                        sum_up += red[(w * rows + r) * (2 * S::Gu) + S::Gu + ch];
-                    }
-                    const float gate = sum * scale;
+                for (int w = 0; w < 8; ++w) sum += at[w * rows * kRedRow];
+                float value = sum * scale;
+                if (half != 0) {
+                    float sum_up = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) sum_up += at[w * rows * kRedRow + S::Gu];
                     const float up = sum_up * scale_up;
-                    put_values(gate / (1.0f + expf(-gate)) * up, 24, group_at(kAtAct, kG, b, rank, r) + 4 * (warp % kChunks), flag);
+                    value = value / (1.0f + expf(-value)) * up;
                 }
-                release_full<S::GuTiles>();
-                collect_group<kG, S::Gu / 2>(kAtAct, b, flag, reinterpret_cast<uint32_t*>(smem + L::AtAct), S::Slice / 2);
-                slice_to_limbs<S::Slice / 64>(smem + L::AtAct, S::Slice * 2);
+                put_values(value, n, group_at(kAtGroup, kGroupRow, b, rank, r) + 4 * chunk, flag_g);
             }
+            end_full(half == 0 ? 2 : S::GuTiles);
+            if (half == 0) {
+                if constexpr (!L::LocalKv) {
+                    if (walk.any) {
+                        if (!TALKER && index == 0 && pos > 0) await_appended();
+                        page::load(f, walk.k + layer_elems, walk.v + layer_elems, TALKER ? older_in(walk.row, walk.page) : pos, lane);
+                    }
+                }
+            }
+            collect_group(half == 0 ? 6 : S::Gu / 6, half == 0 ? 16 : S::Gu / 2, b, flag_g,
+                          reinterpret_cast<uint32_t*>(smem + (half == 0 ? L::AtQkv : L::AtAct)), half == 0 ? 256 : S::Slice / 2);
+            if (half == 0) {
+                if constexpr (TALKER) talker_attention(hn, layer_elems, f, walk);
+                else if constexpr (L::LocalKv) local_attention(hn, index, pos);
+                else predictor_attention(hn, f, walk.k + layer_elems, walk.v + layer_elems, pos);
+            }
+            // the o projection is over the group's 256 attention values, the down projection over its channels
+            slice_to_limbs<S::Slice / 64>(smem + (half == 0 ? L::AtAtt : L::AtAct), S::Slice * 2);
             const uint32_t flag = next_flag();
-            mma_slice(half == 0 ? 4 : S::Slice / 64, bp, flag);
+            mma_slice(half == 0 ? 4 : kSliceBlocks, bp, flag);
+            hold_ahead(half == 0 ? S::GuTiles : next_tiles, half == 0 ? kSliceBlocks : (next_tiles == 2 ? 4 : 0));
             collect_partials(half == 0 ? lc.o_s : lc.down_s, bp, flag);
         }
-        lc = next;
     }
 
     // input rows of the first layer: `row_of(r)` in global memory -> U and Own
@@ -1132,7 +1333,7 @@ struct Chain {
         const float scale = scales[blockIdx.x * 16 + (lane & 15)];
         const float u = norm_to_limbs(nw, nullptr);
         sync_workers();
-        mma_full<S::HeadTiles, S::HeadTiles>(u);
+        mma_full(S::HeadTiles, u);
         sync_workers();
         const int b = flip(kLogits);
         const uint32_t flag = next_flag();
@@ -1140,10 +1341,11 @@ struct Chain {
         if (warp < rows) {
             float sum = 0.0f;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) sum += red[(w * rows + warp) * 16 + (lane & 15)];
+            for (int w = 0; w < 8; ++w) sum += red[(w * rows + warp) * kRedRow + (lane & 15)];
             put_values(sum * scale, 16, a.exchange + kAtLogits + ((b * kCtas + (int)blockIdx.x) * kRowsMost + warp) * 3, flag);
         }
-        release_full<S::HeadTiles>();
+        end_full(S::HeadTiles);
+        if (p + 1 < kCodebooks) hold_ahead(2, 4);                // the next position's q/k/v
         const int bt = flip(kTokens);
         const uint32_t flag_t = next_flag();
         // one row: every CTA draws for itself (same logits, same state, same token); several: group r draws row r
@@ -1199,12 +1401,7 @@ struct Chain {
             misc->token[tid] = min(max((int)poll_one(a.exchange + kAtTokens + bt * kRowsMost + tid, flag_t).x, 0), 2047);
         }
         sync_workers();
-        if (blockIdx.x == 0 && tid < rows) store_code(tid, p, misc->token[tid]);
-    }
-    __device__ __forceinline__ void store_code(int row, int p, int token) {
-        a.table->frame_tokens[row][p] = token;
-        a.table->frame_codes[row][p] = (unsigned short)token;
-        if (a.table->host_codes[row] != nullptr) a.table->host_codes[row][p] = (unsigned short)token;
+        if (tid < rows) misc->codes[tid][p] = (unsigned short)misc->token[tid];
     }
 
     // ---- the whole chain ------------------------------------------------------------------------------------------
@@ -1212,15 +1409,13 @@ struct Chain {
         if (tid == 0) {
             for (int s = 0; s < L::Slots; ++s) {
                 mbar_init(&misc->full[s], 1);
-                misc->read[s] = 0u;
+                mbar_init(&misc->empty[s], kSlotUnits);
                 misc->asked[s] = 0u;
             }
             misc->abort = 0;
             misc->base = *reinterpret_cast<volatile uint32_t*>(a.epoch);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll 1
-            for (uint32_t s = 0; s < L::Slots; ++s) request(s);
         }
         if (tid < rows) {
             if (TALKER) {
@@ -1233,19 +1428,32 @@ struct Chain {
         __syncthreads();
         base = misc->base;
         deadline = now_ns() + kBudgetNs;
-        LayerConst lc = a.layers[0];
+        if (warp >= kWorkers / kWarp) {
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRequestRegisters));
+            if (warp == kWorkers / kWarp && tc::elect_one()) request_weights();
+            __syncwarp();
+            __syncthreads();
+            return;
+        }
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegisters));
         uint32_t nw[S::J];
-        load_norm(lc.in_norm, nw);
+        load_norm(a.layers[0].in_norm, nw);
+        for (int i = tid; i < S::Layers * (int)(sizeof(LayerConst) / 8); i += kWorkers) {
+            reinterpret_cast<uint64_t*>(smem + L::AtConst)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
+        }
+        // behind a row's attention values: zeros, so that its conversion is the next slice's (barriers follow)
+        for (int i = tid; i < L::AttBytes / 4; i += kWorkers) reinterpret_cast<uint32_t*>(smem + L::AtAtt)[i] = 0u;
+        hold_ahead(2, 4);
         if constexpr (TALKER) {
             const Walk walk = first_page();
             load_rotations();
             load_hidden([&](int r) { return a.hidden + (size_t)r * S::H; });
 #pragma unroll 1
-            for (int l = 0; l < S::Layers; ++l) layer(l, 0, lc, nw, walk);
+            for (int l = 0; l < S::Layers; ++l) layer(l, 0, l + 1 < S::Layers ? 2 : S::HeadTiles, nw, walk);
             load_norm(a.final_norm, nw);
             const float u = norm_to_limbs(nw, blockIdx.x == 0 ? a.normalized : nullptr);
             sync_workers();
-            mma_full<S::HeadTiles, S::HeadTiles>(u);
+            mma_full(S::HeadTiles, u);
             sync_workers();
             const float* red = reinterpret_cast<const float*>(smem + L::AtU);
 #pragma unroll 1
@@ -1253,17 +1461,18 @@ struct Chain {
                 const int r = i / S::HeadRows, n = i % S::HeadRows;
                 float sum = 0.0f;
 #pragma unroll
-                for (int w = 0; w < 8; ++w) sum += red[(w * rows + r) * (S::HeadTiles * 16) + n];
+                for (int w = 0; w < 8; ++w) sum += red[(w * rows + r) * kRedRow + n];
                 const int channel = blockIdx.x * S::HeadRows + n;
                 a.logits[(size_t)r * (kCtas * S::HeadRows) + channel] = f2bf(sum * a.head_s[0][channel]);
             }
         } else {
-            Walk walk{warp, 0, nullptr, nullptr, warp < rows};
+            Walk walk{warp, 0, nullptr, nullptr, !L::LocalKv && warp < rows};
+            if constexpr (L::LocalKv) clear_local_values();        // (several barriers ahead of the first use)
             if (walk.any) {
                 walk.k = page_at(a.kv, warp, 0, false);
                 walk.v = page_at(a.kv, warp, 0, true);
             }
-            if (blockIdx.x == 0 && tid < rows) store_code(tid, 0, misc->token[tid]);
+            if (tid < rows) misc->codes[tid][0] = (unsigned short)misc->token[tid];
 #pragma unroll 1
             for (int p = 0; p < kCodebooks; ++p) {
                 const float* head_scales = p > 0 ? a.head_s[p - 1] : nullptr;
@@ -1275,16 +1484,25 @@ struct Chain {
                 sync_workers();
                 load_rotations();
 #pragma unroll 1
-                for (int l = 0; l < S::Layers; ++l) layer(l, p, lc, nw, walk);
+                for (int l = 0; l < S::Layers; ++l) layer(l, p, l + 1 < S::Layers || p == 0 ? 2 : S::HeadTiles, nw, walk);
                 if (p > 0) predictor_head(p, head_scales);
-                say_appended(p + 1 == kCodebooks);
+                if constexpr (!L::LocalKv) say_appended(p + 1 == kCodebooks);
             }
             if (ROWS == 1 ? blockIdx.x == 0 && tid == 0 : rank == 0 && slice < rows && tid == 0) {
                 const int r = ROWS == 1 ? 0 : slice;
                 *a.table->rng[r] = misc->rng[r];
             }
+            // the frame's codes, once all are drawn: sixteen stores in the way of the draws cost a microsecond each
+            sync_workers();
+            if (blockIdx.x == 0 && tid < rows * kCodebooks) {
+                const int r = tid / kCodebooks, p = tid % kCodebooks;
+                const unsigned short code = misc->codes[r][p];
+                a.table->frame_tokens[r][p] = code;
+                a.table->frame_codes[r][p] = code;
+                if (a.table->host_codes[r] != nullptr) a.table->host_codes[r][p] = code;
+            }
         }
-        sync_workers();
+        __syncthreads();        // no further requests
         if (given_up() && tid < L::Slots && misc->asked[tid] > 0) {
             // a copy that nobody waited for must have landed before the CTA leaves
             for (uint32_t polls = 0; polls < (1u << 14) && !mbar_try_wait(&misc->full[tid], (misc->asked[tid] - 1) & 1u); ++polls) {}
@@ -1301,7 +1519,7 @@ struct Chain {
 };
 
 template <bool TALKER, int ROWS>
-__global__ void __launch_bounds__(kWorkers, 1) decode_chain_kernel(const __grid_constant__ ChainArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) decode_chain_kernel(const __grid_constant__ ChainArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     Chain<TALKER, ROWS> chain(a, smem);
     chain.run();
@@ -1364,7 +1582,7 @@ template <bool TALKER, int ROWS>
 cudaError_t launch_variant(const ChainArgs& a, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kCtas);
-    cfg.blockDim = dim3(kWorkers);
+    cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = Layout<TALKER, ROWS>::Bytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

@@ -71,6 +71,39 @@ __device__ __forceinline__ void patch(Fragments& f, const bf16* krow, const bf16
             }
 }
 
+// A page's scores (columns 2 tig, + 1 of tokens 8 nt ..) -> its maximum, the sum of its weights over the first `count` tokens,
+// and the weights as bf16 hi + lo.
+__device__ __forceinline__ void probabilities(const float (&sc)[2][4], int count, float scale, int tig, float& mx, float& lsum,
+                                              uint32_t (&ph)[2], uint32_t (&pl)[2]) {
+    mx = -INFINITY;
+    lsum = 0.0f;
+    float pr[2][2];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const bool valid = 8 * nt + 2 * tig + e < count;
+            pr[nt][e] = valid ? sc[nt][e] * scale : -INFINITY;
+            mx = fmaxf(mx, pr[nt][e]);
+        }
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            pr[nt][e] = pr[nt][e] == -INFINITY ? 0.0f : expf(pr[nt][e] - mx);
+            lsum += pr[nt][e];
+        }
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+        ph[nt] = pack_bf16x2(pr[nt][0], pr[nt][1]);
+        pl[nt] = pack_bf16x2(pr[nt][0] - __uint_as_float(ph[nt] << 16), pr[nt][1] - __uint_as_float(ph[nt] & 0xffff0000u));
+    }
+}
+
 // Scores, softmax within the page and weighted V over its first `count` tokens.  mx, lsum: of head gid (lanes of
 // gid < 2); o[x][0], o[x][2]: head 2 tig, dims 8 gid + x and 64 + 8 gid + x; o[x][1], o[x][3]: head 2 tig + 1.
 // q: [2][128] fp32 (bf16-valued) in shared memory, 16-byte aligned.
@@ -96,34 +129,8 @@ __device__ __forceinline__ void attend(const Fragments& f, const float* q, int c
             mma_bf16_16816(sc[nt], a10, 0u, a11, 0u, (uint32_t)f.k[nt][jj].z, (uint32_t)f.k[nt][jj].w);
         }
     }
-    mx = -INFINITY;
-    lsum = 0.0f;
-    float pr[2][2];
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const bool valid = 8 * nt + 2 * tig + e < count;
-            pr[nt][e] = valid ? sc[nt][e] * scale : -INFINITY;
-            mx = fmaxf(mx, pr[nt][e]);
-        }
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            pr[nt][e] = pr[nt][e] == -INFINITY ? 0.0f : expf(pr[nt][e] - mx);
-            lsum += pr[nt][e];
-        }
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
     uint32_t ph[2], pl[2];
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-        ph[nt] = pack_bf16x2(pr[nt][0], pr[nt][1]);
-        pl[nt] = pack_bf16x2(pr[nt][0] - __uint_as_float(ph[nt] << 16), pr[nt][1] - __uint_as_float(ph[nt] & 0xffff0000u));
-    }
+    probabilities(sc, count, scale, tig, mx, lsum, ph, pl);
     uint32_t tv[2][2][2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
