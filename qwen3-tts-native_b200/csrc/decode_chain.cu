@@ -212,7 +212,7 @@ struct Layout {
     static constexpr int AtStage = AtKNew + KNewBytes;
     static constexpr int AtSample = AtStage + StageBytes;
     static constexpr int AtMisc = AtSample + (SampleBytes + 15) / 16 * 16;
-    static constexpr int MiscBytes = 1024;
+    static constexpr int MiscBytes = 1280;
     // One or two rows of the predictor: every CTA of a group keeps the group's cache, one page of 16 tokens a layer, to
     // itself (K as rows, V with the tokens of a dimension side by side): nothing to fetch, nothing to publish.
     static constexpr bool LocalKv = !TALKER && ROWS <= 2;
@@ -243,8 +243,9 @@ struct Misc {
     float inverse[kRowsMost];      // of the rows' root mean squares
     unsigned long long rng[kRowsMost];
     unsigned short codes[kRowsMost][kCodebooks];
+    SamplingParams sampling[kRowsMost];
 };
-static_assert(sizeof(Misc) <= 1024, "misc area");
+static_assert(sizeof(Misc) <= 1280, "misc area");
 
 __device__ __forceinline__ void imma(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -897,13 +898,14 @@ struct Chain {
         bf16 q[4], k[4];
     };
     // cos | sin of the head vectors this warp rotates: fixed for a launch (talker) or a position (predictor)
-    static constexpr int kJobs = L::LocalKv ? 1 : (3 * ROWS + 7) / 8;       // (LocalKv: the rows are at one position)
-    uint32_t cs[kJobs][2];
-    __device__ __forceinline__ void load_rotations() {
+    static constexpr int kJobs = (3 * ROWS + 7) / 8;
+    uint32_t cs[TALKER ? kJobs : 1][2];                      // (the predictor's rows are all at one position)
+    __device__ __forceinline__ void load_rotations(int position) {
 #pragma unroll
-        for (int i = 0; i < kJobs; ++i) {
+        for (int i = 0; i < (TALKER ? kJobs : 1); ++i) {
             const int job = warp + 8 * i;
-            const uint32_t* at = a.rope_table + (size_t)misc->position[job < 3 * rows ? job / 3 : 0] * 64 + lane;
+            if (TALKER) position = misc->position[job < 3 * rows ? job / 3 : 0];
+            const uint32_t* at = a.rope_table + (size_t)position * 64 + lane;
             cs[i][0] = at[0];
             cs[i][1] = at[32];
         }
@@ -928,7 +930,7 @@ struct Chain {
                 x[j] = bf2f(src[lane + 32 * j]);
                 w[j] = h == 2 ? hn.k[j] : hn.q[j];
             }
-            page::rotate(x, w, cs[i][0], cs[i][1], a.eps, o);
+            page::rotate(x, w, cs[TALKER ? i : 0][0], cs[TALKER ? i : 0][1], a.eps, o);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (h == 2) knew[r * 128 + lane + 32 * j] = f2bf(o[j]);
@@ -1327,9 +1329,7 @@ struct Chain {
     }
 
     // ---- predictor head and draw ---------------------------------------------------------------------------------
-    __device__ __forceinline__ void predictor_head(int p, const float* scales) {
-        uint32_t nw[S::J];
-        load_norm(a.final_norm, nw);
+    __device__ __forceinline__ void predictor_head(int p, const float* scales, const uint32_t (&nw)[S::J]) {
         const float scale = scales[blockIdx.x * 16 + (lane & 15)];
         const float u = norm_to_limbs(nw, nullptr);
         sync_workers();
@@ -1353,21 +1353,29 @@ struct Chain {
         if (draws >= 0) {
             unsigned int* keys = reinterpret_cast<unsigned int*>(smem + L::AtSample);
             TopKScratch& scratch = *reinterpret_cast<TopKScratch*>(smem + L::AtSample + 2048 * 4);
-#pragma unroll 1
-            for (int i = tid; i < kCtas * 3; i += kWorkers) {
-                const int cta = i / 3, g = i % 3;
-                const Quad v = poll_one(a.exchange + kAtLogits + ((b * kCtas + cta) * kRowsMost + draws) * 3 + g, flag);
-                const uint32_t w[3] = {v.x, v.y, v.z};
+            const Quad* at[2];
+            Quad v[2];
+            int quad[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                quad[k] = min(tid + k * kWorkers, kCtas * 3 - 1);
+                at[k] = a.exchange + kAtLogits + ((b * kCtas + quad[k] / 3) * kRowsMost + draws) * 3 + quad[k] % 3;
+            }
+            static_assert(kCtas * 3 <= 2 * kWorkers, "two quads a thread");
+            poll(at, v, flag);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t w[3] = {v[k].x, v[k].y, v[k].z};
+                const int first = quad[k] / 3 * 16 + quad[k] % 3 * 6;
 #pragma unroll
                 for (int e = 0; e < 3; ++e) {
-                    if (6 * g + 2 * e < 16) {
-                        keys[cta * 16 + 6 * g + 2 * e] = order_key(bf_lo(w[e]));
-                        keys[cta * 16 + 6 * g + 2 * e + 1] = order_key(bf_hi(w[e]));
+                    if (quad[k] % 3 * 6 + 2 * e < 16) {
+                        *reinterpret_cast<uint2*>(keys + first + 2 * e) = make_uint2(order_key(bf_lo(w[e])), order_key(bf_hi(w[e])));
                     }
                 }
             }
             sync_workers();
-            const SamplingParams sp = a.table->predictor[draws];
+            const SamplingParams sp = misc->sampling[draws];
             int token;
             if (sp.do_sample == 0) {
                 unsigned long long best = 0ull;
@@ -1387,7 +1395,7 @@ struct Chain {
                 for (int w = 0; w < 8; ++w) best = scratch.warp_best[w] > best ? scratch.warp_best[w] : best;
                 token = 4095 - (int)(best & 0xfffull);
             } else {
-                token = sample_top_k_block<kWorkers>(keys, 2048, min(sp.top_k, 2048), sp.top_p, sp.temperature, &misc->rng[draws],
+                token = sample_top_k_block<kWorkers, 2048 / kWorkers>(keys, 2048, min(sp.top_k, 2048), sp.top_p, sp.temperature, &misc->rng[draws],
                                                      scratch, tid, [] { sync_workers(); });
             }
             token = min(max(token, 0), 2047);
@@ -1422,6 +1430,7 @@ struct Chain {
                 misc->position[tid] = a.positions[tid];
             } else {
                 misc->rng[tid] = *a.table->rng[tid];
+                misc->sampling[tid] = a.table->predictor[tid];
                 misc->token[tid] = *a.table->sampled[tid];
             }
         }
@@ -1446,7 +1455,7 @@ struct Chain {
         hold_ahead(2, 4);
         if constexpr (TALKER) {
             const Walk walk = first_page();
-            load_rotations();
+            load_rotations(0);
             load_hidden([&](int r) { return a.hidden + (size_t)r * S::H; });
 #pragma unroll 1
             for (int l = 0; l < S::Layers; ++l) layer(l, 0, l + 1 < S::Layers ? 2 : S::HeadTiles, nw, walk);
@@ -1473,6 +1482,9 @@ struct Chain {
                 walk.v = page_at(a.kv, warp, 0, true);
             }
             if (tid < rows) misc->codes[tid][0] = (unsigned short)misc->token[tid];
+            load_rotations(0);
+            uint32_t head_norm[S::J];
+            load_norm(a.final_norm, head_norm);
 #pragma unroll 1
             for (int p = 0; p < kCodebooks; ++p) {
                 const float* head_scales = p > 0 ? a.head_s[p - 1] : nullptr;
@@ -1480,12 +1492,10 @@ struct Chain {
                     const int most = p == 1 ? kMaxVocab - 1 : kPredictorVocab - 1;
                     return p == 0 ? a.hidden + (size_t)r * S::H : a.projected[p - 1] + (size_t)min(max(misc->token[r], 0), most) * S::H;
                 });
-                if (tid < rows) misc->position[tid] = p;
-                sync_workers();
-                load_rotations();
 #pragma unroll 1
                 for (int l = 0; l < S::Layers; ++l) layer(l, p, l + 1 < S::Layers || p == 0 ? 2 : S::HeadTiles, nw, walk);
-                if (p > 0) predictor_head(p, head_scales);
+                load_rotations(min(p + 1, kCodebooks - 1));              // the next position's
+                if (p > 0) predictor_head(p, head_scales, head_norm);
                 if constexpr (!L::LocalKv) say_appended(p + 1 == kCodebooks);
             }
             if (ROWS == 1 ? blockIdx.x == 0 && tid == 0 : rank == 0 && slice < rows && tid == 0) {

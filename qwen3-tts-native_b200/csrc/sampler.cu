@@ -112,7 +112,7 @@ __device__ __forceinline__ void sample_one(const SamplerRow& r, unsigned char* s
     if (small_k) {
         // the usual case: a handful of candidates, see q3t_sampler.cuh
         TopKScratch& scratch = *reinterpret_cast<TopKScratch*>(smem_raw + (size_t)kMaxVocab * sizeof(unsigned int));
-        const int token = sample_top_k_block<kSampleThreads>(short_keys, V, min(r.top_k, V), r.top_p, r.temperature, r.rng,
+        const int token = sample_top_k_block<kSampleThreads, kMaxVocab / kSampleThreads>(short_keys, V, min(r.top_k, V), r.top_p, r.temperature, r.rng,
                                                              scratch, tid, [] { __syncthreads(); });
         if (tid == 0) {
             *r.selected = token;
