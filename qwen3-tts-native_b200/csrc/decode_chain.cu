@@ -235,7 +235,7 @@ struct Misc {
     uint64_t full[24];
     uint64_t empty[24];            // counts the units of the slot that have been read
     unsigned int asked[24];        // copies requested into the slot
-    uint32_t base;
+    uint32_t base, landed;         // landed: slots of the stream, in order
     int abort;
     int position[kRowsMost];
     int token[kRowsMost];
@@ -367,17 +367,13 @@ struct Chain {
         }
         __syncwarp();
     }
-    // WRAPS: the phase is longer than the ring, so the slot's fill before this one may still be in flight for another
-    // warp, and its parity would pass for this one's.  A fill is asked for only once the one before it has been read.
-    template <bool WRAPS = false>
+    // Slot `s` and all before it have landed.  (A warp of its own counts them: looking at the count costs those that compute 30
+    // cycles, a wait on the slot's own barrier 110, data there or not.)
     __device__ __forceinline__ void wait_slot(uint32_t s) {
-        const uint32_t fill = s / L::Slots;
-        if (WRAPS) {
-            for (uint32_t polls = 0; *reinterpret_cast<volatile unsigned int*>(&misc->asked[s % L::Slots]) <= fill;) {
-                if ((++polls & 63u) == 0u && slow_check()) return;
-            }
-        }
-        for (uint32_t polls = 0; !mbar_try_wait(&misc->full[s % L::Slots], fill & 1u);) {
+        uint32_t landed;
+        for (uint32_t polls = 0;;) {
+            asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(landed) : "r"(smem_u32(&misc->landed)) : "memory");
+            if (landed > s) return;
             if ((++polls & 63u) == 0u && slow_check()) return;
         }
     }
@@ -434,6 +430,21 @@ struct Chain {
             }
         }
     }
+    // The counting warp's one thread.
+    __device__ __forceinline__ void count_landed() {
+        uint32_t at = 0, fill = 0;
+#pragma unroll 1
+        for (uint32_t s = 0; s < kAllSlots; ++s) {
+            for (uint32_t polls = 0; !mbar_try_wait(&misc->full[at], fill & 1u);) {
+                if ((++polls & 15u) == 0u && slow_check()) return;
+            }
+            asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(&misc->landed)), "r"(s + 1) : "memory");
+            if (++at == L::Slots) {
+                at = 0;
+                ++fill;
+            }
+        }
+    }
     // Gives back bytes [off, off + len) of the phase that started at slot `first`, lane i the i-th slot touched.
     __device__ __forceinline__ void release(uint32_t first, uint32_t off, uint32_t len) {
         __syncwarp();
@@ -482,16 +493,14 @@ struct Chain {
     // to the compiler, so that all projections of this kind share one copy of the code.
     //
     // kAhead: one or two rows of the predictor take the weights of a projection and of the K-split one behind it from the ring
-    // to registers while the exchange before them is under way.  The wait for a slot (110 cycles, data there or not) and the
-    // reads then cost nothing between one exchange and the next (a predictor layer at one row 18.2 -> 16.9 thousand cycles).
+    // to registers while the exchange before them is under way.  The wait for the slots and the reads
+    // then cost nothing between one exchange and the next (a predictor layer at one row 18.2 -> 16.9 thousand cycles).
     static constexpr int kRedRow = L::RedRows;
     static constexpr bool kAhead = !TALKER && ROWS <= 2;
     static constexpr int kSide = TALKER ? 2 : S::GuTiles;      // tiles side by side (the predictor: all of a phase)
     static constexpr int kSliceBlocks = S::Slice / 64;         // of the down projection; the o projection has 4
     static constexpr int kSliceSide = TALKER ? 2 : kSliceBlocks;
     static constexpr uint32_t kTile = S::J * 1024;              // a tile's blocks lie in one slot
-    // A phase longer than the ring: its later slots come in only once the earlier ones of other warps have been used.
-    static constexpr bool kWraps = S::GuTiles * S::J > L::Slots;
     static_assert(S::OutTiles * kSliceBlocks <= 8 * L::Slots && (TALKER || 2 * S::LayerSlots / 3 <= L::Slots), "phases held fit the ring");
     int4 held_full[2 * kSide * S::J], held_slice[2 * kSliceSide];
     __device__ __forceinline__ const int4* ring_at(uint32_t first, uint32_t at) {
@@ -499,23 +508,23 @@ struct Chain {
     }
     __device__ __forceinline__ void hold_full(uint32_t first, int tiles, int t0) {
         const uint32_t off = (warp * tiles + t0) * kTile;
+        if (!kAhead) wait_slot(first + (off + min(kSide, tiles) * kTile - 1) / kSlot);
 #pragma unroll
         for (int i = 0; i < kSide; ++i) {
             if (!TALKER && i >= tiles) break;
             const uint32_t at = off + i * kTile;
-            if (i == 0 || at % kSlot < kTile) wait_slot<kWraps>(first + at / kSlot);
             const int4* w = ring_at(first, at);
 #pragma unroll
             for (int j = 0; j < 2 * S::J; ++j) held_full[2 * S::J * i + j] = w[kWarp * j];
         }
     }
     __device__ __forceinline__ void hold_slice(uint32_t first, int blocks, int j0) {
+        if (!kAhead) wait_slot(first + ((warp % S::OutTiles * blocks + j0 + min(kSliceSide, blocks)) * 1024u - 1u) / kSlot);
         // two blocks at a time: 2 KB units never cross a slot
 #pragma unroll
         for (int j = 0; j < kSliceSide; j += 2) {
             if (!TALKER && j >= blocks) break;
             const uint32_t at = (warp % S::OutTiles * blocks + j0 + j) * 1024u;
-            if ((kAhead ? j : j0 + j) == 0 || at % kSlot == 0) wait_slot(first + at / kSlot);
             const int4* w = ring_at(first, at);
 #pragma unroll
             for (int i = 0; i < 4; ++i) held_slice[2 * j + i] = w[kWarp * i];
@@ -524,6 +533,7 @@ struct Chain {
     // the weights of a layer's half, or of a head (blocks = 0)
     __device__ __forceinline__ void hold_ahead(int tiles, int blocks) {
         if constexpr (kAhead) {
+            wait_slot(seq + tiles * S::J + S::OutTiles * blocks * 1024 / kSlot - 1);
             hold_full(seq, tiles, 0);
             if (blocks > 0 && warp < S::OutTiles) hold_slice(seq + tiles * S::J, blocks, 0);
         }
@@ -1421,6 +1431,7 @@ struct Chain {
                 misc->asked[s] = 0u;
             }
             misc->abort = 0;
+            misc->landed = 0u;
             misc->base = *reinterpret_cast<volatile uint32_t*>(a.epoch);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1440,6 +1451,7 @@ struct Chain {
         if (warp >= kWorkers / kWarp) {
             asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRequestRegisters));
             if (warp == kWorkers / kWarp && tc::elect_one()) request_weights();
+            if (warp == kWorkers / kWarp + 1 && tc::elect_one()) count_landed();
             __syncwarp();
             __syncthreads();
             return;
