@@ -644,7 +644,8 @@ int32_t q3t_test_prompt_gemm(const Q3tGemmDesc* d, int32_t kernel, void* stream)
     GemvArgs a;
     if (const int32_t e = gemm_args(d, a)) return e;
     if (kernel == 0) return static_cast<int32_t>(launch_int8_gemm_prompt(a, S(stream)));
-    return static_cast<int32_t>(kernel == 3 ? launch_int8_gemm_tc(a, S(stream)) : launch_int8_gemm_wide(a, S(stream), kernel));
+    if (kernel >= 3) return static_cast<int32_t>(launch_int8_gemm_tc(a, S(stream), kernel == 3 ? 0 : kernel));
+    return static_cast<int32_t>(launch_int8_gemm_wide(a, S(stream), kernel));
 }
 
 int32_t q3t_launch_quantize_weight_rows(const uint16_t* weight, int8_t* quantized, float* scales,

@@ -1,8 +1,11 @@
-// Skinny int8 weight-only GEMM for 9..64 activation rows on the 5th-generation tensor cores.
+// Skinny int8 weight-only GEMM for 9..64 activation rows, and for prompt passes of some hundred, on the 5th-generation
+// tensor cores.
 //
 // y[r][n] = epilogue( scale[n] * sum_k W[n][k] * x[r][k] ) like the SIMT kernels, but the weights
 // are the UMMA "A" operand: a CTA owns 128 output channels (one TMEM lane each) and a slice of K,
-// the sessions are the UMMA "N" dimension (16, 32, 48 or 64 columns of fp32 accumulators in TMEM).
+// the sessions are the UMMA "N" dimension (16, 32, 48 or 64 columns of fp32 accumulators in TMEM; prompt passes 96, 128 or
+// 160: a weight is then converted once for 160 rows instead of once for 64, and K can be split where blocks of 64 filled the
+// GPU.  150 rows: q/k/v 11.1 -> 9.3 us, o 8.3 -> 7.8, gate/up 18.6 -> 16.3, down 14.4 -> 11.2).
 //
 //   TMA, 128-byte swizzle           int8 W tile 128 x 128 -> shared ring (6 stages of 16 KB)
 //   TMA, 128-byte swizzle           bf16 x tile MT x 128  -> shared ring (4 stages), UMMA K-major
@@ -32,6 +35,7 @@
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
+#include <utility>
 
 namespace q3t {
 namespace {
@@ -45,16 +49,28 @@ constexpr int kGroups = 2;
 constexpr int kTcThreads = 128 + 128 * kGroups;
 constexpr int kTileN = 128;            // output channels per CTA = TMEM lanes
 constexpr int kBK = 128;               // K elements per pipeline step
-constexpr int kWStages = 6;            // int8 ring in shared memory
-constexpr int kXStages = 4;            // activation ring in shared memory (stage i pairs with A stage i)
-constexpr int kAStages = 4;            // dequantised A stages in TMEM
 constexpr int kWStageBytes = kTileN * kBK;          // 16 KB
-static_assert(kWStages % kGroups == 0 && kAStages % kGroups == 0, "a stage is always consumed by the same group");
-static_assert(kXStages == kAStages, "activation stage i and TMEM A stage i share their barriers");
 constexpr int kAStageCols = kBK / 2;   // 64 TMEM columns: two bf16 per 32-bit column
-constexpr int kAccCols = 64;           // accumulators sit in columns [0, 64), A stages follow
-constexpr uint32_t kTmemCols = 512;    // 64 + 4 * 64 rounded up to a power of two
-constexpr int kRedBytes = 44 * 1024;   // K-slice exchange: up to 8 slices x ceil(64 / slices) rows, in fours, x 128 fp32
+constexpr uint32_t kTmemCols = 512;
+// What a tile of MT rows has.  Up to 64 rows the exchange of the K-slices has memory of its own.  Prompt passes take tiles of
+// up to 160: their activations leave no room for it, and it lies over the rings, which costs a barrier of the cluster between
+// the last product and the first part sent.
+template <int MT>
+struct Tile {
+    static constexpr bool kTall = MT > 64;
+    static constexpr int kWStages = MT == 160 ? 4 : 6;       // int8 ring in shared memory
+    static constexpr int kStages = 4;                        // activations in shared memory; dequantised A in TMEM: stage i of one pairs with stage i of the other
+    static constexpr int kAccCols = kTall ? 256 : 64;        // accumulators first, A stages behind them
+    static constexpr int kXAtomBytes = MT * 128;             // MT rows x 64 bf16, one 128-byte-swizzled atom
+    static constexpr int kXStageBytes = 2 * kXAtomBytes;     // 128 K elements per step
+    static constexpr int kRings = kWStages * kWStageBytes + kStages * kXStageBytes;
+    // up to 8 slices x ceil(MT / slices) rows, in fours, x 128 fp32
+    static constexpr int kRedBytes = kTall ? 0 : 44 * 1024;
+    static constexpr size_t kSmem = 1024 + (size_t)kRings + kRedBytes + (2 * kWStages + 3 * kStages + 2) * sizeof(uint64_t) + 64;
+    static_assert(kWStages % kGroups == 0 && kStages % kGroups == 0, "a stage is always consumed by the same group");
+    static_assert(kAccCols >= MT && kAccCols + kStages * kAStageCols <= (int)kTmemCols && kSmem <= 227 * 1024, "fits");
+    static_assert(!kTall || (MT + 8 * 4) * kTileN * 4 <= kRings, "the exchange lies over the rings");
+};
 constexpr unsigned long long kBudgetNs = 2000000000ull;   // 2 s for the whole kernel
 
 __device__ unsigned int g_tc_errors = 0;
@@ -88,6 +104,9 @@ __device__ __forceinline__ float finish(float acc, float scale, float bias, floa
     return acc * scale;
 }
 
+// Everybody's products are done: what their rings held has been used.
+__device__ __forceinline__ void cluster_meet() { cluster_sync(); }
+
 __device__ __forceinline__ void dequant_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(128 * kGroups) : "memory");
 }
@@ -96,8 +115,9 @@ template <int MT, bool GATEUP>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map,
                const TcParams p) {
-    constexpr int kXAtomBytes = MT * 128;          // MT rows x 64 bf16, one 128-byte-swizzled atom
-    constexpr int kXStageBytes = 2 * kXAtomBytes;  // 128 K elements per step
+    using T = Tile<MT>;
+    constexpr int kWStages = T::kWStages, kStages = T::kStages, kAccCols = T::kAccCols;
+    constexpr int kXAtomBytes = T::kXAtomBytes, kXStageBytes = T::kXStageBytes;
     // fp32 accumulate, A and B bf16 (format 1), both K-major
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT >> 3) << 17)
                                 | ((uint32_t)(kTileN >> 4) << 24);
@@ -106,15 +126,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     unsigned char* w8 = smem;
     unsigned char* xs = w8 + kWStages * kWStageBytes;
-    float* red = reinterpret_cast<float*>(xs + kXStages * kXStageBytes);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(red) + kRedBytes);
-    uint64_t* full_w = bars;
+    float* red = reinterpret_cast<float*>(T::kTall ? smem : smem + T::kRings);
+    uint64_t* full_w = reinterpret_cast<uint64_t*>(smem + T::kRings + T::kRedBytes);
     uint64_t* empty_w = full_w + kWStages;
-    uint64_t* full_x = empty_w + kWStages;
-    uint64_t* empty_x = full_x + kXStages;
-    uint64_t* full_a = empty_x + kXStages;
-    uint64_t* empty_a = full_a + kAStages;
-    uint64_t* acc_done = empty_a + kAStages;
+    uint64_t* full_a = empty_w + kWStages;
+    uint64_t* empty_a = full_a + kStages;
+    uint64_t* acc_done = empty_a + kStages;
     uint64_t* red_full = acc_done + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(red_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -158,11 +175,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             mbar_init(&full_w[s], 1);
             mbar_init(&empty_w[s], 4);
         }
-        for (int s = 0; s < kXStages; ++s) {
-            mbar_init(&full_x[s], 1);
-            mbar_init(&empty_x[s], 1);
-        }
-        for (int s = 0; s < kAStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             mbar_init(&full_a[s], 4 + 1);     // four dequantiser warps + the activation copy (bytes)
             mbar_init(&empty_a[s], 1);
         }
@@ -183,8 +196,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    // a peer's barriers have to be set up before anything is sent to it: waited for just before that
-    cluster_arrive();
+    // a peer's barriers have to be set up before anything is sent to it (tall tiles: its rings used up): waited for just
+    // before that
+    if (!T::kTall) cluster_arrive();
     // The weight copies (warp 0) start at once: weights never depend on the kernel before this
     // one.  Everyone else first waits for that kernel to complete (activations, residual), and
     // only then is the kernel after this one let in: every kernel of the library but the norm
@@ -217,8 +231,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         if (elect_one()) {
             // ---- activation producer ------------------------------------------------------
             for (int i = 0; i < nk; ++i) {
-                const int sx = i % kXStages;
-                if (i >= kXStages && !guard.wait(&empty_a[sx], ((i / kXStages) - 1) & 1)) break;
+                const int sx = i % kStages;
+                if (i >= kStages && !guard.wait(&empty_a[sx], ((i / kStages) - 1) & 1)) break;
                 // the activation tile lands on the same barrier the dequantisers arrive on, so
                 // that the MMA issuer has one thing to wait for per step
                 mbar_expect_tx(&full_a[sx], kXStageBytes);
@@ -231,14 +245,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         if (elect_one()) {
             // ---- MMA issuer ---------------------------------------------------------------
             for (int i = 0; i < nk; ++i) {
-                const int sa = i % kAStages;
-                const int sx = i % kXStages;
-                bool ok = true;
-                ok = ok && guard.wait(&full_a[sa], (i / kAStages) & 1);
-                if (!ok) break;
+                const int sa = i % kStages;
+                if (!guard.wait(&full_a[sa], (i / kStages) & 1)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a_col = tmem_base + kAccCols + sa * kAStageCols;
-                const uint32_t b_addr = smem_u32(xs + sx * kXStageBytes);
+                const uint32_t b_addr = smem_u32(xs + sa * kXStageBytes);
 #pragma unroll
                 for (int j = 0; j < kBK / 16; ++j) {
                     // 16 K elements = 8 TMEM columns of A, 32 bytes within a row of the B atom
@@ -258,7 +269,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         bool ok = true;
         for (int i = group; i < nk && ok; i += kGroups) {
             const int s = i % kWStages;
-            const int sa = i % kAStages;
+            const int sa = i % kStages;
             // a wait that gives up does so for the whole warp: the warp-level syncs below must be
             // reached by all 32 lanes or by none
             if (!__all_sync(0xffffffffu, guard.wait(&full_w[s], (i / kWStages) & 1))) { ok = false; break; }
@@ -269,8 +280,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             for (int c = 0; c < 8; ++c) {
                 raw[c] = *reinterpret_cast<const int4*>(rowp + ((c ^ (t & 7)) << 4));
             }
-            if (i >= kAStages
-                && !__all_sync(0xffffffffu, guard.wait(&empty_a[sa], ((i / kAStages) - 1) & 1))) {
+            if (i >= kStages
+                && !__all_sync(0xffffffffu, guard.wait(&empty_a[sa], ((i / kStages) - 1) & 1))) {
                 ok = false;
                 break;
             }
@@ -302,39 +313,47 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         dequant_barrier();
         if (__all_sync(0xffffffffu, *abort_flag == 0)) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // each group takes half of the accumulator columns (= activation rows); every row of
+            // each group takes half of the accumulator columns (= activation rows), some at a time; every row of
             // this K-slice goes to the shared memory of the CTA that owns the row
-            constexpr int kCols = MT / kGroups;
-            float v[kCols];
-            tmem_load_row<kCols>(lane_base + group * kCols, v);
-            cluster_wait();
+            constexpr int kCols = MT / kGroups, kChunk = T::kTall ? 16 : kCols;
+            float v[kChunk];
+            tmem_load_row<kChunk>(lane_base + group * kCols, v);
+            if (T::kTall) cluster_meet();
+            else cluster_wait();
             const uint32_t mine = smem_u32(red) + (uint32_t)((split * share_groups * kTileN + t) * 16);
             int owner = (group * kCols / 4) / share_groups;      // one division, then counted up
             int within = group * kCols / 4 - owner * share_groups;
+#pragma unroll 1
+            for (int j0 = 0; j0 < kCols; j0 += kChunk) {
+                if (j0 > 0) tmem_load_row<kChunk>(lane_base + group * kCols + j0, v);
 #pragma unroll
-            for (int j = 0; j < kCols; j += 4) {
-                if (group * kCols + j < rows) {
-                    const uint32_t at = mine + (uint32_t)(within * kTileN * 16);
-                    if (owner == split) {
-                        *reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(red) + (at - smem_u32(red)))
-                            = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else {
-                        st_async_v4(peer_smem(at, (uint32_t)owner), v[j], v[j + 1], v[j + 2], v[j + 3],
-                                    peer_smem(smem_u32(red_full), (uint32_t)owner));
+                for (int j = 0; j < kChunk; j += 4) {
+                    if (group * kCols + j0 + j < rows) {
+                        const uint32_t at = mine + (uint32_t)(within * kTileN * 16);
+                        if (owner == split) {
+                            *reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(red) + (at - smem_u32(red)))
+                                = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                        } else {
+                            st_async_v4(peer_smem(at, (uint32_t)owner), v[j], v[j + 1], v[j + 2], v[j + 3],
+                                        peer_smem(smem_u32(red_full), (uint32_t)owner));
+                        }
+                    }
+                    if (++within == share_groups) {
+                        within = 0;
+                        ++owner;
                     }
                 }
-                if (++within == share_groups) {
-                    within = 0;
-                    ++owner;
-                }
             }
+        } else if (T::kTall) {
+            cluster_meet();
         } else {
             cluster_wait();
         }
     }
     if (warp < 4) {
         __syncwarp();
-        cluster_wait();
+        if (T::kTall) cluster_meet();
+        else cluster_wait();
     }
 
     // ---- the K-slices of a channel tile live in the CTAs of one cluster; each CTA sums the rows it owns over all slices
@@ -444,14 +463,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
 
 // ---------------------------------------------------------------------------------- host side
 
+// Rows of a tile.  Over 64: prompt passes only.
+constexpr int kTileRows[] = {16, 32, 48, 64, 96, 128, 160};
+constexpr int kVariants = sizeof(kTileRows) / sizeof(kTileRows[0]);
+int variant_of(int mt) {
+    for (int i = 0; i < kVariants; ++i)
+        if (kTileRows[i] == mt) return i;
+    return -1;
+}
+
 // Per-device scratch of the tensor-core path: a buffer for normalised activations.  Allocated
 // once per device by configure_tc_kernels(); launches on one device that use it must be ordered
 // (the engine issues them on one stream).
 struct TcScratch {
     bf16* normalized = nullptr;
     int sms = 148;
-    // clusters of 1..8 CTAs that the device can hold at once, per kernel variant [MT index][GATEUP]
-    int resident_clusters[4][2][9] = {};
+    // clusters of 1..8 CTAs that the device can hold at once, per kernel variant [index in kTileRows][GATEUP]
+    int resident_clusters[kVariants][2][9] = {};
     bool ready = false;
 };
 constexpr size_t kNormalizedElems = (size_t)kMaxRows * 8192;
@@ -465,20 +493,14 @@ TcScratch* scratch_for_current_device() {
 }
 
 template <int MT, bool GATEUP>
-size_t tc_smem_bytes() {
-    return 1024 + (size_t)kWStages * kWStageBytes + (size_t)kXStages * MT * 256 + kRedBytes
-        + (2 * kWStages + 2 * kAStages + 2 * kXStages + 2) * sizeof(uint64_t) + 64;
-}
-
-template <int MT, bool GATEUP>
 cudaError_t configure_one(int (&resident)[9]) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<MT, GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(tc_smem_bytes<MT, GATEUP>()));
+                                         static_cast<int>(Tile<MT>::kSmem));
     for (int size = 1; size <= 8 && e == cudaSuccess; ++size) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(size * 64), 1, 1);
         cfg.blockDim = dim3(kTcThreads, 1, 1);
-        cfg.dynamicSmemBytes = tc_smem_bytes<MT, GATEUP>();
+        cfg.dynamicSmemBytes = Tile<MT>::kSmem;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)size;
@@ -498,7 +520,7 @@ cudaError_t launch_mt(const CUtensorMap& wm, const CUtensorMap& xm, const TcPara
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.tiles * p.splits), (unsigned)((p.rows + MT - 1) / MT), 1);
     cfg.blockDim = dim3(kTcThreads, 1, 1);
-    cfg.dynamicSmemBytes = tc_smem_bytes<MT, GATEUP>();
+    cfg.dynamicSmemBytes = Tile<MT>::kSmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -510,6 +532,27 @@ cudaError_t launch_mt(const CUtensorMap& wm, const CUtensorMap& xm, const TcPara
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MT, GATEUP>, wm, xm, p);
+}
+
+template <int... MTS>
+cudaError_t configure_all(TcScratch& s, std::integer_sequence<int, MTS...>) {
+    cudaError_t e = cudaSuccess;
+    int v = 0;
+    ((e = e == cudaSuccess ? configure_one<MTS, false>(s.resident_clusters[v][0]) : e,
+      e = e == cudaSuccess ? configure_one<MTS, true>(s.resident_clusters[v][1]) : e, ++v), ...);
+    return e;
+}
+template <bool GATEUP>
+cudaError_t launch_tile(int mt, const CUtensorMap& wm, const CUtensorMap& xm, const TcParams& p, cudaStream_t stream) {
+    switch (mt) {
+        case 16: return launch_mt<16, GATEUP>(wm, xm, p, stream);
+        case 32: return launch_mt<32, GATEUP>(wm, xm, p, stream);
+        case 48: return launch_mt<48, GATEUP>(wm, xm, p, stream);
+        case 96: return launch_mt<96, GATEUP>(wm, xm, p, stream);
+        case 128: return launch_mt<128, GATEUP>(wm, xm, p, stream);
+        case 160: return launch_mt<160, GATEUP>(wm, xm, p, stream);
+        default: return launch_mt<64, GATEUP>(wm, xm, p, stream);
+    }
 }
 
 int g_tc_min_rows = 9;
@@ -527,14 +570,7 @@ cudaError_t configure_tc_kernels() {
     std::lock_guard<std::mutex> lock(g_scratch_guard);
     TcScratch& s = g_scratch[device];
     if (s.ready) return cudaSuccess;
-    e = configure_one<16, false>(s.resident_clusters[0][0]);
-    if (e == cudaSuccess) e = configure_one<16, true>(s.resident_clusters[0][1]);
-    if (e == cudaSuccess) e = configure_one<32, false>(s.resident_clusters[1][0]);
-    if (e == cudaSuccess) e = configure_one<32, true>(s.resident_clusters[1][1]);
-    if (e == cudaSuccess) e = configure_one<48, false>(s.resident_clusters[2][0]);
-    if (e == cudaSuccess) e = configure_one<48, true>(s.resident_clusters[2][1]);
-    if (e == cudaSuccess) e = configure_one<64, false>(s.resident_clusters[3][0]);
-    if (e == cudaSuccess) e = configure_one<64, true>(s.resident_clusters[3][1]);
+    e = configure_all(s, std::integer_sequence<int, 16, 32, 48, 64, 96, 128, 160>());
     if (e != cudaSuccess) return e;
     e = cudaMalloc(&s.normalized, kNormalizedElems * sizeof(bf16));
     if (e != cudaSuccess) return e;
@@ -560,11 +596,11 @@ int tile_rows(int rows) {
 }
 // K-slices per tile = cluster size: as many as still let every cluster be resident at once (a second wave would
 // double the time); slices and row shares may be ragged
-int choose_splits(const TcScratch& scratch, const GemvArgs& a) {
+int choose_splits(const TcScratch& scratch, const GemvArgs& a, int mt) {
     const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
-    const int mt = tile_rows(a.rows), nk = a.in_features / kBK;
+    const int nk = a.in_features / kBK;
     const int clusters = (gateup ? (a.out_features + 63) / 64 : (a.out_features + kTileN - 1) / kTileN) * ((a.rows + mt - 1) / mt);
-    const int (&resident)[9] = scratch.resident_clusters[mt / 16 - 1][gateup ? 1 : 0];
+    const int (&resident)[9] = scratch.resident_clusters[variant_of(mt)][gateup ? 1 : 0];
     static const int split_cap = [] {
         const char* v = std::getenv("QWEN3_TTS_TC_MAX_SPLITS");
         const int n = v != nullptr ? std::atoi(v) : 8;
@@ -578,20 +614,23 @@ int choose_splits(const TcScratch& scratch, const GemvArgs& a) {
 }
 }  // namespace
 
-float gemm_tc_estimate_us(const GemvArgs& a) {
+float gemm_tc_estimate_us(const GemvArgs& a, int tile) {
     TcScratch* scratch = scratch_for_current_device();
     if (scratch == nullptr || a.in_features % kBK != 0) return 1.0e9f;
     const bool gateup = a.epilogue == EPI_GATE_UP_SILU;
-    const int mt = tile_rows(a.rows), splits = choose_splits(*scratch, a);
+    const int mt = tile > 0 ? tile : tile_rows(a.rows), splits = choose_splits(*scratch, a, mt);
     const int ctas = (gateup ? (a.out_features + 63) / 64 : (a.out_features + kTileN - 1) / kTileN) * ((a.rows + mt - 1) / mt) * splits;
     const int waves = (ctas + scratch->sms - 1) / scratch->sms;
     const int steps = (a.in_features / kBK + splits - 1) / splits;
-    return waves * ((splits > 1 ? 6.4f : 4.0f) + 0.5f * steps);
+    if (mt <= 64) return waves * (splits > 1 ? 5.3f + 0.39f * steps : 4.5f + 0.43f * steps);
+    // tall tiles: the exchange and the epilogue grow with the rows; a residual is another read of them
+    const bool adds = a.epilogue == EPI_ADD || a.epilogue == EPI_BIAS_ADD;
+    return waves * ((adds || gateup ? 3.0f : 2.1f) + 0.0385f * mt + 0.42f * steps);
 }
 
-cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
+cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream, int tile) {
     TcScratch* scratch = scratch_for_current_device();
-    if (scratch == nullptr || !gemm_tc_supports(a) || a.out_features < 1 || a.w == nullptr
+    if (scratch == nullptr || (tile > 0 && variant_of(tile) < 0) || !gemm_tc_supports(a) || a.out_features < 1 || a.w == nullptr
         || a.scales == nullptr || a.x == nullptr) {
         return cudaErrorInvalidValue;
     }
@@ -613,14 +652,14 @@ cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
         if (e != cudaSuccess) return e;
         x = normalized;
     }
-    const int mt = tile_rows(a.rows);
+    const int mt = tile > 0 ? tile : tile_rows(a.rows);
     TcParams p;
     p.scales = a.scales; p.y = a.y; p.y32 = a.y32; p.bias = a.bias; p.resid = a.resid;
     p.out_features = N; p.rows = a.rows; p.epilogue = a.epilogue;
     p.tiles = gateup ? (N + 63) / 64 : (N + kTileN - 1) / kTileN;
     p.residual_settled = a.residual_settled ? 1 : 0;
     const int nk = K / kBK;
-    p.splits = choose_splits(*scratch, a);
+    p.splits = choose_splits(*scratch, a, mt);
     p.chunks = nk;
 
     alignas(64) CUtensorMap wm, xm;
@@ -631,20 +670,7 @@ cudaError_t launch_int8_gemm_tc(const GemvArgs& a, cudaStream_t stream) {
                      CU_TENSOR_MAP_SWIZZLE_128B)) {
         return cudaErrorInvalidValue;
     }
-    if (gateup) {
-        switch (mt) {
-            case 16: return launch_mt<16, true>(wm, xm, p, stream);
-            case 32: return launch_mt<32, true>(wm, xm, p, stream);
-            case 48: return launch_mt<48, true>(wm, xm, p, stream);
-            default: return launch_mt<64, true>(wm, xm, p, stream);
-        }
-    }
-    switch (mt) {
-        case 16: return launch_mt<16, false>(wm, xm, p, stream);
-        case 32: return launch_mt<32, false>(wm, xm, p, stream);
-        case 48: return launch_mt<48, false>(wm, xm, p, stream);
-        default: return launch_mt<64, false>(wm, xm, p, stream);
-    }
+    return gateup ? launch_tile<true>(mt, wm, xm, p, stream) : launch_tile<false>(mt, wm, xm, p, stream);
 }
 
 unsigned int gemm_tc_error_count() {

@@ -33,6 +33,7 @@ constexpr int kTileN = 128;                   // channels per tile
 constexpr int kTileM = 128;                   // activation rows per CTA
 constexpr int kBK = 128;                      // K elements per step
 constexpr int kSms = 148;
+constexpr int kTallRowsMost = 640;            // see launch_int8_gemm_prompt
 constexpr int kWStages = 8;
 constexpr int kXStages = 3;
 constexpr int kAStages = 4;
@@ -383,13 +384,13 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
 
 // Which kernel takes a projection of a prompt pass: the one with the shortest estimate.  A wave of CTAs of this
 // file's kernel costs its steps (0.50 us each with one channel tile, 0.82 us with two: what an SM takes in) and 4
-// to 6 us of start and epilogue; the 64-row kernel of gemm_int8_tc.cu, its row blocks side by side and K split where
-// that fits one wave, is estimated there.  For the talker's shapes that puts the lines at 65 rows (gate/up; two tiles
-// from 129), 257 (q/k/v; two tiles from 513) and 577 (o, down and the text projection; two tiles from about 1,200).
-// Measured from 65 to 2000 rows (us, row blocks / one tile / two tiles): gate/up 128 rows 20.7 / 15.4 / 17.9, 129
-// 21.3 / 27.0 / 18.2; q/k/v 256 11.8 / 11.7 / 18.4, 257 18.4 / 12.4 / 18.2; down 576 26.4 / 29.4 / 45.1, 577
-// 45.7 / 29.2 / 45.1.  The choice is within 2 % of the best everywhere but for o between 384 and 576 rows (3 to 6 %:
-// 13.1 to 13.9 us against 12.7 to 13.3 by one tile).
+// to 7 us of start and epilogue; the kernel of gemm_int8_tc.cu, in blocks of up to 64 rows or of 96, 128 or 160 side by side
+// and with K split where that fits one wave, is estimated there.  Above 640 rows this file's kernel always has the waves.
+// Measured from 65 to 640 rows (us, blocks of 64 / best of the tall ones / one tile / two tiles of this file): gate/up 65 rows
+// 19.0 / 12.5 / 14.8 / 17.2, 128 21.1 / 14.7 / 15.6 / 18.0, 150 22.3 / 16.3 / 27.3 / 18.6, 300 41.5 / 27.2 / 29.6 / 19.8, 448
+// 53.7 / 31.3 / 43.2 / 36.8; q/k/v 128 8.3 / 9.0 / 11.6 / 18.2, 300 20.8 / 11.3 / 12.5 / 18.2, 512 23.2 / 15.0 / 13.1 / 18.6;
+// down 128 10.6 / 10.8 / 28.2 / 44.3, 300 25.4 / 14.5 / 28.7 / 45.0, 640 49.7 / 20.2 / 29.9 / 44.9; o 150 8.3 / 7.8 / 12.6 /
+// 19.9, 300 12.6 / 10.0 / 12.7 / 19.9.
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     GemvArgs a = args;
     if (a.norm_w != nullptr) {
@@ -405,10 +406,19 @@ cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     auto waves = [&](int tiles) {
         return ((a.out_features + tiles * per_single - 1) / (tiles * per_single) * row_blocks + kSms - 1) / kSms;
     };
-    const float one = waves(1) * (a.epilogue == EPI_GATE_UP_SILU ? 6.0f + 0.50f * steps : 4.3f + 0.50f * steps);
+    const float one = waves(1) * (a.epilogue == EPI_GATE_UP_SILU ? 6.8f + 0.50f * steps : 4.3f + 0.50f * steps);
     const float two = waves(2) * (5.5f + 0.82f * steps);
-    if (gemm_tc_estimate_us(a) <= (one < two ? one : two)) return launch_int8_gemm_tc(a, stream);
-    return launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
+    float best = one < two ? one : two;
+    int tile = -1;
+    for (int t : {0, 96, 128, 160}) {
+        if (t > 0 && a.rows > kTallRowsMost) break;
+        const float estimate = gemm_tc_estimate_us(a, t);
+        if (estimate <= best) {
+            best = estimate;
+            tile = t;
+        }
+    }
+    return tile >= 0 ? launch_int8_gemm_tc(a, stream, tile) : launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
 }
 
 unsigned int gemm_wide_error_count() {

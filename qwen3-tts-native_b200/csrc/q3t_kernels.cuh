@@ -88,7 +88,8 @@ int set_gemv_mode(int mode);
 int gemv_mode();
 // tensor-core path (tcgen05, TMEM accumulators): rows >= tc_min_rows() and K % 64 == 0
 bool gemm_tc_supports(const GemvArgs& args);
-cudaError_t launch_int8_gemm_tc(const GemvArgs& args, cudaStream_t stream);
+// `tile`: rows of a tile, 0 for the smallest that takes them all (up to 64)
+cudaError_t launch_int8_gemm_tc(const GemvArgs& args, cudaStream_t stream, int tile = 0);
 cudaError_t configure_tc_kernels();      // also allocates the per-device scratch of that path
 void set_tc_min_rows(int rows);          // 65 or more: never use the tensor-core path
 int tc_min_rows();
@@ -96,7 +97,7 @@ unsigned int gemm_tc_error_count();
 // more than kMaxRows rows (prompt passes), K % 128 == 0, no norm prologue, no fp32 output
 // (gemm_int8_wide.cu); channel_tiles 1 or 2
 cudaError_t launch_int8_gemm_wide(const GemvArgs& args, cudaStream_t stream, int channel_tiles);
-float gemm_tc_estimate_us(const GemvArgs& args);     // what launch_int8_gemm_tc would take, for that choice
+float gemm_tc_estimate_us(const GemvArgs& args, int tile = 0);     // what launch_int8_gemm_tc would take, for that choice
 cudaError_t configure_wide_kernels();
 // projections of a prompt pass of more than kMaxRows rows (needs norm_out when norm_w is given)
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream);

@@ -145,6 +145,27 @@ def test_prompt_kernels(q3t, orc, ops, kernel, n, k, rows):
     assert q3t.library().q3t_kernel_error_count() == 0
 
 
+@pytest.mark.parametrize("kernel", [96, 128, 160])
+@pytest.mark.parametrize("n,k,rows", [(300, 384, 65), (128, 128, 97), (129, 1152, 161), (257, 512, 300), (2048, 6144, 150), (4096, 2048, 640)])
+def test_tall_tiles(q3t, orc, ops, kernel, n, k, rows):
+    """The lockstep kernel in blocks of 96, 128 or 160 rows: one step of K and many, K unsplit and in up to eight slices (whose
+    exchange lies over the rings), rows that end inside a block and inside an owner's share, channels that end inside a tile."""
+    w, s, x, bias, base = prompt_case(orc, n, k, rows)
+    plain = orc.int8_gemm_rows(w, s, x)
+    check_bf16(orc, ops.int8_gemm(w, s, x, prompt_kernel=kernel)["y"], plain)
+    out = ops.int8_gemm(w, s, x, epilogue=ops.EPI_ADD, y_in=base, prompt_kernel=kernel)["y"]
+    check_bf16(orc, out, orc.int8_gemm_rows(w, s, x, y_in=base, mode=1), summand=base)
+    assert np.array_equal(out, ops.int8_gemm(w, s, x, epilogue=ops.EPI_ADD, y_in=base, prompt_kernel=kernel)["y"])
+    # tolerance: as in test_prompt_kernels
+    summand = orc.to_bf16(1.6 * (np.abs(orc.from_bf16(plain)) + np.abs(orc.from_bf16(bias))).astype(np.float32))
+    check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=ops.EPI_BIAS_SILU, bias=bias, prompt_kernel=kernel)["y"],
+               orc.bias_activation_rows(plain, bias, True), summand=summand)
+    w, s, x, _, _ = prompt_case(orc, n, k, rows, gate_up=True)
+    check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=ops.EPI_GATE_UP_SILU, prompt_kernel=kernel)["y"],
+               orc.int8_gate_up_silu_rows(w, s, x))
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
 @pytest.mark.parametrize("n,k,rows,gate_up", [(2048, 6144, 700, False), (4096, 2048, 1200, False), (2048, 2048, 2048, False), (6144, 2048, 600, True)])
 def test_prompt_kernels_over_several_waves(q3t, orc, ops, n, k, rows, gate_up):
     """More CTAs than the GPU holds at once, at the talker's shapes; rows are compared with the lockstep kernel's, each within
