@@ -1,0 +1,144 @@
+// Which of the GPU's two dies an SM lies on, and on which a page of memory is at home.
+//
+// An atomic operation is done where its word is at home: on a B200 it takes an SM of that die 210 to 330 cycles, one of the
+// other die 400 to 540; homes alternate by pages of 4 KB.  The decode chain puts the CTAs that exchange most, and their
+// buffers, on one die (decode_chain.cu).  What is found here changes the time of a frame, not its results.  SMs are compared
+// with each other, and pages with each other, at the same time and as ratios, since the clocks may be on their way up.
+// Nothing here waits for another CTA.  Takes a millisecond, once for each model.
+
+#include "q3t_kernels.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <vector>
+
+namespace q3t {
+namespace {
+
+constexpr int kProbePages = 8, kProbeLines = 4;          // for telling SMs apart
+constexpr int kPageLines = 8;                            // for telling pages apart
+constexpr int kChain = 4;                                // atomics one behind the other
+constexpr size_t kAlone = 120 * 1024;                    // shared memory of a CTA: one an SM
+
+struct Latencies {
+    uint32_t of_sm[kPlaceSms][kProbePages];              // cycles, 0: no CTA ran there
+    uint32_t of_page[kPoolPages];
+    uint32_t by[kPoolPages];                             // the SM that measured the page
+};
+
+__device__ uint32_t atomic_cycles(uint32_t* word) {
+    uint32_t v = 0;
+    const long long t0 = clock64();
+#pragma unroll
+    for (int i = 0; i < kChain; ++i) v = atomicAdd(word + v, 0u);        // (words are zero)
+    long long t1;
+    asm volatile("{\n\t.reg .u64 t, w;\n\tcvt.u64.u32 w, %1;\n\tmov.u64 t, %%clock64;\n\tadd.u64 %0, t, w;\n\t}" : "=l"(t1) : "r"(v) : "memory");
+    return (uint32_t)(t1 - t0);
+}
+__device__ uint32_t best_of(uint32_t* word, int rounds) {
+    uint32_t best = atomic_cycles(word);
+    for (int r = 1; r < rounds; ++r) best = min(best, atomic_cycles(word));
+    return best;
+}
+
+__global__ void home_latency_kernel(uint32_t* pool, Latencies* out) {
+    if (threadIdx.x != 0) return;
+    uint32_t sm;
+    asm("mov.u32 %0, %%smid;" : "=r"(sm));
+    sm %= kPlaceSms;
+    // every SM the same pages, each from another one on
+    for (int i = 0; i < kProbePages; ++i) {
+        const int page = (i + (int)blockIdx.x) % kProbePages;
+        uint32_t sum = 0;
+        for (int l = 0; l < kProbeLines; ++l) sum += best_of(pool + (size_t)page * (kPlacePage / 4) + l * 64, 6);
+        out->of_sm[sm][page] = sum;
+    }
+    // every page one SM
+    for (int page = (int)blockIdx.x; page < kPoolPages; page += (int)gridDim.x) {
+        uint32_t sum = 0;
+        for (int l = 0; l < kPageLines; ++l) sum += best_of(pool + (size_t)page * (kPlacePage / 4) + l * 64, 3);
+        out->of_page[page] = sum;
+        out->by[page] = sm;
+    }
+}
+
+struct Scratch {
+    void* p = nullptr;
+    ~Scratch() {
+        if (p != nullptr) cudaFree(p);
+    }
+};
+
+}  // namespace
+
+cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t stream) {
+    constexpr int kGroups = 8, kRanks = 16;
+    const size_t pool_at = chain_pool_at(exchange);
+    const uint32_t pool_quad = (uint32_t)(pool_at / 16), page_quads = kPlacePage / 16;
+    // any place will do
+    std::fill(out->die_of_sm, out->die_of_sm + kPlaceSms, (uint8_t)0);
+    out->on_first = kGroups * kRanks;
+    for (int g = 0; g < kGroups; ++g)
+        for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = pool_quad + (uint32_t)(g * kGroupPages + i) * page_quads;
+    static_assert(kGroups * kGroupPages <= kPoolPages, "pages of all groups");
+
+    int device = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return e;
+    std::vector<Latencies> host(1);
+    Latencies& h = host[0];
+    Scratch scratch;
+    e = cudaMalloc(&scratch.p, sizeof(Latencies));
+    if (e != cudaSuccess) return e;
+    Latencies* d = static_cast<Latencies*>(scratch.p);
+    uint32_t* pool = reinterpret_cast<uint32_t*>(static_cast<char*>(exchange) + pool_at);
+    e = cudaMemsetAsync(d, 0, sizeof(Latencies), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(pool, 0, (size_t)kPoolPages * kPlacePage, stream);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(home_latency_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone);
+    if (e == cudaSuccess) {
+        home_latency_kernel<<<sms, kWarp, kAlone, stream>>>(pool, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(Latencies), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return e;
+
+    // SMs of one die agree within a tenth on every page; the other die's take 1.4 to 2.4 times as long, or as little
+    std::vector<int> of_die[2];
+    std::vector<uint8_t> die_of_sm(kPlaceSms, 0);
+    int reference = -1;
+    for (int sm = 0; sm < kPlaceSms; ++sm) {
+        if (h.of_sm[sm][0] == 0) continue;
+        if (reference < 0) reference = sm;
+        double apart = 0.0;
+        for (int p = 0; p < kProbePages; ++p)
+            apart += std::fabs(std::log((double)std::max(h.of_sm[sm][p], 1u) / std::max(h.of_sm[reference][p], 1u)));
+        die_of_sm[sm] = apart / kProbePages > 0.25 ? 1 : 0;
+        of_die[die_of_sm[sm]].push_back(sm);
+    }
+    const int first = (int)of_die[0].size(), second = (int)of_die[1].size();
+    const int groups_first = std::max(std::min(first / kRanks, kGroups / 2), kGroups - second / kRanks);     // as even as they allow
+    if (first + second != sms || groups_first < 1 || groups_first >= kGroups || groups_first * kRanks > first
+        || (kGroups - groups_first) * kRanks > second) {
+        return cudaSuccess;
+    }
+    // an SM's pages fall into two bands
+    std::vector<uint32_t> least(kPlaceSms, 0xffffffffu), home[2];
+    for (int p = 0; p < kPoolPages; ++p) least[h.by[p]] = std::min(least[h.by[p]], h.of_page[p]);
+    for (int p = 0; p < kPoolPages; ++p) {
+        const bool far = h.of_page[p] > least[h.by[p]] * 1.35;
+        home[far ? 1 - die_of_sm[h.by[p]] : die_of_sm[h.by[p]]].push_back(pool_quad + (uint32_t)p * page_quads);
+    }
+    if ((int)home[0].size() < groups_first * kGroupPages || (int)home[1].size() < (kGroups - groups_first) * kGroupPages) return cudaSuccess;
+    std::copy(die_of_sm.begin(), die_of_sm.end(), out->die_of_sm);
+    out->on_first = groups_first * kRanks;
+    size_t next[2] = {0, 0};
+    for (int g = 0; g < kGroups; ++g) {
+        const int die = g < groups_first ? 0 : 1;
+        for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = home[die][next[die]++];
+    }
+    return cudaSuccess;
+}
+
+}  // namespace q3t

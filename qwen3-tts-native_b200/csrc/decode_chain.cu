@@ -37,6 +37,12 @@
 // ring in shared memory in 8 KB bulk copies, requested by a warp of their own as far ahead as the ring
 // reaches, so that HBM (talker) or the L2 (predictor) keeps delivering while the CTAs wait for each other.
 //
+// Where the CTAs and the buffers are.  The GPU is two dies.  A word written on one die and read on the same one from memory
+// that is at home there is read 550 cycles after the store; where one of the three lies on the other die it is 950 to 1,050.
+// Homes alternate by pages of 4 KB.  So a group's CTAs are taken from one die and its buffers from pages of that die: each CTA
+// claims a place of its SM's die at the start, and the launch has a CTA for every SM, those without a place leave at once.
+// chain_places.cu measures which SM and which page lies where; where it cannot tell, any place will do.
+//
 // The launch is cooperative (all CTAs resident or none) and the engine orders the chains of a device one
 // after the other.  Every wait is bounded by a deadline; a wait that gives up marks the run, all others then
 // give up at once, the kernel runs through on whatever it holds and the host refuses the result.
@@ -105,22 +111,25 @@ struct alignas(16) Quad {
     uint32_t x, y, z, flag;
 };
 constexpr int kPartQuads = 2 * kSlices * kRanks * kRowsMost * 48;
-constexpr int kHiddenQuads = 2 * kSlices * kRanks * kRowsMost * 24;
+constexpr int kHiddenQuads = 2 * kRanks * kRowsMost * 24;
 constexpr int kGroupRow = 8;                         // quads of a CTA's q/k/v rows (6) or gate/up channels (4 or 8) of an activation row
-constexpr int kGroupQuads = 2 * kSlices * kRanks * kRowsMost * kGroupRow;
-constexpr int kAttnPartQuads = 2 * kSlices * kRanks * kRowsMost * 88;
-constexpr int kAttnQuads = 2 * kSlices * kRanks * 22;
+constexpr int kGroupQuads = 2 * kRanks * kRowsMost * kGroupRow;
+constexpr int kAttnPartQuads = 2 * kRanks * kRowsMost * 88;
+constexpr int kAttnQuads = 2 * kRanks * 22;
 constexpr int kLogitQuads = 2 * kCtas * kRowsMost * 3;
 constexpr int kTokenQuads = 2 * kRowsMost;
 constexpr int kAppendedQuads = 2 * kSlices * kRowsMost;
-constexpr int kAtHidden = kPartQuads;
+// what stays in a group: behind the rest, in pages of the group's die; offsets in a group's own space
+constexpr int kAtHidden = 0;
 constexpr int kAtGroup = kAtHidden + kHiddenQuads;
 constexpr int kAtAttnPart = kAtGroup + kGroupQuads;
 constexpr int kAtAttn = kAtAttnPart + kAttnPartQuads;
-constexpr int kAtLogits = kAtAttn + kAttnQuads;
+constexpr int kPageQuads = kPlacePage / 16;
+static_assert((kAtAttn + kAttnQuads + kPageQuads - 1) / kPageQuads <= kGroupPages, "pages of a group");
+constexpr int kAtLogits = kPartQuads;
 constexpr int kAtTokens = kAtLogits + kLogitQuads;
 constexpr int kAtAppended = kAtTokens + kTokenQuads;
-constexpr int kExchangeQuads = kAtAppended + kAppendedQuads;
+constexpr int kSharedQuads = (kAtAppended + kAppendedQuads + kPageQuads - 1) / kPageQuads * kPageQuads;
 
 __device__ unsigned int g_chain_errors = 0;
 __device__ unsigned int* g_chain_error_sink = nullptr;
@@ -178,6 +187,8 @@ struct ChainArgs {
     const uint32_t* rope_table;      // [positions][64] bf16 cos | sin
     Quad* exchange;
     uint32_t* epoch;                 // [0] number of the last exchange, [1] the run that was given up
+    const ChainPlaces* places;
+    uint32_t* claims;                // [0], [1] places taken on a die, [2] CTAs that have asked
     int rows;
     float eps;
 };
@@ -217,7 +228,8 @@ struct Layout {
     // itself (K as rows, V with the tokens of a dimension side by side): nothing to fetch, nothing to publish.
     static constexpr bool LocalKv = !TALKER && ROWS <= 2;
     static constexpr int KvPage = 2 * kPageTokens * 128 * 2;
-    static constexpr int AtConst = AtMisc + MiscBytes;             // the layers' constants
+    static constexpr int AtPages = AtMisc + MiscBytes;             // of the group's buffers
+    static constexpr int AtConst = AtPages + kGroupPages * 4;      // the layers' constants
     static constexpr int AtKv = (AtConst + S::Layers * (int)sizeof(LayerConst) + 127) / 128 * 128;
     static constexpr int AtRing = AtKv + (LocalKv ? ROWS * S::Layers * KvPage : 0);
     static constexpr int Budget = 227 * 1024;
@@ -235,6 +247,7 @@ struct Misc {
     uint64_t full[24];
     uint64_t empty[24];            // counts the units of the slot that have been read
     unsigned int asked[24];        // copies requested into the slot
+    int place;
     uint32_t base, landed;         // landed: slots of the stream, in order
     int abort;
     int position[kRowsMost];
@@ -312,7 +325,8 @@ struct Chain {
     const ChainArgs& a;
     unsigned char* smem;
     Misc* misc;
-    int tid, lane, warp, slice, rank, rows;
+    int tid, lane, warp, rows;
+    int cta = 0, slice = 0, rank = 0;                   // the CTA's place among the kCtas
     uint32_t seq = 0;              // ring slots consumed by the phases so far
     uint32_t step = 0;             // exchanges so far
     uint32_t base = 0;
@@ -323,7 +337,7 @@ struct Chain {
 
     __device__ Chain(const ChainArgs& args, unsigned char* s)
         : a(args), smem(s), misc(reinterpret_cast<Misc*>(s + L::AtMisc)), tid(threadIdx.x), lane(threadIdx.x % kWarp),
-          warp(__shfl_sync(0xffffffffu, (int)threadIdx.x / kWarp, 0)), slice(blockIdx.x / kRanks), rank(blockIdx.x % kRanks),
+          warp(__shfl_sync(0xffffffffu, (int)threadIdx.x / kWarp, 0)),
           rows(ROWS <= 2 ? ROWS : args.rows) {}
 
     // ---- bounded waits -------------------------------------------------------------------------------------
@@ -390,8 +404,8 @@ struct Chain {
     static constexpr uint32_t kAllSlots = TALKER ? kLayerSlots + S::HeadSlots : kCodebooks * kLayerSlots + 15 * S::HeadSlots;
     // The requesting warp's one thread: slot after slot of the CTA's stream, each once what lay in its place has been read.
     __device__ __forceinline__ void request_weights() {
-        const uint8_t* layers = a.stream + (size_t)blockIdx.x * S::Layers * S::LayerBytes;
-        const uint8_t* heads = a.heads + (size_t)blockIdx.x * (TALKER ? 1 : 15) * S::HeadBytes;
+        const uint8_t* layers = a.stream + (size_t)cta * S::Layers * S::LayerBytes;
+        const uint8_t* heads = a.heads + (size_t)cta * (TALKER ? 1 : 15) * S::HeadBytes;
         // the layers, then a head; the predictor's sixteen positions all read the layers, and position 0 has no head
         const uint8_t* src = layers;
         uint32_t left = kLayerSlots, at = 0, fill = 0;
@@ -769,8 +783,11 @@ struct Chain {
     __device__ __forceinline__ Quad* part_at(int b, int s, int rk, int r) {
         return a.exchange + (((b * kSlices + s) * kRanks + rk) * kRowsMost + r) * (2 * S::Groups);
     }
-    __device__ __forceinline__ Quad* group_at(int kind_base, int quads_per_row, int b, int rk, int r) {
-        return a.exchange + kind_base + (((b * kSlices + slice) * kRanks + rk) * kRowsMost + r) * quads_per_row;
+    __device__ __forceinline__ Quad* group_quad(int at) {
+        return a.exchange + reinterpret_cast<const uint32_t*>(smem + L::AtPages)[at / kPageQuads] + at % kPageQuads;
+    }
+    __device__ __forceinline__ Quad* group_at(int kind_base, int quads_per_row, int b, int rk, int r, int quad) {
+        return group_quad(kind_base + ((b * kRanks + rk) * kRowsMost + r) * quads_per_row + quad);
     }
     // One value per lane (lanes < n, n a multiple of 2) -> quads of six bf16, sent by the first ceil(n / 6) lanes
     __device__ __forceinline__ void put_values(float v, int n, Quad* dst, uint32_t flag) {
@@ -844,7 +861,7 @@ struct Chain {
                 bf16* mine = own + r * S::Out;
                 sum_group(rank, r, g, mine, packed);
                 store_group(mine, g, packed);
-                put_quad(group_at(kAtHidden, S::Groups, bh, rank, r) + g, packed[0], packed[1], packed[2], flag_h);
+                put_quad(group_at(kAtHidden, S::Groups, bh, rank, r, g), packed[0], packed[1], packed[2], flag_h);
             }
             // a thread's quads, up to six, requested together
             constexpr int kEach = (ROWS * kRanks * S::Groups + kWorkers - 1) / kWorkers < 6 ? (ROWS * kRanks * S::Groups + kWorkers - 1) / kWorkers : 6;
@@ -858,7 +875,7 @@ struct Chain {
                     const int n = min(i + k * kWorkers, kRanks * rows * S::Groups - 1);
                     g[k] = n % S::Groups;
                     const int r = n / S::Groups % rows, rk = n / S::Groups / rows;
-                    p[k] = group_at(kAtHidden, S::Groups, bh, rk, r) + g[k];
+                    p[k] = group_at(kAtHidden, S::Groups, bh, rk, r, g[k]);
                     at[k] = r * S::H + rk * S::Out;
                 }
                 poll(p, v, flag_h);
@@ -881,7 +898,7 @@ struct Chain {
         const int r0 = tid / (kGroupRow * kRanks);
         if (g < per_row && r0 < rows) {
 #pragma unroll
-            for (int i = 0; i < kEach; ++i) p[i] = group_at(kAtGroup, kGroupRow, b, rk, min(r0 + 2 * i, rows - 1)) + g;
+            for (int i = 0; i < kEach; ++i) p[i] = group_at(kAtGroup, kGroupRow, b, rk, min(r0 + 2 * i, rows - 1), g);
             poll(p, v, flag);
 #pragma unroll
             for (int i = 0; i < kEach; ++i) {
@@ -1167,7 +1184,7 @@ struct Chain {
             const int r = i / 88, q = i % 88;
             if (my_slot(r) >= slots_of(r)) continue;
             const float* src = out_s + (r * 2 + q / 44) * 132 + 3 * (q % 44);
-            put_quad(group_at(kAtAttnPart, 88, b, rank, r) + q, __float_as_uint(src[0]), __float_as_uint(src[1]), __float_as_uint(src[2]), flag);
+            put_quad(group_at(kAtAttnPart, 88, b, rank, r, q), __float_as_uint(src[0]), __float_as_uint(src[1]), __float_as_uint(src[2]), flag);
         }
         float* gathered = reinterpret_cast<float*>(smem + L::AtX);              // [rank][132] of a head
         auto fold = [&](const float* from, int stride, int ranks, int dim) {
@@ -1185,7 +1202,7 @@ struct Chain {
                 for (int k = 0; k < 3; ++k) {
                     const int n = min(i + k * kWorkers, ranks * 88 - 1);
                     const int rk = n / 88, q = n % 88;
-                    p[k] = group_at(kAtAttnPart, 88, b, rank_of(0, rk), 0) + q;
+                    p[k] = group_at(kAtAttnPart, 88, b, rank_of(0, rk), 0, q);
                     dst[k] = gathered + (rk * 2 + q / 44) * 132 + 3 * (q % 44);
                 }
                 poll(p, v, flag);
@@ -1209,7 +1226,7 @@ struct Chain {
 #pragma unroll 1
                 for (int i = tid; i < ranks * 44; i += kWorkers) {
                     const int rk = i / 44, q = i % 44;
-                    const Quad v = poll_one(group_at(kAtAttnPart, 88, b, rank_of(row, rk), row) + head * 44 + q, flag);
+                    const Quad v = poll_one(group_at(kAtAttnPart, 88, b, rank_of(row, rk), row, head * 44 + q), flag);
                     float* dst = gathered + rk * 132 + 3 * q;
                     dst[0] = __uint_as_float(v.x);
                     dst[1] = __uint_as_float(v.y);
@@ -1221,13 +1238,13 @@ struct Chain {
                 sync_workers();
                 if (tid < 22) {
                     const uint32_t* w = reinterpret_cast<const uint32_t*>(mine) + 3 * tid;
-                    put_quad(a.exchange + kAtAttn + ((bo * kSlices + slice) * kRanks + rank) * 22 + tid, w[0], w[1], w[2], flag_o);
+                    put_quad(group_quad(kAtAttn + (bo * kRanks + rank) * 22 + tid), w[0], w[1], w[2], flag_o);
                 }
             }
 #pragma unroll 1
             for (int i = tid; i < 2 * rows * 22; i += kWorkers) {
                 const int rk = i / 22, q = i % 22;
-                const Quad v = poll_one(a.exchange + kAtAttn + ((bo * kSlices + slice) * kRanks + rk) * 22 + q, flag_o);
+                const Quad v = poll_one(group_quad(kAtAttn + (bo * kRanks + rk) * 22 + q), flag_o);
                 uint32_t* dst = reinterpret_cast<uint32_t*>(att + (rk >> 1) * S::Slice + (rk & 1) * 128) + 3 * q;
                 dst[0] = v.x;
                 if (q < 21) {
@@ -1291,7 +1308,7 @@ struct Chain {
                     const float up = sum_up * scale_up;
                     value = value / (1.0f + expf(-value)) * up;
                 }
-                put_values(value, n, group_at(kAtGroup, kGroupRow, b, rank, r) + 4 * chunk, flag_g);
+                put_values(value, n, group_at(kAtGroup, kGroupRow, b, rank, r, 4 * chunk), flag_g);
             }
             end_full(half == 0 ? 2 : S::GuTiles);
             if (half == 0) {
@@ -1340,7 +1357,7 @@ struct Chain {
 
     // ---- predictor head and draw ---------------------------------------------------------------------------------
     __device__ __forceinline__ void predictor_head(int p, const float* scales, const uint32_t (&nw)[S::J]) {
-        const float scale = scales[blockIdx.x * 16 + (lane & 15)];
+        const float scale = scales[cta * 16 + (lane & 15)];
         const float u = norm_to_limbs(nw, nullptr);
         sync_workers();
         mma_full(S::HeadTiles, u);
@@ -1352,7 +1369,7 @@ struct Chain {
             float sum = 0.0f;
 #pragma unroll
             for (int w = 0; w < 8; ++w) sum += red[(w * rows + warp) * kRedRow + (lane & 15)];
-            put_values(sum * scale, 16, a.exchange + kAtLogits + ((b * kCtas + (int)blockIdx.x) * kRowsMost + warp) * 3, flag);
+            put_values(sum * scale, 16, a.exchange + kAtLogits + ((b * kCtas + cta) * kRowsMost + warp) * 3, flag);
         }
         end_full(S::HeadTiles);
         if (p + 1 < kCodebooks) hold_ahead(2, 4);                // the next position's q/k/v
@@ -1423,8 +1440,25 @@ struct Chain {
     }
 
     // ---- the whole chain ------------------------------------------------------------------------------------------
+    // A place of the die that the SM lies on, or none (-1).  Who asks last finds all places given out and clears the counts for
+    // the next launch.
+    __device__ __forceinline__ int claim_place() {
+        uint32_t sm;
+        asm("mov.u32 %0, %%smid;" : "=r"(sm));
+        const int die = a.places->die_of_sm[sm % kPlaceSms];
+        const int first = die == 0 ? 0 : a.places->on_first, most = die == 0 ? a.places->on_first : kCtas - a.places->on_first;
+        const int n = (int)atomicAdd(a.claims + die, 1u);
+        if (n < 0) return -1;                      // (the answer is here before the CTA is counted)
+        __threadfence();
+        if (atomicInc(a.claims + 2, gridDim.x - 1) == gridDim.x - 1) {
+            *reinterpret_cast<volatile uint32_t*>(a.claims) = 0u;
+            *reinterpret_cast<volatile uint32_t*>(a.claims + 1) = 0u;
+        }
+        return n < most ? first + n : -1;
+    }
     __device__ __forceinline__ void run() {
-        if (tid == 0) {
+        if (tid == 0) misc->place = claim_place();
+        if (tid == 32) {
             for (int s = 0; s < L::Slots; ++s) {
                 mbar_init(&misc->full[s], 1);
                 mbar_init(&misc->empty[s], kSlotUnits);
@@ -1435,6 +1469,14 @@ struct Chain {
             misc->base = *reinterpret_cast<volatile uint32_t*>(a.epoch);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncthreads();
+        cta = misc->place;
+        if (cta < 0) return;
+        slice = cta / kRanks;
+        rank = cta % kRanks;
+        if (tid >= kWorkers && tid < kWorkers + kGroupPages) {
+            reinterpret_cast<uint32_t*>(smem + L::AtPages)[tid - kWorkers] = a.places->pages[slice][tid - kWorkers];
         }
         if (tid < rows) {
             if (TALKER) {
@@ -1472,7 +1514,7 @@ struct Chain {
 #pragma unroll 1
             for (int l = 0; l < S::Layers; ++l) layer(l, 0, l + 1 < S::Layers ? 2 : S::HeadTiles, nw, walk);
             load_norm(a.final_norm, nw);
-            const float u = norm_to_limbs(nw, blockIdx.x == 0 ? a.normalized : nullptr);
+            const float u = norm_to_limbs(nw, cta == 0 ? a.normalized : nullptr);
             sync_workers();
             mma_full(S::HeadTiles, u);
             sync_workers();
@@ -1483,7 +1525,7 @@ struct Chain {
                 float sum = 0.0f;
 #pragma unroll
                 for (int w = 0; w < 8; ++w) sum += red[(w * rows + r) * kRedRow + n];
-                const int channel = blockIdx.x * S::HeadRows + n;
+                const int channel = cta * S::HeadRows + n;
                 a.logits[(size_t)r * (kCtas * S::HeadRows) + channel] = f2bf(sum * a.head_s[0][channel]);
             }
         } else {
@@ -1510,13 +1552,13 @@ struct Chain {
                 if (p > 0) predictor_head(p, head_scales, head_norm);
                 if constexpr (!L::LocalKv) say_appended(p + 1 == kCodebooks);
             }
-            if (ROWS == 1 ? blockIdx.x == 0 && tid == 0 : rank == 0 && slice < rows && tid == 0) {
+            if (ROWS == 1 ? cta == 0 && tid == 0 : rank == 0 && slice < rows && tid == 0) {
                 const int r = ROWS == 1 ? 0 : slice;
                 *a.table->rng[r] = misc->rng[r];
             }
             // the frame's codes, once all are drawn: sixteen stores in the way of the draws cost a microsecond each
             sync_workers();
-            if (blockIdx.x == 0 && tid < rows * kCodebooks) {
+            if (cta == 0 && tid < rows * kCodebooks) {
                 const int r = tid / kCodebooks, p = tid % kCodebooks;
                 const unsigned short code = misc->codes[r][p];
                 a.table->frame_tokens[r][p] = code;
@@ -1530,7 +1572,7 @@ struct Chain {
             for (uint32_t polls = 0; polls < (1u << 14) && !mbar_try_wait(&misc->full[tid], (misc->asked[tid] - 1) & 1u); ++polls) {}
         }
         sync_workers();
-        if (blockIdx.x == 0 && tid == 0) {
+        if (cta == 0 && tid == 0) {
             if (given_up()) {
                 atomicAdd(&g_chain_errors, 1u);
                 if (g_chain_error_sink != nullptr) atomicAdd_system(g_chain_error_sink, 1u);
@@ -1600,10 +1642,12 @@ cudaError_t configure_variant() {
     return cudaFuncSetAttribute(decode_chain_kernel<TALKER, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<TALKER, ROWS>::Bytes);
 }
 
+int g_chain_sms = kCtas;             // a CTA for every SM (the same on all devices that the chain runs on)
+
 template <bool TALKER, int ROWS>
 cudaError_t launch_variant(const ChainArgs& a, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kCtas);
+    cfg.gridDim = dim3((unsigned)g_chain_sms);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = Layout<TALKER, ROWS>::Bytes;
     cfg.stream = stream;
@@ -1638,7 +1682,8 @@ cudaError_t configure_chain_kernels() {
     if (e == cudaSuccess) e = configure_variant<false, 2>();
     if (e == cudaSuccess) e = configure_variant<false, 4>();
     if (e == cudaSuccess) e = configure_variant<false, 8>();
-    if (e == cudaSuccess && device >= 0 && device < 64) g_chain_fits[device] = cooperative != 0 && sms >= kCtas;
+    if (e == cudaSuccess && device >= 0 && device < 64) g_chain_fits[device] = cooperative != 0 && sms >= kCtas && sms <= kPlaceSms;
+    if (e == cudaSuccess && sms >= kCtas) g_chain_sms = sms;
     return e;
 }
 
@@ -1651,7 +1696,11 @@ size_t chain_stream_bytes(bool talker) {
     return (size_t)kCtas * (talker ? (size_t)Shape<true>::Layers * Shape<true>::LayerBytes : (size_t)Shape<false>::Layers * Shape<false>::LayerBytes);
 }
 size_t chain_head_bytes(bool talker) { return (size_t)kCtas * (talker ? Shape<true>::HeadBytes : 15 * Shape<false>::HeadBytes); }
-size_t chain_exchange_bytes() { return (size_t)kExchangeQuads * sizeof(Quad); }
+size_t chain_exchange_bytes() { return (size_t)kSharedQuads * sizeof(Quad) + (size_t)kPoolPages * kPlacePage + kPlacePage; }
+size_t chain_pool_at(const void* exchange) {
+    const size_t at = reinterpret_cast<uintptr_t>(exchange) + (size_t)kSharedQuads * sizeof(Quad);
+    return (at + kPlacePage - 1) / kPlacePage * kPlacePage - reinterpret_cast<uintptr_t>(exchange);
+}
 
 cudaError_t launch_pack_layer(bool talker, int layer, const int8_t* qkv, const int8_t* o, const int8_t* gate_up, const int8_t* down,
                               uint8_t* stream_base, cudaStream_t stream) {
@@ -1687,7 +1736,7 @@ cudaError_t launch_decode_chain(const ChainLaunch& c, cudaStream_t stream) {
     a.stream = c.stream; a.heads = c.heads; a.layers = reinterpret_cast<const LayerConst*>(c.layers); a.final_norm = c.final_norm;
     a.head_s = c.head_scales; a.hidden = c.hidden; a.normalized = c.normalized; a.logits = c.logits; a.projected = c.projected;
     a.table = c.table; a.positions = c.positions; a.kv = c.kv; a.kv_layer_elems = c.kv_layer_elems; a.rope_table = c.rope_table;
-    a.exchange = static_cast<Quad*>(c.exchange); a.epoch = c.epoch; a.rows = c.rows; a.eps = kRmsEps;
+    a.exchange = static_cast<Quad*>(c.exchange); a.epoch = c.epoch; a.places = c.places; a.claims = c.claims; a.rows = c.rows; a.eps = kRmsEps;
     return c.talker ? launch_rows<true>(a, stream) : launch_rows<false>(a, stream);
 }
 

@@ -721,6 +721,11 @@ void Model::build_chain() {
     table(chain.projected, rows.data(), rows.size() * sizeof(const bf16*));
     chain.exchange = DeviceBuffer(chain_exchange_bytes());
     chain.epoch = DeviceBuffer(2 * sizeof(uint32_t));
+    ChainPlaces places;
+    check_cuda(find_chain_places(chain.exchange.as<void>(), &places, upload_stream_), "chain places");
+    table(chain.places, &places, sizeof(places));
+    const uint32_t none[3] = {0, 0, 0};
+    table(chain.claims, none, sizeof(none));
     check_cuda(restart_chain_numbers(chain.exchange.as<void>(), chain.epoch.as<uint32_t>(), upload_stream_), "chain numbers");
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(decode chain)");
     chain.ready = true;
@@ -895,6 +900,7 @@ void enqueue_chain(Workspace& w, Model& m, bool talker, int n, cudaStream_t s) {
     }
     a.kv_layer_elems = 2 * pool.plane_elems();
     a.exchange = c.exchange.as<void>(); a.epoch = c.epoch.as<uint32_t>();
+    a.places = c.places.as<const ChainPlaces>(); a.claims = c.claims.as<uint32_t>();
     a.rows = n;
     check_launch(launch_decode_chain(a, s), talker ? "talker chain" : "predictor chain");
 }

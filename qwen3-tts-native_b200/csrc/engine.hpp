@@ -231,7 +231,7 @@ public:
     struct DecodeChain {
         bool ready = false;
         DeviceBuffer streams[2], heads[2], layers[2], head_scales[2];     // 0 predictor, 1 talker
-        DeviceBuffer projected_rows, projected, exchange, epoch;
+        DeviceBuffer projected_rows, projected, exchange, epoch, places, claims;
         uint64_t numbers = 0;           // of exchanges, at most, since they were restarted (guarded as the device's chains are)
     } chain;
     std::mutex mutex;               // pools, workspaces
