@@ -4,9 +4,9 @@
 // A frame of few sessions is a chain of some 540 dependent projections and attentions whose bytes are few:
 // launched one by one, each costs 0.6 us of hand-over, 0.9 us until its activations are fetched and
 // converted, and its exchange and epilogue, 3.5-9 us a link whatever it streams.  Here 128 CTAs stay on
-// their SMs for the whole chain.  What bounds it now is the number of exchanges between them: a value
-// written by one SM is read by another 0.9 us later (1.2 us when everybody reads 43 KB).  So the split of the
-// work is the one that needs fewest:
+// their SMs for the whole chain.  What bounds it now is what a hand-over between them costs: 0.3 us for a word within a
+// die and 0.5 across, 0.4 to 1.1 us with the wait for the slowest, and 0.3 to 1.5 us of instructions on either side.  So
+// the split of the work is the one that needs fewest:
 //
 //   8 groups of 16 CTAs; group c owns KV head c (and its two query heads), i.e. slice c of eight of every
 //   contraction whose input it produced itself.
@@ -401,14 +401,18 @@ struct Chain {
 
     // ---- ring ----------------------------------------------------------------------------------------------
     static constexpr uint32_t kLayerSlots = S::Layers * S::LayerSlots;
-    static constexpr uint32_t kAllSlots = TALKER ? kLayerSlots + S::HeadSlots : kCodebooks * kLayerSlots + 15 * S::HeadSlots;
+    // Of the predictor's position 0 only the keys and values are needed: its last layer ends with them.  (3 and 8 sessions 2,140
+    // -> 2,123 and 3,207 -> 3,176 us; with one or two rows it gains nothing, 1,569 and 1,575.)
+    static constexpr bool kEndsEarly = !TALKER && !L::LocalKv;
+    static constexpr uint32_t kUnused = kEndsEarly ? S::LayerSlots - S::QkvBytes / kSlot : 0;
+    static constexpr uint32_t kAllSlots = TALKER ? kLayerSlots + S::HeadSlots : kCodebooks * kLayerSlots + 15 * S::HeadSlots - kUnused;
     // The requesting warp's one thread: slot after slot of the CTA's stream, each once what lay in its place has been read.
     __device__ __forceinline__ void request_weights() {
         const uint8_t* layers = a.stream + (size_t)cta * S::Layers * S::LayerBytes;
         const uint8_t* heads = a.heads + (size_t)cta * (TALKER ? 1 : 15) * S::HeadBytes;
         // the layers, then a head; the predictor's sixteen positions all read the layers, and position 0 has no head
         const uint8_t* src = layers;
-        uint32_t left = kLayerSlots, at = 0, fill = 0;
+        uint32_t left = kLayerSlots - kUnused, at = 0, fill = 0;
         bool in_layers = true, headless = !TALKER;
 #pragma unroll 1
         for (uint32_t s = 0; s < kAllSlots; ++s) {
@@ -1325,6 +1329,11 @@ struct Chain {
                 if constexpr (TALKER) talker_attention(hn, layer_elems, f, walk);
                 else if constexpr (L::LocalKv) local_attention(hn, index, pos);
                 else predictor_attention(hn, f, walk.k + layer_elems, walk.v + layer_elems, pos);
+                if (kEndsEarly && pos == 0 && index + 1 == S::Layers) {
+                    static_assert(!kEndsEarly || !kAhead, "nothing is held for what is left out");
+                    load_norm(constants(0).in_norm, nw);
+                    return;
+                }
             }
             // the o projection is over the group's 256 attention values, the down projection over its channels
             slice_to_limbs<S::Slice / 64>(smem + (half == 0 ? L::AtAtt : L::AtAct), S::Slice * 2);

@@ -780,10 +780,11 @@ struct Probe {
     std::function<void(const char* stage, int layer, const bf16* values, int width)> emit;
 };
 
+// `last_keys_only`: nothing behind the last layer's cache rows is needed (the predictor's position 0, whose hidden row no head reads)
 void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWeights>& layers,
                     const uint32_t* rope_table, const KvPool& pool, const int* page_table, int table_stride,
                     const int* positions, int n, int splits, cudaStream_t s, int prompt_base = -1,
-                    const Probe* probe = nullptr, bool chain_order = false) {
+                    const Probe* probe = nullptr, bool chain_order = false, bool last_keys_only = false) {
     const int qkv_width = d.q_width + 2 * d.kv_width;
     // a prompt pass (prompt_base >= 0): the rows are consecutive positions of one session
     const bool shared_cache = prompt_base >= 0;
@@ -845,6 +846,7 @@ void enqueue_layers(Workspace& w, const ModelDims& d, const std::vector<LayerWei
             check_launch(launch_attention(a, s), "decode attention");
         }
         observe("attention", w.attention.as<bf16>(), d.q_width, d.q_width);
+        if (last_keys_only && l + 1 == layers.size()) break;
 
         GemvArgs o;
         o.w = lw.o.data; o.scales = lw.o.scales;
@@ -933,7 +935,7 @@ void enqueue_predictor(Workspace& w, Model& m, int n, cudaStream_t s) {
         check_launch(launch_int8_gemm(g, s), "predictor input projection");
         enqueue_layers(w, m.predictor, m.predictor_layers, m.predictor_rope, *m.predictor_pool,
                        w.predictor_pages.as<int>(), 1,
-                       w.predictor_positions.as<int>() + (size_t)p * kMaxRows, n, 1, s);
+                       w.predictor_positions.as<int>() + (size_t)p * kMaxRows, n, 1, s, -1, nullptr, false, p == 0);
         if (p >= 1) {
             GemvArgs h;
             h.w = m.predictor_heads[p - 1].data; h.scales = m.predictor_heads[p - 1].scales;
