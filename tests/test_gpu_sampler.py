@@ -80,6 +80,19 @@ def test_config_defaults_paths(orc, ops):
                 history.append(got_tok)
 
 
+@pytest.mark.parametrize("spread", [2.0 ** -7, 2.0 ** -4, 0.5, 4.0, 40.0, 3e4])
+def test_selection_at_every_distance(orc, ops, spread):
+    """The k-th key is found by its distance from the largest, in steps that double with every octave beyond 127 ulps: from a
+    few ulps, where hundreds of keys share a step, to the far side of zero; k at the edges of what is drawn this way."""
+    rng = np.random.default_rng(int(spread * 128))
+    for top_k in (1, 2, 50, 127, 128):
+        for vocab in (128, 2048, 3072):
+            logits = orc.to_bf16((1.0 - spread * np.abs(rng.standard_normal(vocab))).astype(np.float32))
+            state = int(rng.integers(0, 2 ** 63))
+            cfg = dict(do_sample=1, top_k=top_k, top_p=0.95, temperature=float(max(spread, 0.5)), penalty=1.0)
+            assert ops.sample(logits, state, **cfg) == orc.sample(logits, state, suppress=False, history=[], **cfg)
+
+
 def test_greedy_does_not_draw(orc, ops):
     logits = orc.to_bf16(np.random.default_rng(2).standard_normal(2048).astype(np.float32))
     tok, state = ops.sample(logits, 777, do_sample=0, top_k=0)
