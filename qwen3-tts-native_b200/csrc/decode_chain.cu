@@ -1294,7 +1294,7 @@ struct Chain {
             sync_workers();           // everybody has read the hidden rows: their place takes the sums
             mma_full(half == 0 ? 2 : S::GuTiles, u);
             sync_workers();
-            const int bp = flip(kPart), b = flip(kGroup);
+            const int b = flip(kGroup);
             const uint32_t flag_g = next_flag();
             const float* red = reinterpret_cast<const float*>(smem + L::AtU);
 #pragma unroll 1
@@ -1337,6 +1337,7 @@ struct Chain {
             }
             // the o projection is over the group's 256 attention values, the down projection over its channels
             slice_to_limbs<S::Slice / 64>(smem + (half == 0 ? L::AtAtt : L::AtAct), S::Slice * 2);
+            const int bp = flip(kPart);               // (here and not ahead of the early end: a buffer is taken for what is sent)
             const uint32_t flag = next_flag();
             mma_slice(half == 0 ? 4 : kSliceBlocks, bp, flag);
             hold_ahead(half == 0 ? S::GuTiles : next_tiles, half == 0 ? kSliceBlocks : (next_tiles == 2 ? 4 : 0));
