@@ -428,6 +428,13 @@ QWEN3_TTS_API int32_t q3t_test_report_device_wait_failure(int32_t device_index);
  * started at number `given_up` having been given up.  No frame may be in flight. */
 QWEN3_TTS_API int32_t q3t_test_set_chain_numbers(Qwen3TtsModelHandle model, uint64_t used, uint32_t given_up);
 
+/* Test hooks.  set_chain_places: the die (0 or 1) that a model's decode chain takes each of 256 SMs to lie on, and the 124
+ * pages (of 2304, none twice) for the buffers of each of its 8 groups (both NULL: as measured); only the time of a frame
+ * depends on them, and no frame may be in flight.  hold_sms: a kernel on `stream` that takes `ctas` SMs for `ns`
+ * nanoseconds, 10^9 at most. */
+QWEN3_TTS_API int32_t q3t_test_set_chain_places(Qwen3TtsModelHandle model, const uint8_t* die_of_sm, const uint32_t* pages);
+QWEN3_TTS_API int32_t q3t_test_hold_sms(int32_t ctas, uint64_t ns, void* stream);
+
 /* Number of this library's kernels launched so far through frame graphs of the model. */
 QWEN3_TTS_API int32_t q3t_model_kernel_launches(Qwen3TtsModelHandle model, uint64_t* launches,
                                                 char* error, size_t error_capacity);

@@ -1126,6 +1126,12 @@ int32_t q3t_test_set_chain_numbers(Qwen3TtsModelHandle model, uint64_t used, uin
     return protect([&] { model_of(model)->set_chain_numbers(used, given_up); }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
 }
 
+int32_t q3t_test_set_chain_places(Qwen3TtsModelHandle model, const uint8_t* die_of_sm, const uint32_t* pages) {
+    if ((die_of_sm == nullptr) != (pages == nullptr)) return QWEN3_TTS_TALKER_STATUS_INVALID_ARGUMENT;
+    return protect([&] { model_of(model)->set_chain_places(die_of_sm, pages); }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
+}
+int32_t q3t_test_hold_sms(int32_t ctas, uint64_t ns, void* stream) { return static_cast<int32_t>(launch_hold_sms(ctas, ns, S(stream))); }
+
 uint32_t q3t_kernel_error_count(void) {
     return gemm_tc_error_count() + gemm_wide_error_count() + gemv_mma_error_count() + chain_error_count();
 }

@@ -7,6 +7,7 @@
 // Nothing here waits for another CTA.  Takes a millisecond, once for each model.
 
 #include "q3t_kernels.cuh"
+#include "q3t_tcgen05.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -62,6 +63,12 @@ __global__ void home_latency_kernel(uint32_t* pool, Latencies* out) {
     }
 }
 
+__global__ void hold_sm_kernel(unsigned long long ns) {
+    if (threadIdx.x != 0) return;
+    const unsigned long long until = tc::now_ns() + ns;
+    for (unsigned long long i = 0; i < ns / 100 && tc::now_ns() < until; ++i) __nanosleep(200);
+}
+
 struct Scratch {
     void* p = nullptr;
     ~Scratch() {
@@ -77,7 +84,6 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
     const uint32_t pool_quad = (uint32_t)(pool_at / 16), page_quads = kPlacePage / 16;
     // any place will do
     std::fill(out->die_of_sm, out->die_of_sm + kPlaceSms, (uint8_t)0);
-    out->on_first = kGroups * kRanks;
     for (int g = 0; g < kGroups; ++g)
         for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = pool_quad + (uint32_t)(g * kGroupPages + i) * page_quads;
     static_assert(kGroups * kGroupPages <= kPoolPages, "pages of all groups");
@@ -118,11 +124,10 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
         of_die[die_of_sm[sm]].push_back(sm);
     }
     const int first = (int)of_die[0].size(), second = (int)of_die[1].size();
-    const int groups_first = std::max(std::min(first / kRanks, kGroups / 2), kGroups - second / kRanks);     // as even as they allow
-    if (first + second != sms || groups_first < 1 || groups_first >= kGroups || groups_first * kRanks > first
-        || (kGroups - groups_first) * kRanks > second) {
-        return cudaSuccess;
-    }
+    // a launch of 128 CTAs lies evenly on the dies as far as they have the SMs
+    const int ctas_first = std::min(first, std::max(kGroups * kRanks / 2, kGroups * kRanks - second));
+    const int groups_first = (ctas_first + kRanks / 2) / kRanks;
+    if (first + second != sms || groups_first < 1 || groups_first >= kGroups) return cudaSuccess;
     // an SM's pages fall into two bands
     std::vector<uint32_t> least(kPlaceSms, 0xffffffffu), home[2];
     for (int p = 0; p < kPoolPages; ++p) least[h.by[p]] = std::min(least[h.by[p]], h.of_page[p]);
@@ -132,13 +137,20 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
     }
     if ((int)home[0].size() < groups_first * kGroupPages || (int)home[1].size() < (kGroups - groups_first) * kGroupPages) return cudaSuccess;
     std::copy(die_of_sm.begin(), die_of_sm.end(), out->die_of_sm);
-    out->on_first = groups_first * kRanks;
     size_t next[2] = {0, 0};
     for (int g = 0; g < kGroups; ++g) {
         const int die = g < groups_first ? 0 : 1;
         for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = home[die][next[die]++];
     }
     return cudaSuccess;
+}
+
+cudaError_t launch_hold_sms(int ctas, unsigned long long ns, cudaStream_t stream) {
+    if (ctas < 1 || ctas > kPlaceSms || ns > 1000000000ull) return cudaErrorInvalidValue;
+    const cudaError_t e = cudaFuncSetAttribute(hold_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone);
+    if (e != cudaSuccess) return e;
+    hold_sm_kernel<<<ctas, kWarp, kAlone, stream>>>(ns);
+    return cudaGetLastError();
 }
 
 }  // namespace q3t

@@ -40,8 +40,8 @@
 // Where the CTAs and the buffers are.  The GPU is two dies.  A word written on one die and read on the same one from memory
 // that is at home there is read 550 cycles after the store; where one of the three lies on the other die it is 950 to 1,050.
 // Homes alternate by pages of 4 KB.  So a group's CTAs are taken from one die and its buffers from pages of that die: each CTA
-// claims a place of its SM's die at the start, and the launch has a CTA for every SM, those without a place leave at once.
-// chain_places.cu measures which SM and which page lies where; where it cannot tell, any place will do.
+// claims a place on its SM's die at the start (claim_place).  chain_places.cu measures which SM and which page lies where; where
+// it cannot tell, any place will do.
 //
 // The launch is cooperative (all CTAs resident or none) and the engine orders the chains of a device one
 // after the other.  Every wait is bounded by a deadline; a wait that gives up marks the run, all others then
@@ -188,7 +188,7 @@ struct ChainArgs {
     Quad* exchange;
     uint32_t* epoch;                 // [0] number of the last exchange, [1] the run that was given up
     const ChainPlaces* places;
-    uint32_t* claims;                // [0], [1] places taken on a die, [2] CTAs that have asked
+    uint32_t* claims;                // [0], [1] CTAs of a die that have a place, [2] CTAs that have asked
     int rows;
     float eps;
 };
@@ -1450,21 +1450,22 @@ struct Chain {
     }
 
     // ---- the whole chain ------------------------------------------------------------------------------------------
-    // A place of the die that the SM lies on, or none (-1).  Who asks last finds all places given out and clears the counts for
-    // the next launch.
+    // A place on the die that the SM lies on: CTAs of the first die take them from the first one up, those of the second from the
+    // last one down, so that every CTA gets one, however many lie on either die.  (A quiet device puts 64 on each, so groups
+    // 0 to 3 are the first die's; where other kernels hold SMs, or the dies are uneven, one group is of both.)  Who asks last
+    // clears the counts for the next launch.
     __device__ __forceinline__ int claim_place() {
         uint32_t sm;
         asm("mov.u32 %0, %%smid;" : "=r"(sm));
         const int die = a.places->die_of_sm[sm % kPlaceSms];
-        const int first = die == 0 ? 0 : a.places->on_first, most = die == 0 ? a.places->on_first : kCtas - a.places->on_first;
         const int n = (int)atomicAdd(a.claims + die, 1u);
-        if (n < 0) return -1;                      // (the answer is here before the CTA is counted)
         __threadfence();
-        if (atomicInc(a.claims + 2, gridDim.x - 1) == gridDim.x - 1) {
+        if (atomicInc(a.claims + 2, kCtas - 1) == kCtas - 1) {
+            __threadfence();
             *reinterpret_cast<volatile uint32_t*>(a.claims) = 0u;
             *reinterpret_cast<volatile uint32_t*>(a.claims + 1) = 0u;
         }
-        return n < most ? first + n : -1;
+        return die == 0 ? n : kCtas - 1 - n;
     }
     __device__ __forceinline__ void run() {
         if (tid == 0) misc->place = claim_place();
@@ -1482,7 +1483,7 @@ struct Chain {
         }
         __syncthreads();
         cta = misc->place;
-        if (cta < 0) return;
+        __builtin_assume(cta >= 0 && cta < kCtas);         // (without it registers spill: one session 1,544 -> 1,593 us)
         slice = cta / kRanks;
         rank = cta % kRanks;
         if (tid >= kWorkers && tid < kWorkers + kGroupPages) {
@@ -1652,12 +1653,10 @@ cudaError_t configure_variant() {
     return cudaFuncSetAttribute(decode_chain_kernel<TALKER, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<TALKER, ROWS>::Bytes);
 }
 
-int g_chain_sms = kCtas;             // a CTA for every SM (the same on all devices that the chain runs on)
-
 template <bool TALKER, int ROWS>
 cudaError_t launch_variant(const ChainArgs& a, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)g_chain_sms);
+    cfg.gridDim = dim3((unsigned)kCtas);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = Layout<TALKER, ROWS>::Bytes;
     cfg.stream = stream;
@@ -1693,7 +1692,6 @@ cudaError_t configure_chain_kernels() {
     if (e == cudaSuccess) e = configure_variant<false, 4>();
     if (e == cudaSuccess) e = configure_variant<false, 8>();
     if (e == cudaSuccess && device >= 0 && device < 64) g_chain_fits[device] = cooperative != 0 && sms >= kCtas && sms <= kPlaceSms;
-    if (e == cudaSuccess && sms >= kCtas) g_chain_sms = sms;
     return e;
 }
 

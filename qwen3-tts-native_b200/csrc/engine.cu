@@ -721,14 +721,39 @@ void Model::build_chain() {
     table(chain.projected, rows.data(), rows.size() * sizeof(const bf16*));
     chain.exchange = DeviceBuffer(chain_exchange_bytes());
     chain.epoch = DeviceBuffer(2 * sizeof(uint32_t));
-    ChainPlaces places;
-    check_cuda(find_chain_places(chain.exchange.as<void>(), &places, upload_stream_), "chain places");
-    table(chain.places, &places, sizeof(places));
+    chain.places = DeviceBuffer(sizeof(ChainPlaces));
     const uint32_t none[3] = {0, 0, 0};
     table(chain.claims, none, sizeof(none));
+    place_chain();
+    chain.ready = true;
+}
+
+void Model::place_chain() {
+    ChainPlaces places;
+    check_cuda(find_chain_places(chain.exchange.as<void>(), &places, upload_stream_), "chain places");
+    set_now(chain.places.as<void>(), &places, sizeof(places), upload_stream_, "chain places");
     check_cuda(restart_chain_numbers(chain.exchange.as<void>(), chain.epoch.as<uint32_t>(), upload_stream_), "chain numbers");
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(decode chain)");
-    chain.ready = true;
+    chain.numbers = 0;
+}
+
+void Model::set_chain_places(const uint8_t* die_of_sm, const uint32_t* pages) {
+    if (!chain.ready) return;
+    check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(chain places)");
+    if (die_of_sm == nullptr) return place_chain();
+    ChainPlaces places;
+    std::vector<bool> taken(kPoolPages, false);
+    for (int sm = 0; sm < kPlaceSms; ++sm) {
+        if (die_of_sm[sm] > 1) throw std::invalid_argument("a die that is neither 0 nor 1");
+        places.die_of_sm[sm] = die_of_sm[sm];
+    }
+    const uint32_t first = static_cast<uint32_t>(chain_pool_at(chain.exchange.as<void>()) / 16);
+    for (int i = 0; i < 8 * kGroupPages; ++i) {
+        if (pages[i] >= (uint32_t)kPoolPages || taken[pages[i]]) throw std::invalid_argument("a page that is not there or taken");
+        taken[pages[i]] = true;
+        places.pages[i / kGroupPages][i % kGroupPages] = first + pages[i] * (kPlacePage / 16);
+    }
+    set_now(chain.places.as<void>(), &places, sizeof(places), upload_stream_, "chain places");
 }
 
 void Model::set_chain_numbers(uint64_t used, uint32_t given_up) {

@@ -205,6 +205,8 @@ public:
     unsigned int device_errors() const;
     // Test hook: as if `used` numbers had gone by and the run that started at `given_up` had been given up.
     void set_chain_numbers(uint64_t used, uint32_t given_up);
+    // Test hook: other places for the chain (see q3t_ops.h); null: those that are measured at a load.
+    void set_chain_places(const uint8_t* die_of_sm, const uint32_t* pages);
     void check_device_errors(unsigned int count_at_enqueue) const;
     int prefill_chunk = kMaxPromptRows; // prompt positions per pass (1: one position at a time)
     Workspace* batch_workspace_if_any() {
@@ -258,6 +260,7 @@ private:
     Quantized allocate_quantized(uint64_t rows, uint64_t cols);
     Quantized add_quant_matrix(const std::string& name, uint64_t rows, uint64_t cols);
     void build_chain();
+    void place_chain();
     void plan_layers(const std::string& prefix, const ModelDims& d, std::vector<LayerWeights>& out);
 
     int device_;

@@ -303,19 +303,20 @@ struct ChainLaunch {
     uint32_t* claims = nullptr;               // three words, zero before the first launch
     int rows = 0;
 };
-// Which die an SM and a page of memory are at home on (chain_places.cu), and what the chain makes of it: places 0 ..
-// on_first - 1 (whole groups of 16) are the first die's, and the pages of a group's exchange buffers are of its die.
+// Which die an SM and a page of memory are at home on (chain_places.cu), and what the chain makes of it: groups of 16 places
+// from the first one up are the first die's, and the pages of a group's exchange buffers are of its die.
 constexpr int kPlaceSms = 256, kPlacePage = 4096, kGroupPages = 124;
 constexpr int kPoolPages = 2304;              // of which 8 groups take 992
 struct ChainPlaces {
-    uint8_t die_of_sm[kPlaceSms];
-    int on_first;
+    uint8_t die_of_sm[kPlaceSms];             // 0 or 1
     uint32_t pages[8][kGroupPages];           // offsets from the exchange, in units of 16 bytes
 };
 // Measures them; `exchange` is overwritten.  Where nothing can be told apart every SM is of the first die and pages follow
 // each other.
 cudaError_t find_chain_places(void* exchange, ChainPlaces* places, cudaStream_t stream);
 size_t chain_pool_at(const void* exchange);   // bytes from the exchange to its first page
+// For tests: `ctas` SMs are taken by a kernel that leaves nothing of them to the chain, for `ns` (a second at most)
+cudaError_t launch_hold_sms(int ctas, unsigned long long ns, cudaStream_t stream);
 constexpr int kChainRows = 8;
 constexpr int kChainTopK = 128;               // larger or unlimited top-k draws run outside the chain
 bool chain_available();

@@ -1,5 +1,7 @@
 """The decode chain (frames of up to eight sessions as two cooperative launches) against the frame made
 launch by launch, at the context lengths where its page walk and merges change."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -93,7 +95,6 @@ def test_draws_inside_and_outside_the_chain(q3t, model, config):
 def test_exchange_numbers_start_again(q3t, model, used, given_up):
     """Exchanges are numbered in 32 bits.  At the last frame before a restart, at the first behind it, and where numbers
     would come round within a frame; the latter two where the run that was once given up bore the next run's number."""
-    import ctypes as C
     lib = q3t.library()
     lib.q3t_test_set_chain_numbers.argtypes = [C.c_void_p, C.c_uint64, C.c_uint32]
     want = frame(q3t, model, [40, 9, 700], 1, frames=3)
@@ -202,3 +203,78 @@ def test_frame_loop_behind_other_frames(q3t, model, rows):
 
     quiet = run(0)
     assert run(1) == quiet and run(2) == quiet and run(4) == quiet
+
+
+def set_places(q3t, model, die_of_sm=None, pages=None):
+    lib = q3t.library()
+    lib.q3t_test_set_chain_places.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+    die = None if die_of_sm is None else np.ascontiguousarray(die_of_sm, dtype=np.uint8)
+    page = None if pages is None else np.ascontiguousarray(pages, dtype=np.uint32)
+    return lib.q3t_test_set_chain_places(model._handle, None if die is None else die.ctypes.data, None if page is None else page.ctypes.data)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 8])
+def test_places_change_no_bit(q3t, model, rows):
+    """Wherever the CTAs and the buffers are taken to lie, every CTA gets a place of its own and a frame has the same bits: all
+    SMs on either die (what is assumed where the dies cannot be told apart), one SM, a third and half of them on the other."""
+    rng = np.random.default_rng(rows)
+    positions = POSITIONS[-rows:]
+    want = frame(q3t, model, positions, 1, frames=2)
+    sms = np.arange(256)
+    try:
+        for die, pages in ((0 * sms, np.arange(992)), (0 * sms + 1, np.arange(2303, 1311, -1)), (sms == 17, rng.permutation(2304)[:992]),
+                           (sms % 3 == 0, np.arange(992)), (rng.integers(0, 2, 256), rng.permutation(2304)[:992])):
+            assert set_places(q3t, model, die, pages) == 0
+            for a, b in zip(frame(q3t, model, positions, 1, frames=2), want):
+                assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2]) and a[4] == b[4]
+        assert set_places(q3t, model, 0 * sms + 2, np.arange(992)) != 0
+        assert set_places(q3t, model, 0 * sms, np.zeros(992)) != 0 and set_places(q3t, model, 0 * sms, np.arange(1313, 2305)) != 0
+    finally:
+        assert set_places(q3t, model) == 0
+    for a, b in zip(frame(q3t, model, positions, 1, frames=2), want):
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2]) and a[4] == b[4]
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 3])
+def test_frames_beside_a_kernel_that_holds_sms(q3t, model, rows):
+    """A chain needs 128 SMs.  What a host runs on a few of the others (its codec) does not hold a frame up, whichever die it
+    lies on, and changes none of its bits."""
+    import time
+    import torch
+    lib = q3t.library()
+    lib.q3t_test_hold_sms.argtypes = [C.c_int32, C.c_uint64, C.c_void_p]
+    model.set_option("decode_chain", 1)
+    stream = torch.cuda.Stream()
+
+    def run(held):
+        ss = []
+        for i in range(rows):
+            s = model.create_session(256, 40 + i)
+            s.talker_sampling = q3t.SamplingConfig(True, 50, 0.9, 0.9, 1.05)
+            s.predictor_sampling = q3t.SamplingConfig(True, 50, 1.0, 0.9, 1.0)
+            s.synthetic_prefill(60 + 30 * i, 40 + i)
+            ss.append(s)
+        done = torch.cuda.Event()
+        torch.cuda.synchronize()
+        if held:
+            assert lib.q3t_test_hold_sms(held, 500_000_000, stream.cuda_stream) == 0
+            done.record(stream)
+            time.sleep(0.02)
+        out = []
+        for f in range(4):
+            if rows == 1:
+                out.append(ss[0].next_frame(7 + f).codes)
+            else:
+                out.append([p.finish_without_consumer().next_semantic_token for p in model.batch_begin_device_frames(ss, [7 + f] * rows)])
+        assert not held or not done.query()
+        torch.cuda.synchronize()
+        out.append([tuple(np.array(x).tobytes() for x in s.read_state()) for s in ss])
+        for s in ss:
+            s.close()
+        return out
+
+    want = run(0)
+    for held in (1, 7, 20):
+        assert run(held) == want
+    assert lib.q3t_kernel_error_count() == 0
