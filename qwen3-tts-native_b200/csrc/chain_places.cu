@@ -69,13 +69,6 @@ __global__ void hold_sm_kernel(unsigned long long ns) {
     for (unsigned long long i = 0; i < ns / 100 && tc::now_ns() < until; ++i) __nanosleep(200);
 }
 
-struct Scratch {
-    void* p = nullptr;
-    ~Scratch() {
-        if (p != nullptr) cudaFree(p);
-    }
-};
-
 }  // namespace
 
 cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t stream) {
@@ -94,10 +87,9 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
     if (e != cudaSuccess) return e;
     std::vector<Latencies> host(1);
     Latencies& h = host[0];
-    Scratch scratch;
-    e = cudaMalloc(&scratch.p, sizeof(Latencies));
-    if (e != cudaSuccess) return e;
-    Latencies* d = static_cast<Latencies*>(scratch.p);
+    // (what lies ahead of the pages is not in use yet)
+    if (pool_at < sizeof(Latencies)) return cudaErrorInvalidValue;
+    Latencies* d = static_cast<Latencies*>(exchange);
     uint32_t* pool = reinterpret_cast<uint32_t*>(static_cast<char*>(exchange) + pool_at);
     e = cudaMemsetAsync(d, 0, sizeof(Latencies), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(pool, 0, (size_t)kPoolPages * kPlacePage, stream);

@@ -122,3 +122,10 @@ def test_no_buffer_is_written_before_its_readers_are_known_to_have_read_it():
     assert walk_predictor(source, one_hop=True, ends_early=False) == 16 * 5 * 4 + 15
     assert walk_predictor(source, one_hop=False, ends_early=False) == 16 * 5 * 6 + 15
     assert walk_predictor(source, one_hop=False, ends_early=True) == 16 * 5 * 6 + 15 - 5
+
+
+def test_setting_up_the_chain_allocates_through_the_engine_alone():
+    """A chain that finds no memory is done without; only the engine's own buffers report that as what it is."""
+    for name in ("decode_chain.cu", "chain_places.cu"):
+        with open(os.path.join(CSRC, name)) as f:
+            assert not re.search(r"\bcuda(Malloc|HostAlloc|Free)\w*\(", f.read()), name
