@@ -1130,6 +1130,20 @@ int32_t q3t_test_set_chain_places(Qwen3TtsModelHandle model, const uint8_t* die_
     if ((die_of_sm == nullptr) != (pages == nullptr)) return QWEN3_TTS_TALKER_STATUS_INVALID_ARGUMENT;
     return protect([&] { model_of(model)->set_chain_places(die_of_sm, pages); }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
 }
+int32_t q3t_test_sort_chain_places(const uint32_t* of_sm, const uint32_t* of_page, const uint32_t* by, int32_t sms, uint8_t* die_of_sm,
+                                   uint32_t* pages) {
+    std::vector<HomeLatencies> measured(1);
+    std::vector<ChainPlaces> places(1);
+    std::memcpy(measured[0].of_sm, of_sm, sizeof(measured[0].of_sm));
+    std::memcpy(measured[0].of_page, of_page, sizeof(measured[0].of_page));
+    for (int p = 0; p < kPoolPages; ++p) measured[0].by[p] = by[p] % kPlaceSms;
+    const int groups = sort_chain_places(measured[0], sms, &places[0]);
+    if (groups != kPlaceGroups) {
+        std::memcpy(die_of_sm, places[0].die_of_sm, sizeof(places[0].die_of_sm));
+        std::memcpy(pages, places[0].pages, sizeof(places[0].pages));
+    }
+    return groups;
+}
 int32_t q3t_test_hold_sms(int32_t ctas, uint64_t ns, void* stream) { return static_cast<int32_t>(launch_hold_sms(ctas, ns, S(stream))); }
 
 uint32_t q3t_kernel_error_count(void) {

@@ -16,16 +16,10 @@
 namespace q3t {
 namespace {
 
-constexpr int kProbePages = 8, kProbeLines = 4;          // for telling SMs apart
+constexpr int kProbeLines = 4;                           // for telling SMs apart
 constexpr int kPageLines = 8;                            // for telling pages apart
 constexpr int kChain = 4;                                // atomics one behind the other
 constexpr size_t kAlone = 120 * 1024;                    // shared memory of a CTA: one an SM
-
-struct Latencies {
-    uint32_t of_sm[kPlaceSms][kProbePages];              // cycles, 0: no CTA ran there
-    uint32_t of_page[kPoolPages];
-    uint32_t by[kPoolPages];                             // the SM that measured the page
-};
 
 __device__ uint32_t atomic_cycles(uint32_t* word) {
     uint32_t v = 0;
@@ -42,7 +36,7 @@ __device__ uint32_t best_of(uint32_t* word, int rounds) {
     return best;
 }
 
-__global__ void home_latency_kernel(uint32_t* pool, Latencies* out) {
+__global__ void home_latency_kernel(uint32_t* pool, HomeLatencies* out) {
     if (threadIdx.x != 0) return;
     uint32_t sm;
     asm("mov.u32 %0, %%smid;" : "=r"(sm));
@@ -54,8 +48,9 @@ __global__ void home_latency_kernel(uint32_t* pool, Latencies* out) {
         for (int l = 0; l < kProbeLines; ++l) sum += best_of(pool + (size_t)page * (kPlacePage / 4) + l * 64, 6);
         out->of_sm[sm][page] = sum;
     }
-    // every page one SM
-    for (int page = (int)blockIdx.x; page < kPoolPages; page += (int)gridDim.x) {
+    // every page one SM, a run of them each: homes follow the bits of the page number, so that there are both kinds in a run
+    const int run = (kPoolPages + (int)gridDim.x - 1) / (int)gridDim.x;
+    for (int page = (int)blockIdx.x * run; page < min(((int)blockIdx.x + 1) * run, kPoolPages); ++page) {
         uint32_t sum = 0;
         for (int l = 0; l < kPageLines; ++l) sum += best_of(pool + (size_t)page * (kPlacePage / 4) + l * 64, 3);
         out->of_page[page] = sum;
@@ -71,41 +66,11 @@ __global__ void hold_sm_kernel(unsigned long long ns) {
 
 }  // namespace
 
-cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t stream) {
-    constexpr int kGroups = 8, kRanks = 16;
-    const size_t pool_at = chain_pool_at(exchange);
-    const uint32_t pool_quad = (uint32_t)(pool_at / 16), page_quads = kPlacePage / 16;
-    // any place will do
-    std::fill(out->die_of_sm, out->die_of_sm + kPlaceSms, (uint8_t)0);
-    for (int g = 0; g < kGroups; ++g)
-        for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = pool_quad + (uint32_t)(g * kGroupPages + i) * page_quads;
-    static_assert(kGroups * kGroupPages <= kPoolPages, "pages of all groups");
-
-    int device = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e != cudaSuccess) return e;
-    std::vector<Latencies> host(1);
-    Latencies& h = host[0];
-    // (what lies ahead of the pages is not in use yet)
-    if (pool_at < sizeof(Latencies)) return cudaErrorInvalidValue;
-    Latencies* d = static_cast<Latencies*>(exchange);
-    uint32_t* pool = reinterpret_cast<uint32_t*>(static_cast<char*>(exchange) + pool_at);
-    e = cudaMemsetAsync(d, 0, sizeof(Latencies), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(pool, 0, (size_t)kPoolPages * kPlacePage, stream);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(home_latency_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone);
-    if (e == cudaSuccess) {
-        home_latency_kernel<<<sms, kWarp, kAlone, stream>>>(pool, d);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(Latencies), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-
+int sort_chain_places(const HomeLatencies& h, int sms, ChainPlaces* out) {
+    constexpr int kRanks = 16, kCtas = kPlaceGroups * kRanks;
     // SMs of one die agree within a tenth on every page; the other die's take 1.4 to 2.4 times as long, or as little
-    std::vector<int> of_die[2];
     std::vector<uint8_t> die_of_sm(kPlaceSms, 0);
-    int reference = -1;
+    int count[2] = {0, 0}, reference = -1;
     for (int sm = 0; sm < kPlaceSms; ++sm) {
         if (h.of_sm[sm][0] == 0) continue;
         if (reference < 0) reference = sm;
@@ -113,27 +78,70 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
         for (int p = 0; p < kProbePages; ++p)
             apart += std::fabs(std::log((double)std::max(h.of_sm[sm][p], 1u) / std::max(h.of_sm[reference][p], 1u)));
         die_of_sm[sm] = apart / kProbePages > 0.25 ? 1 : 0;
-        of_die[die_of_sm[sm]].push_back(sm);
+        ++count[die_of_sm[sm]];
     }
-    const int first = (int)of_die[0].size(), second = (int)of_die[1].size();
     // a launch of 128 CTAs lies evenly on the dies as far as they have the SMs
-    const int ctas_first = std::min(first, std::max(kGroups * kRanks / 2, kGroups * kRanks - second));
+    const int ctas_first = std::min(count[0], std::max(kCtas / 2, kCtas - count[1]));
     const int groups_first = (ctas_first + kRanks / 2) / kRanks;
-    if (first + second != sms || groups_first < 1 || groups_first >= kGroups) return cudaSuccess;
-    // an SM's pages fall into two bands
-    std::vector<uint32_t> least(kPlaceSms, 0xffffffffu), home[2];
+    if (count[0] + count[1] != sms || groups_first < 1 || groups_first >= kPlaceGroups) return kPlaceGroups;
+    // An SM's pages fall into two bands, the near one up to 1.24 wide and the far one twice as long.  Pages of an SM that saw no
+    // such bands count for nothing.
+    std::vector<uint32_t> least(kPlaceSms, 0xffffffffu), near_most(kPlaceSms, 0), far_least(kPlaceSms, 0xffffffffu);
+    std::vector<uint32_t> home[2];
+    auto far = [&](int p) { return h.of_page[p] > least[h.by[p]] * 1.5; };
     for (int p = 0; p < kPoolPages; ++p) least[h.by[p]] = std::min(least[h.by[p]], h.of_page[p]);
     for (int p = 0; p < kPoolPages; ++p) {
-        const bool far = h.of_page[p] > least[h.by[p]] * 1.35;
-        home[far ? 1 - die_of_sm[h.by[p]] : die_of_sm[h.by[p]]].push_back(pool_quad + (uint32_t)p * page_quads);
+        if (far(p)) far_least[h.by[p]] = std::min(far_least[h.by[p]], h.of_page[p]);
+        else near_most[h.by[p]] = std::max(near_most[h.by[p]], h.of_page[p]);
     }
-    if ((int)home[0].size() < groups_first * kGroupPages || (int)home[1].size() < (kGroups - groups_first) * kGroupPages) return cudaSuccess;
+    for (int p = 0; p < kPoolPages; ++p) {
+        const uint32_t sm = h.by[p];
+        if (h.of_page[p] == 0 || far_least[sm] == 0xffffffffu || far_least[sm] < near_most[sm] * 1.35) continue;
+        home[far(p) ? 1 - die_of_sm[sm] : die_of_sm[sm]].push_back((uint32_t)p);
+    }
+    if ((int)home[0].size() < groups_first * kGroupPages || (int)home[1].size() < (kPlaceGroups - groups_first) * kGroupPages) return kPlaceGroups;
     std::copy(die_of_sm.begin(), die_of_sm.end(), out->die_of_sm);
     size_t next[2] = {0, 0};
-    for (int g = 0; g < kGroups; ++g) {
+    for (int g = 0; g < kPlaceGroups; ++g) {
         const int die = g < groups_first ? 0 : 1;
         for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = home[die][next[die]++];
     }
+    return groups_first;
+}
+
+cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t stream) {
+    const size_t pool_at = chain_pool_at(exchange);
+    const uint32_t pool_quad = (uint32_t)(pool_at / 16), page_quads = kPlacePage / 16;
+    // any place will do
+    std::fill(out->die_of_sm, out->die_of_sm + kPlaceSms, (uint8_t)0);
+    for (int g = 0; g < kPlaceGroups; ++g)
+        for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = pool_quad + (uint32_t)(g * kGroupPages + i) * page_quads;
+    static_assert(kPlaceGroups * kGroupPages <= kPoolPages, "pages of all groups");
+
+    int device = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return e;
+    std::vector<HomeLatencies> host(1);
+    HomeLatencies& h = host[0];
+    // (what lies ahead of the pages is not in use yet)
+    if (pool_at < sizeof(HomeLatencies)) return cudaErrorInvalidValue;
+    HomeLatencies* d = static_cast<HomeLatencies*>(exchange);
+    uint32_t* pool = reinterpret_cast<uint32_t*>(static_cast<char*>(exchange) + pool_at);
+    e = cudaMemsetAsync(d, 0, sizeof(HomeLatencies), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(pool, 0, (size_t)kPoolPages * kPlacePage, stream);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(home_latency_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone);
+    if (e == cudaSuccess) {
+        home_latency_kernel<<<sms, kWarp, kAlone, stream>>>(pool, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(HomeLatencies), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return e;
+
+    if (sort_chain_places(h, sms, out) == kPlaceGroups) return cudaSuccess;
+    for (auto& group : out->pages)
+        for (uint32_t& page : group) page = pool_quad + page * page_quads;
     return cudaSuccess;
 }
 

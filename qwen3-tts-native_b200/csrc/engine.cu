@@ -748,7 +748,7 @@ void Model::set_chain_places(const uint8_t* die_of_sm, const uint32_t* pages) {
         places.die_of_sm[sm] = die_of_sm[sm];
     }
     const uint32_t first = static_cast<uint32_t>(chain_pool_at(chain.exchange.as<void>()) / 16);
-    for (int i = 0; i < 8 * kGroupPages; ++i) {
+    for (int i = 0; i < kPlaceGroups * kGroupPages; ++i) {
         if (pages[i] >= (uint32_t)kPoolPages || taken[pages[i]]) throw std::invalid_argument("a page that is not there or taken");
         taken[pages[i]] = true;
         places.pages[i / kGroupPages][i % kGroupPages] = first + pages[i] * (kPlacePage / 16);

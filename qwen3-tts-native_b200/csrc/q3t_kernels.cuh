@@ -305,12 +305,21 @@ struct ChainLaunch {
 };
 // Which die an SM and a page of memory are at home on (chain_places.cu), and what the chain makes of it: groups of 16 places
 // from the first one up are the first die's, and the pages of a group's exchange buffers are of its die.
-constexpr int kPlaceSms = 256, kPlacePage = 4096, kGroupPages = 124;
+constexpr int kPlaceSms = 256, kPlacePage = 4096, kGroupPages = 124, kPlaceGroups = 8;
 constexpr int kPoolPages = 2304;              // of which 8 groups take 992
 struct ChainPlaces {
     uint8_t die_of_sm[kPlaceSms];             // 0 or 1
-    uint32_t pages[8][kGroupPages];           // offsets from the exchange, in units of 16 bytes
+    uint32_t pages[kPlaceGroups][kGroupPages];           // offsets from the exchange, in units of 16 bytes
 };
+constexpr int kProbePages = 8;
+struct HomeLatencies {
+    uint32_t of_sm[kPlaceSms][kProbePages];   // cycles that an SM needs for each of a few pages, 0: not measured
+    uint32_t of_page[kPoolPages];             // and for each page, those that one SM needs
+    uint32_t by[kPoolPages];                  // that SM (below kPlaceSms)
+};
+// Host only.  What the measurements of a device of `sms` SMs say, pages by their numbers: how many groups are the first die's.
+// kPlaceGroups, and nothing written: they do not tell the dies apart, or too few pages.
+int sort_chain_places(const HomeLatencies& measured, int sms, ChainPlaces* places);
 // Measures them; `exchange` is overwritten.  Where nothing can be told apart every SM is of the first die and pages follow
 // each other.
 cudaError_t find_chain_places(void* exchange, ChainPlaces* places, cudaStream_t stream);
