@@ -519,7 +519,12 @@ struct Chain {
     static constexpr int kSliceBlocks = S::Slice / 64;         // of the down projection; the o projection has 4
     static constexpr int kSliceSide = TALKER ? 2 : kSliceBlocks;
     static constexpr uint32_t kTile = S::J * 1024;              // a tile's blocks lie in one slot
-    static_assert(S::OutTiles * kSliceBlocks <= 8 * L::Slots && (TALKER || 2 * S::LayerSlots / 3 <= L::Slots), "phases held fit the ring");
+    // The predictor's slots are given back behind a projection over all of K.  What is asked for before the next of these has to
+    // fit the ring beside what has not been given back: held ahead, everything to the end of the K-split one behind it.
+    static constexpr int kUnreleasedSlots = (S::OBytes + S::GuBytes + (kAhead ? S::DownBytes : 0)) / kSlot;
+    static constexpr int kUnreleasedNext = (S::DownBytes + (S::QkvBytes > S::HeadBytes ? S::QkvBytes : S::HeadBytes) + (kAhead ? S::OBytes : 0)) / kSlot;
+    static_assert(TALKER || (kUnreleasedSlots <= L::Slots && kUnreleasedNext <= L::Slots), "phases held fit the ring");
+    static_assert(S::OutTiles * kSliceBlocks <= 8 * L::Slots, "a K-split phase fits the ring");
     int4 held_full[2 * kSide * S::J], held_slice[2 * kSliceSide];
     __device__ __forceinline__ const int4* ring_at(uint32_t first, uint32_t at) {
         return reinterpret_cast<const int4*>(smem + L::AtRing + (first + at / kSlot) % L::Slots * kSlot + at % kSlot) + lane;
