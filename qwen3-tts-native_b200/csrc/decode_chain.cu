@@ -1653,8 +1653,14 @@ __global__ void pack_stream_kernel(const int8_t* __restrict__ w, uint8_t* __rest
     }
 }
 
+// `fits`: false where the kernel was compiled (with other flags than the library's) for fewer registers than its warps hand out
+// among themselves; they would wait for the rest of them for good.
 template <bool TALKER, int ROWS>
-cudaError_t configure_variant() {
+cudaError_t configure_variant(bool& fits) {
+    cudaFuncAttributes built;
+    const cudaError_t e = cudaFuncGetAttributes(&built, decode_chain_kernel<TALKER, ROWS>);
+    if (e != cudaSuccess) return e;
+    fits = fits && kThreads * built.numRegs >= kWorkers * kWorkerRegisters + 4 * kWarp * kRequestRegisters;
     return cudaFuncSetAttribute(decode_chain_kernel<TALKER, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<TALKER, ROWS>::Bytes);
 }
 
@@ -1685,18 +1691,19 @@ bool g_chain_fits[64] = {};
 
 cudaError_t configure_chain_kernels() {
     int device = 0, sms = 0, cooperative = 0;
+    bool fits = true;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device);
-    if (e == cudaSuccess) e = configure_variant<true, 1>();
-    if (e == cudaSuccess) e = configure_variant<true, 2>();
-    if (e == cudaSuccess) e = configure_variant<true, 4>();
-    if (e == cudaSuccess) e = configure_variant<true, 8>();
-    if (e == cudaSuccess) e = configure_variant<false, 1>();
-    if (e == cudaSuccess) e = configure_variant<false, 2>();
-    if (e == cudaSuccess) e = configure_variant<false, 4>();
-    if (e == cudaSuccess) e = configure_variant<false, 8>();
-    if (e == cudaSuccess && device >= 0 && device < 64) g_chain_fits[device] = cooperative != 0 && sms >= kCtas && sms <= kPlaceSms;
+    if (e == cudaSuccess) e = configure_variant<true, 1>(fits);
+    if (e == cudaSuccess) e = configure_variant<true, 2>(fits);
+    if (e == cudaSuccess) e = configure_variant<true, 4>(fits);
+    if (e == cudaSuccess) e = configure_variant<true, 8>(fits);
+    if (e == cudaSuccess) e = configure_variant<false, 1>(fits);
+    if (e == cudaSuccess) e = configure_variant<false, 2>(fits);
+    if (e == cudaSuccess) e = configure_variant<false, 4>(fits);
+    if (e == cudaSuccess) e = configure_variant<false, 8>(fits);
+    if (e == cudaSuccess && device >= 0 && device < 64) g_chain_fits[device] = fits && cooperative != 0 && sms >= kCtas && sms <= kPlaceSms;
     return e;
 }
 
