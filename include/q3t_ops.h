@@ -428,13 +428,14 @@ QWEN3_TTS_API int32_t q3t_test_report_device_wait_failure(int32_t device_index);
  * started at number `given_up` having been given up.  No frame may be in flight. */
 QWEN3_TTS_API int32_t q3t_test_set_chain_numbers(Qwen3TtsModelHandle model, uint64_t used, uint32_t given_up);
 
-/* Test hooks.  set_chain_places: the die (0 or 1) that a model's decode chain takes each of 256 SMs to lie on, and the 124
- * pages (of 2304, none twice) for the buffers of each of its 8 groups (both NULL: as measured); only the time of a frame
- * depends on them, and no frame may be in flight.  sort_chain_places: what a load makes of the cycles that each of 256 SMs
+/* Test hooks.  set_chain_places: the die (0 or 1) that a model's decode chain takes each of 256 SMs to lie on, the 124
+ * pages (of 2304, none twice) for the buffers of each of its 8 groups, and the CTAs of a launch, 128 up to the SMs (both NULL:
+ * all as measured); only the time of a frame depends on them, and no frame may be in flight.  sort_chain_places: what a load makes of the cycles that each of 256 SMs
  * needs for 8 pages (0: no such SM) and one SM, by[page], for each of 2304 pages; the groups that are die 0's, or 8, and
  * nothing written, where the dies cannot be told apart; on the host alone.  hold_sms: a kernel on `stream` that takes `ctas` SMs for `ns`
  * nanoseconds, 10^9 at most. */
-QWEN3_TTS_API int32_t q3t_test_set_chain_places(Qwen3TtsModelHandle model, const uint8_t* die_of_sm, const uint32_t* pages);
+QWEN3_TTS_API int32_t q3t_test_set_chain_places(Qwen3TtsModelHandle model, const uint8_t* die_of_sm, const uint32_t* pages,
+                                                int32_t grid);
 QWEN3_TTS_API int32_t q3t_test_sort_chain_places(const uint32_t* of_sm, const uint32_t* of_page, const uint32_t* by, int32_t sms,
                                                  uint8_t* die_of_sm, uint32_t* pages);
 QWEN3_TTS_API int32_t q3t_test_hold_sms(int32_t ctas, uint64_t ns, void* stream);

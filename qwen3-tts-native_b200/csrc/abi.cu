@@ -1126,9 +1126,9 @@ int32_t q3t_test_set_chain_numbers(Qwen3TtsModelHandle model, uint64_t used, uin
     return protect([&] { model_of(model)->set_chain_numbers(used, given_up); }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
 }
 
-int32_t q3t_test_set_chain_places(Qwen3TtsModelHandle model, const uint8_t* die_of_sm, const uint32_t* pages) {
+int32_t q3t_test_set_chain_places(Qwen3TtsModelHandle model, const uint8_t* die_of_sm, const uint32_t* pages, int32_t grid) {
     if ((die_of_sm == nullptr) != (pages == nullptr)) return QWEN3_TTS_TALKER_STATUS_INVALID_ARGUMENT;
-    return protect([&] { model_of(model)->set_chain_places(die_of_sm, pages); }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
+    return protect([&] { model_of(model)->set_chain_places(die_of_sm, pages, grid); }, QWEN3_TTS_TALKER_STATUS_STATE, nullptr, 0);
 }
 int32_t q3t_test_sort_chain_places(const uint32_t* of_sm, const uint32_t* of_page, const uint32_t* by, int32_t sms, uint8_t* die_of_sm,
                                    uint32_t* pages) {

@@ -4,7 +4,7 @@
 // other die 400 to 540; homes alternate by pages of 4 KB.  The decode chain puts the CTAs that exchange most, and their
 // buffers, on one die (decode_chain.cu).  What is found here changes the time of a frame, not its results.  SMs are compared
 // with each other, and pages with each other, at the same time and as ratios, since the clocks may be on their way up.
-// Nothing here waits for another CTA.  Takes a millisecond, once for each model.
+// No CTA here waits for another.  Takes a millisecond, once for each model.
 
 #include "q3t_kernels.cuh"
 #include "q3t_tcgen05.cuh"
@@ -20,6 +20,7 @@ constexpr int kProbeLines = 4;                           // for telling SMs apar
 constexpr int kPageLines = 8;                            // for telling pages apart
 constexpr int kChain = 4;                                // atomics one behind the other
 constexpr size_t kAlone = 120 * 1024;                    // shared memory of a CTA: one an SM
+constexpr int kRanks = 16, kCtas = kPlaceGroups * kRanks;
 
 __device__ uint32_t atomic_cycles(uint32_t* word) {
     uint32_t v = 0;
@@ -58,6 +59,12 @@ __global__ void home_latency_kernel(uint32_t* pool, HomeLatencies* out) {
     }
 }
 
+__global__ void sm_of_cta_kernel(uint32_t* sm_of) {
+    uint32_t sm;
+    asm("mov.u32 %0, %%smid;" : "=r"(sm));
+    if (threadIdx.x == 0) sm_of[blockIdx.x] = sm % kPlaceSms;
+}
+
 __global__ void hold_sm_kernel(unsigned long long ns) {
     if (threadIdx.x != 0) return;
     const unsigned long long until = tc::now_ns() + ns;
@@ -67,7 +74,6 @@ __global__ void hold_sm_kernel(unsigned long long ns) {
 }  // namespace
 
 int sort_chain_places(const HomeLatencies& h, int sms, ChainPlaces* out) {
-    constexpr int kRanks = 16, kCtas = kPlaceGroups * kRanks;
     // SMs of one die agree within a tenth on every page; the other die's take 1.4 to 2.4 times as long, or as little
     std::vector<uint8_t> die_of_sm(kPlaceSms, 0);
     int count[2] = {0, 0}, reference = -1;
@@ -114,6 +120,7 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
     const uint32_t pool_quad = (uint32_t)(pool_at / 16), page_quads = kPlacePage / 16;
     // any place will do
     std::fill(out->die_of_sm, out->die_of_sm + kPlaceSms, (uint8_t)0);
+    out->on_first = out->grid = kCtas;
     for (int g = 0; g < kPlaceGroups; ++g)
         for (int i = 0; i < kGroupPages; ++i) out->pages[g][i] = pool_quad + (uint32_t)(g * kGroupPages + i) * page_quads;
     static_assert(kPlaceGroups * kGroupPages <= kPoolPages, "pages of all groups");
@@ -131,6 +138,7 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
     e = cudaMemsetAsync(d, 0, sizeof(HomeLatencies), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(pool, 0, (size_t)kPoolPages * kPlacePage, stream);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(home_latency_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sm_of_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone);
     if (e == cudaSuccess) {
         home_latency_kernel<<<sms, kWarp, kAlone, stream>>>(pool, d);
         e = cudaGetLastError();
@@ -139,9 +147,36 @@ cudaError_t find_chain_places(void* exchange, ChainPlaces* out, cudaStream_t str
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return e;
 
-    if (sort_chain_places(h, sms, out) == kPlaceGroups) return cudaSuccess;
+    const int groups_first = sort_chain_places(h, sms, out);
+    if (groups_first == kPlaceGroups) return cudaSuccess;
     for (auto& group : out->pages)
         for (uint32_t& page : group) page = pool_quad + page * page_quads;
+    // how a launch lies on the dies
+    out->on_first = groups_first * kRanks;
+    uint32_t sm_of[kPlaceSms];
+    for (int grid = kCtas; grid <= std::min(sms, kPlaceSms); ++grid) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(384);                        // as the chain's
+        cfg.dynamicSmemBytes = kAlone;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        uint32_t* on_device = static_cast<uint32_t*>(exchange);
+        e = cudaLaunchKernelEx(&cfg, sm_of_cta_kernel, on_device);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(sm_of, on_device, sizeof(sm_of), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return e;
+        int on_die[2] = {0, 0};
+        for (int cta = 0; cta < grid; ++cta) ++on_die[out->die_of_sm[sm_of[cta]]];
+        if (on_die[0] >= out->on_first && on_die[1] >= kCtas - out->on_first) {
+            out->grid = grid;
+            break;
+        }
+    }
     return cudaSuccess;
 }
 

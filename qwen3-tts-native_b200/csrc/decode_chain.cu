@@ -188,7 +188,7 @@ struct ChainArgs {
     Quad* exchange;
     uint32_t* epoch;                 // [0] number of the last exchange, [1] the run that was given up
     const ChainPlaces* places;
-    uint32_t* claims;                // [0], [1] CTAs of a die that have a place, [2] CTAs that have asked
+    uint32_t* claims;                // [0], [1] CTAs of a die that have asked for a place, [2] CTAs that have an answer
     int rows;
     float eps;
 };
@@ -1455,22 +1455,42 @@ struct Chain {
     }
 
     // ---- the whole chain ------------------------------------------------------------------------------------------
-    // A place on the die that the SM lies on: CTAs of the first die take them from the first one up, those of the second from the
-    // last one down, so that every CTA gets one, however many lie on either die.  (A quiet device puts 64 on each, so groups
-    // 0 to 3 are the first die's; where other kernels hold SMs, or the dies are uneven, one group is of both.)  Who asks last
-    // clears the counts for the next launch.
+    // A place on the die that the SM lies on, or none (-1).  CTAs of the first die take places from the first one up, those of the
+    // second from the last one down.  The launch has as many CTAs as give both dies all of their places on a quiet device:
+    // 128 where these lie as the places do, more on a part whose dies are filled unevenly (128 lie 60 and 68 on one of 72 and 76
+    // SMs, where one session's frame was 1.5 % longer and three sessions' up to 4 %; 140 are enough there).  Where more CTAs
+    // lie on a die than it has places, they wait until all have asked and take what the other die's left over, so that all
+    // places are taken however the CTAs lie.  Who is done last clears the counts for the next launch.
     __device__ __forceinline__ int claim_place() {
         uint32_t sm;
         asm("mov.u32 %0, %%smid;" : "=r"(sm));
         const int die = a.places->die_of_sm[sm % kPlaceSms];
+        const int share = die == 0 ? a.places->on_first : kCtas - a.places->on_first;
         const int n = (int)atomicAdd(a.claims + die, 1u);
+        int most = share;
+        if (n >= share) {
+            // (all CTAs of the launch are resident, so this takes a microsecond; a run that is given up goes on with what it has)
+            const unsigned long long until = now_ns() + kBudgetNs;
+            int asked[2];
+            for (;;) {
+                asked[0] = (int)*reinterpret_cast<volatile uint32_t*>(a.claims);
+                asked[1] = (int)*reinterpret_cast<volatile uint32_t*>(a.claims + 1);
+                if (asked[0] + asked[1] >= (int)gridDim.x) break;
+                if (now_ns() > until) {
+                    *reinterpret_cast<volatile uint32_t*>(a.epoch + 1) = *reinterpret_cast<volatile uint32_t*>(a.epoch);
+                    break;
+                }
+                __nanosleep(100);
+            }
+            most = max(share, kCtas - asked[1 - die]);
+        }
         __threadfence();
-        if (atomicInc(a.claims + 2, kCtas - 1) == kCtas - 1) {
+        if (atomicInc(a.claims + 2, gridDim.x - 1) == gridDim.x - 1) {
             __threadfence();
             *reinterpret_cast<volatile uint32_t*>(a.claims) = 0u;
             *reinterpret_cast<volatile uint32_t*>(a.claims + 1) = 0u;
         }
-        return die == 0 ? n : kCtas - 1 - n;
+        return n >= most ? -1 : (die == 0 ? n : kCtas - 1 - n);
     }
     __device__ __forceinline__ void run() {
         if (tid == 0) misc->place = claim_place();
@@ -1488,7 +1508,7 @@ struct Chain {
         }
         __syncthreads();
         cta = misc->place;
-        __builtin_assume(cta >= 0 && cta < kCtas);         // (without it registers spill: one session 1,544 -> 1,593 us)
+        if (cta < 0) return;
         slice = cta / kRanks;
         rank = cta % kRanks;
         if (tid >= kWorkers && tid < kWorkers + kGroupPages) {
@@ -1665,9 +1685,9 @@ cudaError_t configure_variant(bool& fits) {
 }
 
 template <bool TALKER, int ROWS>
-cudaError_t launch_variant(const ChainArgs& a, cudaStream_t stream) {
+cudaError_t launch_variant(const ChainArgs& a, int grid, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)kCtas);
+    cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = Layout<TALKER, ROWS>::Bytes;
     cfg.stream = stream;
@@ -1680,9 +1700,9 @@ cudaError_t launch_variant(const ChainArgs& a, cudaStream_t stream) {
 }
 
 template <bool TALKER>
-cudaError_t launch_rows(const ChainArgs& a, cudaStream_t stream) {
-    if (a.rows <= 2) return a.rows == 1 ? launch_variant<TALKER, 1>(a, stream) : launch_variant<TALKER, 2>(a, stream);
-    return a.rows <= 4 ? launch_variant<TALKER, 4>(a, stream) : launch_variant<TALKER, 8>(a, stream);
+cudaError_t launch_rows(const ChainArgs& a, int grid, cudaStream_t stream) {
+    if (a.rows <= 2) return a.rows == 1 ? launch_variant<TALKER, 1>(a, grid, stream) : launch_variant<TALKER, 2>(a, grid, stream);
+    return a.rows <= 4 ? launch_variant<TALKER, 4>(a, grid, stream) : launch_variant<TALKER, 8>(a, grid, stream);
 }
 
 bool g_chain_fits[64] = {};
@@ -1757,7 +1777,7 @@ cudaError_t launch_decode_chain(const ChainLaunch& c, cudaStream_t stream) {
     a.head_s = c.head_scales; a.hidden = c.hidden; a.normalized = c.normalized; a.logits = c.logits; a.projected = c.projected;
     a.table = c.table; a.positions = c.positions; a.kv = c.kv; a.kv_layer_elems = c.kv_layer_elems; a.rope_table = c.rope_table;
     a.exchange = static_cast<Quad*>(c.exchange); a.epoch = c.epoch; a.places = c.places; a.claims = c.claims; a.rows = c.rows; a.eps = kRmsEps;
-    return c.talker ? launch_rows<true>(a, stream) : launch_rows<false>(a, stream);
+    return c.talker ? launch_rows<true>(a, c.grid, stream) : launch_rows<false>(a, c.grid, stream);
 }
 
 // The last number used becomes 0, the run given up one that no launch reaches before the next restart, and no word of

@@ -732,16 +732,23 @@ void Model::place_chain() {
     ChainPlaces places;
     check_cuda(find_chain_places(chain.exchange.as<void>(), &places, upload_stream_), "chain places");
     set_now(chain.places.as<void>(), &places, sizeof(places), upload_stream_, "chain places");
+    chain.grid = places.grid;
     check_cuda(restart_chain_numbers(chain.exchange.as<void>(), chain.epoch.as<uint32_t>(), upload_stream_), "chain numbers");
     check_cuda(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize(decode chain)");
     chain.numbers = 0;
 }
 
-void Model::set_chain_places(const uint8_t* die_of_sm, const uint32_t* pages) {
+void Model::set_chain_places(const uint8_t* die_of_sm, const uint32_t* pages, int grid) {
     if (!chain.ready) return;
     check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(chain places)");
+    ++option_epoch;                 // captured graphs launch the grid of before
     if (die_of_sm == nullptr) return place_chain();
+    int sms = 0;
+    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
+    if (grid < 128 || grid > sms) throw std::invalid_argument("a chain of fewer than 128 CTAs, or more than SMs");
     ChainPlaces places;
+    places.on_first = 64;
+    chain.grid = places.grid = grid;
     std::vector<bool> taken(kPoolPages, false);
     for (int sm = 0; sm < kPlaceSms; ++sm) {
         if (die_of_sm[sm] > 1) throw std::invalid_argument("a die that is neither 0 nor 1");
@@ -927,7 +934,7 @@ void enqueue_chain(Workspace& w, Model& m, bool talker, int n, cudaStream_t s) {
     }
     a.kv_layer_elems = 2 * pool.plane_elems();
     a.exchange = c.exchange.as<void>(); a.epoch = c.epoch.as<uint32_t>();
-    a.places = c.places.as<const ChainPlaces>(); a.claims = c.claims.as<uint32_t>();
+    a.places = c.places.as<const ChainPlaces>(); a.claims = c.claims.as<uint32_t>(); a.grid = c.grid;
     a.rows = n;
     check_launch(launch_decode_chain(a, s), talker ? "talker chain" : "predictor chain");
 }

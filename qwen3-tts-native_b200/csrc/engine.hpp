@@ -206,7 +206,7 @@ public:
     // Test hook: as if `used` numbers had gone by and the run that started at `given_up` had been given up.
     void set_chain_numbers(uint64_t used, uint32_t given_up);
     // Test hook: other places for the chain (see q3t_ops.h); null: those that are measured at a load.
-    void set_chain_places(const uint8_t* die_of_sm, const uint32_t* pages);
+    void set_chain_places(const uint8_t* die_of_sm, const uint32_t* pages, int grid);
     void check_device_errors(unsigned int count_at_enqueue) const;
     int prefill_chunk = kMaxPromptRows; // prompt positions per pass (1: one position at a time)
     Workspace* batch_workspace_if_any() {
@@ -234,6 +234,7 @@ public:
         bool ready = false;
         DeviceBuffer streams[2], heads[2], layers[2], head_scales[2];     // 0 predictor, 1 talker
         DeviceBuffer projected_rows, projected, exchange, epoch, places, claims;
+        int grid = 0;                   // CTAs of a launch
         uint64_t numbers = 0;           // of exchanges, at most, since they were restarted (guarded as the device's chains are)
     } chain;
     std::mutex mutex;               // pools, workspaces

@@ -275,7 +275,7 @@ struct FrameTable {
 
 // ---------------------------------------------------------------- decode chain (decode_chain.cu)
 // The predictor's 16 positions with their draws, or the talker's layers and head, of 1..8 rows in one
-// cooperative launch of 128 CTAs.  At most one chain may run on a device at a time.
+// cooperative launch, 128 CTAs of which do the work.  At most one chain may run on a device at a time.
 struct ChainLayer {                  // device array, one per layer
     const float *qkv_s, *o_s, *gu_s, *down_s;
     const bf16 *in_norm, *post_norm, *q_norm, *k_norm;
@@ -301,14 +301,17 @@ struct ChainLaunch {
     uint32_t* epoch = nullptr;                // two words
     const struct ChainPlaces* places = nullptr;
     uint32_t* claims = nullptr;               // three words, zero before the first launch
+    int grid = 0;                             // CTAs of the launch (ChainPlaces)
     int rows = 0;
 };
-// Which die an SM and a page of memory are at home on (chain_places.cu), and what the chain makes of it: groups of 16 places
-// from the first one up are the first die's, and the pages of a group's exchange buffers are of its die.
+// Which die an SM and a page of memory are at home on (chain_places.cu), and what the chain makes of it: places 0 ..
+// on_first - 1 (whole groups of 16) are the first die's, and the pages of a group's exchange buffers are of its die.
 constexpr int kPlaceSms = 256, kPlacePage = 4096, kGroupPages = 124, kPlaceGroups = 8;
 constexpr int kPoolPages = 2304;              // of which 8 groups take 992
 struct ChainPlaces {
     uint8_t die_of_sm[kPlaceSms];             // 0 or 1
+    int on_first;
+    int grid;                                 // CTAs of a launch, as few as give both dies all of their places
     uint32_t pages[kPlaceGroups][kGroupPages];           // offsets from the exchange, in units of 16 bytes
 };
 constexpr int kProbePages = 8;

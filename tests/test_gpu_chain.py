@@ -205,29 +205,32 @@ def test_frame_loop_behind_other_frames(q3t, model, rows):
     assert run(1) == quiet and run(2) == quiet and run(4) == quiet
 
 
-def set_places(q3t, model, die_of_sm=None, pages=None):
+def set_places(q3t, model, die_of_sm=None, pages=None, grid=128):
     lib = q3t.library()
-    lib.q3t_test_set_chain_places.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.q3t_test_set_chain_places.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32]
     die = None if die_of_sm is None else np.ascontiguousarray(die_of_sm, dtype=np.uint8)
     page = None if pages is None else np.ascontiguousarray(pages, dtype=np.uint32)
-    return lib.q3t_test_set_chain_places(model._handle, None if die is None else die.ctypes.data, None if page is None else page.ctypes.data)
+    return lib.q3t_test_set_chain_places(model._handle, None if die is None else die.ctypes.data, None if page is None else page.ctypes.data, grid)
 
 
 @pytest.mark.parametrize("rows", [1, 2, 3, 8])
 def test_places_change_no_bit(q3t, model, rows):
-    """Wherever the CTAs and the buffers are taken to lie, every CTA gets a place of its own and a frame has the same bits: all
-    SMs on either die (what is assumed where the dies cannot be told apart), one SM, a third and half of them on the other."""
+    """Wherever the CTAs and the buffers are taken to lie, and however many CTAs more than needed there are, every place is
+    taken once and a frame has the same bits: all SMs on either die, one SM, a third and half of them on the other."""
     rng = np.random.default_rng(rows)
     positions = POSITIONS[-rows:]
     want = frame(q3t, model, positions, 1, frames=2)
     sms = np.arange(256)
     try:
-        for die, pages in ((0 * sms, np.arange(992)), (0 * sms + 1, np.arange(2303, 1311, -1)), (sms == 17, rng.permutation(2304)[:992]),
-                           (sms % 3 == 0, np.arange(992)), (rng.integers(0, 2, 256), rng.permutation(2304)[:992])):
-            assert set_places(q3t, model, die, pages) == 0
+        for die, pages, grid in ((0 * sms, np.arange(992), 128), (0 * sms, np.arange(992), 148), (0 * sms + 1, np.arange(2303, 1311, -1), 128),
+                                 (0 * sms + 1, np.arange(992), 140), (sms == 17, rng.permutation(2304)[:992], 128), (sms != 17, np.arange(992), 148),
+                                 (sms % 3 == 0, np.arange(992), 128), (sms % 3 == 0, np.arange(992), 133),
+                                 (rng.integers(0, 2, 256), rng.permutation(2304)[:992], 128), (rng.integers(0, 2, 256), np.arange(992), 148)):
+            assert set_places(q3t, model, die, pages, grid) == 0
             for a, b in zip(frame(q3t, model, positions, 1, frames=2), want):
                 assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(a[2], b[2]) and a[4] == b[4]
         assert set_places(q3t, model, 0 * sms + 2, np.arange(992)) != 0
+        assert set_places(q3t, model, 0 * sms, np.arange(992), 127) != 0 and set_places(q3t, model, 0 * sms, np.arange(992), 149) != 0
         assert set_places(q3t, model, 0 * sms, np.zeros(992)) != 0 and set_places(q3t, model, 0 * sms, np.arange(1313, 2305)) != 0
     finally:
         assert set_places(q3t, model) == 0
@@ -238,8 +241,8 @@ def test_places_change_no_bit(q3t, model, rows):
 
 @pytest.mark.parametrize("rows", [1, 3])
 def test_frames_beside_a_kernel_that_holds_sms(q3t, model, rows):
-    """A chain needs 128 SMs.  What a host runs on a few of the others (its codec) does not hold a frame up, whichever die it
-    lies on, and changes none of its bits."""
+    """A launch of 128 CTAs needs as many SMs.  What a host runs on some of the others (its codec) does not hold a frame up,
+    whichever die it lies on, and changes none of its bits."""
     import time
     import torch
     lib = q3t.library()
@@ -275,6 +278,10 @@ def test_frames_beside_a_kernel_that_holds_sms(q3t, model, rows):
         return out
 
     want = run(0)
-    for held in (1, 7, 20):
-        assert run(held) == want
+    try:
+        assert set_places(q3t, model, np.arange(256) // 2 % 2, np.arange(992), 128) == 0
+        for held in (1, 7, 20):
+            assert run(held) == want
+    finally:
+        assert set_places(q3t, model) == 0
     assert lib.q3t_kernel_error_count() == 0
