@@ -369,7 +369,8 @@ QWEN3_TTS_API int32_t q3t_launch_sample_logits_at(
  * "decode_chain" (1, default: frames of up to 8 sessions run as two cooperative launches, or, while the
  * device is at work on a prompt, on larger frames or on three and more sessions stepped alone, launch by launch with
  * the same results to the bit; 2: always the latter; 0: launch by launch with the operators' attention; with
- * "use_graphs" 0 always as with 0),
+ * "use_graphs" 0 always as with 0.  Also with 1, the predictor's part of frames of 9 and more sessions runs as one cooperative
+ * launch while the device is at work on nothing else, with the bits of launch by launch),
  * "batch_host_codes" (1: lockstep batches also mirror each frame's 16 codes to host memory),
  * "gemv_mode" (process-wide, see q3t_set_gemv_mode),
  * "attention_mode" (process-wide, see q3t_set_attention_mode),

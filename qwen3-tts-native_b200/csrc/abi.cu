@@ -32,6 +32,7 @@ cudaError_t set_gemv_mma_error_sink(unsigned int* device_visible_word);
 cudaError_t set_tc_error_sink(unsigned int* device_visible_word);
 cudaError_t set_wide_error_sink(unsigned int* device_visible_word);
 cudaError_t set_chain_error_sink(unsigned int* device_visible_word);
+cudaError_t set_lockstep_error_sink(unsigned int* device_visible_word);
 
 namespace {
 std::atomic<unsigned int*> g_error_words[64];
@@ -54,6 +55,7 @@ cudaError_t configure_device() {
     if (e == cudaSuccess) e = configure_wide_kernels();
     if (e == cudaSuccess) e = configure_prompt_kernels();
     if (e == cudaSuccess) e = configure_chain_kernels();
+    if (e == cudaSuccess) e = configure_lockstep_kernels();
     if (e == cudaSuccess) e = configure_gemv_mma_kernels();
     if (e == cudaSuccess) e = configure_sampler_kernels();
     if (e == cudaSuccess && device >= 0 && device < 64 && g_error_words[device].load() == nullptr) {
@@ -67,6 +69,7 @@ cudaError_t configure_device() {
             if (e == cudaSuccess) e = set_tc_error_sink(word);
             if (e == cudaSuccess) e = set_wide_error_sink(word);
             if (e == cudaSuccess) e = set_chain_error_sink(word);
+            if (e == cudaSuccess) e = set_lockstep_error_sink(word);
             if (e == cudaSuccess) e = set_attention_error_sink(word);
             if (e == cudaSuccess) g_error_words[device].store(word, std::memory_order_release);
         }
@@ -1147,7 +1150,7 @@ int32_t q3t_test_sort_chain_places(const uint32_t* of_sm, const uint32_t* of_pag
 int32_t q3t_test_hold_sms(int32_t ctas, uint64_t ns, void* stream) { return static_cast<int32_t>(launch_hold_sms(ctas, ns, S(stream))); }
 
 uint32_t q3t_kernel_error_count(void) {
-    return gemm_tc_error_count() + gemm_wide_error_count() + gemv_mma_error_count() + chain_error_count();
+    return gemm_tc_error_count() + gemm_wide_error_count() + gemv_mma_error_count() + chain_error_count() + lockstep_error_count();
 }
 
 uint32_t q3t_attention_range_error_count(void) { return attention_range_error_count(); }

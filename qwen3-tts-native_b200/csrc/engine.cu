@@ -130,6 +130,18 @@ struct Traffic {
         if (alone >= 3) crowd_until = now + std::chrono::milliseconds(20);
         return !launches && now >= crowd_until;
     }
+    // Whether nothing else is at work, nor was a moment ago: the lockstep chain takes 128 SMs for the predictor's part of a
+    // frame, and what runs beside it gets the rest.  Launch by launch such a frame has the same bits.
+    bool alone(const Workspace* w) {
+        const auto now = std::chrono::steady_clock::now();
+        drop_finished();
+        for (const Entry& e : entries) {
+            if (e.workspace == w) continue;
+            shared_until = now + std::chrono::milliseconds(5);
+            return false;
+        }
+        return now >= shared_until;
+    }
     void enter(const Workspace* w, int rows, Kind kind) {
         Entry* e = find(w);
         if (e != nullptr) *e = Entry{w, rows, kind, false};
@@ -325,6 +337,7 @@ Workspace::Workspace(int capacity_, int device_, int rows_) : capacity(capacity_
         {&hidden, c * 2048 * e}, {&qkv, c * 4096 * e}, {&attention, c * 2048 * e}, {&gate, c * 6144 * e},
         {&logits, one * kTalkerVocab * e}, {&x_in, c * 2048 * e}, {&projection, c * 2048 * e}, {&normalized, c * 2048 * e},
         {&prompt_positions, c * sizeof(int)}, {&talker_pages, one * kMaxPagesPerRow * sizeof(int)},
+        {&lockstep_exchange, capacity > kChainRows ? lockstep_exchange_bytes() : 0},
         {&predictor_pages, one * sizeof(int)}, {&predictor_positions, (size_t)kPredictorSequence * kMaxRows * sizeof(int)}};
     size_t total = 0;
     for (const auto& part : parts) total += align_up(part.second, 1024);
@@ -414,7 +427,7 @@ uint64_t Workspace::bytes() const {
     return hidden.bytes() + qkv.bytes() + attention.bytes() + gate.bytes() + logits.bytes()
         + x_in.bytes() + projection.bytes() + normalized.bytes() + table.bytes()
         + talker_pages.bytes() + predictor_pages.bytes() + predictor_positions.bytes()
-        + counters.bytes() + scratch.bytes() + chain_order_scratch.bytes();
+        + counters.bytes() + scratch.bytes() + chain_order_scratch.bytes() + lockstep_exchange.bytes();
 }
 
 // ------------------------------------------------------------------ Model
@@ -654,6 +667,7 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
         cudaStreamSynchronize(upload_stream_);
         chain = DecodeChain();
     }
+    build_lockstep();
     talker_pool.reset(new KvPool(talker.layers, talker.kv_width, 8, upload_stream_));
     predictor_pool.reset(new KvPool(predictor.layers, predictor.kv_width, 6, upload_stream_));
     finalized_ = true;
@@ -726,6 +740,32 @@ void Model::build_chain() {
     table(chain.claims, none, sizeof(none));
     place_chain();
     chain.ready = true;
+}
+
+void Model::build_lockstep() {
+    if (predictor.head_dim != 128) return;
+    std::unique_ptr<LockstepModel> host(new LockstepModel());
+    const int PH = predictor.hidden, PI = predictor.intermediate, qkv = predictor.q_width + 2 * predictor.kv_width;
+    bool ok = true;
+    for (int l = 0; l < predictor.layers; ++l) {
+        const LayerWeights& lw = predictor_layers[l];
+        ok = ok && make_lockstep_map(host.get(), 4 * l, lw.qkv.data, PH, qkv, true)
+             && make_lockstep_map(host.get(), 4 * l + 1, lw.o.data, predictor.q_width, PH, false)
+             && make_lockstep_map(host.get(), 4 * l + 2, lw.gate_up.data, PH, 2 * PI, false)
+             && make_lockstep_map(host.get(), 4 * l + 3, lw.down.data, PI, PH, false);
+        host->layers[l] = {lw.qkv.scales, lw.o.scales, lw.gate_up.scales, lw.down.scales, lw.input_norm, lw.post_norm, lw.q_norm, lw.k_norm};
+    }
+    for (int h = 0; h < kResidualCodebooks; ++h) {
+        ok = ok && make_lockstep_map(host.get(), kLockstepHeadMap + h, predictor_heads[h].data, PH, kPredictorVocab, true);
+        host->head_scales[h] = predictor_heads[h].scales;
+    }
+    ok = ok && make_lockstep_map(host.get(), kLockstepMtpMap, small_to_mtp.data, talker.hidden, PH, false);
+    host->mtp_scales = small_to_mtp.scales;
+    host->mtp_bias = small_to_mtp_bias;
+    host->final_norm = predictor_norm;
+    if (!ok) return;
+    lockstep = DeviceBuffer(sizeof(LockstepModel));
+    set_now(lockstep.as<void>(), host.get(), sizeof(LockstepModel), upload_stream_, "lockstep table");
 }
 
 void Model::place_chain() {
@@ -952,12 +992,55 @@ void enqueue_predictor_chain(Workspace& w, Model& m, int n, cudaStream_t s) {
     enqueue_chain(w, m, false, n, s);
 }
 
+// How a frame's predictor is made: launch by launch, a launch of the lockstep chain for each position with the draws between
+// them, or one launch for all.
+enum class Lockstep { kNone, kPositions, kWhole };
+// Whether it may run on the lockstep chain: enough rows, the default kernels (it computes what they compute).
+bool lockstep_may_run(const Workspace& w, const Model& m, int n) {
+    return n > kChainRows && n >= tc_min_rows() && m.use_chain == 1 && attention_mode() == 1 && m.lockstep.bytes() != 0
+           && w.lockstep_exchange.bytes() != 0 && lockstep_chain_available(n);
+}
+
+// Whether the chains make these draws of the predictor: greedy ones, and from no more candidates than their sampler ranks.
+bool draws_fit_chains(const FrameTable& t, int n) {
+    for (int i = 0; i < n; ++i) {
+        const SamplingParams& p = t.predictor[i];
+        if (p.do_sample != 0 && (p.top_k < 1 || p.top_k > kChainTopK)) return false;
+    }
+    return true;
+}
+
 // 16 predictor positions, 15 sampled codebooks, packed codes (talker.cu:1549-1701)
-void enqueue_predictor(Workspace& w, Model& m, int n, cudaStream_t s) {
+void enqueue_predictor(Workspace& w, Model& m, int n, Lockstep lockstep, cudaStream_t s) {
     const FrameTable* table = w.table.as<FrameTable>();
     const int H = m.talker.hidden, PH = m.predictor.hidden;
     check_launch(launch_frame_begin(table, n, s), "frame begin");
-    for (int p = 0; p < kPredictorSequence; ++p) {
+    LockstepLaunch c;
+    if (lockstep != Lockstep::kNone) {
+        c.model = m.lockstep.as<LockstepModel>();
+        c.table = table; c.pages = w.predictor_pages.as<int>();
+        c.kv = m.predictor_pool->layout(0, c.pages, 1);
+        c.kv_layer_elems = 2 * m.predictor_pool->plane_elems();
+        c.rope_table = m.predictor_rope;
+        c.codec_embedding = m.codec_embedding; c.embeddings = m.predictor_embedding_table;
+        c.logits = w.logits.as<bf16>(); c.exchange = w.lockstep_exchange.as<void>();
+        c.rows = n;
+    }
+    if (lockstep == Lockstep::kWhole) {
+        c.last = kPredictorSequence - 1;
+        c.draws = true;
+        check_launch(launch_lockstep_chain(c, s), "lockstep chain");
+    }
+    for (int p = 0; p < kPredictorSequence && lockstep != Lockstep::kWhole; ++p) {
+        if (lockstep == Lockstep::kPositions) {
+            c.first = c.last = p;
+            check_launch(launch_lockstep_chain(c, s), "lockstep chain");
+            if (p >= 1) {
+                check_launch(launch_sample_table(table, w.logits.as<bf16>(), kPredictorVocab, kPredictorVocab, 0, p, 0, kEos, n, s),
+                             "sample predictor logits");
+            }
+            continue;
+        }
         check_launch(launch_predictor_input(table, p, m.codec_embedding, m.predictor_embedding_table,
                                           w.x_in.as<bf16>(), H, n, s), "predictor input");
         GemvArgs g;
@@ -1051,11 +1134,7 @@ bool frame_may_chain(const Model& m, const FrameTable& t, int n) {
         || traffic_of(m.device()) == nullptr) {
         return false;
     }
-    for (int i = 0; i < n; ++i) {
-        const SamplingParams& p = t.predictor[i];
-        if (p.do_sample != 0 && (p.top_k < 1 || p.top_k > kChainTopK)) return false;
-    }
-    return true;
+    return draws_fit_chains(t, n);
 }
 
 // one prompt position of row 0 (talker.cu:1058-1064 + one decoder pass)
@@ -1400,15 +1479,15 @@ void Session::bind_rows(Workspace& w, Session** s, int n) {
     for (int i = 0; i < n; ++i) w.bound[i] = s[i]->id_;
 }
 
-Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int splits, Way way) {
+Workspace::Graphs& Session::frame_graphs(Workspace& w, Model& m, int n, int splits, Way way, int lockstep) {
     const bool chain = way == Way::kChain;
-    const auto key = std::make_pair(n, chain ? 0 : (way == Way::kInItsPlace ? -1 : splits));
+    const auto key = std::make_tuple(n, chain ? 0 : (way == Way::kInItsPlace ? -1 : splits), lockstep);
     auto found = w.graphs.find(key);
     if (found != w.graphs.end()) return found->second;
     Workspace::Graphs g;
     g.predictor = capture(w.stream, [&] {
                               if (chain) enqueue_predictor_chain(w, m, n, w.stream);
-                              else enqueue_predictor(w, m, n, w.stream);
+                              else enqueue_predictor(w, m, n, static_cast<Lockstep>(lockstep), w.stream);
                           },
                           &g.predictor_kernels);
     try {
@@ -1439,15 +1518,20 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
     Traffic* const traffic = traffic_of(m.device());
     std::unique_ptr<InFlight> in_flight;
     Way way = Way::kLaunches;
+    Lockstep lockstep = Lockstep::kNone;
     if (frame_may_chain(m, *w.host_table, n)) {
         in_flight.reset(new InFlight(traffic, w, n, m.use_chain == 2));
         way = in_flight->kind() == Traffic::kChain ? Way::kChain : Way::kInItsPlace;
     } else {
+        if (lockstep_may_run(w, m, n) && traffic != nullptr) {
+            std::lock_guard<std::mutex> lock(traffic->mutex);
+            if (traffic->alone(&w)) lockstep = draws_fit_chains(*w.host_table, n) ? Lockstep::kWhole : Lockstep::kPositions;
+        }
         in_flight.reset(new InFlight(traffic, w, n, Traffic::kOther));
     }
     if (way == Way::kLaunches) w.ensure_scratch(splits);
     bind_rows(w, s, n);
-    Workspace::Graphs* const g = m.use_graphs ? &frame_graphs(w, m, n, splits, way) : nullptr;
+    Workspace::Graphs* const g = m.use_graphs ? &frame_graphs(w, m, n, splits, way, static_cast<int>(lockstep)) : nullptr;
     {
         const ChainTurn turn(way == Way::kChain ? traffic : nullptr, w);
         if (upload_table) {
@@ -1459,9 +1543,14 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
             check_cuda(restart_chain_numbers(m.chain.exchange.as<void>(), m.chain.epoch.as<uint32_t>(), w.stream), "chain numbers");
             m.chain.numbers = kChainNumbersPerFrame;
         }
+        if (lockstep != Lockstep::kNone && (w.lockstep_rows != n || w.lockstep_errors != m.device_errors())) {
+            w.lockstep_errors = m.device_errors();
+            check_cuda(restart_lockstep(w.lockstep_exchange.as<void>(), w.stream), "lockstep exchange");
+            w.lockstep_rows = n;
+        }
         check_cuda(cudaEventRecord(w.predictor_start, w.stream), "cudaEventRecord");
         if (g != nullptr) check_cuda(cudaGraphLaunch(g->predictor, w.stream), "cudaGraphLaunch(predictor)");
-        else enqueue_predictor(w, m, n, w.stream);
+        else enqueue_predictor(w, m, n, lockstep, w.stream);
         check_cuda(cudaEventRecord(w.predictor_stop, w.stream), "cudaEventRecord");
         if (record_session_events) {
             for (int i = 0; i < n; ++i) {

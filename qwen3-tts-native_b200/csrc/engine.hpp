@@ -23,6 +23,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <unordered_map>
 #include <vector>
 
@@ -145,6 +146,9 @@ struct Workspace {
     DeviceBuffer prompt_positions;      // [activation rows], positions of the rows of a prompt chunk
     DeviceBuffer scratch;
     DeviceBuffer chain_order_scratch;   // of frames that stand in for the chain's
+    DeviceBuffer lockstep_exchange;     // of frames of more rows than a chain takes
+    int lockstep_rows = 0;              // row count that it is set up for
+    unsigned int lockstep_errors = 0;   // device errors seen by then
     DeviceBuffer counters;
     int scratch_splits = 0;
     int option_epoch = 0;            // Model::option_epoch the captured graphs were built under
@@ -155,8 +159,8 @@ struct Workspace {
         int predictor_kernels = 0;   // kernel nodes in each graph
         int talker_kernels = 0;
     };
-    // (rows, talker splits; 0: the decode chain, -1: launch by launch in its place) -> graphs
-    std::map<std::pair<int, int>, Graphs> graphs;
+    // (rows, talker splits; 0: the decode chain, -1: launch by launch in its place; how the predictor's part is made) -> graphs
+    std::map<std::tuple<int, int, int>, Graphs> graphs;
     cudaEvent_t predictor_start = nullptr, predictor_stop = nullptr;
     // frames launched on this workspace, and the GPU times of the frame `timed_frame` (every
     // session of a lockstep frame reports the same two numbers: they are read from the events once)
@@ -237,6 +241,8 @@ public:
         int grid = 0;                   // CTAs of a launch
         uint64_t numbers = 0;           // of exchanges, at most, since they were restarted (guarded as the device's chains are)
     } chain;
+    // What the lockstep chain reads of the predictor; empty where it cannot run.
+    DeviceBuffer lockstep;
     std::mutex mutex;               // pools, workspaces
     int mask_eos = 0;
     int use_graphs = 1;
@@ -261,6 +267,7 @@ private:
     Quantized allocate_quantized(uint64_t rows, uint64_t cols);
     Quantized add_quant_matrix(const std::string& name, uint64_t rows, uint64_t cols);
     void build_chain();
+    void build_lockstep();
     void place_chain();
     void plan_layers(const std::string& prefix, const ModelDims& d, std::vector<LayerWeights>& out);
 
@@ -345,7 +352,7 @@ private:
                   const SamplingParams& predictor, bool host_codes) const;
     static void bind_rows(Workspace& w, Session** s, int n);
     enum class Way { kChain, kInItsPlace, kLaunches };      // of a frame
-    static Workspace::Graphs& frame_graphs(Workspace& w, Model& m, int n, int splits, Way way);
+    static Workspace::Graphs& frame_graphs(Workspace& w, Model& m, int n, int splits, Way way, int lockstep);
     // `ahead`: frames enqueued since the host table was filled (their rows advance on the device; the host table stays as
     // it is, since its upload may not have run yet)
     static void launch_frame(Workspace& w, Model& m, Session** s, int n, bool upload_table,

@@ -608,11 +608,21 @@ int choose_splits(const TcScratch& scratch, const GemvArgs& a, int mt) {
     }();
     int splits = 1;
     for (int s = 2; s <= split_cap && s <= nk; ++s) {
-        if (clusters <= resident[s]) splits = s;
+        // (as few as have the longest slice this short: each one more is another part to exchange)
+        if (clusters <= resident[s] && (nk + s - 1) / s < (nk + splits - 1) / splits) splits = s;
     }
     return splits;
 }
 }  // namespace
+
+int gemm_tc_tile(int rows) { return tile_rows(rows); }
+int gemm_tc_slices(int out_features, int in_features, int rows, bool gate_up) {
+    TcScratch* scratch = scratch_for_current_device();
+    if (scratch == nullptr || rows < g_tc_min_rows || in_features % kBK != 0) return 0;
+    GemvArgs a;
+    a.out_features = out_features; a.in_features = in_features; a.rows = rows; a.epilogue = gate_up ? EPI_GATE_UP_SILU : EPI_PLAIN;
+    return choose_splits(*scratch, a, tile_rows(rows));
+}
 
 float gemm_tc_estimate_us(const GemvArgs& a, int tile) {
     TcScratch* scratch = scratch_for_current_device();

@@ -94,6 +94,9 @@ cudaError_t configure_tc_kernels();      // also allocates the per-device scratc
 void set_tc_min_rows(int rows);          // 65 or more: never use the tensor-core path
 int tc_min_rows();
 unsigned int gemm_tc_error_count();
+int gemm_tc_tile(int rows);              // rows of the tile that it takes for up to kMaxRows rows
+// K-slices that it sums for a projection of these sizes, 0 where it does not take it
+int gemm_tc_slices(int out_features, int in_features, int rows, bool gate_up);
 // more than kMaxRows rows (prompt passes), K % 128 == 0, no norm prologue, no fp32 output
 // (gemm_int8_wide.cu); channel_tiles 1 or 2
 cudaError_t launch_int8_gemm_wide(const GemvArgs& args, cudaStream_t stream, int channel_tiles);
@@ -346,6 +349,42 @@ constexpr uint64_t kChainNumbers = 1ull << 31;
 constexpr uint64_t kChainNumbersPerFrame = 1024;     // at most: 16 x (5 x 6 + 1) + 15 x 2 by the predictor, 28 x 8 by the talker
 cudaError_t restart_chain_numbers(void* exchange, uint32_t* epoch, cudaStream_t stream);
 unsigned int chain_error_count();
+
+// ---------------------------------------------------------------- lockstep chain (lockstep_chain.cu)
+// Positions of the predictor for 9..64 rows, input projections to heads and draws, in one cooperative launch; same bits as
+// launch by launch.  Launches that share an exchange run one after the other.
+constexpr int kLockstepHeadMap = 20, kLockstepMtpMap = 35, kLockstepMaps = 36;
+struct LockstepModel {               // device memory; maps first, aligned as tensor maps are
+    alignas(64) unsigned char maps[kLockstepMaps][128];     // [layer][qkv, o, gate/up, down], heads, input projection
+    ChainLayer layers[5];
+    const float* head_scales[15];
+    const float* mtp_scales;
+    const bf16 *mtp_bias, *final_norm;
+};
+struct LockstepLaunch {
+    const LockstepModel* model = nullptr;
+    const FrameTable* table = nullptr;
+    const int* pages = nullptr;               // [rows] page of the predictor's cache
+    KvLayout kv;                              // paged; offsets of layer 0
+    long long kv_layer_elems = 0;
+    const uint32_t* rope_table = nullptr;
+    const bf16* codec_embedding = nullptr;
+    const bf16* const* embeddings = nullptr;  // device array: [15]
+    bf16* logits = nullptr;                   // out, without draws: [rows][kPredictorVocab], positions from 1
+    void* exchange = nullptr;                 // lockstep_exchange_bytes(), set up by restart_lockstep
+    int rows = 0;
+    int first = 0, last = 0;                  // positions
+    bool draws = false;                       // their tokens are drawn in the launch (greedy, or top-k draws of 1..kChainTopK)
+};
+cudaError_t configure_lockstep_kernels();
+bool lockstep_chain_available(int rows);
+bool make_lockstep_map(LockstepModel* host_model, int index, const int8_t* weights, int in_features, int matrix_rows, bool wide);
+size_t lockstep_exchange_bytes();
+// Before the first launch, one of another row count, and one behind a launch that was given up.
+cudaError_t restart_lockstep(void* exchange, cudaStream_t stream);
+cudaError_t launch_lockstep_chain(const LockstepLaunch& chain, cudaStream_t stream);
+unsigned int lockstep_error_count();
+
 // The talker's decode attention with the bits of the chain's, as a launch (attention_blocks.cu): fused, paged, settled
 // inputs, a.scratch of chain_order_scratch_floats().
 size_t chain_order_scratch_floats(int rows, int kv_heads);
