@@ -79,7 +79,7 @@ typedef struct Q3tGemmDesc {
 QWEN3_TTS_API int32_t q3t_launch_int8_gemm_ex(const Q3tGemmDesc* desc, void* stream);
 /* Test hook: a projection of a prompt pass, up to 2048 rows.  kernel 0: the one that a prompt takes; 1 and 2: 128 rows and
  * one or two tiles of channels a CTA; 3: the lockstep kernel with its row blocks side by side; 96, 128, 160: the same in
- * blocks of so many rows. */
+ * blocks of so many rows; 256: pairs of CTAs. */
 QWEN3_TTS_API int32_t q3t_test_prompt_gemm(const Q3tGemmDesc* desc, int32_t kernel, void* stream);
 
 /* launch_quantize_weight_rows (int8_gemv.cu:302-317) */

@@ -31,6 +31,7 @@ namespace q3t {
 cudaError_t set_gemv_mma_error_sink(unsigned int* device_visible_word);
 cudaError_t set_tc_error_sink(unsigned int* device_visible_word);
 cudaError_t set_wide_error_sink(unsigned int* device_visible_word);
+cudaError_t set_pair_error_sink(unsigned int* device_visible_word);
 cudaError_t set_chain_error_sink(unsigned int* device_visible_word);
 cudaError_t set_lockstep_error_sink(unsigned int* device_visible_word);
 
@@ -53,6 +54,7 @@ cudaError_t configure_device() {
     e = configure_gemv_kernels();
     if (e == cudaSuccess) e = configure_tc_kernels();
     if (e == cudaSuccess) e = configure_wide_kernels();
+    if (e == cudaSuccess) e = configure_pair_kernels();
     if (e == cudaSuccess) e = configure_prompt_kernels();
     if (e == cudaSuccess) e = configure_chain_kernels();
     if (e == cudaSuccess) e = configure_lockstep_kernels();
@@ -68,6 +70,7 @@ cudaError_t configure_device() {
             e = set_gemv_mma_error_sink(word);
             if (e == cudaSuccess) e = set_tc_error_sink(word);
             if (e == cudaSuccess) e = set_wide_error_sink(word);
+            if (e == cudaSuccess) e = set_pair_error_sink(word);
             if (e == cudaSuccess) e = set_chain_error_sink(word);
             if (e == cudaSuccess) e = set_lockstep_error_sink(word);
             if (e == cudaSuccess) e = set_attention_error_sink(word);
@@ -647,6 +650,7 @@ int32_t q3t_test_prompt_gemm(const Q3tGemmDesc* d, int32_t kernel, void* stream)
     GemvArgs a;
     if (const int32_t e = gemm_args(d, a)) return e;
     if (kernel == 0) return static_cast<int32_t>(launch_int8_gemm_prompt(a, S(stream)));
+    if (kernel == 256) return static_cast<int32_t>(launch_int8_gemm_pair(a, S(stream)));
     if (kernel >= 3) return static_cast<int32_t>(launch_int8_gemm_tc(a, S(stream), kernel == 3 ? 0 : kernel));
     return static_cast<int32_t>(launch_int8_gemm_wide(a, S(stream), kernel));
 }
@@ -1150,7 +1154,7 @@ int32_t q3t_test_sort_chain_places(const uint32_t* of_sm, const uint32_t* of_pag
 int32_t q3t_test_hold_sms(int32_t ctas, uint64_t ns, void* stream) { return static_cast<int32_t>(launch_hold_sms(ctas, ns, S(stream))); }
 
 uint32_t q3t_kernel_error_count(void) {
-    return gemm_tc_error_count() + gemm_wide_error_count() + gemv_mma_error_count() + chain_error_count() + lockstep_error_count();
+    return gemm_tc_error_count() + gemm_wide_error_count() + gemm_pair_error_count() + gemv_mma_error_count() + chain_error_count() + lockstep_error_count();
 }
 
 uint32_t q3t_attention_range_error_count(void) { return attention_range_error_count(); }

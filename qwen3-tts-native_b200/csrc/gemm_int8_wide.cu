@@ -5,19 +5,18 @@
 // tiles here to fill the GPU.  A CTA owns NT tiles of 128 output channels (TMEM lanes) by 128
 // activation rows (TMEM columns).
 //
-// What bounds it: the tensor cores, if the operands arrive in time.  Per element of K a CTA with NT
-// = 2 fetches 256 bytes of weights and 256 bytes of activations for 8 cycles of MMA (4096 bf16 MACs a
-// cycle and SM), 64 bytes a cycle, about what the L2 delivers to one SM; with one channel tile of 128 the
-// same activations cost 96.  So NT = 2 wherever its tiles fill the GPU, NT = 1 for passes of few rows.
+// What bounds it: the way of a step through conversion, tensor memory and products.  A step of 128 x 128 weights is 512 cycles of
+// products and some 500 of integer instructions on every scheduler; it takes 0.32 us with NT = 2 and 0.46 with NT = 1, of one CTA
+// alone as of 148.  The issuing thread does not look at barriers (await_step), and weights are converted ahead of the wait for
+// their place (1,500 rows of down 48 -> 41 us, gate/up 75.5 -> 69, q/k/v 37 -> 34).  NT = 2 has its activations once for two steps;
+// NT = 1 has more CTAs, for passes of few rows.
 // The two tiles of a gate/up projection are the gate rows and the up rows of the same 128 channels, so
 // that a thread finds both values of a channel in its own TMEM lane; with NT = 1 a tile holds 64 of
 // each and the up half crosses over through shared memory.
 //
 // Warp roles as in gemm_int8_tc.cu: 0 weight copies, 1 MMA issue, 2 activation copies, 3 TMEM; 4..19 in four
 // groups dequantise (a thread turns 128 int8 of its channel into bf16 and stores them to tensor memory as the
-// A operand), then read the accumulators.  Every wait is bounded.
-// Measured (B200, 1500 rows): gate/up 2048 -> 2 x 6144 74 us, q/k/v 37 us, o 21 us, down 47 us, 0.6-1.0 PFLOP/s; a step
-// of 64 KB takes about 1350 cycles with or without its MMAs, the rate at which an SM takes data in.
+// A operand), then read the accumulators; 3 is also the look-out for steps whose operands are all there.  Every wait is bounded.
 
 #include "q3t_kernels.cuh"
 #include "q3t_tcgen05.cuh"
@@ -89,6 +88,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
     uint64_t* acc_done = empty_a + kAStages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint32_t* steps_ready = tmem_slot + 2;
 
     const int tid = threadIdx.x;
     const int warp = __shfl_sync(0xffffffffu, tid / kWarp, 0);
@@ -119,6 +119,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         }
         mbar_init(acc_done, 1);
         *abort_flag = 0;
+        *steps_ready = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -170,16 +171,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
     } else if (warp == 1) {
         if (elect_one()) {
             bool ok = true;
+            uint32_t seen = 0;
             for (int i = 0; i < nk && ok; ++i) {
                 const int sx = i % kXStages;
-                ok = guard.wait(&full_x[sx], (i / kXStages) & 1);
-                if (!ok) break;
                 const uint32_t b_addr = smem_u32(xs + sx * kXStageBytes);
 #pragma unroll
                 for (int u = 0; u < NT; ++u) {
                     const int item = i * NT + u;
                     const int sa = item % kAStages;
-                    ok = ok && guard.wait(&full_a[sa], (item / kAStages) & 1);
+                    ok = ok && await_step(guard, steps_ready, (uint32_t)item, seen);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t a_col = tmem_base + kAStageBase + sa * kAStageCols;
@@ -195,6 +195,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
             }
             umma_commit(acc_done);
         }
+    } else if (warp == 3) {
+        if (elect_one()) {
+            for (int item = 0; item < nk * NT; ++item) {
+                const int i = item / NT;
+                if (item % NT == 0 && !guard.wait(&full_x[i % kXStages], (i / kXStages) & 1)) break;
+                if (!guard.wait(&full_a[item % kAStages], (item / kAStages) & 1)) break;
+                publish_steps(steps_ready, (uint32_t)item + 1);
+            }
+        }
     } else if (warp >= 4) {
         const int group = (warp - 4) / 4;
         const int t = (warp % 4) * 32 + lane;        // channel within the tile = TMEM lane
@@ -205,30 +214,26 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
             const int sa = item % kAStages;
             if (!__all_sync(0xffffffffu, guard.wait(&full_w[s], (item / kWStages) & 1))) { ok = false; break; }
             const unsigned char* rowp = w8 + s * kWStageBytes + t * 128;
-            int4 raw[8];
+            // converted ahead of the wait for its place: what the place still holds is being multiplied meanwhile
+            uint32_t out[2][32];
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                raw[c] = *reinterpret_cast<const int4*>(rowp + ((c ^ (t & 7)) << 4));
+                const int4 v = *reinterpret_cast<const int4*>(rowp + ((c ^ (t & 7)) << 4));
+                uint32_t* to = out[c / 4] + 8 * (c & 3);
+                dequant4(static_cast<uint32_t>(v.x), to[0], to[1]);
+                dequant4(static_cast<uint32_t>(v.y), to[2], to[3]);
+                dequant4(static_cast<uint32_t>(v.z), to[4], to[5]);
+                dequant4(static_cast<uint32_t>(v.w), to[6], to[7]);
             }
-            if (item >= kAStages
-                && !__all_sync(0xffffffffu, guard.wait(&empty_a[sa], ((item / kAStages) - 1) & 1))) {
+            compute_now(out[0]);
+            compute_now(out[1]);
+            if (item >= kAStages && !__all_sync(0xffffffffu, guard.wait(&empty_a[sa], ((item / kAStages) - 1) & 1))) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t out[32];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int4 v = raw[4 * h + c];
-                    dequant4(static_cast<uint32_t>(v.x), out[8 * c + 0], out[8 * c + 1]);
-                    dequant4(static_cast<uint32_t>(v.y), out[8 * c + 2], out[8 * c + 3]);
-                    dequant4(static_cast<uint32_t>(v.z), out[8 * c + 4], out[8 * c + 5]);
-                    dequant4(static_cast<uint32_t>(v.w), out[8 * c + 6], out[8 * c + 7]);
-                }
-                tmem_store_32(lane_base + kAStageBase + sa * kAStageCols + 32 * h, out);
-            }
+            tmem_store_32(lane_base + kAStageBase + sa * kAStageCols, out[0]);
+            tmem_store_32(lane_base + kAStageBase + sa * kAStageCols + 32, out[1]);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -316,6 +321,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
+    __syncwarp();
     __syncthreads();
     if (*abort_flag) {
         // copies still in flight get time to land before the CTA's memory is released
@@ -383,9 +389,11 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
 }
 
 // Which kernel takes a projection of a prompt pass: the one with the shortest estimate.  A wave of CTAs of this
-// file's kernel costs its steps (0.50 us each with one channel tile, 0.82 us with two: what an SM takes in) and 4
-// to 7 us of start and epilogue; the kernel of gemm_int8_tc.cu, in blocks of up to 64 rows or of 96, 128 or 160 side by side
-// and with K split where that fits one wave, is estimated there.  Above 640 rows this file's kernel always has the waves.
+// file's kernel costs its steps (0.46 us each with one channel tile, 0.63 us with two) and 5 to 7 us of start and epilogue;
+// the kernel of gemm_int8_tc.cu, in blocks of up to 64 rows or of 96, 128 or 160 side by side and with K split where that fits
+// one wave, and the one of gemm_int8_pair.cu are estimated there.  Above 640 rows tc's never has fewer waves.  Measured there (us, one tile /
+// two tiles / pairs): 700 rows q/k/v 20.8 / 17.2 / 15.2, o 13.2 / 17.6 / 13.7, gate/up 53.6 / 34.9 / 34.2, down 28.4 / 38.1 / 25.7;
+// 2,048 rows 42.6 / 34.6 / 32.8, 25.6 / 19.4 / 20.6, 142 / 99.9 / 93.8, 56.6 / 41.8 / 38.6.
 // Measured from 65 to 640 rows (us, blocks of 64 / best of the tall ones / one tile / two tiles of this file): gate/up 65 rows
 // 19.0 / 12.5 / 14.8 / 17.2, 128 21.1 / 14.7 / 15.6 / 18.0, 150 22.3 / 16.3 / 27.3 / 18.6, 300 41.5 / 27.2 / 29.6 / 19.8, 448
 // 53.7 / 31.3 / 43.2 / 36.8; q/k/v 128 8.3 / 9.0 / 11.6 / 18.2, 300 20.8 / 11.3 / 12.5 / 18.2, 512 23.2 / 15.0 / 13.1 / 18.6;
@@ -406,9 +414,13 @@ cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     auto waves = [&](int tiles) {
         return ((a.out_features + tiles * per_single - 1) / (tiles * per_single) * row_blocks + kSms - 1) / kSms;
     };
-    const float one = waves(1) * (a.epilogue == EPI_GATE_UP_SILU ? 6.8f + 0.50f * steps : 4.3f + 0.50f * steps);
-    const float two = waves(2) * (5.5f + 0.82f * steps);
+    const bool adds = a.epilogue == EPI_ADD || a.epilogue == EPI_BIAS_ADD;         // another read of the rows
+    const float one = waves(1) * (4.9f + (adds ? 1.5f : 0.0f) + 0.456f * steps);
+    const float two = waves(2) * (7.2f + (adds ? 2.0f : 0.0f) + 0.63f * steps);
+    const float pairs = gemm_pair_estimate_us(a);
     float best = one < two ? one : two;
+    const bool paired = pairs < best;
+    if (paired) best = pairs;
     int tile = -1;
     for (int t : {0, 96, 128, 160}) {
         if (t > 0 && a.rows > kTallRowsMost) break;
@@ -418,7 +430,8 @@ cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
             tile = t;
         }
     }
-    return tile >= 0 ? launch_int8_gemm_tc(a, stream, tile) : launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
+    if (tile >= 0) return launch_int8_gemm_tc(a, stream, tile);
+    return paired ? launch_int8_gemm_pair(a, stream) : launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
 }
 
 unsigned int gemm_wide_error_count() {

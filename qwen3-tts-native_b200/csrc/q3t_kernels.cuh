@@ -102,6 +102,11 @@ int gemm_tc_slices(int out_features, int in_features, int rows, bool gate_up);
 cudaError_t launch_int8_gemm_wide(const GemvArgs& args, cudaStream_t stream, int channel_tiles);
 float gemm_tc_estimate_us(const GemvArgs& args, int tile = 0);     // what launch_int8_gemm_tc would take, for that choice
 cudaError_t configure_wide_kernels();
+// the same by pairs of CTAs (gemm_int8_pair.cu)
+cudaError_t launch_int8_gemm_pair(const GemvArgs& args, cudaStream_t stream);
+float gemm_pair_estimate_us(const GemvArgs& args);
+cudaError_t configure_pair_kernels();
+unsigned int gemm_pair_error_count();
 // projections of a prompt pass of more than kMaxRows rows (needs norm_out when norm_w is given)
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream);
 unsigned int gemm_wide_error_count();

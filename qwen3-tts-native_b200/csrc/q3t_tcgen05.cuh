@@ -39,6 +39,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+// 1 if that phase is complete; does not wait
+__device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok;
+}
+
 // One lane of a converged warp.  Unlike a test of the lane index, this tells the compiler that
 // the code below runs in exactly one thread, which the instructions that take their operands
 // from uniform registers (TMA copies, MMA issue) need in order to be emitted without a loop
@@ -72,6 +85,33 @@ struct Guard {
         return true;
     }
 };
+
+// How many steps have all of their operands, for the thread that issues the products.  A look at a barrier costs 110 cycles even
+// when it is complete (200 and more at cluster scope), twice a step, and the tensor cores' queue holds only a few products;
+// a thread of its own looks at the barriers, and the issuing one at a word.
+__device__ __forceinline__ void publish_steps(uint32_t* word, uint32_t steps) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(word)), "r"(steps) : "memory");
+}
+__device__ __forceinline__ uint32_t published_steps(const uint32_t* word) {
+    uint32_t steps;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(steps) : "r"(smem_u32(word)) : "memory");
+    return steps;
+}
+// until `word` has passed `step`; `seen` is what it was at the last look
+__device__ __forceinline__ bool await_step(const Guard& g, const uint32_t* word, uint32_t step, uint32_t& seen) {
+    uint32_t polls = 0;
+    while (seen <= step) {
+        seen = published_steps(word);
+        if (seen > step) break;
+        if ((++polls & 255u) != 0) continue;
+        if (*g.abort_flag) return false;
+        if ((polls & 16383u) == 0 && now_ns() > g.deadline) {
+            *g.abort_flag = 1;
+            return false;
+        }
+    }
+    return true;
+}
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
@@ -154,6 +194,12 @@ __device__ __forceinline__ void dequant4(uint32_t word, uint32_t& lo, uint32_t& 
     const uint32_t p = __byte_perm(word, 0x43434343u, 0x4140), q = __byte_perm(word, 0x43434343u, 0x4342);
     asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(p & 0xff7fff7fu), "r"(p & 0xff80ff80u));
     asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"(q & 0xff7fff7fu), "r"(q & 0xff80ff80u));
+}
+
+// Keeps the computation of these values ahead of what follows (the compiler would move it behind a wait, next to the store).
+__device__ __forceinline__ void compute_now(uint32_t (&r)[32]) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));
 }
 
 // NCOL consecutive fp32 accumulator columns of this thread's TMEM lane

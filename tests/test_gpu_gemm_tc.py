@@ -166,6 +166,41 @@ def test_tall_tiles(q3t, orc, ops, kernel, n, k, rows):
     assert q3t.library().q3t_kernel_error_count() == 0
 
 
+@pytest.mark.parametrize("n,k,rows", [(256, 128, 1), (300, 384, 65), (129, 1152, 161), (257, 512, 300), (512, 2048, 257)])
+def test_pairs(q3t, orc, ops, n, k, rows):
+    """Pairs of CTAs: one step of K and many, rows and channels that end inside a block, a chunk of sixteen and a CTA's half; each
+    value within a rounding step of the oracle's, and the same twice.  Tolerance: as in test_prompt_kernels."""
+    w, s, x, bias, base = prompt_case(orc, n, k, rows)
+    plain = orc.int8_gemm_rows(w, s, x)
+    check_bf16(orc, ops.int8_gemm(w, s, x, prompt_kernel=256)["y"], plain)
+    out = ops.int8_gemm(w, s, x, epilogue=ops.EPI_ADD, y_in=base, prompt_kernel=256)["y"]
+    check_bf16(orc, out, orc.int8_gemm_rows(w, s, x, y_in=base, mode=1), summand=base)
+    assert np.array_equal(out, ops.int8_gemm(w, s, x, epilogue=ops.EPI_ADD, y_in=base, prompt_kernel=256)["y"])
+    summand = orc.to_bf16(1.6 * (np.abs(orc.from_bf16(plain)) + np.abs(orc.from_bf16(bias))).astype(np.float32))
+    for epilogue, silu in ((ops.EPI_BIAS, False), (ops.EPI_BIAS_SILU, True)):
+        check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=epilogue, bias=bias, prompt_kernel=256)["y"],
+                   orc.bias_activation_rows(plain, bias, silu), summand=summand)
+    got = ops.int8_gemm(w, s, x, epilogue=ops.EPI_BIAS_ADD, bias=bias, resid=base, prompt_kernel=256)["resid"]
+    check_bf16(orc, got, orc.add(base, orc.bias_activation_rows(plain, bias, False)).reshape(rows, n),
+               summand=orc.to_bf16(np.maximum(np.abs(orc.from_bf16(base)), orc.from_bf16(summand)).astype(np.float32)))
+    w, s, x, _, _ = prompt_case(orc, n, k, rows, gate_up=True)
+    check_bf16(orc, ops.int8_gemm(w, s, x, epilogue=ops.EPI_GATE_UP_SILU, prompt_kernel=256)["y"],
+               orc.int8_gate_up_silu_rows(w, s, x))
+    for bad in (dict(epilogue=ops.EPI_BIAS_ADD, bias=bias), dict(want_f32=True), dict(epilogue=ops.EPI_BIAS)):
+        with pytest.raises(RuntimeError):
+            ops.int8_gemm(w[:n], s[:n], x, prompt_kernel=256, **bad)
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
+@pytest.mark.parametrize("n,k,rows,gate_up", [(4096, 256, 1500, False), (2048, 1152, 2048, False), (4097, 384, 1201, False), (6144, 256, 1500, True), (6100, 640, 700, True)])
+def test_pairs_of_several_tiles(q3t, orc, ops, n, k, rows, gate_up):
+    """More tiles than pairs: every sum is made of the same products in the same order as with one tile a CTA, so every bit is."""
+    w, s, x, _, base = prompt_case(orc, n, k, rows, gate_up)
+    args = dict(epilogue=ops.EPI_GATE_UP_SILU) if gate_up else dict(epilogue=ops.EPI_ADD, y_in=base)
+    assert np.array_equal(ops.int8_gemm(w, s, x, prompt_kernel=256, **args)["y"], ops.int8_gemm(w, s, x, prompt_kernel=1, **args)["y"])
+    assert q3t.library().q3t_kernel_error_count() == 0
+
+
 @pytest.mark.parametrize("n,k,rows,gate_up", [(2048, 6144, 700, False), (4096, 2048, 1200, False), (2048, 2048, 2048, False), (6144, 2048, 600, True)])
 def test_prompt_kernels_over_several_waves(q3t, orc, ops, n, k, rows, gate_up):
     """More CTAs than the GPU holds at once, at the talker's shapes; rows are compared with the lockstep kernel's, each within
