@@ -33,6 +33,7 @@ cudaError_t set_tc_error_sink(unsigned int* device_visible_word);
 cudaError_t set_wide_error_sink(unsigned int* device_visible_word);
 cudaError_t set_pair_error_sink(unsigned int* device_visible_word);
 cudaError_t set_chain_error_sink(unsigned int* device_visible_word);
+cudaError_t set_prompt_attention_error_sink(unsigned int* device_visible_word);
 cudaError_t set_lockstep_error_sink(unsigned int* device_visible_word);
 
 namespace {
@@ -72,6 +73,7 @@ cudaError_t configure_device() {
             if (e == cudaSuccess) e = set_wide_error_sink(word);
             if (e == cudaSuccess) e = set_pair_error_sink(word);
             if (e == cudaSuccess) e = set_chain_error_sink(word);
+            if (e == cudaSuccess) e = set_prompt_attention_error_sink(word);
             if (e == cudaSuccess) e = set_lockstep_error_sink(word);
             if (e == cudaSuccess) e = set_attention_error_sink(word);
             if (e == cudaSuccess) g_error_words[device].store(word, std::memory_order_release);
@@ -1154,7 +1156,7 @@ int32_t q3t_test_sort_chain_places(const uint32_t* of_sm, const uint32_t* of_pag
 int32_t q3t_test_hold_sms(int32_t ctas, uint64_t ns, void* stream) { return static_cast<int32_t>(launch_hold_sms(ctas, ns, S(stream))); }
 
 uint32_t q3t_kernel_error_count(void) {
-    return gemm_tc_error_count() + gemm_wide_error_count() + gemm_pair_error_count() + gemv_mma_error_count() + chain_error_count() + lockstep_error_count();
+    return gemm_tc_error_count() + gemm_wide_error_count() + gemm_pair_error_count() + gemv_mma_error_count() + chain_error_count() + lockstep_error_count() + prompt_attention_error_count();
 }
 
 uint32_t q3t_attention_range_error_count(void) { return attention_range_error_count(); }

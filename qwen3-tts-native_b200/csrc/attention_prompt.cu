@@ -5,47 +5,47 @@
 // native/qwen3-tts-native/native/src/talker_kernels.cu:506-595, after the per-head RMSNorm, RoPE and
 // cache append of :50-70, :597-658); the decode kernel there treats every row as a session of its own
 // and reads its whole context again, which for a prompt of n positions is n^2 / 2 cache rows a layer.
-// Here a CTA takes 32 positions of the two query heads of a KV head (64 rows of MMA) and walks their
+// Here a CTA takes 64 positions of the two query heads of a KV head, 128 rows of the tensor cores, and walks their
 // common context once, 64 tokens at a time, with a running softmax.
 //
-// What bounds it: the chain of a step, 64 tokens' scores, softmax and products, times the steps of the longest
-// context.  The probabilities go through the second product as bf16 hi + lo (16 bits kept), so a 64-row, 64-token step is
-// 3 x 64 x 64 x 128 MACs: 0.9 us of an SM's mma.sync rate, 31 steps an SM for 1500 positions.  Two groups of four
-// warps of 16 rows take half of every step's tokens each and meet at the end; K and V of the next step are in flight
-// (cp.async, two buffers of 32 KB); two CTAs fit an SM at 128 registers (the query fragments come from shared memory).
-// 1500 positions: 71 us a layer; four warps on whole steps 81, with a page lookup per token, masks on every score
-// and heads one after the other 118.
+//   scores    S = Q K^T, tcgen05.mma from shared memory into 64 columns of tensor memory
+//   softmax   two threads a row, half of the step's tokens each: S to registers (the next step's products may begin), weights as bf16 hi + lo (16 bits kept) back to
+//             tensor memory
+//   output    O += P V, hi and lo as the A operand from tensor memory, V as it lies in its pages
+//   copies    K and V, by two warps each, two steps ahead of their products (cp.async: the pages lie anywhere)
+// A row's reference is its first maximum until a score exceeds it by 2^8: weights above one cost no precision in floating point,
+// and an output in tensor memory is rescaled at almost no step instead of almost every one (some row of 32 has a new maximum).
+//
+// What bounds it: the chain of a step in its softmax threads, times the steps of the longest context; two CTAs an SM take turns
+// at the issue slots.  1,500 positions: 68 us a layer with mma.sync (32 positions a CTA, the weights' two halves as 3 x 64 x 64 x 128
+// products a step at the legacy rate), 54 so with K and V in one buffer, 45 with a buffer each, 43 with two threads a row.
 
 #include "q3t_kernels.cuh"
+#include "q3t_tcgen05.cuh"
 
 namespace q3t {
 namespace {
 
 constexpr int kHd = 128;
-constexpr int kBlockPositions = 32;
+constexpr int kBlockPositions = 64;
 constexpr int kStepTokens = 64;
-constexpr int kFlashThreads = 256;
-constexpr int kTileBytes = kStepTokens * kHd * 2;       // 16 KB of K or V
+constexpr int kRows = 2 * kBlockPositions;              // of the tensor cores: position + 64 * head
+constexpr int kFlashThreads = 416;                      // warps 0..7 softmax, 8..11 copies, 12 products
+constexpr int kCopyWarp = 8, kProductWarp = 12;
+constexpr int kHalf = kStepTokens / 2;                  // tokens of a step, to each of a row's two threads
+constexpr int kTileBytes = kStepTokens * kHd * 2;       // 16 KB of K or V: [64 dims][token][128 bytes, swizzled]
+constexpr int kQueryBytes = kRows * kHd * 2;
+constexpr int kBuffers = 2;
 constexpr int kFlashCtas = 2;
-constexpr int kHalfTokens = kStepTokens / 2;            // of a step, to each group of four warps
-constexpr size_t kFlashSmem = 5 * kTileBytes;           // two buffers of (K, V), the queries
+constexpr uint32_t kTmemCols = 256, kScores = 0, kHi = 64, kLo = 96, kOut = 128;
+constexpr float kSlack = 8.0f;                          // log2 of the largest weight
+constexpr unsigned long long kBudgetNs = 2000000000ull;
+constexpr size_t kFlashSmem = 1024 + kQueryBytes + kBuffers * 2 * kTileBytes + 4 * kRows * 4 + 128;
+
+__device__ unsigned int g_prompt_attention_errors = 0;
+__device__ unsigned int* g_prompt_attention_error_sink = nullptr;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
 __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -160,223 +160,300 @@ __global__ void __launch_bounds__(256) prompt_append_kernel(const PromptArgs a) 
     }
 }
 
-// 16-byte piece `piece` (0..15) of token `t` in a K or V tile: pieces are XORed with the token so that the
-// eight rows of an ldmatrix fall into different banks
-__device__ __forceinline__ uint32_t tile_offset(int t, int piece) { return (uint32_t)(t * 256 + ((piece ^ (t & 7)) << 4)); }
+// 16-byte piece `piece` (0..15) of row `t` of a tile of `rows`: K-major for the products over dims, and for those over tokens
+// as it is, with the dims contiguous
+__device__ __forceinline__ uint32_t tile_offset(int rows, int t, int piece) {
+    return (uint32_t)((piece >> 3) * rows * 128 + t * 128 + (((piece & 7) ^ (t & 7)) << 4));
+}
+// B operand whose rows are contiguous: 64 of them in 128 bytes (swizzled), the next 64 a tile of tokens further on, eight of K 1024 bytes
+__device__ __forceinline__ uint64_t desc_rows_contiguous(uint32_t smem) {
+    return (uint64_t)((smem >> 4) & 0x3FFFu) | ((uint64_t)(kStepTokens * 128 / 16) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_store_16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 
 __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_kernel(const PromptArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* queries = smem;
+    unsigned char* tiles = smem + kQueryBytes;                // buffer: K, V
+    float* tops = reinterpret_cast<float*>(tiles + kBuffers * 2 * kTileBytes);             // [step % 2][half][row]
+    uint64_t* full_k = reinterpret_cast<uint64_t*>(tops + 4 * kRows);
+    uint64_t* full_v = full_k + kBuffers;
+    uint64_t* empty_k = full_v + kBuffers;
+    uint64_t* empty_v = empty_k + kBuffers;
+    uint64_t* s_ready = empty_v + kBuffers;                   // scores in tensor memory
+    uint64_t* s_free = s_ready + 1;                           // and in registers
+    uint64_t* p_ready = s_free + 1;                           // weights in tensor memory
+    uint64_t* o_ready = p_ready + 1;                          // multiplied
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_ready + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
     const int tid = threadIdx.x;
+    const int warp = __shfl_sync(0xffffffffu, tid / kWarp, 0);
     const int lane = tid % kWarp;
-    const int group = tid / (kFlashThreads / 2);          // tokens 32 group .. + 31 of every step
-    const int warp = tid / kWarp % 4;
-    const int gid = lane >> 2;
-    const int tig = lane & 3;
     // the last positions have the longest context: they go first, all KV heads of a block together
     const int kvh = (int)blockIdx.x % a.kv_heads;
     const int block = ((int)gridDim.x - 1 - (int)blockIdx.x) / a.kv_heads;
     const int row0 = block * kBlockPositions;
-    const int head = kvh * 2 + (warp >> 1);
-    const int my_row = row0 + (warp & 1) * 16;            // rows my_row + gid and + 8 of this lane
     const int length = a.base + min(a.rows, row0 + kBlockPositions);      // tokens the CTA walks
     const int steps = (length + kStepTokens - 1) / kStepTokens;
 
+    tc::Guard guard;
+    guard.deadline = tc::now_ns() + kBudgetNs;
+    guard.abort_flag = abort_flag;
+    if (tid == 0) {
+        for (int i = 0; i < kBuffers; ++i) {
+            tc::mbar_init(&full_k[i], 2);
+            tc::mbar_init(&full_v[i], 2);
+            tc::mbar_init(&empty_k[i], 1);
+            tc::mbar_init(&empty_v[i], 1);
+        }
+        tc::mbar_init(s_ready, 1);
+        tc::mbar_init(s_free, 8);
+        tc::mbar_init(p_ready, 8);
+        tc::mbar_init(o_ready, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kProductWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
     pdl_wait();
     pdl_trigger();
 
-    auto load_step = [&](int step, int buffer) {
-        const uint32_t kdst = smem_addr(smem) + buffer * 2 * kTileBytes;
-        // 64 tokens x 16 pieces of K and as many of V: thread t takes piece t % 16 of token t / 16 of every page
-        const int piece = tid & 15;
+    if (warp >= kCopyWarp && warp < kProductWarp) {
+        // ---- copies: K by the first two warps, behind the queries, V by the others; thread t takes piece t % 16 of tokens t / 16,
+        // + 4, + 8, + 12 of every page.  Pages are looked up a step ahead.
+        const bool values = warp >= kCopyWarp + 2;
+        const int t = (tid - kCopyWarp * kWarp) % (2 * kWarp), piece = t & 15;
+        uint64_t* const landed = values ? full_v : full_k;
+        uint64_t* const used = values ? empty_v : empty_k;
+        if (!values) {
 #pragma unroll
-        for (int page = 0; page < kStepTokens / kPageTokens; ++page) {
-            const int t = page * kPageTokens + (tid >> 4);
-            const uint32_t off = tile_offset(t, piece);
-            if (step * kStepTokens + t < length) {
-                const bf16* k = page_of(a, step * kStepTokens + page * kPageTokens, kvh, false) + (size_t)(tid >> 4) * kHd + piece * 8;
-                copy16(kdst + off, k);
-                copy16(kdst + kTileBytes + off, k + (a.kv.v_offset - a.kv.k_offset));
-            } else {
-                // past the end: the scores are masked, but 0 * (stale bits that decode as NaN) is not zero
-                *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + off) = make_int4(0, 0, 0, 0);
-                *reinterpret_cast<int4*>(smem + buffer * 2 * kTileBytes + kTileBytes + off) = make_int4(0, 0, 0, 0);
+            for (int i = 0; i < kRows / 4; ++i) {
+                const int row = (t >> 4) + 4 * i;
+                const bf16* q = a.qkv + (size_t)min(row0 + row % kBlockPositions, a.rows - 1) * a.qkv_stride + (size_t)(kvh * 2 + row / kBlockPositions) * kHd;
+                copy16(smem_addr(queries) + tile_offset(kRows, row, piece), q + 8 * piece);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    // the queries: row 32 head + position, as the K tiles
-    {
-        const uint32_t to = smem_addr(smem) + 4 * kTileBytes;
+        constexpr int kPages = kStepTokens / kPageTokens;
+        const bf16* pages[kPages];
+        auto look_up = [&](int step) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row = (tid >> 4) + 16 * i;
-            const bf16* q = a.qkv + (size_t)min(row0 + row % kBlockPositions, a.rows - 1) * a.qkv_stride
-                            + (size_t)(kvh * 2 + row / kBlockPositions) * kHd;
-            copy16(to + tile_offset(row, tid & 15), q + 8 * (tid & 15));
+            for (int page = 0; page < kPages; ++page) {
+                const int first = step * kStepTokens + page * kPageTokens;
+                pages[page] = first < length ? page_of(a, first, kvh, values) + piece * 8 : nullptr;
+            }
+        };
+        look_up(0);
+        for (int step = 0; step < steps; ++step) {
+            const int buffer = step % kBuffers;
+            if (step >= kBuffers && !__all_sync(0xffffffffu, guard.wait(&used[buffer], ((step / kBuffers) - 1) & 1))) break;
+            unsigned char* tile = tiles + (buffer * 2 + (values ? 1 : 0)) * kTileBytes;
+#pragma unroll
+            for (int page = 0; page < kPages; ++page) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int in_page = (t >> 4) + 4 * u;
+                    const uint32_t off = tile_offset(kStepTokens, page * kPageTokens + in_page, piece);
+                    if (step * kStepTokens + page * kPageTokens + in_page < length) {
+                        copy16(smem_addr(tile) + off, pages[page] + (size_t)in_page * kHd);
+                    } else {
+                        // past the end: the scores are masked, but 0 * (stale bits that decode as NaN) is not zero
+                        *reinterpret_cast<int4*>(tile + off) = make_int4(0, 0, 0, 0);
+                    }
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            look_up(step + 1);
+            if (step > 0) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&landed[(step - 1) % kBuffers]);
+            }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0 && *abort_flag == 0) tc::mbar_arrive(&landed[(steps - 1) % kBuffers]);
+    } else if (warp == kProductWarp) {
+        if (tc::elect_one()) {
+            // ---- products
+            const uint32_t scores_idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kStepTokens >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+            // B with its rows (dims) contiguous: bit 16
+            const uint32_t out_idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(kHd >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+            auto scores = [&](int step) {
+                const uint32_t q = tc::smem_u32(queries), k = tc::smem_u32(tiles + (step % kBuffers) * 2 * kTileBytes);
+#pragma unroll
+                for (int j = 0; j < kHd / 16; ++j) {
+                    umma_ss(tmem + kScores, tc::umma_desc(q + (j / 4) * kRows * 128 + 32 * (j % 4)),
+                            tc::umma_desc(k + (j / 4) * kStepTokens * 128 + 32 * (j % 4)), scores_idesc, j != 0 ? 1u : 0u);
+                }
+                tc::umma_commit(s_ready);
+                tc::umma_commit(&empty_k[step % kBuffers]);
+            };
+            bool ok = guard.wait(&full_k[0], 0);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (ok) scores(0);
+            for (int step = 0; step < steps && ok; ++step) {
+                if (step + 1 < steps) {
+                    ok = guard.wait(&full_k[(step + 1) % kBuffers], ((step + 1) / kBuffers) & 1) && guard.wait(s_free, step & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    scores(step + 1);
+                }
+                ok = guard.wait(&full_v[step % kBuffers], (step / kBuffers) & 1) && guard.wait(p_ready, step & 1);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t v = tc::smem_u32(tiles + (step % kBuffers) * 2 * kTileBytes + kTileBytes);
+#pragma unroll
+                for (int j = 0; j < kStepTokens / 16; ++j) {
+                    const uint64_t tokens = desc_rows_contiguous(v + j * 16 * 128);
+                    tc::umma_f16_ts(tmem + kOut, tmem + kHi + 8 * j, tokens, out_idesc, (step | j) != 0 ? 1u : 0u);
+                    tc::umma_f16_ts(tmem + kOut, tmem + kLo + 8 * j, tokens, out_idesc, 1u);
+                }
+                tc::umma_commit(&empty_v[step % kBuffers]);
+                tc::umma_commit(o_ready);
+            }
+        }
+    } else {
+        // ---- softmax: two threads a row, each half of a step's tokens
+        const int half = warp >> 2, quarter = warp & 3;
+        const int row = quarter * kWarp + lane;
+        const int position = row % kBlockPositions;
+        const int last = a.base + row0 + position;            // the newest token that the row sees
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * kWarp) << 16);
+        // scores are kept in units of log2(e) / sqrt(128), so that exp is one exp2
+        const float scale = rsqrtf(static_cast<float>(kHd)) * 1.4426950408889634f;
+        auto meet = [&]() {                                   // the two warps of these rows
+            __syncwarp();
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
+        };
+        float m = -INFINITY, l = 0.0f;                        // of both; of this half
+        for (int step = 0; step < steps; ++step) {
+            guard.wait(s_ready, step & 1);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float sc[kHalf];
+            tc::tmem_load_row<kHalf>(lanes + kScores + half * kHalf, sc);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(s_free);
+            const int t0 = step * kStepTokens + half * kHalf;
+            if (t0 + kHalf - 1 > a.base + row0 + (quarter & 1) * kWarp) {          // some row of the warp ends in this half
+#pragma unroll
+                for (int j = 0; j < kHalf; ++j)
+                    if (t0 + j > last) sc[j] = -INFINITY;
+            }
+            float mx[4] = {sc[0], sc[1], sc[2], sc[3]};
+#pragma unroll
+            for (int j = 4; j < kHalf; ++j) mx[j & 3] = fmaxf(mx[j & 3], sc[j]);
+            float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale;
+            float* const at = tops + (step & 1) * 2 * kRows + row;
+            at[half * kRows] = top;
+            meet();
+            top = fmaxf(top, at[(half ^ 1) * kRows]);
+            const float moved = step == 0 || top > m + kSlack ? top : m;
+            const bool rescale = __any_sync(0xffffffffu, moved != m) && step > 0;
+            const float f = moved == m ? 1.0f : (step == 0 ? 0.0f : exp2_ftz(m - moved));
+            m = moved;
+            // (nothing but -inf so far: weights of zero)
+            const float reference = m == -INFINITY ? 0.0f : m;
+            float sums[4] = {l * f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int j = 0; j < kHalf; ++j) {
+                sc[j] = exp2_ftz(fmaf(sc[j], scale, -reference));
+                sums[j & 3] += sc[j];
+            }
+            l = (sums[0] + sums[1]) + (sums[2] + sums[3]);
+            uint32_t hi[kHalf / 2], lo[kHalf / 2];
+#pragma unroll
+            for (int j = 0; j < kHalf / 2; ++j) {
+                const float p0 = sc[2 * j], p1 = sc[2 * j + 1];
+                hi[j] = pack_pair(p0, p1);
+                lo[j] = pack_pair(p0 - __uint_as_float(hi[j] << 16), p1 - __uint_as_float(hi[j] & 0xffff0000u));
+            }
+            // what the step before has left in tensor memory is being multiplied up to here
+            if (step > 0) guard.wait(o_ready, (step - 1) & 1);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (rescale) {
+#pragma unroll 1
+                for (int c = half * (kHd / 2); c < (half + 1) * (kHd / 2); c += 16) {
+                    float o[16];
+                    uint32_t bits[16];
+                    tc::tmem_load_row<16>(lanes + kOut + c, o);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) bits[j] = __float_as_uint(o[j] * f);
+                    tmem_store_16(lanes + kOut + c, bits);
+                }
+            }
+            tmem_store_16(lanes + kHi + 16 * half, hi);
+            tmem_store_16(lanes + kLo + 16 * half, lo);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(p_ready);
+        }
+        float* const sum_at = tops + (steps & 1) * 2 * kRows + row;
+        sum_at[half * kRows] = l;
+        meet();
+        const float inv = 1.0f / (tops[(steps & 1) * 2 * kRows + row] + tops[(steps & 1) * 2 * kRows + kRows + row]);
+        guard.wait(o_ready, (steps - 1) & 1);
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        bf16* dst = a.out + (size_t)(row0 + position) * a.q_heads * kHd + (size_t)(kvh * 2 + row / kBlockPositions) * kHd;
+#pragma unroll 1
+        for (int c = half * (kHd / 2); c < (half + 1) * (kHd / 2); c += 16) {
+            float o[16];
+            tc::tmem_load_row<16>(lanes + kOut + c, o);
+            if (row0 + position < a.rows && *abort_flag == 0) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 8) {
+                    int4 v;
+                    v.x = (int)pack_pair(o[j] * inv, o[j + 1] * inv);
+                    v.y = (int)pack_pair(o[j + 2] * inv, o[j + 3] * inv);
+                    v.z = (int)pack_pair(o[j + 4] * inv, o[j + 5] * inv);
+                    v.w = (int)pack_pair(o[j + 6] * inv, o[j + 7] * inv);
+                    *reinterpret_cast<int4*>(dst + c + j) = v;
+                }
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
-    load_step(0, 0);
-
-    float o[16][4];
-#pragma unroll
-    for (int n = 0; n < 16; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[n][e] = 0.0f;
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
-    // scores are kept in units of log2(e) / sqrt(128), so that exp is one exp2
-    const float scale = rsqrtf(static_cast<float>(kHd)) * 1.4426950408889634f;
-    const int last_lo = a.base + my_row + gid;            // the newest token each of the lane's two rows sees
-    const int last_hi = last_lo + 8;
-
-    for (int step = 0; step < steps; ++step) {
-        const int buffer = step & 1;
-        if (step + 1 < steps) {
-            load_step(step + 1, buffer ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const uint32_t kt = smem_addr(smem) + buffer * 2 * kTileBytes + group * kHalfTokens * 256;
-        const uint32_t vt = kt + kTileBytes;
-        const uint32_t qt = smem_addr(smem) + 4 * kTileBytes;
-        const int t0 = step * kStepTokens + group * kHalfTokens;
-        // ---- scores of 16 rows x 32 tokens
-        float s[4][4];
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s[n][e] = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            // matrices: rows 16 warp .. + 7 and + 8 .. + 15, dims 16 k .. + 7, then dims 16 k + 8 .. + 15
-            uint32_t qa[4];
-            ldmatrix_x4(qt + tile_offset(16 * warp + (lane & 15), 2 * k + (lane >> 4)), qa);
-#pragma unroll
-            for (int n2 = 0; n2 < 2; ++n2) {
-                // matrices: tokens 16 n2 .. + 7 and + 8 .. + 15, dims 16 k .. + 7 and + 8 .. + 15
-                const int t = 16 * n2 + (lane & 7) + ((lane >> 4) << 3);
-                const int piece = 2 * k + ((lane >> 3) & 1);
-                uint32_t b[4];
-                ldmatrix_x4(kt + tile_offset(t, piece), b);
-                mma_16816(s[2 * n2], qa, b[0], b[1]);
-                mma_16816(s[2 * n2 + 1], qa, b[2], b[3]);
-            }
-        }
-        // ---- running softmax
-        const bool masked = t0 + kHalfTokens - 1 > a.base + my_row;       // some row of the warp ends in this step
-        if (masked) {
-#pragma unroll
-            for (int n = 0; n < 4; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (t0 + 8 * n + 2 * tig + (e & 1) > (e < 2 ? last_lo : last_hi)) s[n][e] = -INFINITY;
-        }
-        float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-            mx[h] = fmaxf(m[h], mx[h] * scale);
-        }
-        if (__any_sync(0xffffffffu, mx[0] != m[0] || mx[1] != m[1])) {       // seldom, once the context is some steps long
-            float f[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                // a half whose tokens so far all lie past the row has no maximum yet, and zeros to scale
-                f[h] = m[h] == -INFINITY ? 0.0f : exp2_ftz(m[h] - mx[h]);
-                m[h] = mx[h];
-                l[h] *= f[h];
-            }
-#pragma unroll
-            for (int n = 0; n < 16; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) o[n][e] *= f[e >> 1];
-        }
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float pr = s[n][e] == -INFINITY ? 0.0f : exp2_ftz(fmaf(s[n][e], scale, -m[e >> 1]));
-                s[n][e] = pr;
-                l[e >> 1] += pr;
-            }
-        // ---- output: P (16 x 32) V (32 x 128), P as hi + lo
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float p0 = s[2 * k + (q >> 1)][2 * (q & 1)], p1 = s[2 * k + (q >> 1)][2 * (q & 1) + 1];
-                hi[q] = pack_pair(p0, p1);
-                lo[q] = pack_pair(p0 - __uint_as_float(hi[q] << 16), p1 - __uint_as_float(hi[q] & 0xffff0000u));
-            }
-#pragma unroll
-            for (int n2 = 0; n2 < 8; ++n2) {
-                // matrices: tokens 16 k .. + 7 and + 8 .. + 15, dims 16 n2 .. + 7 and + 8 .. + 15
-                const int t = 16 * k + (lane & 15);
-                const int piece = 2 * n2 + (lane >> 4);
-                uint32_t b[4];
-                ldmatrix_x4_trans(vt + tile_offset(t, piece), b);
-                mma_16816(o[2 * n2], hi, b[0], b[1]);
-                mma_16816(o[2 * n2], lo, b[0], b[1]);
-                mma_16816(o[2 * n2 + 1], hi, b[2], b[3]);
-                mma_16816(o[2 * n2 + 1], lo, b[2], b[3]);
-            }
-        }
-        __syncthreads();        // the buffer is refilled by the step after the next
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-    }
-    // ---- the two halves of every row meet: the second group's in shared memory (the last barrier of the loop has freed it)
-    float* meet = reinterpret_cast<float*>(smem) + (warp * kWarp + lane);
-    constexpr int kPlane = 4 * kWarp;                     // one value of every thread of a group
-    if (group == 1) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            meet[h * kPlane] = m[h];
-            meet[(2 + h) * kPlane] = l[h];
-        }
-#pragma unroll
-        for (int n = 0; n < 16; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) meet[(4 + 4 * n + e) * kPlane] = o[n][e];
-    }
+    __syncwarp();
     __syncthreads();
-    if (group == 1) return;
-    float inv[2], f1[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        // token 0 is visible to every row: the first group's maximum is finite
-        const float m1 = meet[h * kPlane];
-        const float top = fmaxf(m[h], m1);
-        const float f0 = exp2_ftz(m[h] - top);
-        f1[h] = exp2_ftz(m1 - top);
-        inv[h] = 1.0f / (l[h] * f0 + meet[(2 + h) * kPlane] * f1[h]);
-        f1[h] *= inv[h];
-        inv[h] *= f0;
+    if (*abort_flag != 0 && tid == 0) {
+        atomicAdd(&g_prompt_attention_errors, 1u);
+        if (g_prompt_attention_error_sink != nullptr) atomicAdd_system(g_prompt_attention_error_sink, 1u);
+        const unsigned long long until = tc::now_ns() + 200000ull;       // products that are still under way
+        while (tc::now_ns() < until) __nanosleep(1000);
     }
-#pragma unroll
-    for (int n = 0; n < 16; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[n][e] = fmaf(meet[(4 + 4 * n + e) * kPlane], f1[e >> 1], o[n][e] * inv[e >> 1]);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int row = my_row + gid + 8 * h;
-        if (row < a.rows) {
-            bf16* dst = a.out + (size_t)row * a.q_heads * kHd + (size_t)head * kHd + 2 * tig;
-#pragma unroll
-            for (int n = 0; n < 16; ++n) {
-                *reinterpret_cast<uint32_t*>(dst + 8 * n) = pack_pair(o[n][2 * h], o[n][2 * h + 1]);
-            }
-        }
+    if (*abort_flag != 0) __syncthreads();
+    if (warp == kProductWarp) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
 }
 
@@ -407,6 +484,16 @@ cudaError_t launch_prompt_attention(const AttentionArgs& a, int base, cudaStream
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((a.rows + kBlockPositions - 1) / kBlockPositions * a.kv_heads));
     return launch_pdl(prompt_attention_kernel, grid, dim3(kFlashThreads), kFlashSmem, stream, p);
+}
+
+unsigned int prompt_attention_error_count() {
+    unsigned int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_prompt_attention_errors, sizeof(v)) != cudaSuccess) return ~0u;
+    return v;
+}
+
+cudaError_t set_prompt_attention_error_sink(unsigned int* device_visible_word) {
+    return cudaMemcpyToSymbol(g_prompt_attention_error_sink, &device_visible_word, sizeof(device_visible_word));
 }
 
 }  // namespace q3t

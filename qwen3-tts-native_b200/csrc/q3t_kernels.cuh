@@ -221,6 +221,7 @@ cudaError_t launch_attention(const AttentionArgs& args, cudaStream_t stream);
 bool prompt_attention_supports(const AttentionArgs& args);
 cudaError_t launch_prompt_attention(const AttentionArgs& args, int base, cudaStream_t stream);
 cudaError_t configure_prompt_kernels();
+unsigned int prompt_attention_error_count();
 // cos/sin of every (position, rotary pair), rounded to bf16 as the fused prologue rounds them;
 // computed by the same device expressions, so using the table changes no bit
 cudaError_t launch_build_rope_table(uint32_t* table, int positions, int head_dim, float theta,
