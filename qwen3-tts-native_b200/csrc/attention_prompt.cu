@@ -380,20 +380,26 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
             m = moved;
             // (nothing but -inf so far: weights of zero)
             const float reference = m == -INFINITY ? 0.0f : m;
-            float sums[4] = {l * f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int j = 0; j < kHalf; ++j) {
-                sc[j] = exp2_ftz(fmaf(sc[j], scale, -reference));
-                sums[j & 3] += sc[j];
-            }
-            l = (sums[0] + sums[1]) + (sums[2] + sums[3]);
+            // (pairs of ordinary operations: this part is bound by the issue of its instructions)
+            const unsigned long long scale2 = pack2(scale, scale), minus2 = pack2(-reference, -reference), negative2 = pack2(-1.0f, -1.0f);
+            unsigned long long sums[2] = {pack2(l * f, 0.0f), pack2(0.0f, 0.0f)};
             uint32_t hi[kHalf / 2], lo[kHalf / 2];
 #pragma unroll
             for (int j = 0; j < kHalf / 2; ++j) {
-                const float p0 = sc[2 * j], p1 = sc[2 * j + 1];
+                float p0, p1, rest0, rest1;
+                unpack2(fma2(pack2(sc[2 * j], sc[2 * j + 1]), scale2, minus2), p0, p1);
+                p0 = exp2_ftz(p0);
+                p1 = exp2_ftz(p1);
+                const unsigned long long weights = pack2(p0, p1);
+                sums[j & 1] = add2(sums[j & 1], weights);
                 hi[j] = pack_pair(p0, p1);
-                lo[j] = pack_pair(p0 - __uint_as_float(hi[j] << 16), p1 - __uint_as_float(hi[j] & 0xffff0000u));
+                unpack2(fma2(pack2(bf_lo(hi[j]), bf_hi(hi[j])), negative2, weights), rest0, rest1);       // exact
+                lo[j] = pack_pair(rest0, rest1);
             }
+            float s0, s1, s2, s3;
+            unpack2(sums[0], s0, s1);
+            unpack2(sums[1], s2, s3);
+            l = (s0 + s1) + (s2 + s3);
             // what the step before has left in tensor memory is being multiplied up to here
             if (step > 0) guard.wait(o_ready, (step - 1) & 1);
             __syncwarp();

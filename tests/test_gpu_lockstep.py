@@ -1,5 +1,5 @@
-"""The lockstep chain (the predictor's positions of 9 to 64 sessions, a cooperative launch each) against the frame made
-launch by launch: the same sums in the same order, so the same bits."""
+"""The lockstep chain (the predictor's part of 9 to 64 sessions in one cooperative launch) against the frame made launch by
+launch: the same sums in the same order, so the same bits."""
 import numpy as np
 import pytest
 
@@ -46,11 +46,22 @@ def test_lockstep_chain_equals_launch_by_launch(q3t, model, rows):
     assert q3t.library().q3t_kernel_error_count() == 0
 
 
-def test_every_draw(q3t, model):
-    """Draws that differ between the rows of a frame: greedy, a few, many, all of the vocabulary."""
-    kinds = [q3t.SamplingConfig.greedy(), q3t.SamplingConfig(True, 1, 1.0, 0.9, 1.0), q3t.SamplingConfig(True, 128, 0.8, 1.1, 1.0),
-             q3t.SamplingConfig(True, 300, 0.9, 1.0, 1.0), q3t.SamplingConfig(True, 0, 1.0, 1.0, 1.0)]
+@pytest.mark.parametrize("inside", [True, False])
+def test_every_draw(q3t, model, inside):
+    """Draws that differ between the rows of a frame: greedy, a few and many, which the chain makes itself, and more than it
+    ranks, with which the sampler runs between its positions."""
+    kinds = [q3t.SamplingConfig.greedy(), q3t.SamplingConfig(True, 1, 1.0, 0.9, 1.0), q3t.SamplingConfig(True, 128, 0.8, 1.1, 1.0)]
+    if not inside:
+        kinds += [q3t.SamplingConfig(True, 300, 0.9, 1.0, 1.0), q3t.SamplingConfig(True, 0, 1.0, 1.0, 1.0)]
     pick = lambda i: kinds[i % len(kinds)]
     chained, launched = frames(q3t, model, 20, 1, 2, pick), frames(q3t, model, 20, 0, 2, pick)
     assert chained[0] == launched[0]
     assert all(np.array_equal(a[0], b[0]) and a[1] == b[1] for a, b in zip(chained[1], launched[1]))
+
+
+def test_row_counts_in_turn(q3t, model):
+    """The chain's places are marked for one row count: another count, and the first again, start with all of them marked."""
+    want = {n: frames(q3t, model, n, 0, 1)[0] for n in (12, 40, 9)}
+    for n in (12, 40, 9, 40, 12):
+        assert frames(q3t, model, n, 1, 1)[0] == want[n]
+    assert q3t.library().q3t_kernel_error_count() == 0
