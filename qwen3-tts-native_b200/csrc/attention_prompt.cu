@@ -99,9 +99,10 @@ __global__ void __launch_bounds__(256) prompt_append_kernel(const PromptArgs a) 
     uint32_t cs[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) cs[j] = a.rope_table[(size_t)pos * (kHd / 2) + lane + 32 * j];
+    // where the position lies in its page, of KV head 0: looked up ahead of the wait, two loads one behind the other
+    bf16* const place = page_of(a, pos, 0, false) + (size_t)(pos % kPageTokens) * kHd;
     pdl_wait();
     pdl_trigger();
-    const int t = pos % kPageTokens;
     // three heads a warp at a time (all of the talker's 16 + 8), requested together: one latency
     constexpr int kJobs = 3;
     const int total = a.q_heads + a.kv_heads;
@@ -144,8 +145,8 @@ __global__ void __launch_bounds__(256) prompt_append_kernel(const PromptArgs a) 
             }
             if (is_key) {
                 const int kvh = job - a.q_heads;
-                bf16* kdst = page_of(a, pos, kvh, false) + (size_t)t * kHd;
-                bf16* vdst = page_of(a, pos, kvh, true) + (size_t)t * kHd;
+                bf16* kdst = place + (size_t)kvh * (kPageTokens * kHd);
+                bf16* vdst = kdst + (a.kv.v_offset - a.kv.k_offset);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     kdst[lane + 32 * j] = f2bf(y[j]);
