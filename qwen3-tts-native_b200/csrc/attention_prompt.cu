@@ -9,8 +9,8 @@
 // common context once, 64 tokens at a time, with a running softmax.
 //
 //   scores    S = Q K^T, tcgen05.mma from shared memory into 64 columns of tensor memory
-//   softmax   two threads a row, half of the step's tokens each: S to registers (the next step's products may begin), weights as bf16 hi + lo (16 bits kept) back to
-//             tensor memory
+//   softmax   two threads a row, half of the step's tokens each: S to registers (the next step's products may begin), weights as
+//             bf16 hi + lo (16 bits kept) back to tensor memory
 //   output    O += P V, hi and lo as the A operand from tensor memory, V as it lies in its pages
 //   copies    K and V, by two warps each, two steps ahead of their products (cp.async: the pages lie anywhere)
 // A row's reference is its first maximum until a score exceeds it by 2^8: weights above one cost no precision in floating point,

@@ -16,8 +16,9 @@
 // this one's products (110 cycles an answer, three a step).
 //
 // Warp roles: 0 weight copies, 1 product issue (in the first CTA only), 2 activation copies, 3 tensor memory, then in the second CTA the
-// relay that tells the first one of activations that have landed; 4..19 in four groups dequantise, then read the accumulators.  A pair of CTAs stays for all of its tiles: weights and
-// activations of the next one are on their way while the last one's accumulators are read.  The two tiles of gate/up lie side by
+// relay that tells the first one of activations that have landed; 4..19 in four groups dequantise, then read the accumulators.
+// A pair of CTAs stays for all of its tiles: weights and activations of the next one are on their way while the last one's
+// accumulators are read.  The two tiles of gate/up lie side by
 // side in the lanes (64 channels each a CTA); the values that a channel's other lane finishes cross through
 // shared memory.  Every wait is bounded.
 
