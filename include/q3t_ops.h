@@ -81,6 +81,8 @@ QWEN3_TTS_API int32_t q3t_launch_int8_gemm_ex(const Q3tGemmDesc* desc, void* str
  * one or two tiles of channels a CTA; 3: the lockstep kernel with its row blocks side by side; 96, 128, 160: the same in
  * blocks of so many rows; 256: pairs of CTAs. */
 QWEN3_TTS_API int32_t q3t_test_prompt_gemm(const Q3tGemmDesc* desc, int32_t kernel, void* stream);
+/* Test hook: which of these a prompt takes; launches nothing.  Negative: not a projection. */
+QWEN3_TTS_API int32_t q3t_test_prompt_gemm_kernel(const Q3tGemmDesc* desc);
 
 /* launch_quantize_weight_rows (int8_gemv.cu:302-317) */
 QWEN3_TTS_API int32_t q3t_launch_quantize_weight_rows(const uint16_t* weight, int8_t* quantized,

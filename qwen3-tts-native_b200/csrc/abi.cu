@@ -657,6 +657,11 @@ int32_t q3t_test_prompt_gemm(const Q3tGemmDesc* d, int32_t kernel, void* stream)
     return static_cast<int32_t>(launch_int8_gemm_wide(a, S(stream), kernel));
 }
 
+int32_t q3t_test_prompt_gemm_kernel(const Q3tGemmDesc* d) {
+    GemvArgs a;
+    return gemm_args(d, a) != 0 ? -1 : gemm_prompt_kernel(a);
+}
+
 int32_t q3t_launch_quantize_weight_rows(const uint16_t* weight, int8_t* quantized, float* scales,
                                         int32_t in_features, int32_t out_features, void* stream) {
     return static_cast<int32_t>(launch_quantize_weight_rows(B(weight), quantized, scales, in_features,

@@ -389,7 +389,7 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
 }
 
 // Which kernel takes a projection of a prompt pass: the one with the shortest estimate.  A wave of CTAs of this
-// file's kernel costs its steps (0.46 us each with one channel tile, 0.63 us with two) and 5 to 7 us of start and epilogue;
+// file's kernel costs its steps (0.46 us each with one channel tile, 0.63 us with two) and 5 to 9 us of start and epilogue;
 // the kernel of gemm_int8_tc.cu, in blocks of up to 64 rows or of 96, 128 or 160 side by side and with K split where that fits
 // one wave, and the one of gemm_int8_pair.cu are estimated there.  Above 640 rows tc's never has fewer waves.  Measured there (us, one tile /
 // two tiles / pairs): 700 rows q/k/v 20.8 / 17.2 / 15.2, o 13.2 / 17.6 / 13.7, gate/up 53.6 / 34.9 / 34.2, down 28.4 / 38.1 / 25.7;
@@ -398,7 +398,37 @@ cudaError_t launch_int8_gemm_wide(const GemvArgs& a, cudaStream_t stream, int ch
 // 19.0 / 12.5 / 14.8 / 17.2, 128 21.1 / 14.7 / 15.6 / 18.0, 150 22.3 / 16.3 / 27.3 / 18.6, 300 41.5 / 27.2 / 29.6 / 19.8, 448
 // 53.7 / 31.3 / 43.2 / 36.8; q/k/v 128 8.3 / 9.0 / 11.6 / 18.2, 300 20.8 / 11.3 / 12.5 / 18.2, 512 23.2 / 15.0 / 13.1 / 18.6;
 // down 128 10.6 / 10.8 / 28.2 / 44.3, 300 25.4 / 14.5 / 28.7 / 45.0, 640 49.7 / 20.2 / 29.9 / 44.9; o 150 8.3 / 7.8 / 12.6 /
-// 19.9, 300 12.6 / 10.0 / 12.7 / 19.9.
+// 19.9, 300 12.6 / 10.0 / 12.7 / 19.9.  Gate/up again, out of more weights than the L2 holds (best tall tile / one tile / pairs): 65 rows
+// 11.8 / 13.5 / 13.0, 96 12.5 / 13.8 / 13.1, 112 13.5 / 14.3 / 13.2, 128 14.1 / 14.3 / 13.3, 150 15.5 / 24.8 / 15.6.  One tile's
+// estimate errs on the same side as theirs, by 0.5 to 1.3 us (without the 2.6 us it took 65 to 128 rows, a prompt of 65 1,575 us for 1,505).
+int gemm_prompt_kernel(const GemvArgs& a) {
+    const int per_single = a.epilogue == EPI_GATE_UP_SILU ? 64 : kTileN;
+    const int row_blocks = (a.rows + kTileM - 1) / kTileM, steps = a.in_features / kBK;
+    auto waves = [&](int tiles) {
+        return ((a.out_features + tiles * per_single - 1) / (tiles * per_single) * row_blocks + kSms - 1) / kSms;
+    };
+    const bool adds = a.epilogue == EPI_ADD || a.epilogue == EPI_BIAS_ADD;         // another read of the rows
+    const bool crosses = a.epilogue == EPI_GATE_UP_SILU;                           // the up half, through shared memory
+    const float one = waves(1) * (4.9f + (adds ? 1.5f : 0.0f) + (crosses ? 2.6f : 0.0f) + 0.456f * steps);
+    const float two = waves(2) * (7.2f + (adds ? 2.0f : 0.0f) + 0.63f * steps);
+    int kernel = one <= two ? 1 : 2;
+    float best = one < two ? one : two;
+    const float pairs = gemm_pair_estimate_us(a);
+    if (pairs < best) {
+        best = pairs;
+        kernel = 256;
+    }
+    for (int t : {0, 96, 128, 160}) {
+        if (t > 0 && a.rows > kTallRowsMost) break;
+        const float estimate = gemm_tc_estimate_us(a, t);
+        if (estimate <= best) {
+            best = estimate;
+            kernel = t > 0 ? t : 3;
+        }
+    }
+    return kernel;
+}
+
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
     GemvArgs a = args;
     if (a.norm_w != nullptr) {
@@ -409,29 +439,9 @@ cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream) {
         a.norm_w = nullptr;
         a.norm_out = nullptr;
     }
-    const int per_single = a.epilogue == EPI_GATE_UP_SILU ? 64 : kTileN;
-    const int row_blocks = (a.rows + kTileM - 1) / kTileM, steps = a.in_features / kBK;
-    auto waves = [&](int tiles) {
-        return ((a.out_features + tiles * per_single - 1) / (tiles * per_single) * row_blocks + kSms - 1) / kSms;
-    };
-    const bool adds = a.epilogue == EPI_ADD || a.epilogue == EPI_BIAS_ADD;         // another read of the rows
-    const float one = waves(1) * (4.9f + (adds ? 1.5f : 0.0f) + 0.456f * steps);
-    const float two = waves(2) * (7.2f + (adds ? 2.0f : 0.0f) + 0.63f * steps);
-    const float pairs = gemm_pair_estimate_us(a);
-    float best = one < two ? one : two;
-    const bool paired = pairs < best;
-    if (paired) best = pairs;
-    int tile = -1;
-    for (int t : {0, 96, 128, 160}) {
-        if (t > 0 && a.rows > kTallRowsMost) break;
-        const float estimate = gemm_tc_estimate_us(a, t);
-        if (estimate <= best) {
-            best = estimate;
-            tile = t;
-        }
-    }
-    if (tile >= 0) return launch_int8_gemm_tc(a, stream, tile);
-    return paired ? launch_int8_gemm_pair(a, stream) : launch_int8_gemm_wide(a, stream, one <= two ? 1 : 2);
+    const int kernel = gemm_prompt_kernel(a);
+    if (kernel == 256) return launch_int8_gemm_pair(a, stream);
+    return kernel < 3 ? launch_int8_gemm_wide(a, stream, kernel) : launch_int8_gemm_tc(a, stream, kernel == 3 ? 0 : kernel);
 }
 
 unsigned int gemm_wide_error_count() {

@@ -109,6 +109,8 @@ cudaError_t configure_pair_kernels();
 unsigned int gemm_pair_error_count();
 // projections of a prompt pass of more than kMaxRows rows (needs norm_out when norm_w is given)
 cudaError_t launch_int8_gemm_prompt(const GemvArgs& args, cudaStream_t stream);
+// the kernel that takes one: 1 or 2 (channel tiles, gemm_int8_wide.cu), 256 (pairs), 3 (blocks of up to 64 rows), 96, 128, 160 (tall ones)
+int gemm_prompt_kernel(const GemvArgs& args);
 unsigned int gemm_wide_error_count();
 
 cudaError_t launch_quantize_weight_rows(const bf16* weight, int8_t* quantized, float* scales,

@@ -5,6 +5,8 @@ the SIMT kernels and from the reference: the checks are the north-star tolerance
 before the final round within 1e-3 of fp64 truth, relative to |value| + the row's RMS) and bf16
 outputs within one rounding step of bf16(oracle).  Rows are independent in the reference kernel,
 so the oracle for more than 8 rows is the reference arithmetic applied row by row."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -199,6 +201,16 @@ def test_pairs_of_several_tiles(q3t, orc, ops, n, k, rows, gate_up):
     args = dict(epilogue=ops.EPI_GATE_UP_SILU) if gate_up else dict(epilogue=ops.EPI_ADD, y_in=base)
     assert np.array_equal(ops.int8_gemm(w, s, x, prompt_kernel=256, **args)["y"], ops.int8_gemm(w, s, x, prompt_kernel=1, **args)["y"])
     assert q3t.library().q3t_kernel_error_count() == 0
+
+
+@pytest.mark.parametrize("rows,kernels", [(65, (96,)), (96, (96,)), (97, (128, 256)), (128, (128, 256))])
+def test_gate_up_of_short_prompts(q3t, ops, rows, kernels):
+    """The talker's gate/up of 65 to 128 rows goes to a kernel that was measured the shortest there or within 0.8 us of it, not to
+    one tile a CTA (1.7 us longer than the tall tiles at 65 rows); the bits are the same, so they do not tell."""
+    d = ops.GemmDescC()
+    d.struct_size = C.sizeof(d)
+    d.epilogue, d.in_features, d.out_features, d.rows = ops.EPI_GATE_UP_SILU, 2048, 6144, rows
+    assert q3t.library().q3t_test_prompt_gemm_kernel(C.byref(d)) in kernels
 
 
 @pytest.mark.parametrize("n,k,rows,gate_up", [(2048, 6144, 700, False), (4096, 2048, 1200, False), (2048, 2048, 2048, False), (6144, 2048, 600, True)])
