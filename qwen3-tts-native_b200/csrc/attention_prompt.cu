@@ -12,11 +12,16 @@
 //   softmax   two threads a row, half of the step's tokens each: S to registers (the next step's products may begin), weights as
 //             bf16 hi + lo (16 bits kept) back to tensor memory
 //   output    O += P V, hi and lo as the A operand from tensor memory, V as it lies in its pages
-//   copies    K and V, by two warps each, two steps ahead of their products (cp.async: the pages lie anywhere)
+//   copies    K and V, by two warps each, two steps ahead of their products (cp.async: the pages lie anywhere), the queries by the softmax's
 // A row's reference is its first maximum until a score exceeds it by 2^8: weights above one cost no precision in floating point,
 // and an output in tensor memory is rescaled at almost no step instead of almost every one (some row of 32 has a new maximum).
 //
-// What bounds it: the chain of a step in its softmax threads, times the steps of the longest context; two CTAs an SM take turns
+// Short passes are one or two steps a CTA, bound by the way of the first operands from the L2: the first pages are looked up ahead
+// of the launch's wait, the softmax warps bring the queries, and a CTA takes 32 positions (half of its rows idle) while twice as
+// many CTAs fit the SMs.  A prompt of 64 positions (us) 1,441 -> 1,406, 12 1,162 -> 1,151, 128 1,648 -> 1,628 (halves against whole
+// blocks: 64 1,431 -> 1,406, 128 1,646 -> 1,628); with mma.sync 1,412, 1,155 and 1,690.
+//
+// What bounds it else: the chain of a step in its softmax threads, times the steps of the longest context; two CTAs an SM take turns
 // at the issue slots.  1,500 positions: 68 us a layer with mma.sync (32 positions a CTA, the weights' two halves as 3 x 64 x 64 x 128
 // products a step at the legacy rate), 54 so with K and V in one buffer, 45 with a buffer each, 43 with two threads a row.
 
@@ -31,12 +36,16 @@ constexpr int kBlockPositions = 64;
 constexpr int kStepTokens = 64;
 constexpr int kRows = 2 * kBlockPositions;              // of the tensor cores: position + 64 * head
 constexpr int kFlashThreads = 416;                      // warps 0..7 softmax, 8..11 copies, 12 products
+// Registers: 72 a thread at launch (two CTAs an SM); the copying warps hand 16 each to the softmax's, which spill with 72
+constexpr int kLaunchRegisters = 72, kSoftmaxRegisters = 80, kCopyRegisters = 56;
+static_assert(2 * kSoftmaxRegisters + kCopyRegisters <= 3 * kLaunchRegisters, "registers of the three groups of four warps");
 constexpr int kCopyWarp = 8, kProductWarp = 12;
 constexpr int kHalf = kStepTokens / 2;                  // tokens of a step, to each of a row's two threads
 constexpr int kTileBytes = kStepTokens * kHd * 2;       // 16 KB of K or V: [64 dims][token][128 bytes, swizzled]
 constexpr int kQueryBytes = kRows * kHd * 2;
 constexpr int kBuffers = 2;
 constexpr int kFlashCtas = 2;
+constexpr int kSms = 148;
 constexpr uint32_t kTmemCols = 256, kScores = 0, kHi = 64, kLo = 96, kOut = 128;
 constexpr float kSlack = 8.0f;                          // log2 of the largest weight
 constexpr unsigned long long kBudgetNs = 2000000000ull;
@@ -187,6 +196,7 @@ __device__ __forceinline__ void tmem_store_16(uint32_t taddr, const uint32_t (&r
         : "memory");
 }
 
+template <int BLOCK>                                          // positions of a CTA: kBlockPositions, or half of them
 __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_kernel(const PromptArgs a) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -201,7 +211,8 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
     uint64_t* s_free = s_ready + 1;                           // and in registers
     uint64_t* p_ready = s_free + 1;                           // weights in tensor memory
     uint64_t* o_ready = p_ready + 1;                          // multiplied
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_ready + 1);
+    uint64_t* q_ready = o_ready + 1;                          // queries in shared memory
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_ready + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x;
@@ -210,8 +221,9 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
     // the last positions have the longest context: they go first, all KV heads of a block together
     const int kvh = (int)blockIdx.x % a.kv_heads;
     const int block = ((int)gridDim.x - 1 - (int)blockIdx.x) / a.kv_heads;
-    const int row0 = block * kBlockPositions;
-    const int length = a.base + min(a.rows, row0 + kBlockPositions);      // tokens the CTA walks
+    const int row0 = block * BLOCK;
+    const int rows_end = BLOCK == kBlockPositions ? a.rows : min(a.rows, row0 + BLOCK);
+    const int length = a.base + min(a.rows, row0 + BLOCK);      // tokens the CTA walks
     const int steps = (length + kStepTokens - 1) / kStepTokens;
 
     tc::Guard guard;
@@ -228,6 +240,7 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
         tc::mbar_init(s_free, 8);
         tc::mbar_init(p_ready, 8);
         tc::mbar_init(o_ready, 1);
+        tc::mbar_init(q_ready, 8);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -239,49 +252,44 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    pdl_wait();
-    pdl_trigger();
 
     if (warp >= kCopyWarp && warp < kProductWarp) {
-        // ---- copies: K by the first two warps, behind the queries, V by the others; thread t takes piece t % 16 of tokens t / 16,
-        // + 4, + 8, + 12 of every page.  Pages are looked up a step ahead.
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCopyRegisters));
+        // ---- copies: K by the first two warps, V by the others; thread t takes piece t % 16 of tokens t / 16, + 4, + 8, + 12 of every
+        // page.  Pages are looked up a step ahead, two loads one behind the other; the first step's ahead of the launch's wait, since the
+        // page table is older than the launch before.
         const bool values = warp >= kCopyWarp + 2;
         const int t = (tid - kCopyWarp * kWarp) % (2 * kWarp), piece = t & 15;
         uint64_t* const landed = values ? full_v : full_k;
         uint64_t* const used = values ? empty_v : empty_k;
-        if (!values) {
-#pragma unroll
-            for (int i = 0; i < kRows / 4; ++i) {
-                const int row = (t >> 4) + 4 * i;
-                const bf16* q = a.qkv + (size_t)min(row0 + row % kBlockPositions, a.rows - 1) * a.qkv_stride + (size_t)(kvh * 2 + row / kBlockPositions) * kHd;
-                copy16(smem_addr(queries) + tile_offset(kRows, row, piece), q + 8 * piece);
-            }
-        }
         constexpr int kPages = kStepTokens / kPageTokens;
         const bf16* pages[kPages];
         auto look_up = [&](int step) {
 #pragma unroll
             for (int page = 0; page < kPages; ++page) {
                 const int first = step * kStepTokens + page * kPageTokens;
-                pages[page] = first < length ? page_of(a, first, kvh, values) + piece * 8 : nullptr;
+                pages[page] = first < length ? page_of(a, first, kvh, values) + (t >> 4) * kHd + piece * 8 : nullptr;
             }
         };
+        const uint32_t at = tile_offset(kStepTokens, t >> 4, piece);
         look_up(0);
+        pdl_wait();
+        pdl_trigger();
         for (int step = 0; step < steps; ++step) {
             const int buffer = step % kBuffers;
             if (step >= kBuffers && !__all_sync(0xffffffffu, guard.wait(&used[buffer], ((step / kBuffers) - 1) & 1))) break;
-            unsigned char* tile = tiles + (buffer * 2 + (values ? 1 : 0)) * kTileBytes;
+            unsigned char* const tile = tiles + (buffer * 2 + (values ? 1 : 0)) * kTileBytes;
 #pragma unroll
             for (int page = 0; page < kPages; ++page) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const int in_page = (t >> 4) + 4 * u;
-                    const uint32_t off = tile_offset(kStepTokens, page * kPageTokens + in_page, piece);
-                    if (step * kStepTokens + page * kPageTokens + in_page < length) {
-                        copy16(smem_addr(tile) + off, pages[page] + (size_t)in_page * kHd);
+                    // (four tokens further on: another swizzle of the 16-byte pieces)
+                    unsigned char* const to = tile + (at ^ ((u & 1) * 64)) + (page * kPageTokens + 4 * u) * 128;
+                    if (step * kStepTokens + page * kPageTokens + 4 * u + (t >> 4) < length) {
+                        copy16(smem_addr(to), pages[page] + 4 * u * kHd);
                     } else {
                         // past the end: the scores are masked, but 0 * (stale bits that decode as NaN) is not zero
-                        *reinterpret_cast<int4*>(tile + off) = make_int4(0, 0, 0, 0);
+                        *reinterpret_cast<int4*>(to) = make_int4(0, 0, 0, 0);
                     }
                 }
             }
@@ -314,7 +322,7 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
                 tc::umma_commit(s_ready);
                 tc::umma_commit(&empty_k[step % kBuffers]);
             };
-            bool ok = guard.wait(&full_k[0], 0);
+            bool ok = guard.wait(q_ready, 0) && guard.wait(&full_k[0], 0);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (ok) scores(0);
             for (int step = 0; step < steps && ok; ++step) {
@@ -339,7 +347,19 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
             }
         }
     } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegisters));
         // ---- softmax: two threads a row, each half of a step's tokens
+        pdl_wait();
+#pragma unroll
+        for (int i = 0; i < kRows * kHd / 8 / 256; ++i) {
+            const int q_row = (tid >> 4) + 16 * i, q_piece = tid & 15;
+            const bf16* q = a.qkv + (size_t)min(row0 + q_row % kBlockPositions, rows_end - 1) * a.qkv_stride + (size_t)(kvh * 2 + q_row / kBlockPositions) * kHd;
+            copy16(smem_addr(queries) + tile_offset(kRows, q_row, q_piece), q + 8 * q_piece);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(q_ready);
         const int half = warp >> 2, quarter = warp & 3;
         const int row = quarter * kWarp + lane;
         const int position = row % kBlockPositions;
@@ -435,7 +455,7 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
         for (int c = half * (kHd / 2); c < (half + 1) * (kHd / 2); c += 16) {
             float o[16];
             tc::tmem_load_row<16>(lanes + kOut + c, o);
-            if (row0 + position < a.rows && *abort_flag == 0) {
+            if (row0 + position < rows_end && *abort_flag == 0) {
 #pragma unroll
                 for (int j = 0; j < 16; j += 8) {
                     int4 v;
@@ -466,8 +486,19 @@ __global__ void __launch_bounds__(kFlashThreads, kFlashCtas) prompt_attention_ke
 
 }  // namespace
 
+namespace {
+template <int BLOCK>
+cudaError_t configure_block() {
+    cudaFuncAttributes built;
+    cudaError_t e = cudaFuncGetAttributes(&built, prompt_attention_kernel<BLOCK>);
+    if (e == cudaSuccess && built.numRegs < kLaunchRegisters) e = cudaErrorInvalidConfiguration;     // what setmaxnreg hands out has to be there
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(prompt_attention_kernel<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlashSmem);
+}
+}  // namespace
+
 cudaError_t configure_prompt_kernels() {
-    return cudaFuncSetAttribute(prompt_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlashSmem);
+    const cudaError_t e = configure_block<kBlockPositions>();
+    return e != cudaSuccess ? e : configure_block<kBlockPositions / 2>();
 }
 
 bool prompt_attention_supports(const AttentionArgs& a) {
@@ -489,8 +520,12 @@ cudaError_t launch_prompt_attention(const AttentionArgs& a, int base, cudaStream
     p.q_heads = a.q_heads; p.kv_heads = a.kv_heads; p.eps = a.eps;
     const cudaError_t e = launch_pdl(prompt_append_kernel, dim3((unsigned)a.rows), dim3(256), 0, stream, p);
     if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)((a.rows + kBlockPositions - 1) / kBlockPositions * a.kv_heads));
-    return launch_pdl(prompt_attention_kernel, grid, dim3(kFlashThreads), kFlashSmem, stream, p);
+    // twice as many CTAs of half as many positions, while each has an SM of its own (two on an SM as well: a prompt of 700 positions
+    // the same, of 900 0.9 % longer)
+    const bool halves = a.rows > kBlockPositions / 2 && (a.rows + kBlockPositions - 1) / kBlockPositions * a.kv_heads * 2 <= kSms;
+    const int block = halves ? kBlockPositions / 2 : kBlockPositions;
+    const dim3 grid((unsigned)((a.rows + block - 1) / block * a.kv_heads));
+    return launch_pdl(halves ? prompt_attention_kernel<kBlockPositions / 2> : prompt_attention_kernel<kBlockPositions>, grid, dim3(kFlashThreads), kFlashSmem, stream, p);
 }
 
 unsigned int prompt_attention_error_count() {

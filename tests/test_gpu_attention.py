@@ -308,12 +308,14 @@ def test_scores_of_minus_infinity(orc, ops, length, masked):
     check(orc, got["out"], got["f32"], want, want32, hd)
 
 
-@pytest.mark.parametrize("base,rows", [(0, 9), (0, 32), (0, 33), (0, 64), (0, 97), (31, 40), (64, 65), (100, 70), (250, 129)])
-def test_prompt_attention(orc, ops, base, rows):
+@pytest.mark.parametrize("base,rows,kvh", [(0, 9, 8), (0, 32, 8), (0, 33, 8), (0, 64, 8), (0, 97, 8), (31, 40, 8), (64, 65, 8), (100, 70, 8), (250, 129, 8),
+                                           (3, 31, 8), (17, 128, 37), (0, 65, 38), (40, 129, 38), (70, 64, 75), (0, 63, 74)])
+def test_prompt_attention(orc, ops, base, rows, kvh):
     """Consecutive positions of one session that share their walk over the cache, against the oracle row by row: first and
-    later passes, at the edges of pages, of blocks of 32 positions and of steps of 64 tokens; places behind the last position
-    hold NaN, so that a token let through the mask would show."""
-    qh, kvh, hd = 16, 8, 128
+    later passes, at the edges of pages, of blocks of 32 positions (33 and more, while twice 64 positions' CTAs fit 148 SMs) and of
+    64 (up to 32, and with enough KV heads), and of steps of 64 tokens; places behind the last position hold NaN, so that a token let
+    through the mask would show."""
+    qh, hd = 2 * kvh, 128
     qw, kvw = qh * hd, kvh * hd
     end = base + rows
     cap = (end + 15) // 16 * 16 + 16
