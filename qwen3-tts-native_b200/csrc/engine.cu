@@ -1545,7 +1545,7 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
         }
         if (lockstep != Lockstep::kNone && (w.lockstep_rows != n || w.lockstep_errors != m.device_errors())) {
             w.lockstep_errors = m.device_errors();
-            check_cuda(restart_lockstep(w.lockstep_exchange.as<void>(), w.stream), "lockstep exchange");
+            check_cuda(restart_lockstep(w.lockstep_exchange.as<void>(), n, w.stream), "lockstep exchange");
             w.lockstep_rows = n;
         }
         check_cuda(cudaEventRecord(w.predictor_start, w.stream), "cudaEventRecord");

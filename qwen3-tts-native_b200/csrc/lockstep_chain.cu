@@ -19,10 +19,10 @@
 //   16 of 64 channels, whose finishing threads keep the residual stream in registers; head 16 of 128.
 //   norms: a CTA per row; attention: a warp per (row, KV head), one page of 16 tokens; draws: a CTA per row.
 //
-// Hand-overs.  A reader polls the values themselves: 16 bytes that are no longer the mark (bf16 pairs of all ones, which no
-// rounding yields) have been written, since 16-byte accesses are single.  No fence, no counter, no flag to unpack: with
-// counters and bulk copies a hand-over took 3,700 cycles, so 1,600 to 2,000; with words of six values and a number 5,000, most of
-// it unpacking.  Each kind of value has three buffers that take turns.  Whoever has published use u of a kind marks its own
+// Hand-overs.  A reader polls the values themselves: a word of two bf16 that is no longer the mark (all ones, which no rounding
+// yields) has been written.  Each of a piece's four words is looked at, so nothing rests on 16 bytes arriving at once.  No fence, no
+// counter, no flag to unpack: with counters and bulk copies a hand-over took 3,700 cycles, so 1,600 to 2,000; with words of six
+// values and a number 5,000, most of it unpacking.  Each kind of value has three buffers that take turns.  Whoever has published use u of a kind marks its own
 // places of use u - 1 again, and fences, before it publishes use u + 1: its readers have then all read use u - 1 (between two
 // uses of a kind lies a norm, which takes everybody's results), and nobody polls for use u + 2 before it has seen use u + 1.
 // The next launch takes the turns up where this one ends.  The marks are the rows' of one row count: another count starts with all
@@ -73,7 +73,8 @@ __host__ __device__ constexpr int value_bytes(int v) {
     return kMaxRows * (v == vIn || v == vMid || v == vNormed ? H * 2 : v == vQkv ? kQkvWidth * 2 : v == vLogits ? kPredictorVocab * 2
                        : v == vTokens ? 16 : v == vAtt ? QWidth * 2 : I * 2);
 }
-__host__ __device__ constexpr int at_value(int v) { return v == 0 ? 0 : at_value(v - 1) + 3 * value_bytes(v - 1); }
+constexpr int kTurns = 3;
+__host__ __device__ constexpr int at_value(int v) { return v == 0 ? 0 : at_value(v - 1) + kTurns * value_bytes(v - 1); }
 constexpr int kAtState = at_value(kValues);           // [0] launches begun, [1] the launch that was given up, then a turn a kind
 constexpr int kExchangeBytes = kAtState + 128;
 
@@ -207,16 +208,22 @@ __device__ __forceinline__ int4 get_piece(const void* p) {
         : "memory");
     return v;
 }
-// Pieces of one thread, `apart` bytes from each other: all are asked for again until those wanted have been written.
+// Pieces of one thread, `apart` bytes from each other: all are asked for again until none of their words is the mark.
+// (The largest of all words, in a tree: a comparison for each of them, and a condition for rows that nobody has, took 1.5 to 2.9 % of
+// a frame.  With the tree frames of 40 sessions 3,759 -> 3,561 us, of 64 4,331 -> 4,240, of 12 2,668 -> 2,683.)
 template <int N>
-__device__ __forceinline__ void poll(const unsigned char* at, int apart, const bool (&wanted)[N], int4 (&v)[N], const Waiter& w) {
+__device__ __forceinline__ void poll(const unsigned char* at, int apart, int4 (&v)[N], const Waiter& w) {
     for (uint32_t polls = 0;;) {
-        bool all = true;
+        uint32_t most[N];
 #pragma unroll
         for (int i = 0; i < N; ++i) v[i] = get_piece(at + i * apart);
 #pragma unroll
-        for (int i = 0; i < N; ++i) all = all && (v[i].x != -1 || !wanted[i]);
-        if (all) return;
+        for (int i = 0; i < N; ++i) most[i] = max(max((uint32_t)v[i].x, (uint32_t)v[i].y), max((uint32_t)v[i].z, (uint32_t)v[i].w));
+#pragma unroll
+        for (int half = 1; half < N; half *= 2)
+#pragma unroll
+            for (int i = 0; i + half < N; i += 2 * half) most[i] = max(most[i], most[i + half]);
+        if (most[0] != 0xffffffffu) return;
         if ((++polls & 255u) == 0 && w.gives_up()) return;
     }
 }
@@ -231,9 +238,9 @@ struct Turns {
 #pragma unroll
         for (int v = 0; v < kValues; ++v) now[v] = __ldcg(state + 2 + v);
     }
-    template <Value V> __device__ __forceinline__ void next() { now[V] = now[V] == 2 ? 0 : now[V] + 1; }
+    template <Value V> __device__ __forceinline__ void next() { now[V] = now[V] == kTurns - 1 ? 0 : now[V] + 1; }
     template <Value V> __device__ __forceinline__ int at() const { return at_value(V) + (int)now[V] * value_bytes(V); }
-    template <Value V> __device__ __forceinline__ int before() const { return at_value(V) + (int)(now[V] == 0 ? 2 : now[V] - 1) * value_bytes(V); }
+    template <Value V> __device__ __forceinline__ int before() const { return at_value(V) + (int)(now[V] == 0 ? kTurns - 1 : now[V] - 1) * value_bytes(V); }
 };
 
 // where 16 bytes (8 channels from k of a row) lie in a slice of MT rows
@@ -392,9 +399,8 @@ __global__ void __launch_bounds__(kThreads, 1) lockstep_chain_kernel(const Locks
                 if (is_normed(kind)) {
                     const bf16* norm_w = kind == kHead ? m.final_norm : (kind == kQkv ? m.layers[layer].in_norm : m.layers[layer].post_norm);
                     const int4 nw = __ldg(reinterpret_cast<const int4*>(norm_w) + n);
-                    const bool wanted[1] = {true};
                     int4 mine[1];
-                    poll<1>(ex + (kind == kGateUp ? turns.at<vMid>() : turns.at<vIn>()) + row * (H * 2) + n * 16, 0, wanted, mine, wt);
+                    poll<1>(ex + (kind == kGateUp ? turns.at<vMid>() : turns.at<vIn>()) + row * (H * 2) + n * 16, 0, mine, wt);
                     reinterpret_cast<int4*>(values)[n] = mine[0];
                     norm_barrier();
                     // talker_kernels.cu:27-48: strided sums of 256 threads, then their tree
@@ -487,9 +493,8 @@ __global__ void __launch_bounds__(kThreads, 1) lockstep_chain_kernel(const Locks
                     if (a.draws == 0 || p == 1) {
                         token = a.table->frame_tokens[my_row][p - 1];
                     } else {
-                        const bool wanted[1] = {true};
                         int4 v[1];
-                        poll<1>(ex + turns.before<vTokens>() + my_row * 16, 0, wanted, v, wt);
+                        poll<1>(ex + turns.before<vTokens>() + my_row * 16, 0, v, wt);
                         token = v[0].x;
                     }
                     if (token >= 0 && token < (p == 1 ? kMaxVocab : kPredictorVocab)) {
@@ -517,17 +522,14 @@ __global__ void __launch_bounds__(kThreads, 1) lockstep_chain_kernel(const Locks
             constexpr int kAtoms = PIECES * 32 / MT;
 #pragma unroll 1
             for (int u0 = 0; u0 < PIECES; u0 += kBatch) {
-                bool wanted[kBatch];
                 int4 v[kBatch];
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) wanted[u] = ((tid >> 3) + 32 * (u0 + u)) % MT < rows;
-                poll<kBatch>(src + (tid + kIoThreads * u0) * 16, kIoThreads * 16, wanted, v, wt);
+                poll<kBatch>(src + (tid + kIoThreads * u0) * 16, kIoThreads * 16, v, wt);
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
                     const int i = tid + kIoThreads * (u0 + u), atom = i / (8 * MT);
                     // two K-slices: the rows of the second behind those of the first
                     const int to = narrow ? (atom < kAtoms / 2 ? 2 * atom : 2 * atom - kAtoms + 1) : atom;
-                    if (wanted[u]) *reinterpret_cast<int4*>(xs + to * kXAtom + (i - atom * (8 * MT)) * 16) = v[u];
+                    *reinterpret_cast<int4*>(xs + to * kXAtom + (i - atom * (8 * MT)) * 16) = v[u];
                 }
             }
         };
@@ -703,10 +705,10 @@ __global__ void __launch_bounds__(kThreads, 1) lockstep_chain_kernel(const Locks
                 page::load(f, kdst, vdst, pos, lane);
                 // lanes 0..15 the first query head and the key, the others the second and the value
                 const unsigned char* src = ex + turns.at<vQkv>() + arow * (kQkvWidth * 2) + (lane & 15) * 16;
-                const bool upper = lane >= 16, wanted[2] = {true, true};
+                const bool upper = lane >= 16;
                 int4 v[2];
                 const int q_at = (2 * head + (upper ? 1 : 0)) * 256, kv_at = ((upper ? 24 : 16) + head) * 256;
-                poll<2>(src + q_at, kv_at - q_at, wanted, v, wt);
+                poll<2>(src + q_at, kv_at - q_at, v, wt);
                 __syncwarp();
                 reinterpret_cast<int4*>(raw)[lane] = v[0];
                 reinterpret_cast<int4*>(raw)[32 + lane] = v[1];
@@ -771,9 +773,8 @@ __global__ void __launch_bounds__(kThreads, 1) lockstep_chain_kernel(const Locks
             TopKScratch& scratch = *reinterpret_cast<TopKScratch*>(xs + kPredictorVocab * sizeof(unsigned int));
             static_assert(kPredictorVocab * sizeof(unsigned int) + sizeof(TopKScratch) <= L::XBytes, "the draw lies over the activations");
             const SamplingParams sp = a.table->predictor[draw_row];
-            const bool wanted[1] = {true};
             int4 v[1];
-            poll<1>(ex + turns.at<vLogits>() + draw_row * (kPredictorVocab * 2) + tid * 16, 0, wanted, v, wt);
+            poll<1>(ex + turns.at<vLogits>() + draw_row * (kPredictorVocab * 2) + tid * 16, 0, v, wt);
             const int four[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
             unsigned long long best = 0ull;
 #pragma unroll
@@ -871,6 +872,21 @@ __global__ void __launch_bounds__(kThreads, 1) lockstep_chain_kernel(const Locks
     }
 }
 
+// Every place marked, all turns at their first buffer, no launch given up.  Places of the tile's rows that nobody has are zeros, there
+// from the beginning: whoever polls for a tile takes them as they are.
+__global__ void __launch_bounds__(512) restart_kernel(unsigned char* exchange, int rows, int tile) {
+    static_assert(kAtState % 16 == 0 && 4 * (2 + kValues) <= 128, "the state behind the values");
+    for (int at = 16 * (blockIdx.x * blockDim.x + threadIdx.x); at < kAtState; at += 16 * gridDim.x * blockDim.x) {
+        bool nobodys = false;
+        for (int v : {vNormed, vAtt, vAct}) {
+            if (at >= at_value(v) && at < at_value(v + 1)) nobodys = (at - at_value(v)) % value_bytes(v) % (tile * 128) / 128 >= rows;
+        }
+        *reinterpret_cast<int4*>(exchange + at) = nobodys ? make_int4(0, 0, 0, 0) : mark();
+    }
+    uint32_t* state = reinterpret_cast<uint32_t*>(exchange + kAtState);
+    if (blockIdx.x == 0 && threadIdx.x < 2 + kValues) state[threadIdx.x] = threadIdx.x == 1 ? ~0u : 0u;
+}
+
 // ---------------------------------------------------------------------------------- host side
 
 bool g_lockstep_fits[64] = {};
@@ -955,12 +971,9 @@ bool make_lockstep_map(LockstepModel* model, int index, const int8_t* weights, i
 
 size_t lockstep_exchange_bytes() { return kExchangeBytes; }
 
-cudaError_t restart_lockstep(void* exchange, cudaStream_t stream) {
-    unsigned char* state = static_cast<unsigned char*>(exchange) + kAtState;
-    cudaError_t e = cudaMemsetAsync(exchange, 0xff, kExchangeBytes, stream);       // every place marked, no launch given up
-    if (e == cudaSuccess) e = cudaMemsetAsync(state, 0, sizeof(uint32_t), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(state + 2 * sizeof(uint32_t), 0, kValues * sizeof(uint32_t), stream);
-    return e;
+cudaError_t restart_lockstep(void* exchange, int rows, cudaStream_t stream) {
+    restart_kernel<<<148, 512, 0, stream>>>(static_cast<unsigned char*>(exchange), rows, gemm_tc_tile(rows));
+    return cudaGetLastError();
 }
 
 cudaError_t launch_lockstep_chain(const LockstepLaunch& c, cudaStream_t stream) {

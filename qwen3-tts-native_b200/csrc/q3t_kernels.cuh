@@ -389,7 +389,7 @@ bool lockstep_chain_available(int rows);
 bool make_lockstep_map(LockstepModel* host_model, int index, const int8_t* weights, int in_features, int matrix_rows, bool wide);
 size_t lockstep_exchange_bytes();
 // Before the first launch, one of another row count, and one behind a launch that was given up.
-cudaError_t restart_lockstep(void* exchange, cudaStream_t stream);
+cudaError_t restart_lockstep(void* exchange, int rows, cudaStream_t stream);
 cudaError_t launch_lockstep_chain(const LockstepLaunch& chain, cudaStream_t stream);
 unsigned int lockstep_error_count();
 
