@@ -22,9 +22,16 @@
 // Hand-overs.  A reader polls the values themselves: a word of two bf16 that is no longer the mark (all ones, which no rounding
 // yields) has been written.  Each of a piece's four words is looked at, so nothing rests on 16 bytes arriving at once.  No fence, no
 // counter, no flag to unpack: with counters and bulk copies a hand-over took 3,700 cycles, so 1,600 to 2,000; with words of six
-// values and a number 5,000, most of it unpacking.  Each kind of value has three buffers that take turns.  Whoever has published use u of a kind marks its own
-// places of use u - 1 again, and fences, before it publishes use u + 1: its readers have then all read use u - 1 (between two
-// uses of a kind lies a norm, which takes everybody's results), and nobody polls for use u + 2 before it has seen use u + 1.
+// values and a number 5,000, most of it unpacking.  Each kind of value has buffers that take turns.  Whoever has published use u of
+// a kind marks its own places of use u - 1 again, and fences.
+//   Not too early: everybody who reads use u - 1 has read it, since what leads to use u has been through all of them.  Position 0
+//   ends at its last q/k/v and position 1 begins with what no reader of it has made; there it is the attention of a ninth row, whose
+//   CTAs, clusters 16 and 17, wait for every tile before they take part in position 1's input.  So not for 8 rows and fewer.
+//   Not too late: a reader of the next use of the same buffer knows of the mark.  Nothing is fenced between two polls of a layer:
+//   writers vouch with the fence at the end of a layer for what they had marked by their barrier before, readers count what they
+//   have seen by such a fence and a barrier behind it.  So a buffer comes round only after so many uses that this lies between,
+//   also for the clusters that read but every second normed row and none of the head's: 8 buffers of those, 4 of the others, 3
+//   where a whole position lies between two uses (turns_of; tests/test_lockstep_protocol.py walks through it).
 // The next launch takes the turns up where this one ends.  The marks are the rows' of one row count: another count starts with all
 // places marked (restart_lockstep).  The buffers of the K-slices alternate: a CTA may be one projection ahead of its
 // neighbours (attention ties rows and heads together, not the whole cluster), never two.
@@ -66,15 +73,15 @@ constexpr int kWStageBytes = 128 * kBK;
 constexpr int kAccCols = 128, kAStages = 6, kAStageCols = kBK / 2;
 static_assert(kAccCols + kAStages * kAStageCols <= 512, "tensor memory");
 
-// ---- exchange: three buffers a kind.  What one row's reader wants lies row by row, what all rows' readers want as it lies in
+// ---- exchange: turns_of() buffers a kind.  What one row's reader wants lies row by row, what all rows' readers want as it lies in
 // their shared memory: [64 K][rows of the tile][128 bytes, swizzled]
 enum Value { vIn, vMid, vQkv, vLogits, vTokens, vNormed, vAtt, vAct, kValues };
 __host__ __device__ constexpr int value_bytes(int v) {
     return kMaxRows * (v == vIn || v == vMid || v == vNormed ? H * 2 : v == vQkv ? kQkvWidth * 2 : v == vLogits ? kPredictorVocab * 2
                        : v == vTokens ? 16 : v == vAtt ? QWidth * 2 : I * 2);
 }
-constexpr int kTurns = 3;
-__host__ __device__ constexpr int at_value(int v) { return v == 0 ? 0 : at_value(v - 1) + kTurns * value_bytes(v - 1); }
+__host__ __device__ constexpr int turns_of(int v) { return v == vNormed ? 8 : (v == vLogits || v == vTokens ? 3 : 4); }
+__host__ __device__ constexpr int at_value(int v) { return v == 0 ? 0 : at_value(v - 1) + turns_of(v - 1) * value_bytes(v - 1); }
 constexpr int kAtState = at_value(kValues);           // [0] launches begun, [1] the launch that was given up, then a turn a kind
 constexpr int kExchangeBytes = kAtState + 128;
 
@@ -238,9 +245,9 @@ struct Turns {
 #pragma unroll
         for (int v = 0; v < kValues; ++v) now[v] = __ldcg(state + 2 + v);
     }
-    template <Value V> __device__ __forceinline__ void next() { now[V] = now[V] == kTurns - 1 ? 0 : now[V] + 1; }
+    template <Value V> __device__ __forceinline__ void next() { now[V] = now[V] == turns_of(V) - 1 ? 0 : now[V] + 1; }
     template <Value V> __device__ __forceinline__ int at() const { return at_value(V) + (int)now[V] * value_bytes(V); }
-    template <Value V> __device__ __forceinline__ int before() const { return at_value(V) + (int)(now[V] == 0 ? kTurns - 1 : now[V] - 1) * value_bytes(V); }
+    template <Value V> __device__ __forceinline__ int before() const { return at_value(V) + (int)(now[V] == 0 ? turns_of(V) - 1 : now[V] - 1) * value_bytes(V); }
 };
 
 // where 16 bytes (8 channels from k of a row) lie in a slice of MT rows
