@@ -957,10 +957,10 @@ cudaError_t configure_lockstep_kernels() {
     return e;
 }
 
-// The kernel sums the K-slices that these are.
+// The kernel sums the K-slices that these are.  (8 rows and fewer: see the hand-overs.)
 bool lockstep_chain_available(int rows) {
     int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64 || !g_lockstep_fits[device] || rows < 1 || rows > kMaxRows) return false;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64 || !g_lockstep_fits[device] || rows <= kChainRows || rows > kMaxRows) return false;
     return gemm_tc_slices(4096, H, rows, false) == 4 && gemm_tc_slices(H, QWidth, rows, false) == 8 && gemm_tc_slices(I, H, rows, true) == 2
            && gemm_tc_slices(H, I, rows, false) == 8 && gemm_tc_slices(kPredictorVocab, H, rows, false) == 4
            && gemm_tc_slices(H, TalkerH, rows, false) == 8;

@@ -230,3 +230,9 @@ def test_every_word_of_a_piece_is_looked_at():
     poll = text[text.index("void poll("):text.index("int4 mark()")]
     for word in "xyzw":
         assert "(uint32_t)v[i].%s" % word in poll
+
+
+def test_no_launch_for_rows_that_the_hand_overs_are_not_ordered_for():
+    text = source()
+    rule = text[text.index("bool lockstep_chain_available("):text.index("bool make_lockstep_map(")]
+    assert "rows <= kChainRows" in rule and "lockstep_chain_available(c.rows)" in text[text.index("cudaError_t launch_lockstep_chain("):]
