@@ -997,7 +997,7 @@ void enqueue_predictor_chain(Workspace& w, Model& m, int n, cudaStream_t s) {
 enum class Lockstep { kNone, kPositions, kWhole };
 // Whether it may run on the lockstep chain: enough rows, the default kernels (it computes what they compute).
 bool lockstep_may_run(const Workspace& w, const Model& m, int n) {
-    return n > kChainRows && n >= tc_min_rows() && m.use_chain == 1 && attention_mode() == 1 && m.lockstep.bytes() != 0
+    return n > kChainRows && n >= tc_min_rows() && m.use_chain == 1 && m.use_graphs != 0 && attention_mode() == 1 && m.lockstep.bytes() != 0
            && w.lockstep_exchange.bytes() != 0 && lockstep_chain_available(n);
 }
 

@@ -65,3 +65,24 @@ def test_row_counts_in_turn(q3t, model):
     for n in (12, 40, 9, 40, 12):
         assert frames(q3t, model, n, 1, 1)[0] == want[n]
     assert q3t.library().q3t_kernel_error_count() == 0
+
+
+def test_without_graphs_launch_by_launch(q3t, model):
+    """With "use_graphs" 0 a frame is made launch by launch, as the header has it: the 600th of its launches is there to fail."""
+    lib = q3t.library()
+    model.set_option("decode_chain", 1)
+    model.set_option("use_graphs", 0)
+    sessions = []
+    try:
+        for i in range(12):
+            s = model.create_session(64, 1 + i)
+            s.synthetic_prefill(20 + i, 1 + i)
+            sessions.append(s)
+        lib.q3t_test_fail_launch_after(600)
+        with pytest.raises(q3t.NativeTalkerStatusError):
+            model.batch_begin_device_frames(sessions, [7] * 12)
+    finally:
+        lib.q3t_test_fail_launch_after(0)
+        model.set_option("use_graphs", 1)
+        for s in sessions:
+            s.close()
