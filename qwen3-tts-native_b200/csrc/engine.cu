@@ -177,6 +177,13 @@ public:
         kind_ = !never_chain && traffic_->chain_pays(workspace_, rows) ? Traffic::kChain : Traffic::kInPlaceOfChain;
         traffic_->enter(workspace_, rows, kind_);
     }
+    // a frame of more rows than a chain takes: alone() tells whether nothing else was at work when it entered the census
+    struct Large {};
+    InFlight(Traffic* traffic, const Workspace& w, int rows, Large) : traffic_(traffic), workspace_(&w) {
+        std::lock_guard<std::mutex> lock(traffic_->mutex);
+        alone_ = traffic_->alone(workspace_);
+        traffic_->enter(workspace_, rows, Traffic::kOther);
+    }
     InFlight(const InFlight&) = delete;
     InFlight& operator=(const InFlight&) = delete;
     // from here on the workspace's talker_stop tells the end
@@ -192,10 +199,12 @@ public:
         traffic_->leave(workspace_);
     }
     Traffic::Kind kind() const { return kind_; }
+    bool alone() const { return alone_; }
 private:
     Traffic* traffic_;
     const Workspace* workspace_;
     Traffic::Kind kind_ = Traffic::kOther;
+    bool alone_ = false;
 };
 
 // Held while a frame's chains are enqueued; whatever chain was enqueued by then, the next holder's stream waits for it, and
@@ -1522,11 +1531,10 @@ void Session::launch_frame(Workspace& w, Model& m, Session** s, int n, bool uplo
     if (frame_may_chain(m, *w.host_table, n)) {
         in_flight.reset(new InFlight(traffic, w, n, m.use_chain == 2));
         way = in_flight->kind() == Traffic::kChain ? Way::kChain : Way::kInItsPlace;
+    } else if (lockstep_may_run(w, m, n) && traffic != nullptr) {
+        in_flight.reset(new InFlight(traffic, w, n, InFlight::Large()));
+        if (in_flight->alone()) lockstep = draws_fit_chains(*w.host_table, n) ? Lockstep::kWhole : Lockstep::kPositions;
     } else {
-        if (lockstep_may_run(w, m, n) && traffic != nullptr) {
-            std::lock_guard<std::mutex> lock(traffic->mutex);
-            if (traffic->alone(&w)) lockstep = draws_fit_chains(*w.host_table, n) ? Lockstep::kWhole : Lockstep::kPositions;
-        }
         in_flight.reset(new InFlight(traffic, w, n, Traffic::kOther));
     }
     if (way == Way::kLaunches) w.ensure_scratch(splits);

@@ -236,3 +236,13 @@ def test_no_launch_for_rows_that_the_hand_overs_are_not_ordered_for():
     text = source()
     rule = text[text.index("bool lockstep_chain_available("):text.index("bool make_lockstep_map(")]
     assert "rows <= kChainRows" in rule and "lockstep_chain_available(c.rows)" in text[text.index("cudaError_t launch_lockstep_chain("):]
+
+
+def test_a_frame_sees_whether_it_is_alone_and_is_seen_in_one_step():
+    """Between the look at the census and the entry into it a prompt or a chain could have come in, unseen and not seeing."""
+    with open(os.path.join(CSRC, "engine.cu")) as f:
+        text = f.read()
+    large = text[text.index("InFlight(Traffic* traffic, const Workspace& w, int rows, Large)"):]
+    large = large[:large.index("    }\n")]
+    assert large.count("lock_guard") == 1 and large.index("lock_guard") < large.index("->alone(") < large.index("->enter(")
+    assert text.count("->alone(workspace_)") == 1 and "traffic->alone(" not in text
