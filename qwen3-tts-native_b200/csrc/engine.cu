@@ -334,7 +334,8 @@ uint64_t KvPool::page_bytes() const { return (uint64_t)layers_ * 2 * page_elems_
 
 // ------------------------------------------------------------------ Workspace
 
-Workspace::Workspace(int capacity_, int device_, int rows_) : capacity(capacity_), rows(std::max(capacity_, rows_)), device(device_) {
+Workspace::Workspace(int capacity_, int device_, int rows_, bool lockstep)
+    : capacity(capacity_), rows(std::max(capacity_, rows_)), device(device_) {
     check_cuda(cudaSetDevice(device), "cudaSetDevice(workspace)");
     const size_t e = sizeof(bf16);
     size_t c = rows;
@@ -346,7 +347,7 @@ Workspace::Workspace(int capacity_, int device_, int rows_) : capacity(capacity_
         {&hidden, c * 2048 * e}, {&qkv, c * 4096 * e}, {&attention, c * 2048 * e}, {&gate, c * 6144 * e},
         {&logits, one * kTalkerVocab * e}, {&x_in, c * 2048 * e}, {&projection, c * 2048 * e}, {&normalized, c * 2048 * e},
         {&prompt_positions, c * sizeof(int)}, {&talker_pages, one * kMaxPagesPerRow * sizeof(int)},
-        {&lockstep_exchange, capacity > kChainRows ? lockstep_exchange_bytes() : 0},
+        {&lockstep_exchange, lockstep ? lockstep_exchange_bytes() : 0},
         {&predictor_pages, one * sizeof(int)}, {&predictor_positions, (size_t)kPredictorSequence * kMaxRows * sizeof(int)}};
     size_t total = 0;
     for (const auto& part : parts) total += align_up(part.second, 1024);
@@ -833,7 +834,7 @@ void Model::check_device_errors(unsigned int count_at_enqueue) const {
 
 Workspace& Model::batch_workspace() {
     std::lock_guard<std::mutex> lock(mutex);
-    if (!batch_) batch_.reset(new Workspace(kMaxRows, device_));
+    if (!batch_) batch_.reset(new Workspace(kMaxRows, device_, 0, true));
     return *batch_;
 }
 

@@ -120,8 +120,9 @@ class Session;
 
 // Activation buffers, frame table and captured graphs for up to `capacity` lockstep rows.
 struct Workspace {
-    // `rows`: activation rows of one pass when that is more than the `capacity` table rows (prompts)
-    Workspace(int capacity, int device, int rows = 0);
+    // `rows`: activation rows of one pass when that is more than the `capacity` table rows (prompts); `lockstep`: frames of more
+    // rows than a chain takes run here
+    Workspace(int capacity, int device, int rows = 0, bool lockstep = false);
     ~Workspace();
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
