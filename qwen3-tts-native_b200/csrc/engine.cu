@@ -677,7 +677,11 @@ void Model::finalize(uint64_t* weight_bytes, uint32_t* tensor_count) {
         cudaStreamSynchronize(upload_stream_);
         chain = DecodeChain();
     }
-    build_lockstep();
+    try {
+        build_lockstep();
+    } catch (const std::bad_alloc&) {
+        lockstep = DeviceBuffer();          // frames of 9 and more sessions likewise
+    }
     talker_pool.reset(new KvPool(talker.layers, talker.kv_width, 8, upload_stream_));
     predictor_pool.reset(new KvPool(predictor.layers, predictor.kv_width, 6, upload_stream_));
     finalized_ = true;

@@ -110,6 +110,26 @@ def test_without_memory_for_the_chain_and_for_long_passes(q3t, gpu_model, checkp
         replica.close()
 
 
+def test_without_memory_for_the_lockstep_chains_table(q3t, gpu_model, checkpoint):
+    """The lockstep chain's table of tensor maps is optional too: without it large frames run launch by launch, with the same bits."""
+    lib = q3t.library()
+    want = frames(q3t, gpu_model, 12, count=1)
+    replica = replica_of(q3t, gpu_model, checkpoint.keys())
+    try:
+        lib.q3t_test_fail_allocation_after(17)         # two that every model needs, fourteen of the decode chain, then this one
+        replica.finalize()
+        lib.q3t_test_fail_allocation_after(0)
+        before = replica.kernel_launches()
+        assert same(frames(q3t, replica, 12, count=1), want)
+        assert replica.kernel_launches() - before > 600
+        before = replica.kernel_launches()
+        frames(q3t, replica, 2, count=1)
+        assert replica.kernel_launches() - before < 30
+    finally:
+        lib.q3t_test_fail_allocation_after(0)
+        replica.close()
+
+
 def test_two_models_on_one_device(q3t, gpu_model, checkpoint):
     """Two replicas that decode at the same time from threads of their own, in large batches (tensor cores, norms as launches of
     their own) and in small ones (decode chain), decode what each decodes alone: nothing that a frame writes is shared."""
