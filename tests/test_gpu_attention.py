@@ -341,3 +341,77 @@ def test_prompt_attention(orc, ops, base, rows, kvh):
             pid = int(table[0, t // 16])
             row = got["pages"][pid // 64][which, pid % 64, :, t % 16].reshape(-1)
             assert np.array_equal(row, full[0, t] if t < end else np.full(kvw, 0x7fc0, dtype=np.uint16)), t
+
+
+def prompt_over_cache(orc, ops, rng, base, rows, qkv, wq, wk, k, v):
+    """A prompt pass over given caches (tokens 0 .. base - 1 as they lie there), and the oracle's rows."""
+    qh, kvh, hd = 16, 8, 128
+    qw, kvw, end = qh * hd, kvh * hd, base + rows
+    pos = np.arange(base, end, dtype=np.int32)
+    q2 = ops.rope_rows_at(ops.head_rms_norm_rows(np.ascontiguousarray(qkv[:, :qw]), wq, rows, qh, hd), rows, qh, hd, pos)
+    k2 = ops.rope_rows_at(ops.head_rms_norm_rows(np.ascontiguousarray(qkv[:, qw:qw + kvw]), wk, rows, kvh, hd), rows, kvh, hd, pos)
+    full_k, full_v = k.copy(), v.copy()
+    full_k[0, base:end], full_v[0, base:end] = k2.reshape(rows, kvw), qkv[:, qw + kvw:]
+    k[0, base:], v[0, base:] = 0x7fc0, 0x7fc0
+    slabs, table = paged_copy(k, v, kvw, rng, per_slab=64)
+    got = ops.attention_ex(qkv, pos, qh, kvh, hd, pages=slabs, page_table=table, slab_shift=6, q_norm_w=wq, k_norm_w=wk, fused=True,
+                           q_stride=qw + 2 * kvw, new_stride=qw + 2 * kvw, prompt_base=base)
+    want, _ = orc.attention(q2.reshape(rows, qw), np.repeat(full_k, rows, axis=0), np.repeat(full_v, rows, axis=0), pos, qh, kvh, hd,
+                            fast=True, want_f32=True)
+    return got["out"], want, orc.from_bf16(q2).reshape(rows, qh, hd), orc.from_bf16(full_k).reshape(-1, kvh, hd)
+
+
+SLOW = np.r_[48:64, 112:128]             # dimensions that the rotation hardly turns at these positions
+
+
+@pytest.mark.parametrize("base,rows", [(128, 20), (192, 64), (330, 70), (640, 33), (200, 600)])
+def test_prompt_attention_of_peaked_heads(orc, ops, base, rows):
+    """Scores that rise from one 64-token step to the next: a row's output is rescaled where one exceeds its reference by 2^8.
+    The rows of a warp differ: some rise past it at every step, some at every second one, some never."""
+    kvh, hd = 8, 128
+    qw, kvw = 2 * kvh * hd, kvh * hd
+    rng = np.random.default_rng(base)
+    direction = np.zeros(hd)
+    direction[SLOW] = 1 / np.sqrt(len(SLOW))
+    share = np.array([0.0, 0.97, 0.5, 0.8, 0.25])[np.arange(rows) % 5]                       # of a query along the direction
+    other = rng.standard_normal((rows, 2 * kvh, hd))
+    other[..., SLOW] = 0
+    other /= np.linalg.norm(other, axis=-1, keepdims=True)
+    q = share[:, None, None] * direction + np.sqrt(1 - share ** 2)[:, None, None] * other    # a head's norm makes sqrt(128) of each
+    qkv = np.concatenate([q.reshape(rows, qw), rng.standard_normal((rows, 2 * kvw))], axis=1)
+    wq, wk = bf(orc, np.ones(hd)), bf(orc, np.ones(hd))
+    cap = (base + rows + 15) // 16 * 16 + 16
+    k, v = rng.standard_normal((1, cap, kvh, hd)), rng.standard_normal((1, cap, kvw))
+    k += 11.0 * (np.arange(cap) // 64)[None, :, None, None] * direction                      # a step adds up to 11 x 0.97 / ln 2 in log2
+    got, want, q2, k2 = prompt_over_cache(orc, ops, rng, base, rows, bf(orc, qkv), wq, wk, bf(orc, k.reshape(1, cap, kvw)), bf(orc, v))
+    # the case is what it says: how often a row's reference moves
+    moves = np.zeros((rows, 2 * kvh), dtype=int)
+    for r in range(rows):
+        scores = np.einsum("hd,thd->ht", q2[r], np.repeat(k2[:base + r + 1], 2, axis=1)) / np.sqrt(hd) / np.log(2)
+        tops = np.array([scores[:, t:t + 64].max(axis=1) for t in range(0, base + r + 1, 64)])
+        reference = tops[0]
+        for top in tops[1:]:
+            moves[r] += top > reference + 8
+            reference = np.where(top > reference + 8, top, reference)
+    assert moves[share == 0].max() == 0 and moves[share > 0.9].min() >= min(2, base // 64 - 1)
+    assert 0 < moves[share == 0.5].mean() < moves[share > 0.9].mean()
+    check_bf16(orc, got, want, hd)
+
+
+@pytest.mark.parametrize("masked", [(0, 64), (64, 128), (3, 60), (0, 128)])
+@pytest.mark.parametrize("base,rows", [(150, 9), (150, 40), (130, 64), (192, 600)])
+def test_prompt_attention_of_scores_of_minus_infinity(orc, ops, base, rows, masked):
+    """Keys whose products overflow to -inf have no weight, also where they fill a row's first steps."""
+    kvh, hd = 8, 128
+    qw, kvw = 2 * kvh * hd, kvh * hd
+    rng = np.random.default_rng(rows)
+    q = np.zeros((rows, 2 * kvh, hd))
+    q[..., SLOW] = 1 + rng.random((rows, 2 * kvh, len(SLOW)))
+    qkv = np.concatenate([q.reshape(rows, qw), rng.standard_normal((rows, 2 * kvw))], axis=1)
+    wq, wk = bf(orc, np.ones(hd)), bf(orc, 1 + 0.1 * rng.standard_normal(hd))
+    cap = (base + rows + 15) // 16 * 16 + 16
+    k, v = rng.standard_normal((1, cap, kvh, hd)), rng.standard_normal((1, cap, kvw))
+    k[0, masked[0]:masked[1], :, SLOW] = -1e38
+    got, want, q2, _ = prompt_over_cache(orc, ops, rng, base, rows, bf(orc, qkv), wq, wk, bf(orc, k.reshape(1, cap, kvw)), bf(orc, v))
+    assert (q2[..., SLOW] > 0).all() and np.isfinite(orc.from_bf16(want)).all()
+    check_bf16(orc, got, want, hd)
