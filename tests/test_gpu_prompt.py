@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,chunk", [(n, 2048) for n in (9, 33, 65, 128, 129, 257, 300, 385, 641, 1201)] + [(450, 200), (150, 141)])
 def test_prompt_pass_tracks_single_positions(q3t, orc, gpu_model, n, chunk):
-    """Lengths around the row blocks (64, 128), the attention blocks (32 positions, 64 tokens) and the changes of GEMM kernel
+    """Lengths around the row blocks (64, 128), the attention blocks (32 or 64 positions, 64 tokens) and the changes of GEMM kernel
     (gate/up after 64 rows, q/k/v after 256, the others after 576), and passes behind a longer one, the last of 50 or of 9
     rows.  Layer 0's keys and values have one GEMM chain behind them (text projection, q/k/v) whose fp32 sums differ in order
     only: relative error below one bf16 rounding, 2^-8.  From there to layer 1's lie eight bf16 roundings (attention, o,
