@@ -84,6 +84,7 @@ __host__ __device__ constexpr int turns_of(int v) { return v == vNormed ? 8 : (v
 __host__ __device__ constexpr int at_value(int v) { return v == 0 ? 0 : at_value(v - 1) + turns_of(v - 1) * value_bytes(v - 1); }
 constexpr int kAtState = at_value(kValues);           // [0] launches begun, [1] the launch that was given up, then a turn a kind
 constexpr int kExchangeBytes = kAtState + 128;
+constexpr uint32_t kNoLaunch = ~0u;                  // [1] as long as none was given up: no launch has that number
 
 __device__ unsigned int g_lockstep_errors = 0;
 __device__ unsigned int* g_lockstep_error_sink = nullptr;
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(kThreads, 1) lockstep_chain_kernel(const Locks
     }
     // a neighbour may still send here, and every CTA has read the launch's base by now
     cluster_sync();
-    if (cta == 0 && tid == 0) *state = wt.base + 1;
+    if (cta == 0 && tid == 0) *state = wt.base >= kNoLaunch - 1 ? 0 : wt.base + 1;
     if (warp == kRoleWarp + 2) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
@@ -891,7 +892,7 @@ __global__ void __launch_bounds__(512) restart_kernel(unsigned char* exchange, i
         *reinterpret_cast<int4*>(exchange + at) = nobodys ? make_int4(0, 0, 0, 0) : mark();
     }
     uint32_t* state = reinterpret_cast<uint32_t*>(exchange + kAtState);
-    if (blockIdx.x == 0 && threadIdx.x < 2 + kValues) state[threadIdx.x] = threadIdx.x == 1 ? ~0u : 0u;
+    if (blockIdx.x == 0 && threadIdx.x < 2 + kValues) state[threadIdx.x] = threadIdx.x == 1 ? kNoLaunch : 0u;
 }
 
 // ---------------------------------------------------------------------------------- host side

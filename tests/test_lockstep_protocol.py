@@ -246,3 +246,12 @@ def test_a_frame_sees_whether_it_is_alone_and_is_seen_in_one_step():
     large = large[:large.index("    }\n")]
     assert large.count("lock_guard") == 1 and large.index("lock_guard") < large.index("->alone(") < large.index("->enter(")
     assert text.count("->alone(workspace_)") == 1 and "traffic->alone(" not in text
+
+
+def test_no_launch_has_the_number_of_none():
+    """Launches are numbered in 32 bits, and a frame may be sixteen of them: the number that stands for "none was given up" comes up
+    after some twelve days, and the launch that bore it would give up."""
+    text = source()
+    assert "constexpr uint32_t kNoLaunch = ~0u;" in text and "threadIdx.x == 1 ? kNoLaunch : 0u" in text
+    following = re.search(r"\*state = wt\.base >= kNoLaunch - 1 \? 0 : wt\.base \+ 1;", text)
+    assert following and text.count("*state = ") == 1
