@@ -64,7 +64,8 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// 2^x, x <= 0: as exp2f, but what would be subnormal (below 2^-126 of the largest weight) is zero
+// 2^x, x <= kSlack (the reference may lie that far below a row's maximum, so that weights reach 256): as exp2f, but what would be
+// subnormal is zero
 __device__ __forceinline__ float exp2_ftz(float x) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

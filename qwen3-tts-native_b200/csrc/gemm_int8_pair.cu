@@ -4,7 +4,7 @@
 // rows with tcgen05.mma.cta_group::2: each CTA converts 128 weight rows into its tensor memory (the A operand, and later the
 // accumulators of the same lanes) and fetches half of the activation rows (its half of B), which the tensor cores of both read.
 //
-// What bounds it: the products, 4 cycles for 16 K and a row, at the clock that the power leaves; below 140 rows the conversion of
+// What bounds it: the products, 4 cycles for a step of 128 K and a row, at the clock that the power leaves; below 140 rows the conversion of
 // the weights, 0.36 us a step of 128 K.  A weight is converted once for up to 256 rows, where gemm_int8_wide.cu converts it for
 // 128; its two tiles of 128 x 128 take 0.63 us a step, this kernel's 256 x 256 of two SMs 0.7.
 //

@@ -11,9 +11,10 @@
 //     weights        TMA into a ring, converted to bf16 in tensor memory as far ahead as that reaches: six steps of 128 K, more
 //                    than most projections have, so that conversion and HBM are behind the hand-overs
 //     activations    polled for where they are handed over and copied to shared memory, which they are laid out for
-//     products       tcgen05.mma as in gemm_int8_tc.cu.  Narrow tiles (64 channels) whose rank has two of the K-slices put one into
-//                    the lower and one into the upper half of the lanes, with the rows of both side by side as columns: a
-//                    product takes some 60 cycles whatever its columns, and so do both
+//     products       tcgen05.mma as in gemm_int8_tc.cu (half a cycle a column, 10 at least).  Narrow tiles (64 channels) whose rank
+//                    has two of the K-slices put one into the lower and one into the upper half of the lanes, with the rows of both
+//                    side by side as columns: one product of twice the columns in place of two that leave 64 lanes idle, as long,
+//                    but half the steps of conversion, arrivals and issue
 //     K-slices       meet in the cluster by asynchronous stores counted where they land; each rank finishes a share of the rows
 //   tiles: q/k/v 32 of 128 channels, one a cluster; gate/up 48 of 64 + 64, two a cluster; o, down and the input projection
 //   16 of 64 channels, whose finishing threads keep the residual stream in registers; head 16 of 128.
@@ -37,7 +38,10 @@
 // neighbours (attention ties rows and heads together, not the whole cluster), never two.
 //
 // What bounds it (B200, cycles; 23 rows): a layer takes 29,500, of which products 6,000, K-slices' sums 4,500, attention 4,800, norms
-// 2,000, and the rest hand-overs with the wait for the slowest CTA.  Frames of 23 sessions 4,082 -> 3,583 us, of 64 5,909 -> 5,421.
+// 2,000, and the rest hand-overs with the wait for the slowest CTA.  The predictor's part of a frame by events, launch by launch and
+// here (ms): 9 rows 1.92 / 1.40, 16 2.05 / 1.45, 23 2.16 / 1.65, 32 2.21 / 1.71, 40 2.42 / 1.92, 48 2.46 / 1.98, 64 2.70 / 2.17; whole
+// frames at contexts of 64 to 512 tokens (us) 9 sessions 3,158 / 2,639, 23 3,572 / 3,071, 64 4,803 / 4,249.  96 registers at launch,
+// 8 to 24 bytes spilled.
 //
 // The launch is cooperative.  Every wait is bounded by a deadline; one that gives up marks the run, all others give up too,
 // the kernel runs through on whatever it holds and the host refuses the result.
